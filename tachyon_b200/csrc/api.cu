@@ -155,14 +155,13 @@ void ws_release(tc_ctx* ctx) {
 // layer has asked for. Growing it frees the old buffers, which invalidates graphs
 // captured earlier; create every layer before capturing.
 bool prefill_reserve(tc_ctx* ctx, const tc::MoeDims& d, int max_tokens) {
-    const int tiles = tc::prefill_max_token_tiles(max_tokens * d.topk, d.experts);
-    const int nb = std::max(d.hidden, d.inter) / 32;
+    const int slots = max_tokens * d.topk;
+    const size_t rows = tc::prefill_max_rows(slots, d.experts);
     tc::PrefillScratch& p = ctx->pre;
-    const size_t per_tile = size_t(nb) * tc::prefill_token_tile() * 32;
-    if (p.max_tiles >= tiles && p.xt_bytes >= size_t(tiles) * per_tile && p.tile_bytes >= per_tile) return true;
-    const int T = std::max(tiles, p.max_tiles);
-    const size_t tile_bytes = std::max(per_tile, p.tile_bytes);
-    const size_t xt_bytes = size_t(T) * tile_bytes, xst_elems = xt_bytes / 32;
+    const size_t tiles = size_t(tc::prefill_max_token_tiles(slots, d.experts, true));
+    if (p.max_tiles >= tiles && p.xt_elems >= rows * d.hidden && p.ht_elems >= rows * d.inter) return true;
+    const size_t T = std::max(tiles, p.max_tiles), xt = std::max(rows * d.hidden, p.xt_elems),
+                 ht = std::max(rows * d.inter, p.ht_elems);
     cudaStreamSynchronize(ctx->stream);
     for (void* q : ctx->pre_allocs) cudaFree(q);
     ctx->pre_allocs.clear();
@@ -174,18 +173,16 @@ bool prefill_reserve(tc_ctx* ctx, const tc::MoeDims& d, int max_tokens) {
         dst = static_cast<std::remove_reference_t<decltype(dst)>>(raw);
         return true;
     };
-    if (!(get(p.tile_expert, size_t(T) * 4) && get(p.tile_n, size_t(T) * 4) && get(p.tile_count, 4) &&
-          get(p.tile_p0, size_t(T) * 4) && get(p.xt, xt_bytes) && get(p.xst, xst_elems * 4) &&
-          get(p.xsumt, xst_elems * 4))) {
+    if (!(get(p.tiles, T * sizeof(tc::TokenTile)) && get(p.tile_count, 4) && get(p.xt, xt * 2) && get(p.xst, xt / 8) &&
+          get(p.xsumt, xt / 8) && get(p.ht, ht * 2) && get(p.hst, ht / 8) && get(p.hsumt, ht / 8))) {
         for (void* q : ctx->pre_allocs) cudaFree(q);
         ctx->pre_allocs.clear();
         p = tc::PrefillScratch{};
         return false;
     }
     p.max_tiles = T;
-    p.tile_bytes = tile_bytes;
-    p.xt_bytes = xt_bytes;
-    p.xst_elems = xst_elems;
+    p.xt_elems = xt;
+    p.ht_elems = ht;
     return true;
 }
 
@@ -737,10 +734,9 @@ tc_moe_layer* layer_create(tc_ctx* ctx, int hidden, int experts, int k, int inte
     tc::tile_weights(dl, down->dev, false, l->down_tiled, ctx->stream);
     // (Expert-parallel layers: tiles of this rank's experts; scratch for every rank's tokens.)
     const tc::MoeDims& dp = ep ? dl : d;
-    if (tc::prefill_fits(dp, gate_up->dev.kind == TC_Q4, down->dev.kind == TC_Q4) &&
-        prefill_reserve(ctx, d, ep ? max_tokens * ctx->ep.size : max_tokens)) {
-        // Third copy of the experts, for prefill-size groups: int8 tiles in the tensor core's
-        // canonical order and f32 block scales.
+    if (prefill_reserve(ctx, d, ep ? max_tokens * ctx->ep.size : max_tokens)) {
+        // Third copy of the experts, for prefill-size groups: the values as f16 tiles in the tensor
+        // core's canonical order and f32 block scales.
         auto get = [&](auto*& dst, size_t bytes) {
             void* raw = nullptr;
             if (!cuda_ok(ctx, cudaMalloc(&raw, bytes + 256), "cudaMalloc(prefill weights)")) return false;
@@ -908,7 +904,7 @@ int moe_enqueue(tc_moe_layer* layer, const float* x, const float* norm_w, float 
         const int slots = t * d.topk;
         n += staged(ctx, 2, [&] {
             return tc::launch_prefill(d, true, layer->gu.kind == TC_Q4, layer->pw, ctx->pre, ws, slots,
-                                      ws.hidden_f, nullptr, s);
+                                      nullptr, nullptr, s);
         });
         n += staged(ctx, 4, [&] {
             return tc::launch_prefill(d, false, layer->dn.kind == TC_Q4, layer->pw, ctx->pre, ws, slots,

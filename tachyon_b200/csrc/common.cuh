@@ -259,26 +259,31 @@ __device__ __forceinline__ void peer_scatter_signal(const PeerPlan& a, uint32_t*
 inline bool dense_walk(const MoeDims& d, int t) { return (long long)t * d.topk >= 4LL * d.experts; }
 
 // ---- prefill-size groups on tcgen05 (experts_prefill.cu)
-struct PrefillWeights {  // per layer: int8 tiles + f32 block scales (and 4-bit offsets)
-    int8_t *gu_t = nullptr, *dn_t = nullptr;
+struct PrefillWeights {  // per layer: the 8-bit values as f16 tiles + f32 block scales (and 4-bit offsets)
+    uint16_t *gu_t = nullptr, *dn_t = nullptr;
     float *gu_d = nullptr, *gu_c = nullptr, *dn_d = nullptr, *dn_c = nullptr;
 };
+// A tile of one expert's tokens: n of them (sorted slots p0, p0 + 1, ...) in `cols` columns (32, 64
+// or 128); row0 counts the columns of the tiles before it (where its rows start in the tile buffers).
+struct TokenTile {
+    int expert;
+    uint32_t p0, row0;
+    uint16_t n, cols;
+};
 struct PrefillScratch {  // per context
-    int *tile_expert = nullptr, *tile_n = nullptr, *tile_count = nullptr;
-    uint32_t* tile_p0 = nullptr;
-    int8_t* xt = nullptr;
-    float *xst = nullptr, *xsumt = nullptr;
-    size_t xt_bytes = 0, xst_elems = 0;
-    size_t tile_bytes = 0;  // bytes of one token tile's 8-bit rows at the widest layer so far
-    int max_tiles = 0;
+    TokenTile* tiles = nullptr;
+    int* tile_count = nullptr;
+    uint16_t *xt = nullptr, *ht = nullptr;    // the block's input rows and the SwiGLU rows, 8-bit values as f16, as tiles
+    float *xst = nullptr, *xsumt = nullptr;   // their scales and scaled block sums
+    float *hst = nullptr, *hsumt = nullptr;
+    size_t max_tiles = 0, xt_elems = 0, ht_elems = 0;
 };
 void init_kernels_prefill();
-bool prefill_fits(const MoeDims& d, bool q4_gate_up, bool q4_down);
 size_t prefill_weight_bytes(const MoeDims& d, bool gate_up);
 size_t prefill_scale_elems(const MoeDims& d, bool gate_up);
-int prefill_max_token_tiles(int slots, int experts);
-int prefill_token_tile();  // tokens per tile
-void tile_prefill_weights(const MoeDims& d, const MatrixDev& m, bool gate_up, int8_t* wt, float* wd, float* wc,
+int prefill_max_token_tiles(int slots, int experts, bool q4);
+size_t prefill_max_rows(int slots, int experts);  // columns of all the tiles of a batch, at most
+void tile_prefill_weights(const MoeDims& d, const MatrixDev& m, bool gate_up, uint16_t* wt, float* wd, float* wc,
                           cudaStream_t stream);
 // peer_out (down only): null, or every rank's window for expert outputs; a row whose number in
 // out_rows' numbering is p then goes to rank p / peer_rows, row p % peer_rows.

@@ -585,7 +585,7 @@ const char* ep_forward_peer(EpState& st, EpLayerBuffers& b, const MoeDims& d, co
         // gets is only known on the device, so the grids are sized for all of them; the down
         // kernel's epilogue stores each row into its home rank's window, then one thread announces.
         const int slots = G * d.topk;
-        *launches += launch_prefill(ld, true, gate_up.kind == 2, *pw, *ps, lw, slots, u.hidden_f, nullptr, stream);
+        *launches += launch_prefill(ld, true, gate_up.kind == 2, *pw, *ps, lw, slots, nullptr, nullptr, stream);
         *launches += launch_prefill(ld, false, down.kind == 2, *pw, *ps, lw, slots, nullptr, u.perm, stream, outs, R,
                                     uint32_t(t) * d.topk);
         PeerFlags pf{};
@@ -693,7 +693,7 @@ const char* ep_forward(EpState& st, EpLayerBuffers& b, const MoeDims& d, const u
         lw.out = b.out_recv;
         if (pw && ps && pw->gu_t && received >= size_t(prefill_min_avg) * size_t(b.local)) {
             // Prefill-size groups: the tcgen05 kernels, on this rank's tiles.
-            *launches += launch_prefill(ld, true, gate_up.kind == 2, *pw, *ps, lw, int(received), b.hidden_f, nullptr,
+            *launches += launch_prefill(ld, true, gate_up.kind == 2, *pw, *ps, lw, int(received), nullptr, nullptr,
                                         stream);
             *launches += launch_prefill(ld, false, down.kind == 2, *pw, *ps, lw, int(received), b.out_recv,
                                         b.slot_row, stream);

@@ -1,27 +1,40 @@
 // Grouped expert products for prefill-size groups on the 5th-generation tensor
-// cores (tcgen05): int8 x int8 -> int32 MMAs issued by one thread per CTA,
-// operands staged in shared memory by bulk async copies, accumulators in tensor
-// memory (TMEM), read back with tcgen05.ld for the float work.
+// cores (tcgen05), whose results are scaled and added up block by block on the FP32 pipe.
 //
-// Arithmetic: the same single fma chain per output as the decode-size kernel
-// (experts_fast.cu), so a token's value does not depend on which kernel ran:
+// Arithmetic: the same single fma chain per output as the decode-size kernels
+// (experts_fast.cuh), so a token's value does not depend on which kernel ran:
 //     acc = fma(float(sum_b), ws[row,b] * xs[token,b], acc)      b = 0, 1, ...
-// One MMA has K = 32 = one quantization block, and is issued WITHOUT
-// accumulation into its own TMEM buffer: the per-block integer tile must leave
-// the tensor core to be scaled by (weight scale x activation scale) before it
-// can be added. That float work (about 2.5 instructions per output per block on
-// the CUDA cores) bounds this kernel, not the tensor pipe.
+// One block of 32 columns is one product of its own into its own tensor-memory buffer: the block's
+// sums must leave the tensor core to be scaled before they can be added.
 //
-// Work decomposition: a CTA computes one output tile: 128 weight rows (for
-// gate_up: 64 gate rows interleaved with the 64 matching up rows, so SwiGLU
-// pairs sit in adjacent lanes) x 64 tokens of one expert, over all of K.
-// Roles: warp 16 streams operand chunks (8 blocks: 32 KB of weights + 16 KB of
-// activations) through a 3-stage ring; one thread each of warps 17-20 issues the MMAs
-// into a ring of 8 TMEM buffers (64 columns each, handed over four at a time);
-// warps 0-15 drain the buffers
-// (each TMEM lane quadrant is served by four warps, 16 columns each) and keep
-// the float chains in registers. Every wait is bounded and watches a CTA-wide
-// abort flag; TMEM is freed on every path.
+// What bounds it: that float work, two packed FP32 operations per output pair and block: 139 cycles
+// per 128 x 64 x 32 unit and SM, 180 with the tensor-memory loads. So everything else is kept off the
+// float warps' issue slots and off the FP32 pipe:
+//  - The operands are the 8-bit values as f16 (kind::f16). Products and sums of a block are
+//    integers below 2^20, exact in the f32 accumulator, so the sums arrive as floats. With kind::i8
+//    every sum costs a conversion besides (238 cycles per unit); with mma.sync, which would leave the
+//    sums in registers, conversions and a slower instruction (276).
+//  - Block scales travel with the operands, in the same shared-memory stages.
+//  - A finished tile is only parked in shared memory by the float warps; four other warps take it
+//    from there while the next tile's chains run: for gate_up SwiGLU, 8-bit quantization per
+//    32-block (src/kernels.rs:84-98) and the store in the layout the down product reads, so the
+//    SwiGLU rows never visit memory in f32; for down the rows' stores.
+// Persistent CTAs (one per SM) walk (token tile, 128-row tile) pairs; both rings run across tile
+// boundaries. Roles: warps 0-7 float chains (TMEM lane quadrant = warp % 4, half of the tokens
+// = warp / 4: a row's weight scale, a barrier wait and a release are paid once per 64 outputs of a
+// lane), warp 8 streams operand chunks of 2 blocks, one thread of warp 9 issues the products into a ring
+// of two TMEM halves, warps 12-15 finish tiles. An expert's tokens are cut into tiles of 128 and a
+// remainder of 128, 64 or 32 columns (4-bit: 64 at most, since each output keeps a second chain).
+// Every wait is bounded; TMEM is freed on every path.
+//
+// Measured (granite-1b-a400m, 4096 tokens, int8): gate_up 352 -> 234 us, down 220 -> 103 us against the
+// form with 64-column tiles, kind::i8, one tile per CTA, f32 SwiGLU rows in memory and a
+// kernel that tiled them for down. That is 375-410 cycles per unit: two float warps per scheduler do not
+// cover each other's waits for tensor memory, shared memory (which the products read at
+// 128 bytes a clock a third of the time) and the hand-over. Tried: 16 float warps of 32 columns (as
+// fast, a third more instructions), hand-over block by block (5 % slower), polling instead of suspended
+// waits (no change), mma.sync with the sums in registers (8 % slower), kind::i8 (10 % slower).
+#include <algorithm>
 #include <type_traits>
 
 #include "experts_common.cuh"
@@ -31,38 +44,64 @@ namespace tc {
 
 namespace {
 
-constexpr int P_ROWS = 128;           // MMA M
-constexpr int P_TOK = 64;             // MMA N
-constexpr int P_CHUNK = 8;            // blocks per smem stage
-constexpr int P_STAGES = 3;
-constexpr int P_TBUF = 8;             // TMEM buffers of P_TOK columns
-constexpr int P_GROUP = 4;            // buffers per barrier: the ring is handed over in halves
-constexpr int P_NGRP = P_TBUF / P_GROUP;
-static_assert(P_GROUP == 4 && P_CHUNK % P_GROUP == 0, "block b of a group belongs to issuer b % P_MW");
-constexpr int P_A_BLOCK = P_ROWS * 32;  // bytes of one block of weights
-constexpr int P_B_BLOCK = P_TOK * 32;
-constexpr int P_STAGE_BYTES = P_CHUNK * (P_A_BLOCK + P_B_BLOCK);
-constexpr int P_EW = 16;               // epilogue warps: 4 TMEM lane quadrants x 4 column slices
-constexpr int P_COLS = P_TOK * 4 / P_EW;  // columns (tokens) per epilogue warp
-constexpr int P_MW = 4;                // MMA-issuing warps: block b belongs to warp b % P_MW
-constexpr int P_THREADS = (P_EW + 1 + P_MW) * 32;  // + producer + MMA issuers
+constexpr int P_ROWS = 128;             // MMA M
+constexpr int P_CHUNK = 2;              // blocks per shared-memory stage, and per hand-over of TMEM buffers
+constexpr int P_TBUF = 128;             // columns of a TMEM buffer
+constexpr int P_NGRP = 2;               // groups of P_CHUNK buffers: all 512 columns
+constexpr int P_A_BLOCK = P_ROWS * 64;  // bytes of one block of weights (f16)
+constexpr int P_EW = 8;                 // float warps: 4 TMEM lane quadrants x 2 token halves
+constexpr int P_IW = 4;                 // producer, MMA issuer and two warps that make up their warpgroup
+constexpr int P_FW = 4;                 // finishing warps
+constexpr int P_THREADS = (P_EW + P_IW + P_FW) * 32;
 constexpr uint32_t P_SPIN = 1u << 16;
-constexpr int P_SMEM_LIMIT = 226 * 1024;
+constexpr size_t P_SMEM_LIMIT = 227 * 1024 - 256;  // the kernel also has a few static words
+constexpr int P_HSTRIDE = P_ROWS + 4;   // floats per parked token (the pad keeps 16-byte reads conflict-free)
+
+// Registers: 128 a thread at launch (ptxas gives a 512-thread block that many), then split.
+constexpr int P_REGS_LAUNCH = 128, P_REGS_FLOAT = 168, P_REGS_ISSUE = 64, P_REGS_FINISH = 112;
+static_assert((P_EW * P_REGS_FLOAT + P_IW * P_REGS_ISSUE + P_FW * P_REGS_FINISH) * 32 <= P_THREADS * P_REGS_LAUNCH, "register split");
+
+__host__ __device__ constexpr int prefill_columns(bool q4) { return q4 ? 64 : 128; }  // the largest token tile
+
+// A shared-memory stage: P_CHUNK blocks of weights, activations, and their scales.
+template <bool Q4>
+struct Stage {
+    static constexpr int TOK = prefill_columns(Q4);
+    static constexpr int B = P_CHUNK * P_A_BLOCK;
+    static constexpr int WD = B + P_CHUNK * TOK * 64;
+    static constexpr int XS = WD + P_CHUNK * P_ROWS * 4;
+    static constexpr int WC = XS + P_CHUNK * TOK * 4;      // (4-bit only from here)
+    static constexpr int XSUM = WC + P_CHUNK * P_ROWS * 4;
+    static constexpr int BYTES = Q4 ? XSUM + P_CHUNK * TOK * 4 : WC;
+    static constexpr int N = 4;                             // ring depth
+    static constexpr int PARK = TOK * P_HSTRIDE * 4;
+    static constexpr size_t SMEM = size_t(N) * BYTES + PARK + (2 * N + 2 * P_NGRP + 3) * 8;
+    static_assert(SMEM <= P_SMEM_LIMIT, "stages fit");
+};
+
+// Byte offset of (row, k) in a block's operand tile of `rows` rows x 32 f16: 8-row x 16-byte core matrices.
+__host__ __device__ constexpr uint32_t f16_tile_offset(uint32_t rows, uint32_t row, uint32_t k) {
+    return (k / 8) * (rows * 16) + (row / 8) * 128 + (row % 8) * 16 + (k % 8) * 2;
+}
 
 struct PrefillArgs {
-    const int8_t* wt;        // weight tiles [expert][row tile][block][128 x 32 canonical]
+    const uint16_t* wt;      // weight tiles, f16 [expert][row tile][block][128 x 32 canonical]
     const float* wd;         // weight block scales [expert][row tile][nb][128]
     const float* wc;         // 4-bit block offsets, same shape (null for 8-bit)
-    const int8_t* xt;        // activation tiles [token tile][block][64 x 32 canonical]
-    const float* xst;        // activation scales [token tile][nb][64]
+    const uint16_t* xt;      // activation tiles, f16: tile at row0 * 32 * nb, [block][N x 32 canonical]
+    const float* xst;        // activation scales: tile at row0 * nb, [block][N]
     const float* xsumt;      // scale * sum of quants, same shape (4-bit only)
-    const int* tile_expert;  // per token tile
-    const uint32_t* tile_p0; // first sorted slot of the tile
-    const int* tile_n;       // tokens in the tile (1..64)
+    const TokenTile* tiles;
     const int* tile_count;
-    int nb, row_tiles, rows_per_expert, out_cols;
+    int nb, row_tiles, out_cols;
+    // gate_up: the SwiGLU rows as the down product's activation tiles (nb_out = out_cols / 32 blocks)
+    uint16_t* xt_out;
+    float* xst_out;
+    float* xsumt_out;
+    // down: rows of f32
     float* out;
     const uint32_t* out_rows;
+    float one;               // 1.0f, a value the compiler does not know (see add2_exact)
     int* status;
 };
 
@@ -76,7 +115,6 @@ struct PrefillPeer {
 };
 struct NoPeer {};
 
-// Bounded wait that also gives up when another warp of the CTA has.
 __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
@@ -89,296 +127,468 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
     return ok != 0;
 }
 
-__device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-    if (mbar_test(bar, parity)) return true;  // the common case in steady state: no suspension machinery
-    for (uint32_t i = 0; i < P_SPIN; i++) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if (*abort_flag) return false;
-    }
+// Bounded wait. One that runs out sets the CTA's abort flag, and every wait after that gives up at
+// once; the warps then run on to the end over whatever they find (every address they form stays in
+// bounds) and the kernel reports the failure. Waits that could leave the loops instead would make
+// every loop counter, and with it every address, a per-lane value to the compiler: each tensor
+// memory load would then wait for a move into a uniform register.
+__device__ __forceinline__ void wait_or_abort(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+    if (mbar_test(bar, parity)) return;
+    for (uint32_t i = 0; i < P_SPIN; i++)
+        if (mbar_try_wait(bar, parity) || *abort_flag) return;
     *abort_flag = 1;
-    return false;
 }
 
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
+__device__ __forceinline__ void mbar_arrive_if(uint64_t* bar, bool mine) {  // predicated: no branch around it
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\t@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(
+                     smem_addr(bar)),
+                 "r"(uint32_t(mine))
+                 : "memory");
+}
+
+// The same value in every lane, told to the compiler.
+__device__ __forceinline__ uint32_t warp_uniform(uint32_t v) { return __reduce_or_sync(0xffffffffu, v); }
+
+// Four signed bytes as f16: 1024 + (v + 128) is exact in f16 and is v + 1152.
+__device__ __forceinline__ uint2 f16_from_s8(uint32_t w) {
+    const uint32_t u = w ^ 0x80808080u;
+    const __half2 bias = __halves2half2(__ushort_as_half(0x6480), __ushort_as_half(0x6480));
+    uint32_t lo = __byte_perm(u, 0x64646464u, 0x4140), hi = __byte_perm(u, 0x64646464u, 0x4342);
+    const __half2 l = __hsub2(*reinterpret_cast<__half2*>(&lo), bias), h = __hsub2(*reinterpret_cast<__half2*>(&hi), bias);
+    return make_uint2(*reinterpret_cast<const uint32_t*>(&l), *reinterpret_cast<const uint32_t*>(&h));
+}
+
+__device__ __forceinline__ float2 splat(float v) { return make_float2(v, v); }
+
+// a + b in one packed operation: fma(a, 1, b) with a 1 the compiler cannot see. (It fuses a packed
+// product into a packed addition that follows it, even where fusing is turned off for the scalar
+// forms, and also when the addition is written as an fma by a constant 1.)
+__device__ __forceinline__ float2 add2_exact(float2 a, float2 b, float2 one) { return fma2(a, one, b); }
+
+// exp_poly (experts_common.cuh) on two values: the same operations, packed. Rounding half away from
+// zero is truncation after adding the float below one half with the value's sign, which is exact
+// for the arguments that reach it (|x * log2 e| < 129).
+__device__ __forceinline__ float2 exp_poly2(float2 x, float2 one) {
+    auto clamp = [](float v) {
+        float r;
+        asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(v), "f"(-87.33655f));
+        asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(r), "f"(88.7f));
+        return r;
+    };
+    x.x = clamp(x.x), x.y = clamp(x.y);
+    const float2 z = mul2(x, splat(1.44269504088896340736f));
+    const int n0 = __float2int_rz(z.x + copysignf(0.49999997f, z.x)), n1 = __float2int_rz(z.y + copysignf(0.49999997f, z.y));
+    const float2 n = make_float2(__int2float_rn(n0), __int2float_rn(n1));
+    // x - n * c1 - n * c2, each product rounded first (negating a factor negates the product exactly)
+    const float2 r = add2_exact(mul2(n, splat(2.1219444e-4f)), add2_exact(mul2(n, splat(-0.6933594f)), x, one), one);
+    float2 y = splat(1.9875692e-4f);
+    y = add2_exact(mul2(y, r), splat(1.3981999e-3f), one);
+    y = add2_exact(mul2(y, r), splat(8.333452e-3f), one);
+    y = add2_exact(mul2(y, r), splat(4.1665796e-2f), one);
+    y = add2_exact(mul2(y, r), splat(0.16666665f), one);
+    y = add2_exact(mul2(y, r), splat(0.5f), one);
+    y = add2_exact(add2_exact(mul2(y, mul2(r, r)), r, one), one, one);
+    return make_float2(__int_as_float(__float_as_int(y.x) + (n0 << 23)), __int_as_float(__float_as_int(y.y) + (n1 << 23)));
+}
+
+// silu(g) = g / (1 + exp(-g)) on two values, correctly rounded as the IEEE division is: Markstein's
+// scheme (IBM J. Res. Dev. 34, 1990: a reciprocal refined once, a quotient, one correction by its exact
+// remainder), packed. Not for arguments whose quotient or remainder could leave the normal range:
+// `usable` becomes false for those. (Compared with the division for every float g.)
+__device__ __forceinline__ float2 silu2(float2 g, float2 one, bool& usable) {
+    const float2 den = add2_exact(exp_poly2(make_float2(-g.x, -g.y), one), one, one);
+    float2 y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y.x) : "f"(den.x));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y.y) : "f"(den.y));
+    const float2 nden = make_float2(-den.x, -den.y);
+    y = fma2(y, fma2(nden, y, splat(1.0f)), y);
+    const float2 q = mul2(g, y);
+    usable = usable && fmaxf(den.x, den.y) < 1e18f && fminf(fabsf(g.x), fabsf(g.y)) > 1e-18f &&
+             fmaxf(fabsf(g.x), fabsf(g.y)) < 1e18f;
+    return fma2(fma2(nden, q, g), y, q);
+}
+
+// A role's place in the two rings is one number, the chunks of the CTA's sequence so far, across tiles:
+// chunk c is in operand stage c % 4 and in TMEM half c % 2.
+template <bool Q4>
+__device__ __forceinline__ uint32_t stage_of(uint32_t c) { return c % Stage<Q4>::N; }
+template <bool Q4>
+__device__ __forceinline__ uint32_t stage_par(uint32_t c) { return (c / Stage<Q4>::N) & 1; }
+__device__ __forceinline__ uint32_t half_of(uint32_t c) { return c % P_NGRP; }
+__device__ __forceinline__ uint32_t half_par(uint32_t c) { return (c / P_NGRP) & 1; }
+
+struct Bars {
+    uint64_t *full, *empty;    // [stages] operands landed; left by every float warp (and, before them, by the MMAs)
+    uint64_t *tfull, *tempty;  // [P_NGRP] a chunk's sums are in TMEM; read out by every float warp
+    uint64_t *pfull, *pempty;  // a tile has been parked by every float warp; taken by every finishing warp
+    uint64_t* drain;           // after a failure only: the issuer's MMAs so far are done
+    volatile int* abort_flag;
+};
+
+__device__ __forceinline__ float4 staged_f4(uint32_t addr) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ float staged_f1(uint32_t addr) {
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+    return v;
+}
+
+// One tile's float work for this warp's 32 rows x CW tokens: reads each block's sums from TMEM (a piece
+// ahead of the arithmetic: the load is asynchronous until wait_ld, and two register pieces
+// alternate) and keeps the chains in registers. A barrier is tested one piece of arithmetic before the
+// answer is needed.
+template <bool Q4, int CW>
+__device__ __forceinline__ void float_chains(float (&acc)[64], float (&off)[Q4 ? 32 : 1], uint32_t& c, uint32_t smem,
+                                             const Bars& bars, uint32_t tbase, int nb, int col0, int row, int lane) {
+    using S = Stage<Q4>;
+    constexpr int N = CW * 2, PC = 16, PIECES = CW / PC;
+    float v[2][PC];
+#pragma unroll
+    for (int j = 0; j < CW; j++) {
+        acc[j] = 0.0f;
+        if (Q4) off[j] = 0.0f;
+    }
+    auto fetch = [&](uint32_t half, int k, int p, float (&dst)[PC]) {
+        umma::ld_f32(tbase + (half * P_CHUNK + k) * P_TBUF + col0 + p * PC, dst);
+    };
+    // A piece's scales: one of its row, PC of its tokens (4-bit: and the offsets').
+    struct Scales {
+        float w, c;
+        float4 x[PC / 4], u[Q4 ? PC / 4 : 1];
+    };
+    auto chains = [&](const float (&cur)[PC], int p, const Scales& sc) {
+        const float2 w = make_float2(sc.w, sc.w), cc = make_float2(sc.c, sc.c);
+#pragma unroll
+        for (int j = 0; j < PC / 4; j++) {
+            const float4 x = sc.x[j];
+            const int i = 4 * j, o = p * PC + i;
+            const float2 r0 = fma2(make_float2(cur[i], cur[i + 1]), mul2(w, make_float2(x.x, x.y)), make_float2(acc[o], acc[o + 1]));
+            const float2 r1 = fma2(make_float2(cur[i + 2], cur[i + 3]), mul2(w, make_float2(x.z, x.w)), make_float2(acc[o + 2], acc[o + 3]));
+            acc[o] = r0.x, acc[o + 1] = r0.y, acc[o + 2] = r1.x, acc[o + 3] = r1.y;
+            if (Q4) {
+                const float4 u = sc.u[Q4 ? j : 0];
+                const float2 o0 = fma2(cc, make_float2(u.x, u.y), make_float2(off[o], off[o + 1]));
+                const float2 o1 = fma2(cc, make_float2(u.z, u.w), make_float2(off[o + 2], off[o + 3]));
+                off[o] = o0.x, off[o + 1] = o0.y, off[o + 2] = o1.x, off[o + 3] = o1.y;
+            }
+        }
+    };
+    // A chunk of NBLK blocks in TMEM half HALF (constants keep the addresses out of the loop's
+    // arithmetic); its first piece is already on its way into v[0].
+    auto chunk = [&](bool more, auto nblk_c, auto half_c) {
+        constexpr int NBLK = decltype(nblk_c)::value, ITEMS = NBLK * PIECES;
+        constexpr uint32_t HALF = decltype(half_c)::value;
+        const uint32_t st = smem + stage_of<Q4>(c) * S::BYTES;
+        const uint32_t ws = st + S::WD + row * 4, xs = st + S::XS + col0 * 4;
+        const uint32_t wcs = st + S::WC + row * 4, su = st + S::XSUM + col0 * 4;
+        bool ready = false;
+#pragma unroll
+        for (int i = 0; i < ITEMS; i++) {
+            const int k = i / PIECES, p = i % PIECES;
+            Scales sc;
+            sc.w = staged_f1(ws + k * P_ROWS * 4);
+            sc.c = Q4 ? staged_f1(wcs + k * P_ROWS * 4) : 0.0f;
+#pragma unroll
+            for (int j = 0; j < PC / 4; j++) {
+                sc.x[j] = staged_f4(xs + (k * N + p * PC + 4 * j) * 4);
+                if (Q4) sc.u[j] = staged_f4(su + (k * N + p * PC + 4 * j) * 4);
+            }
+            umma::wait_ld(v[i & 1]);
+            if (i + 1 < ITEMS) {
+                fetch(HALF, (i + 1) / PIECES, (i + 1) % PIECES, v[(i + 1) & 1]);
+                if (i + 2 == ITEMS && more)  // the next chunk's sums, and its scales, which its own copies wrote
+                    ready = mbar_test(bars.tfull + (HALF ^ 1), half_par(c + 1)) &&
+                            mbar_test(bars.full + stage_of<Q4>(c + 1), stage_par<Q4>(c + 1));
+            } else {
+                // The chunk's sums and scales have been read: the issuer may overwrite this half, the
+                // producer this stage (whose MMAs were done before the sums could be read).
+                umma::fence_before_sync();
+                __syncwarp();
+                mbar_arrive_if(bars.tempty + HALF, lane == 0);
+                mbar_arrive_if(bars.empty + stage_of<Q4>(c), lane == 0);
+                if (more) {
+                    if (!ready) {
+                        wait_or_abort(bars.full + stage_of<Q4>(c + 1), stage_par<Q4>(c + 1), bars.abort_flag);
+                        wait_or_abort(bars.tfull + (HALF ^ 1), half_par(c + 1), bars.abort_flag);
+                    }
+                    umma::fence_after_sync();
+                    fetch(HALF ^ 1, 0, 0, v[(i + 1) & 1]);
+                }
+            }
+            chains(v[i & 1], p, sc);
+        }
+        c++;
+    };
+    auto any_half = [&](bool more, auto nblk_c) {
+        if (half_of(c)) chunk(more, nblk_c, std::integral_constant<uint32_t, 1>{});
+        else chunk(more, nblk_c, std::integral_constant<uint32_t, 0>{});
+    };
+    wait_or_abort(bars.full + stage_of<Q4>(c), stage_par<Q4>(c), bars.abort_flag);
+    wait_or_abort(bars.tfull + half_of(c), half_par(c), bars.abort_flag);
+    umma::fence_after_sync();
+    fetch(half_of(c), 0, 0, v[0]);
+#pragma unroll 1
+    for (int b = 0; b + 1 < nb; b += 2) any_half(b + 2 < nb, std::integral_constant<int, 2>{});
+    if (nb & 1) any_half(false, std::integral_constant<int, 1>{});
+}
+
+// silu(gate) * up of 32 hidden columns of one token (the parked row holds gate and up side by side),
+// then quantize_q8 (src/kernels.rs:84-98) of that block, as f16 into the token's row of the tile.
+__device__ __forceinline__ void finish_block(const float4* parked, float2 one, uint8_t* dst, int N, float& scale, float& sum) {
+    float2 h[16];
+    bool usable = true;
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+        const float4 v = parked[i];  // gate, up, gate, up
+        h[i] = mul2(silu2(make_float2(v.x, v.z), one, usable), make_float2(v.y, v.w));
+    }
+    if (!usable) {  // (one test for the block: a branch at every pair would keep them from overlapping)
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+            const float4 v = parked[i];
+            h[i].x = __fdiv_rn(v.x, 1.0f + exp_poly(-v.x)) * v.y;
+            h[i].y = __fdiv_rn(v.z, 1.0f + exp_poly(-v.z)) * v.w;
+        }
+    }
+    float amax = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 16; i++) amax = fmaxf(fmaxf(amax, fabsf(h[i].x)), fabsf(h[i].y));
+    const float d = __fdiv_rn(amax, 127.0f);
+    const float id = d > 0.0f ? __fdiv_rn(1.0f, d) : 0.0f;
+    int qsum = 0;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {  // 8 columns: 16 bytes of f16
+        uint2 f[2];
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            // Rounds half away from zero as exp_poly2 does; NaN becomes 0; the packing saturates.
+            int q[4];
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                const float2 t = mul2(h[4 * i + 2 * u + k], make_float2(id, id));
+                q[2 * k] = __float2int_rz(t.x + copysignf(0.49999997f, t.x));
+                q[2 * k + 1] = __float2int_rz(t.y + copysignf(0.49999997f, t.y));
+            }
+            uint32_t w = 0;
+            asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(w) : "r"(q[3]), "r"(q[2]), "r"(0));
+            asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(w) : "r"(q[1]), "r"(q[0]), "r"(w));
+            qsum = __dp4a(int(w), 0x01010101, qsum);
+            f[u] = f16_from_s8(w);
+        }
+        *reinterpret_cast<uint4*>(dst + i * N * 16) = make_uint4(f[0].x, f[0].y, f[1].x, f[1].y);
+    }
+    scale = d;
+    sum = d * float(qsum);
 }
 
 template <bool Q4, bool GATE_UP, bool PEER = false>
 __global__ void __launch_bounds__(P_THREADS, 1)
     expert_prefill_kernel(const PrefillArgs a, const std::conditional_t<PEER, PrefillPeer, NoPeer> peer) {
+    using S = Stage<Q4>;
     extern __shared__ __align__(128) uint8_t smem[];
-    uint8_t* stages = smem;                                                  // P_STAGES x P_STAGE_BYTES
-    float* s_xs = reinterpret_cast<float*>(smem + P_STAGES * P_STAGE_BYTES);  // [nb][64]
-    float* s_xsum = s_xs + a.nb * P_TOK;                                     // [nb][64] (4-bit)
-    float* s_wd = s_xsum + (Q4 ? a.nb * P_TOK : 0);                          // [nb][128]
-    float* s_wc = s_wd + a.nb * P_ROWS;                                      // [nb][128] (4-bit)
-    uint64_t* bars = reinterpret_cast<uint64_t*>(s_wc + (Q4 ? a.nb * P_ROWS : 0));
-    uint64_t* full = bars;                    // [P_STAGES] operands landed
-    uint64_t* empty = bars + P_STAGES;        // [P_STAGES] MMAs that read the stage are done
-    uint64_t* tfull = bars + 2 * P_STAGES;    // [P_TBUF] a block's integer tile is in TMEM
-    uint64_t* tempty = tfull + P_TBUF;        // [P_TBUF] drained by all epilogue warps
-    uint64_t* xbar = tempty + P_TBUF;         // activation scales landed
-    uint64_t* drain = xbar + 1;               // [P_MW] abort path only: an issuer's MMAs so far are done
+    float* parked = reinterpret_cast<float*>(smem + S::N * S::BYTES);  // [tokens][P_HSTRIDE] a finished tile
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
+    Bars bars;
+    bars.full = reinterpret_cast<uint64_t*>(smem + S::N * S::BYTES + S::PARK);
+    bars.empty = bars.full + S::N;
+    bars.tfull = bars.empty + S::N;
+    bars.tempty = bars.tfull + P_NGRP;
+    bars.pfull = bars.tempty + P_NGRP;
+    bars.pempty = bars.pfull + 1;
+    bars.drain = bars.pempty + 1;
+    bars.abort_flag = &s_abort;
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int tt = blockIdx.y, rt = blockIdx.x;
-    if (tt >= *a.tile_count) return;  // uniform: the whole CTA leaves before touching TMEM
-    const int e = a.tile_expert[tt];
-    const int tile_n = a.tile_n[tt];
-    const uint32_t p0 = a.tile_p0[tt];
-    const int nb = a.nb;
-    const int nchunks = (nb + P_CHUNK - 1) / P_CHUNK;
-
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = int(warp_uniform(uint32_t(tid) >> 5));
+    grid_launch_dependents();
     if (tid == 0) {
-        for (int s = 0; s < P_STAGES; s++) {
-            mbar_init(full + s, 1);
-            mbar_init(empty + s, P_MW);
+        for (int s = 0; s < S::N; s++) {
+            mbar_init(bars.full + s, 1);
+            mbar_init(bars.empty + s, P_EW);
         }
         for (int g = 0; g < P_NGRP; g++) {
-            mbar_init(tfull + g, P_MW);
-            mbar_init(tempty + g, P_EW);
+            mbar_init(bars.tfull + g, 1);
+            mbar_init(bars.tempty + g, P_EW);
         }
-        mbar_init(xbar, 1);
-        for (int i = 0; i < P_MW; i++) mbar_init(drain + i, 1);
+        mbar_init(bars.pfull, P_EW);
+        mbar_init(bars.pempty, P_FW);
+        mbar_init(bars.drain, 1);
         s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    __syncthreads();
-    const size_t tile_index = size_t(e) * a.row_tiles + rt;
-    const int8_t* wsrc = a.wt + tile_index * size_t(nb) * P_A_BLOCK;
-    const int8_t* xsrc = a.xt + size_t(tt) * nb * P_B_BLOCK;
-    auto issue_chunk = [&](int c) {
-        const int s = c % P_STAGES;
-        const int nblk = min(P_CHUNK, nb - c * P_CHUNK);
-        uint8_t* st = stages + s * P_STAGE_BYTES;
-        mbar_expect_tx(full + s, uint32_t(nblk) * (P_A_BLOCK + P_B_BLOCK));
-        bulk_copy(st, wsrc + size_t(c) * P_CHUNK * P_A_BLOCK, uint32_t(nblk) * P_A_BLOCK, full + s);
-        bulk_copy(st + P_CHUNK * P_A_BLOCK, xsrc + size_t(c) * P_CHUNK * P_B_BLOCK, uint32_t(nblk) * P_B_BLOCK,
-                  full + s);
-    };
-    const int first_chunks = min(P_STAGES, nchunks);
     if (warp == P_EW + 1) {
-        umma::tmem_alloc(&s_tmem, P_TBUF * P_TOK);
+        umma::tmem_alloc(&s_tmem, P_NGRP * P_CHUNK * P_TBUF);
         umma::tmem_relinquish();
-    } else if (warp == P_EW && lane == 0) {
-        // The ring starts empty: the scales and the first stages' operands are requested
-        // while TMEM is being allocated.
-        const uint32_t xs_bytes = uint32_t(nb) * P_TOK * 4;
-        const uint32_t ws_bytes = uint32_t(nb) * P_ROWS * 4;
-        mbar_expect_tx(xbar, (Q4 ? 2 : 1) * (xs_bytes + ws_bytes));
-        bulk_copy(s_xs, a.xst + size_t(tt) * nb * P_TOK, xs_bytes, xbar);
-        bulk_copy(s_wd, a.wd + tile_index * nb * P_ROWS, ws_bytes, xbar);
-        if (Q4) {
-            bulk_copy(s_xsum, a.xsumt + size_t(tt) * nb * P_TOK, xs_bytes, xbar);
-            bulk_copy(s_wc, a.wc + tile_index * nb * P_ROWS, ws_bytes, xbar);
-        }
-        for (int c = 0; c < first_chunks; c++) issue_chunk(c);
     }
     umma::fence_before_sync();
     __syncthreads();
     umma::fence_after_sync();
     const uint32_t tmem = s_tmem;
-    volatile int* abort_flag = &s_abort;
-
-    if (warp == P_EW) {
-        // ---- producer: the rest of the operand chunks, each once its stage is free again
-        if (lane == 0) {
-            int c = first_chunks;
-            for (; c < nchunks; c++) {
-                const int s = c % P_STAGES;
-                if (!wait_or_abort(empty + s, ((c / P_STAGES) & 1) ^ 1, abort_flag)) break;
-                issue_chunk(c);
-            }
-            if (*abort_flag) {
-                // Giving up: let the copies already issued land before the CTA's shared memory is released.
-                mbar_wait_bounded(xbar, 0);
-                for (int i = max(0, c - P_STAGES); i < c; i++) mbar_wait_bounded(full + i % P_STAGES, (i / P_STAGES) & 1);
-            }
+    grid_dependency_wait();  // everything below reads what earlier kernels wrote
+    const int nb = a.nb;
+    const int work = int(warp_uniform(uint32_t(*a.tile_count * a.row_tiles)));
+    if (warp < P_EW) {
+        // ---- float warps
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(P_REGS_FLOAT));
+        const int quad = warp & 3, slice = warp >> 2;
+        const int row = quad * 32 + lane;  // row of the tile = TMEM lane
+        const uint32_t tbase = tmem + (uint32_t(quad * 32) << 16);
+        uint32_t c = 0;
+        uint32_t parity = 1;  // of pempty: the first tile finds the parking space free
+        for (int w = blockIdx.x; w < work; w += gridDim.x) {
+            const int N = int(warp_uniform(a.tiles[w / a.row_tiles].cols));
+            const int col0 = slice * (N / 2);  // this warp's first token of the tile
+            float acc[64], off[Q4 ? 32 : 1];
+            if (!Q4 && N == 128) float_chains<Q4, Q4 ? 32 : 64>(acc, off, c, smem_addr(smem), bars, tbase, nb, col0, row, lane);
+            else if (N == 64) float_chains<Q4, 32>(acc, off, c, smem_addr(smem), bars, tbase, nb, col0, row, lane);
+            else float_chains<Q4, 16>(acc, off, c, smem_addr(smem), bars, tbase, nb, col0, row, lane);
+            wait_or_abort(bars.pempty, parity, bars.abort_flag);
+            parity ^= 1;
+            float* dst = parked + col0 * P_HSTRIDE + row;
+#pragma unroll
+            for (int j = 0; j < (Q4 ? 32 : 64); j++)
+                if (j < N / 2) dst[j * P_HSTRIDE] = Q4 ? acc[j] + off[Q4 ? j : 0] : acc[j];
+            __syncwarp();
+            mbar_arrive_if(bars.pfull, lane == 0);
         }
-    } else if (warp > P_EW) {
-        // ---- MMA issuers: one block = one MMA into its own TMEM buffer. A single thread
-        // spends several hundred cycles per block on its waits, fence and commit, far more
-        // than the MMA takes, so P_MW threads (one per warp) take the blocks in turn; the
-        // blocks are independent (different TMEM buffers), so no order among them is needed.
-        if (lane == 0) {
-            const uint32_t idesc = umma::idesc_s8(P_ROWS, P_TOK);
-            const int mw = warp - P_EW - 1;
-            const int ngroups = (nb + P_GROUP - 1) / P_GROUP;
-            for (int g = 0; g < ngroups; g++) {
-                // Block mw of every group of P_GROUP (= P_MW) blocks; the group's TMEM half is
-                // free once the epilogue warps have read group g - P_NGRP out of it.
-                const int b = g * P_GROUP + mw, gi = g % P_NGRP;
-                if (!wait_or_abort(tempty + gi, ((g / P_NGRP) & 1) ^ 1, abort_flag)) break;
-                if (b >= nb) {  // ragged last group: keep the arrival count whole
-                    mbar_arrive(tfull + gi);
-                    continue;
+    } else if (warp < P_EW + P_IW) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(P_REGS_ISSUE));
+        if (warp == P_EW && lane == 0) {
+            // ---- producer: operand chunks, each once its stage is free again
+            asm volatile("fence.proxy.async;" ::: "memory");  // the tiles were written by plain stores
+            uint32_t c = 0;
+            for (int w = blockIdx.x; w < work; w += gridDim.x) {
+                const TokenTile tile = a.tiles[w / a.row_tiles];
+                const size_t wtile = size_t(tile.expert) * a.row_tiles + w % a.row_tiles;
+                const uint32_t N = tile.cols;
+                for (int b0 = 0; b0 < nb; b0 += P_CHUNK, c++) {
+                    const uint32_t nblk = min(P_CHUNK, nb - b0);
+                    uint64_t* full = bars.full + stage_of<Q4>(c);
+                    if (c >= uint32_t(S::N)) wait_or_abort(bars.empty + stage_of<Q4>(c), stage_par<Q4>(c) ^ 1, bars.abort_flag);
+                    uint8_t* st = smem + stage_of<Q4>(c) * S::BYTES;
+                    const uint32_t wb = nblk * P_A_BLOCK, xb = nblk * N * 64, wf = nblk * P_ROWS * 4, xf = nblk * N * 4;
+                    const size_t wo = wtile * nb + b0, xo = size_t(tile.row0) * nb + size_t(b0) * N;
+                    mbar_expect_tx(full, wb + xb + (wf + xf) * (Q4 ? 2 : 1));
+                    bulk_copy(st, a.wt + wo * (P_A_BLOCK / 2), wb, full);
+                    bulk_copy(st + S::B, a.xt + xo * 32, xb, full);
+                    bulk_copy(st + S::WD, a.wd + wo * P_ROWS, wf, full);
+                    bulk_copy(st + S::XS, a.xst + xo, xf, full);
+                    if (Q4) {
+                        bulk_copy(st + S::WC, a.wc + wo * P_ROWS, wf, full);
+                        bulk_copy(st + S::XSUM, a.xsumt + xo, xf, full);
+                    }
                 }
-                const int c = b / P_CHUNK, k = b % P_CHUNK, s = c % P_STAGES, buf = b % P_TBUF;
-                if (k < P_MW && !wait_or_abort(full + s, (c / P_STAGES) & 1, abort_flag)) break;
-                umma::fence_after_sync();
-                const uint32_t sa = smem_addr(stages + s * P_STAGE_BYTES + k * P_A_BLOCK);
-                const uint32_t sb = smem_addr(stages + s * P_STAGE_BYTES + P_CHUNK * P_A_BLOCK + k * P_B_BLOCK);
-                umma::mma_s8(tmem + buf * P_TOK, umma::smem_desc(sa, P_ROWS * 16, 128),
-                             umma::smem_desc(sb, P_TOK * 16, 128), idesc, 0u);
-                umma::commit(tfull + gi);
-                // This thread's last block of the chunk. (A ragged last chunk may leave
-                // `empty` short of arrivals: nothing waits for it.)
-                if (k + P_MW >= P_CHUNK || b + P_MW >= nb) umma::commit(empty + s);
             }
-            if (*abort_flag) {
+            if (s_abort) {
+                // Giving up: let the copies already issued land before the CTA's shared memory is released.
+                for (uint32_t i = c > uint32_t(S::N) ? c - S::N : 0; i < c; i++)
+                    mbar_wait_bounded(bars.full + stage_of<Q4>(i), stage_par<Q4>(i));
+            }
+        } else if (warp == P_EW + 1 && lane == 0) {
+            // ---- MMA issuer: a block = two K = 16 products into its own TMEM buffer, a commit per chunk
+            uint32_t c = 0;
+            for (int w = blockIdx.x; w < work; w += gridDim.x) {
+                const uint32_t N = a.tiles[w / a.row_tiles].cols, idesc = umma::idesc_f16(P_ROWS, int(N));
+                for (int b0 = 0; b0 < nb; b0 += P_CHUNK, c++) {
+                    const int nblk = min(P_CHUNK, nb - b0);
+                    wait_or_abort(bars.full + stage_of<Q4>(c), stage_par<Q4>(c), bars.abort_flag);
+                    if (c >= uint32_t(P_NGRP)) wait_or_abort(bars.tempty + half_of(c), half_par(c) ^ 1, bars.abort_flag);
+                    umma::fence_after_sync();
+                    const uint32_t sa = smem_addr(smem + stage_of<Q4>(c) * S::BYTES), sb = sa + S::B;
+#pragma unroll
+                    for (int k = 0; k < P_CHUNK; k++) {
+                        if (k < nblk) {
+                            const uint32_t d = tmem + (half_of(c) * P_CHUNK + k) * P_TBUF;
+#pragma unroll
+                            for (int h = 0; h < 2; h++)
+                                umma::mma_f16(d, umma::smem_desc(sa + k * P_A_BLOCK + h * P_ROWS * 32, P_ROWS * 16, 128),
+                                              umma::smem_desc(sb + k * N * 64 + h * N * 32, N * 16, 128), idesc, uint32_t(h));
+                        }
+                    }
+                    umma::commit(bars.tfull + half_of(c));
+                }
+            }
+            if (s_abort) {
                 // Giving up: the MMAs in flight must finish before TMEM is freed.
-                umma::commit(drain + mw);
-                mbar_wait_bounded(drain + mw, 0);
+                umma::commit(bars.drain);
+                mbar_wait_bounded(bars.drain, 0);
             }
         }
     } else {
-        // ---- epilogue: warp w drains lanes 32*(w%4).. and columns P_COLS*(w/4)..
-        const int quad = warp & 3, slice = warp >> 2;
-        const int row = quad * 32 + lane;  // row of the tile = TMEM lane
-        float acc[P_COLS], off[Q4 ? P_COLS : 1];
-#pragma unroll
-        for (int j = 0; j < P_COLS; j++) acc[j] = 0.0f;
-        if (Q4) {
-#pragma unroll
-            for (int j = 0; j < P_COLS; j++) off[j] = 0.0f;
-        }
-        bool ok = wait_or_abort(xbar, 0, abort_flag);
-        const uint32_t tbase = tmem + (uint32_t(quad * 32) << 16) + slice * P_COLS;
-        // One block's float work on the integer tile in v.
-        auto consume = [&](int b, const int (&v)[P_COLS]) {
-            const float wdb = s_wd[b * P_ROWS + row];
-            const float wcb = Q4 ? s_wc[b * P_ROWS + row] : 0.0f;
-            const float4* xs4 = reinterpret_cast<const float4*>(s_xs + b * P_TOK + slice * P_COLS);
-            const float4* su4 = reinterpret_cast<const float4*>(s_xsum + b * P_TOK + slice * P_COLS);
-#pragma unroll
-            for (int j = 0; j < P_COLS / 4; j++) {
-                const float4 x = xs4[j];
-                const float2 xlo = make_float2(x.x, x.y), xhi = make_float2(x.z, x.w);
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const int i = 4 * j + 2 * h;
-                    // The conversion unit works beside the FP32 pipe, which the two packed
-                    // operations below keep busy; the add-a-magic-number conversion used
-                    // where issue slots are short would add a third FP32 operation here.
-                    const float2 sum = make_float2(__int2float_rn(v[i]), __int2float_rn(v[i + 1]));
-                    const float2 d = mul2(make_float2(wdb, wdb), h ? xhi : xlo);
-                    const float2 r = fma2(sum, d, make_float2(acc[i], acc[i + 1]));
-                    acc[i] = r.x;
-                    acc[i + 1] = r.y;
-                }
-                if (Q4) {
-                    const float4 u = su4[j];
-                    const float2 o0 = fma2(make_float2(wcb, wcb), make_float2(u.x, u.y),
-                                           make_float2(off[4 * j], off[4 * j + 1]));
-                    const float2 o1 = fma2(make_float2(wcb, wcb), make_float2(u.z, u.w),
-                                           make_float2(off[4 * j + 2], off[4 * j + 3]));
-                    off[4 * j] = o0.x, off[4 * j + 1] = o0.y, off[4 * j + 2] = o1.x, off[4 * j + 3] = o1.y;
-                }
-            }
-        };
-        // Block b's tile is read from TMEM while block b-1's float work runs: the load is
-        // asynchronous until wait_ld, and the two register tiles alternate.
-        auto fetch = [&](int b, int (&v)[P_COLS]) -> bool {
-            if (b % P_GROUP == 0) {  // first block of a group: its MMAs are all done
-                if (!wait_or_abort(tfull + (b / P_GROUP) % P_NGRP, (b / P_TBUF) & 1, abort_flag)) return false;
-                umma::fence_after_sync();
-            }
-            umma::ld_32x16(tbase + (b % P_TBUF) * P_TOK, v);
-            return true;
-        };
-        auto release = [&](int b) {  // after wait_ld of a group's last block: its half may be overwritten
-            if (b % P_GROUP == P_GROUP - 1 || b == nb - 1) {
-                umma::fence_before_sync();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(tempty + (b / P_GROUP) % P_NGRP);
-            }
-        };
-        int va[P_COLS], vb[P_COLS];
-        if (ok) ok = fetch(0, va);
-        for (int b = 0; ok && b < nb; b += 2) {
-            umma::wait_ld(va);
-            release(b);
-            if (b + 1 < nb && !fetch(b + 1, vb)) {
-                ok = false;
-                break;
-            }
-            consume(b, va);
-            if (b + 1 < nb) {
-                umma::wait_ld(vb);
-                release(b + 1);
-                if (b + 2 < nb && !fetch(b + 2, va)) {
-                    ok = false;
-                    break;
-                }
-                consume(b + 1, vb);
-            }
-        }
-        ok = __all_sync(0xffffffffu, ok);
-        if (ok) {
+        // ---- finishing warps
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(P_REGS_FINISH));
+        const int ftid = tid - (P_EW + P_IW) * 32;
+        const float2 one = make_float2(a.one, a.one);
+        uint32_t parity = 0;  // of pfull
+        for (int w = blockIdx.x; w < work; w += gridDim.x, parity ^= 1) {
+            const TokenTile tile = a.tiles[w / a.row_tiles];
+            const int rt = w % a.row_tiles, N = int(tile.cols), tile_n = int(tile.n);
+            wait_or_abort(bars.pfull, parity, bars.abort_flag);
             if (GATE_UP) {
-                // Lanes 2i / 2i+1 hold the gate / up row of hidden column 64*rt + i. The pair
-                // trades halves so that each lane finishes one token of every two: the even
-                // lane token j (its gate, the partner's up), the odd lane token j+1.
-                const bool odd = lane & 1;
-                const int col = rt * 64 + (row >> 1);
-#pragma unroll
-                for (int j = 0; j < P_COLS; j += 2) {
-                    float y0 = acc[j], y1 = acc[j + 1];
-                    if (Q4) y0 = y0 + off[j], y1 = y1 + off[j + 1];
-                    const float got = __shfl_xor_sync(0xffffffffu, odd ? y0 : y1, 1);
-                    const float g = odd ? got : y0, up = odd ? y1 : got;
-                    const int n = slice * P_COLS + j + (odd ? 1 : 0);  // token of the tile
-                    if (n < tile_n && col < a.out_cols) {
-                        const float ex = exp_poly(-g);
-                        a.out[size_t(p0 + n) * a.out_cols + col] = __fdiv_rn(g, 1.0f + ex) * up;
-                    }
+                // A thread per (token, 32-block of hidden columns). Padding tokens are left as they are:
+                // their columns are never stored.
+                const int nb_out = a.out_cols / QK;
+#pragma unroll 1
+                for (int i = ftid; i < N * 2; i += P_FW * 32) {
+                    const int n = i & (N - 1), q = i / N, b = rt * 2 + q;
+                    if (n >= tile_n || b >= nb_out) continue;
+                    uint8_t* dst = reinterpret_cast<uint8_t*>(a.xt_out + size_t(tile.row0) * a.out_cols + size_t(b) * N * 32) +
+                                   f16_tile_offset(N, n, 0);
+                    float d, su;
+                    finish_block(reinterpret_cast<const float4*>(parked + n * P_HSTRIDE + q * 64), one, dst, N, d, su);
+                    const size_t so = size_t(tile.row0) * nb_out + size_t(b) * N + n;
+                    a.xst_out[so] = d;
+                    a.xsumt_out[so] = su;
                 }
             } else {
-                const int r = rt * P_ROWS + row;
-#pragma unroll
-                for (int j = 0; j < P_COLS; j++) {
-                    float y = acc[j];
-                    if (Q4) y = y + off[j];
-                    const int n = slice * P_COLS + j;
-                    if (n < tile_n && r < a.out_cols) {
-                        size_t p = p0 + n;
-                        if (a.out_rows) p = a.out_rows[p];
-                        float* dst = a.out;
-                        if constexpr (PEER) {
-                            const uint32_t home = uint32_t(p) / peer.rows;
-                            p -= size_t(home) * peer.rows;
-                            dst = peer.out[home];
-                        }
-                        dst[p * a.out_cols + r] = y;
+                // A warp per token row, 16 bytes a lane. (out_cols is a multiple of 32.)
+                const int r = rt * P_ROWS + lane * 4;
+#pragma unroll 4
+                for (int n = ftid >> 5; n < tile_n; n += P_FW) {
+                    const float4 v = *reinterpret_cast<const float4*>(parked + n * P_HSTRIDE + lane * 4);
+                    size_t p = tile.p0 + n;
+                    if (a.out_rows) p = a.out_rows[p];
+                    float* dst = a.out;
+                    if constexpr (PEER) {
+                        const uint32_t home = uint32_t(p) / peer.rows;
+                        p -= size_t(home) * peer.rows;
+                        dst = peer.out[home];
                     }
+                    if (r < a.out_cols) *reinterpret_cast<float4*>(dst + p * a.out_cols + r) = v;
                 }
             }
+            __syncwarp();
+            mbar_arrive_if(bars.pempty, lane == 0);
         }
     }
     umma::fence_before_sync();
     __syncthreads();
-    if (warp == P_EW + 1) umma::tmem_dealloc(tmem, P_TBUF * P_TOK);
+    if (warp == P_EW + 1) umma::tmem_dealloc(tmem, P_NGRP * P_CHUNK * P_TBUF);
     if (tid == 0 && s_abort) atomicExch(a.status, ERR_COPY_WAIT_TIMEOUT);
 }
 
 // ---------------------------------------------------------------- tiling kernels
 
-// Weights of one (expert, row tile) into canonical 128 x 32 tiles per block,
-// with their block scales (and 4-bit offsets) as f32 per (block, row). 4-bit
-// values are expanded to int8 (q - 8). One CTA per (expert, row tile).
+// Weights as f16 into canonical 128 x 32 tiles per block, with their block scales (and 4-bit offsets) as
+// f32 per (block, row); gate_up rows interleaved (gate, up, gate, ...). 4-bit values become q - 8. A
+// thread per (row, block), a warp's lanes on 32 consecutive rows: 32-byte reads, 512-byte runs of stores.
+// blockIdx.y: a range of P_WT_BLOCKS blocks.
+constexpr int P_WT_BLOCKS = 8;
 template <bool Q4, bool GATE_UP>
-__global__ void tile_prefill_weights_kernel(const uint8_t* __restrict__ wdata, const void* __restrict__ wscales,
-                                            int cols, int rows_per_expert, int row_tiles,
-                                            int8_t* __restrict__ wt, float* __restrict__ wd,
-                                            float* __restrict__ wc) {
+__global__ void __launch_bounds__(256)
+    tile_prefill_weights_kernel(const uint8_t* __restrict__ wdata, const void* __restrict__ wscales, int cols,
+                                int rows_per_expert, int row_tiles, uint16_t* __restrict__ wt, float* __restrict__ wd,
+                                float* __restrict__ wc) {
     const int rt = blockIdx.x % row_tiles, e = blockIdx.x / row_tiles;
     const int nb = cols / QK;
-    const size_t tile_index = size_t(e) * row_tiles + rt;
-    int8_t* dst = wt + tile_index * size_t(nb) * P_A_BLOCK;
-    for (int r = 0; r < P_ROWS; r++) {
+    const int b_lo = blockIdx.y * P_WT_BLOCKS, b_n = min(P_WT_BLOCKS, nb - b_lo);
+    for (int task = threadIdx.x; task < P_ROWS * b_n; task += 256) {
+        const int r = task % P_ROWS, b = b_lo + task / P_ROWS;
         int row;
         if (GATE_UP) {
             const int inter = rows_per_expert / 2, col = rt * 64 + (r >> 1);
@@ -387,157 +597,127 @@ __global__ void tile_prefill_weights_kernel(const uint8_t* __restrict__ wdata, c
             const int rr = rt * P_ROWS + r;
             row = rr < rows_per_expert ? e * rows_per_expert + rr : -1;
         }
-        for (int i = threadIdx.x; i < cols; i += blockDim.x) {
-            const int b = i / QK, k = i % QK;
-            int8_t v = 0;
-            if (row >= 0) {
-                if (!Q4) {
-                    v = int8_t(wdata[size_t(row) * cols + i]);
-                } else {
-                    const uint8_t byte = wdata[(size_t(row) * cols) / 2 + b * 16 + (k & 15)];
-                    v = int8_t(int(k < 16 ? (byte & 0xF) : (byte >> 4)) - 8);
-                }
-            }
-            dst[size_t(b) * P_A_BLOCK + umma::tile_offset(P_ROWS, r, k)] = v;
-        }
-        for (int b = threadIdx.x; b < nb; b += blockDim.x) {
-            float d = 0.0f, c = 0.0f;
-            if (row >= 0) {
-                if (!Q4) {
-                    d = f16_bits_to_f32(reinterpret_cast<const uint16_t*>(wscales)[size_t(row) * nb + b]);
-                } else {
-                    const int words = (nb + SUPER - 1) / SUPER * SUPER_WORDS;
-                    const uint32_t* w = reinterpret_cast<const uint32_t*>(wscales) + size_t(row) * words +
-                                        (b / SUPER) * SUPER_WORDS;
-                    const int j = b % SUPER;
-                    d = f16_bits_to_f32(uint16_t(w[0])) * float((w[1 + j / 4] >> (8 * (j % 4))) & 0xFFu);
-                    c = f16_bits_to_f32(uint16_t(w[0] >> 16)) *
-                        float(int(int8_t(uint8_t(w[3 + j / 4] >> (8 * (j % 4))))));
-                }
-            }
-            wd[(tile_index * nb + b) * P_ROWS + r] = d;
-            if (Q4) wc[(tile_index * nb + b) * P_ROWS + r] = c;
-        }
-    }
-}
-
-// The token tiles of the experts: expert e with m tokens gets ceil(m / 64) tiles. One CTA.
-__global__ void build_token_tiles_kernel(const uint32_t* __restrict__ counts, const uint32_t* __restrict__ offsets,
-                                         int experts, int* __restrict__ tile_expert,
-                                         uint32_t* __restrict__ tile_p0, int* __restrict__ tile_n,
-                                         int* __restrict__ tile_count) {
-    __shared__ int s_base[MAX_EXPERTS + 1];
-    if (threadIdx.x == 0) {
-        int run = 0;
-        for (int e = 0; e < experts; e++) {
-            s_base[e] = run;
-            run += (int(counts[e]) + P_TOK - 1) / P_TOK;
-        }
-        s_base[experts] = run;
-        *tile_count = run;
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < experts; e += blockDim.x) {
-        const int m = int(counts[e]);
-        for (int i = 0; i * P_TOK < m; i++) {
-            const int tt = s_base[e] + i;
-            tile_expert[tt] = e;
-            tile_p0[tt] = offsets[e] + i * P_TOK;
-            tile_n[tt] = min(P_TOK, m - i * P_TOK);
-        }
-    }
-}
-
-// Activations into canonical 64 x 32 tiles per (token tile, block), scales (and
-// block sums) transposed to [block][token]. Source rows are already 8-bit
-// (xq/xs/xsum through row_of_slot) or f32 rows to quantize here (xf), as
-// quantize_q8 does (src/kernels.rs:84-98). A thread per (token, block).
-template <bool Q4>
-__global__ void tile_activations_kernel(const int8_t* __restrict__ xq, const float* __restrict__ xs,
-                                        const float* __restrict__ xsum, const float* __restrict__ xf,
-                                        const uint32_t* __restrict__ row_of_slot, int cols, int nbp,
-                                        const uint32_t* __restrict__ tile_p0, const int* __restrict__ tile_n,
-                                        const int* __restrict__ tile_count, int8_t* __restrict__ xt,
-                                        float* __restrict__ xst, float* __restrict__ xsumt) {
-    const int nb = cols / QK;
-    const int tt = blockIdx.x;
-    if (tt >= *tile_count) return;
-    const int n_valid = tile_n[tt];
-    const uint32_t p0 = tile_p0[tt];
-    for (int task = threadIdx.x; task < P_TOK * nb; task += blockDim.x) {
-        const int n = task % P_TOK, b = task / P_TOK;
-        uint32_t q[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        float d = 0.0f, su = 0.0f;
-        if (n < n_valid) {
-            const size_t p = p0 + n;
-            const size_t row = row_of_slot ? row_of_slot[p] : p;
-            if (xf) {
-                const float4* src = reinterpret_cast<const float4*>(xf + row * cols + b * QK);
-                float4 v[8];
-#pragma unroll
-                for (int i = 0; i < 8; i++) v[i] = src[i];
-                float amax = 0.0f;
-#pragma unroll
-                for (int i = 0; i < 8; i++)
-                    amax = fmaxf(fmaxf(fmaxf(fmaxf(amax, fabsf(v[i].x)), fabsf(v[i].y)), fabsf(v[i].z)),
-                                 fabsf(v[i].w));
-                d = __fdiv_rn(amax, 127.0f);
-                const float id = d > 0.0f ? __fdiv_rn(1.0f, d) : 0.0f;
-                auto q8 = [&](float x) {
-                    const float rr = roundf(x * id);
-                    return (rr != rr) ? 0 : int(fminf(127.0f, fmaxf(-128.0f, rr)));
-                };
-                int qsum = 0;
-#pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    const int q0 = q8(v[i].x), q1 = q8(v[i].y), q2 = q8(v[i].z), q3 = q8(v[i].w);
-                    qsum += q0 + q1 + q2 + q3;
-                    q[i] = uint32_t(q0 & 0xFF) | (uint32_t(q1 & 0xFF) << 8) | (uint32_t(q2 & 0xFF) << 16) |
-                           (uint32_t(q3 & 0xFF) << 24);
-                }
-                su = d * float(qsum);
-            } else {
-                const uint4* src = reinterpret_cast<const uint4*>(xq + row * cols + b * QK);
+        uint32_t w[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // the block's 32 values as signed bytes
+        float d = 0.0f, c = 0.0f;
+        if (row >= 0) {
+            if (!Q4) {
+                const uint4* src = reinterpret_cast<const uint4*>(wdata + size_t(row) * cols + b * QK);
                 const uint4 lo = src[0], hi = src[1];
-                q[0] = lo.x, q[1] = lo.y, q[2] = lo.z, q[3] = lo.w;
-                q[4] = hi.x, q[5] = hi.y, q[6] = hi.z, q[7] = hi.w;
-                d = xs[row * nbp + b];
-                if (Q4) su = xsum[row * nbp + b];
+                w[0] = lo.x, w[1] = lo.y, w[2] = lo.z, w[3] = lo.w;
+                w[4] = hi.x, w[5] = hi.y, w[6] = hi.z, w[7] = hi.w;
+                d = f16_bits_to_f32(reinterpret_cast<const uint16_t*>(wscales)[size_t(row) * nb + b]);
+            } else {
+                // Low nibbles are elements 0..15, high nibbles 16..31.
+                const uint4 v = *reinterpret_cast<const uint4*>(wdata + (size_t(row) * cols) / 2 + b * 16);
+                const uint32_t n[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    w[i] = uint32_t(nibbles_minus8(n[i] & 0x0F0F0F0Fu));
+                    w[4 + i] = uint32_t(nibbles_minus8((n[i] >> 4) & 0x0F0F0F0Fu));
+                }
+                const int words = (nb + SUPER - 1) / SUPER * SUPER_WORDS;
+                const uint32_t* sw = reinterpret_cast<const uint32_t*>(wscales) + size_t(row) * words + (b / SUPER) * SUPER_WORDS;
+                const int j = b % SUPER;
+                d = f16_bits_to_f32(uint16_t(sw[0])) * float((sw[1 + j / 4] >> (8 * (j % 4))) & 0xFFu);
+                c = f16_bits_to_f32(uint16_t(sw[0] >> 16)) * float(int(int8_t(uint8_t(sw[3 + j / 4] >> (8 * (j % 4))))));
             }
         }
-        // Bytes 0-15 and 16-31 of the token's block are the two K halves of its core-matrix row.
-        int8_t* dst = xt + (size_t(tt) * nb + b) * P_B_BLOCK;
-        *reinterpret_cast<uint4*>(dst + umma::tile_offset(P_TOK, n, 0)) = make_uint4(q[0], q[1], q[2], q[3]);
-        *reinterpret_cast<uint4*>(dst + umma::tile_offset(P_TOK, n, 16)) = make_uint4(q[4], q[5], q[6], q[7]);
-        xst[(size_t(tt) * nb + b) * P_TOK + n] = d;
-        if (Q4) xsumt[(size_t(tt) * nb + b) * P_TOK + n] = su;
+        const size_t at = (size_t(e) * row_tiles + rt) * nb + b;
+        uint8_t* dst = reinterpret_cast<uint8_t*>(wt) + at * P_A_BLOCK + f16_tile_offset(P_ROWS, r, 0);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const uint2 f0 = f16_from_s8(w[2 * i]), f1 = f16_from_s8(w[2 * i + 1]);
+            *reinterpret_cast<uint4*>(dst + i * P_ROWS * 16) = make_uint4(f0.x, f0.y, f1.x, f1.y);
+        }
+        wd[at * P_ROWS + r] = d;
+        if (Q4) wc[at * P_ROWS + r] = c;
     }
 }
 
-size_t prefill_smem(int nb, bool q4) {
-    return size_t(P_STAGES) * P_STAGE_BYTES + size_t(nb) * (P_TOK + P_ROWS) * 4 * (q4 ? 2 : 1) +
-           (2 * P_STAGES + 2 * P_TBUF + 1 + P_MW) * 8 + 64;
+// The token tiles of the experts. Expert e's m tokens: whole tiles of most_cols (128 or 64), then the
+// remainder as one tile of 32, 64 or 128 columns. One CTA, a thread per expert.
+__global__ void __launch_bounds__(MAX_EXPERTS)
+    build_token_tiles_kernel(const uint32_t* counts, const uint32_t* offsets, int experts, int most_cols,
+                             TokenTile* tiles, int* tile_count) {
+    __shared__ int s_tiles[MAX_EXPERTS / 32], s_rows[MAX_EXPERTS / 32];
+    grid_launch_dependents();
+    grid_dependency_wait();
+    const int e = threadIdx.x, lane = e & 31, warp = e >> 5;
+    const int m = e < experts ? int(counts[e]) : 0;
+    const int whole = m / most_cols, rest = m - whole * most_cols;
+    const int mine = whole + (rest ? 1 : 0);
+    const int rows = whole * most_cols + (rest == 0 ? 0 : rest > 64 ? 128 : rest > 32 ? 64 : 32);
+    int t_in = mine, r_in = rows;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t_up = __shfl_up_sync(0xffffffffu, t_in, o), r_up = __shfl_up_sync(0xffffffffu, r_in, o);
+        if (lane >= o) t_in += t_up, r_in += r_up;
+    }
+    if (lane == 31) s_tiles[warp] = t_in, s_rows[warp] = r_in;
+    __syncthreads();
+    int tt = t_in - mine, row0 = r_in - rows;
+    for (int k = 0; k < warp; k++) tt += s_tiles[k], row0 += s_rows[k];
+    if (e == MAX_EXPERTS - 1) *tile_count = tt + mine;
+    if (e >= experts) return;
+    uint32_t p0 = offsets[e];
+    int left = m;
+    for (int i = 0; i < mine; i++) {
+        const int cols = left > 64 ? most_cols : left > 32 ? 64 : 32;
+        const int n = min(left, cols);
+        tiles[tt + i] = TokenTile{e, p0, uint32_t(row0), uint16_t(n), uint16_t(cols)};
+        p0 += n, row0 += cols, left -= n;
+    }
+}
+
+// The 8-bit rows of the block's input (xq/xs/xsum through row_of_slot) as f16 into canonical
+// (columns x 32) tiles per (token tile, block), scales (and block sums) transposed to
+// [block][token]. A thread per (token, block), blockIdx.y a range of blocks. Padding tokens are left as they are.
+constexpr int P_ACT_BLOCKS = 8;
+template <bool Q4>
+__global__ void __launch_bounds__(256)
+    tile_activations_kernel(const int8_t* xq, const float* xs, const float* xsum, const uint32_t* row_of_slot, int cols,
+                            int nbp, const TokenTile* tiles, const int* tile_count, uint16_t* xt, float* xst, float* xsumt) {
+    grid_launch_dependents();
+    grid_dependency_wait();
+    const int nb = cols / QK;
+    if (int(blockIdx.x) >= *tile_count) return;
+    const TokenTile tile = tiles[blockIdx.x];
+    const int N = tile.cols, b_lo = blockIdx.y * P_ACT_BLOCKS, b_n = min(P_ACT_BLOCKS, nb - b_lo);
+    for (int task = threadIdx.x; task < N * b_n; task += 256) {
+        const int n = task & (N - 1), b = b_lo + task / N;
+        if (n >= tile.n) continue;
+        const size_t row = row_of_slot[tile.p0 + n];
+        const uint4* src = reinterpret_cast<const uint4*>(xq + row * cols + b * QK);
+        const uint4 in[2] = {src[0], src[1]};
+        const float d = xs[row * nbp + b];
+        uint8_t* dst = reinterpret_cast<uint8_t*>(xt + size_t(tile.row0) * cols + size_t(b) * N * 32) + f16_tile_offset(N, n, 0);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const uint2 f0 = f16_from_s8(i & 1 ? in[i / 2].z : in[i / 2].x), f1 = f16_from_s8(i & 1 ? in[i / 2].w : in[i / 2].y);
+            *reinterpret_cast<uint4*>(dst + i * N * 16) = make_uint4(f0.x, f0.y, f1.x, f1.y);
+        }
+        const size_t so = size_t(tile.row0) * nb + size_t(b) * N + n;
+        xst[so] = d;
+        if (Q4) xsumt[so] = xsum[row * nbp + b];
+    }
 }
 
 }  // namespace
 
 void init_kernels_prefill() {
-    const int lim = P_SMEM_LIMIT;  // the kernel also has a few static words
-    cudaFuncSetAttribute(expert_prefill_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    cudaFuncSetAttribute(expert_prefill_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    cudaFuncSetAttribute(expert_prefill_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    cudaFuncSetAttribute(expert_prefill_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    cudaFuncSetAttribute(expert_prefill_kernel<true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    cudaFuncSetAttribute(expert_prefill_kernel<false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+    auto opt_in = [](auto kernel, size_t bytes) {
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
+    };
+    opt_in(expert_prefill_kernel<false, true>, Stage<false>::SMEM);
+    opt_in(expert_prefill_kernel<false, false>, Stage<false>::SMEM);
+    opt_in(expert_prefill_kernel<false, false, true>, Stage<false>::SMEM);
+    opt_in(expert_prefill_kernel<true, true>, Stage<true>::SMEM);
+    opt_in(expert_prefill_kernel<true, false>, Stage<true>::SMEM);
+    opt_in(expert_prefill_kernel<true, false, true>, Stage<true>::SMEM);
 }
 
 int prefill_row_tiles(const MoeDims& d, bool gate_up) {
     return gate_up ? (d.inter + 63) / 64 : (d.hidden + P_ROWS - 1) / P_ROWS;
-}
-
-bool prefill_fits(const MoeDims& d, bool q4_gate_up, bool q4_down) {
-    return prefill_smem(d.hidden / QK, q4_gate_up) <= size_t(P_SMEM_LIMIT) &&
-           prefill_smem(d.inter / QK, q4_down) <= size_t(P_SMEM_LIMIT);
 }
 
 size_t prefill_weight_bytes(const MoeDims& d, bool gate_up) {
@@ -550,15 +730,18 @@ size_t prefill_scale_elems(const MoeDims& d, bool gate_up) {
     return size_t(d.experts) * prefill_row_tiles(d, gate_up) * P_ROWS * (cols / QK);
 }
 
-int prefill_max_token_tiles(int slots, int experts) { return (slots + P_TOK - 1) / P_TOK + experts; }
-int prefill_token_tile() { return P_TOK; }
+// Bounds over every routing: an expert adds at most one tile beyond its whole ones, and pads by up to 63 rows.
+int prefill_max_token_tiles(int slots, int experts, bool q4) {
+    return slots / prefill_columns(q4) + std::min(slots, experts);
+}
+size_t prefill_max_rows(int slots, int experts) { return size_t(slots) + 63 * size_t(std::min(slots, experts)); }
 
-void tile_prefill_weights(const MoeDims& d, const MatrixDev& m, bool gate_up, int8_t* wt, float* wd, float* wc,
+void tile_prefill_weights(const MoeDims& d, const MatrixDev& m, bool gate_up, uint16_t* wt, float* wd, float* wc,
                           cudaStream_t stream) {
     const int cols = gate_up ? d.hidden : d.inter;
     const int rpe = gate_up ? 2 * d.inter : d.hidden;
     const int rts = prefill_row_tiles(d, gate_up);
-    const unsigned grid = unsigned(d.experts * rts);
+    const dim3 grid(unsigned(d.experts * rts), unsigned((cols / QK + P_WT_BLOCKS - 1) / P_WT_BLOCKS));
     const uint8_t* data = static_cast<const uint8_t*>(m.data);
     if (m.kind == 1) {
         if (gate_up) tile_prefill_weights_kernel<false, true><<<grid, 256, 0, stream>>>(data, m.scales, cols, rpe, rts, wt, wd, wc);
@@ -569,48 +752,45 @@ void tile_prefill_weights(const MoeDims& d, const MatrixDev& m, bool gate_up, in
     }
 }
 
-// One of the two grouped products on the tensor cores. `src` describes where the
-// activations come from: 8-bit rows through row_of_slot (gate_up), or f32 rows
-// in slot order to quantize (down).
+// One of the two grouped products, gate_up first: it reads the 8-bit rows through
+// slot_token and leaves the SwiGLU rows in s.ht / hst / hsumt, as tiles; down reads those.
 int launch_prefill(const MoeDims& d, bool gate_up, bool q4, const PrefillWeights& w, const PrefillScratch& s,
                    const Workspace& ws, int slots, float* out, const uint32_t* out_rows, cudaStream_t stream,
                    float* const* peer_out, int peer_ranks, uint32_t peer_rows) {
     const int cols = gate_up ? d.hidden : d.inter;
     const int nb = cols / QK, nbp = (nb + 7) / 8 * 8;
-    const int max_tiles = prefill_max_token_tiles(slots, d.experts);
+    const bool narrow = w.gu_c || w.dn_c;  // one tile list serves both products
+    const int max_tiles = prefill_max_token_tiles(slots, d.experts, narrow);
     int launched = 0;
     if (gate_up) {
-        build_token_tiles_kernel<<<1, 256, 0, stream>>>(ws.counts, ws.offsets, d.experts, s.tile_expert, s.tile_p0,
-                                                        s.tile_n, s.tile_count);
-        launched++;
+        launch_overlapped(build_token_tiles_kernel, dim3(1), dim3(MAX_EXPERTS), size_t(0), stream,
+                          static_cast<const uint32_t*>(ws.counts), static_cast<const uint32_t*>(ws.offsets), d.experts,
+                          prefill_columns(narrow), s.tiles, s.tile_count);
+        launch_overlapped(q4 ? tile_activations_kernel<true> : tile_activations_kernel<false>,
+                          dim3(max_tiles, (nb + P_ACT_BLOCKS - 1) / P_ACT_BLOCKS), dim3(256), size_t(0), stream,
+                          static_cast<const int8_t*>(ws.xq), static_cast<const float*>(ws.xs),
+                          static_cast<const float*>(ws.xsum), static_cast<const uint32_t*>(ws.slot_token), cols, nbp,
+                          static_cast<const TokenTile*>(s.tiles), static_cast<const int*>(s.tile_count), s.xt, s.xst,
+                          s.xsumt);
+        launched += 2;
     }
-    if (q4)
-        tile_activations_kernel<true><<<max_tiles, 256, 0, stream>>>(
-            gate_up ? ws.xq : nullptr, gate_up ? ws.xs : nullptr, gate_up ? ws.xsum : nullptr,
-            gate_up ? nullptr : ws.hidden_f, gate_up ? ws.slot_token : nullptr, cols, nbp, s.tile_p0, s.tile_n,
-            s.tile_count, s.xt, s.xst, s.xsumt);
-    else
-        tile_activations_kernel<false><<<max_tiles, 256, 0, stream>>>(
-            gate_up ? ws.xq : nullptr, gate_up ? ws.xs : nullptr, nullptr, gate_up ? nullptr : ws.hidden_f,
-            gate_up ? ws.slot_token : nullptr, cols, nbp, s.tile_p0, s.tile_n, s.tile_count, s.xt, s.xst, s.xsumt);
-    launched++;
     PrefillArgs a{};
     a.wt = gate_up ? w.gu_t : w.dn_t;
     a.wd = gate_up ? w.gu_d : w.dn_d;
     a.wc = gate_up ? w.gu_c : w.dn_c;
-    a.xt = s.xt;
-    a.xst = s.xst;
-    a.xsumt = s.xsumt;
-    a.tile_expert = s.tile_expert;
-    a.tile_p0 = s.tile_p0;
-    a.tile_n = s.tile_n;
+    a.xt = gate_up ? s.xt : s.ht;
+    a.xst = gate_up ? s.xst : s.hst;
+    a.xsumt = gate_up ? s.xsumt : s.hsumt;
+    a.tiles = s.tiles;
     a.tile_count = s.tile_count;
     a.nb = nb;
     a.row_tiles = prefill_row_tiles(d, gate_up);
-    a.rows_per_expert = gate_up ? 2 * d.inter : d.hidden;
     a.out_cols = gate_up ? d.inter : d.hidden;
+    a.xt_out = s.ht, a.xst_out = s.hst, a.xsumt_out = s.hsumt;
     a.out = out;
     a.out_rows = out_rows;
+    a.one = 1.0f;
+    a.status = ws.status;
     PrefillPeer pp{};
     const bool to_peers = peer_out && !gate_up;
     if (to_peers) {
@@ -618,20 +798,19 @@ int launch_prefill(const MoeDims& d, bool gate_up, bool q4, const PrefillWeights
         pp.ranks = peer_ranks;
         pp.rows = peer_rows;
     }
-    a.status = ws.status;
-    const dim3 grid(a.row_tiles, max_tiles);
-    const size_t smem = prefill_smem(nb, q4);
-    if (q4) {
-        if (gate_up) expert_prefill_kernel<true, true><<<grid, P_THREADS, smem, stream>>>(a, NoPeer{});
-        else if (to_peers) expert_prefill_kernel<true, false, true><<<grid, P_THREADS, smem, stream>>>(a, pp);
-        else expert_prefill_kernel<true, false><<<grid, P_THREADS, smem, stream>>>(a, NoPeer{});
-    } else {
-        if (gate_up) expert_prefill_kernel<false, true><<<grid, P_THREADS, smem, stream>>>(a, NoPeer{});
-        else if (to_peers) expert_prefill_kernel<false, false, true><<<grid, P_THREADS, smem, stream>>>(a, pp);
-        else expert_prefill_kernel<false, false><<<grid, P_THREADS, smem, stream>>>(a, NoPeer{});
-    }
+    const int sms = ws.sms > 0 ? ws.sms : 148;
+    const dim3 grid(unsigned(std::min<long long>(sms, (long long)max_tiles * a.row_tiles))), block(P_THREADS);
+    const size_t smem = q4 ? Stage<true>::SMEM : Stage<false>::SMEM;
+    if (to_peers)
+        launch_overlapped(q4 ? expert_prefill_kernel<true, false, true> : expert_prefill_kernel<false, false, true>, grid, block,
+                          smem, stream, a, pp);
+    else if (gate_up)
+        launch_overlapped(q4 ? expert_prefill_kernel<true, true> : expert_prefill_kernel<false, true>, grid, block, smem,
+                          stream, a, NoPeer{});
+    else
+        launch_overlapped(q4 ? expert_prefill_kernel<true, false> : expert_prefill_kernel<false, false>, grid, block, smem,
+                          stream, a, NoPeer{});
     return launched + 1;
 }
 
 }  // namespace tc
-
