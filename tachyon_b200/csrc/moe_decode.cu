@@ -68,7 +68,7 @@ constexpr int D_TOK = 8 * D_GMAX;  // tokens per block this kernel takes; rows s
 constexpr int D_NORM_HELD = 8;     // elements of the norm's weight a thread holds (rows of up to 8 x 256 floats)
 constexpr int D_ROUTE_VEC = 10;    // 16-byte pieces of the router matrix a thread holds at a time
 constexpr int D_NSEG = 4;          // experts of a CTA's range whose slot lists are held at a time
-constexpr size_t D_SMEM_LIMIT = 227 * 1024 - 3072;  // dynamic part: the kernel also has up to 2.5 KB of static shared memory
+constexpr size_t D_SMEM_LIMIT = 227 * 1024 - 3584;  // dynamic part: the kernel also has up to 3.2 KB of static shared memory
 
 constexpr int DECODE_EP_FLAG_ROUTE = 16, DECODE_EP_FLAG_DOWN = 17;  // words of the window's flag area
 
@@ -219,7 +219,8 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
     __shared__ int s_run_len;                           // EP: slots per run (32, 16 or 8)
     __shared__ uint32_t s_cnt[EP ? MAX_EXPERTS : 1];    // EP: slots per local expert
     __shared__ int s_part[EP ? D_NSEG * D_MAX_WARPS : 1];  // EP: a segment's hits per warp's slice of the ids
-    __shared__ uint32_t s_rids[MAX_TOPK];               // the routed token's picks, on their way out
+    __shared__ uint32_t s_rids[MAX_TOPK];               // the routed token's picks ...
+    __shared__ float s_rval[MAX_TOPK];                  // ... and their scores
     __shared__ uint32_t s_cpos[MAX_TOPK];
     __shared__ float s_cgate[MAX_TOPK];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -461,12 +462,12 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
                              min(experts, e_lo + pass_rows), slog, logits_row, tid, nthreads);
                 __syncthreads();  // the staged rows are no longer read; slog is complete up to here
             }
-            if (warp == 0)
-                route_topk_gates(slog, experts, topk, EP ? s_rids : a.ids + size_t(bid) * topk,
-                                 a.gates + size_t(bid) * topk, lane);
+            // The picks by the first warps (a thread per expert), the row's quantization by the others.
+            route_rank_picks(slog, experts, topk, EP ? nullptr : a.ids + size_t(bid) * topk, s_rids, s_rval, tid);
+            const int rank_warps = (experts + 31) >> 5, qfirst = rank_warps < nwarps ? rank_warps : 0;
             if (!EP) {
                 route_quantize_row(xrow, hidden, a.xq + size_t(bid) * hidden, a.xs + size_t(bid) * P0.nbp,
-                                   a.xsum + size_t(bid) * P0.nbp, warp, lane, 1, nwarps - 1);
+                                   a.xsum + size_t(bid) * P0.nbp, warp, lane, qfirst, nwarps - qfirst);
                 __syncthreads();
                 if (tid == 0) grid_arrive(a.sync + 0);
             } else {
@@ -475,7 +476,7 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
                 int8_t* sq = reinterpret_cast<int8_t*>(wsm);
                 float* ss = reinterpret_cast<float*>(wsm + hidden);
                 float* ssum = ss + P0.nbp;
-                route_quantize_row(xrow, hidden, sq, ss, ssum, warp, lane, 1, nwarps - 1);
+                route_quantize_row(xrow, hidden, sq, ss, ssum, warp, lane, qfirst, nwarps - qfirst);
                 __syncthreads();
                 const size_t g = size_t(own + bid);  // this token among all ranks' tokens
                 const int vq = hidden / 16, vs = P0.nbp / 4, per_rank = vq + 2 * vs + topk;
@@ -497,6 +498,19 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
                 __syncthreads();
                 if (tid < ranks && !a.ep.mute)
                     arrive_on_peer(reinterpret_cast<uint32_t*>(a.ep.base[tid] + a.ep.off_flags) + DECODE_EP_FLAG_ROUTE);
+            }
+            // The gates, and the order the combine adds the picks in (ascending expert): wanted by this
+            // CTA's combine only, so they are worked out behind the arrival.
+            if (warp == 1) {
+                const float gate = route_pick_gate(s_rval, topk, lane);
+                if (lane < topk) {
+                    a.gates[size_t(bid) * topk + lane] = gate;
+                    const uint32_t mine = s_rids[lane];
+                    int rank = 0;
+                    for (int j = 0; j < topk; j++) rank += s_rids[j] < mine ? 1 : 0;
+                    s_cpos[rank] = uint32_t(bid * topk + lane);
+                    s_cgate[rank] = gate;
+                }
             }
         }
         if (EP) {
@@ -890,7 +904,9 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
 
     // ---- weighted combine + residual add: CTA i < t takes token i (src/model.rs:513-519, 681),
     // once every CTA's part of the down phase is in global memory.
+    float4 y_ahead = make_float4(0.0f, 0.0f, 0.0f, 0.0f);  // this thread's first part of the residual row
     if (ok && bid < t) {
+        if (tid * 4 < hidden) y_ahead = *reinterpret_cast<const float4*>(a.y + size_t(bid) * hidden + tid * 4);
         if (tid == 0) {
             const bool came = EP ? peer_count_wait(flags + DECODE_EP_FLAG_DOWN, (epoch0 + 1u) * uint32_t(ranks * nctas),
                                                    a.spin_limit)
@@ -902,15 +918,6 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
         if (stamping) a.stamps[4] = wall_clock_ns();
     }
     if (ok && bid < t) {
-        if (tid < topk) {
-            const uint32_t* my_ids = s_ids + (own + bid) * topk;
-            const uint32_t mine = my_ids[tid];
-            int rank = 0;
-            for (int j = 0; j < topk; j++) rank += my_ids[j] < mine ? 1 : 0;
-            s_cpos[rank] = uint32_t(bid * topk + tid);
-            s_cgate[rank] = __ldcg(a.gates + size_t(bid) * topk + tid);
-        }
-        __syncthreads();
         float* yr = a.y + size_t(bid) * hidden;
 #pragma unroll 1
         for (int c = tid * 4; c < hidden; c += nthreads * 4) {
@@ -924,7 +931,7 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
                 proj.z = proj.z + gt * v.z;
                 proj.w = proj.w + gt * v.w;
             }
-            float4 r = *reinterpret_cast<float4*>(yr + c);
+            float4 r = c == tid * 4 ? y_ahead : *reinterpret_cast<float4*>(yr + c);
             r.x = r.x + proj.x;
             r.y = r.y + proj.y;
             r.z = r.z + proj.z;
@@ -955,22 +962,6 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
     }
 }
 
-// Rows of the router matrix the router phase stages at a time: the whole matrix, or the
-// fewest equal parts, within what the token area offers anyway (a dense walk, where the
-// ring's depth matters) or within 72 KB (a sparse walk, where the ring is mostly idle).
-template <int KIND>
-int decode_route_rows(const MoeDims& d, int t, int xcap, int nthreads) {
-    const int held = D_ROUTE_VEC * nthreads / (d.hidden / 8);  // rows the CTA's registers hold at a time
-    const int tokens = DLayout<KIND>::token_bytes(xcap, d.hidden, d.inter);
-    const int base = DLayout<KIND>::route_base(d.hidden, d.experts) + 64, wstride = 2 * d.hidden + 32;
-    const int budget = dense_walk(d, t) ? tokens + 2048 : max(tokens, 72 * 1024);
-    for (int parts = 1; parts <= 8; parts++) {
-        const int rows = (d.experts + parts - 1) / parts;
-        if (rows <= held && base + rows * wstride <= budget) return rows;
-    }
-    return max(0, min(held, (tokens - base) / wstride));
-}
-
 // Warps per CTA, ring depth and staged rows: as many warps as possible while each still
 // gets a ring of at least two stages; then the deepest ring that fits.
 template <int KIND>
@@ -986,8 +977,15 @@ bool decode_config(const MoeDims& d, int t, int ids_slots, int& nwarps, int& sta
     };
     int best_w = 0, best_s = 0, best_r = 0;
     for (int w = D_MAX_WARPS; w >= 8; w -= 2) {
-        const int rr = decode_route_rows<KIND>(d, t, xcap, w * 32);
-        const int s = deepest(w, rr);
+        // Rows of the router matrix staged at a time: the whole matrix or the fewest equal parts that
+        // leave the ring two stages (each part is a pass of the logits: 1.6 us at 16 rows of 1024).
+        const int held = D_ROUTE_VEC * w * 32 / (d.hidden / 8);  // rows the CTA's registers hold at a time
+        int rr = 0, s = 0;
+        for (int parts = 1; parts <= 8 && s < 2; parts++) {
+            rr = (d.experts + parts - 1) / parts;
+            if (rr <= held) s = deepest(w, rr);
+        }
+        if (s < 2) rr = 0, s = deepest(w, 0);  // (the logits read global memory)
         // (More warps matter more than a third stage: an expert's units are cut into parts of 16
         // where they can be, one per warp. Measured at granite-1b-a400m, batch 32: 0.83 ms per
         // step with 16 warps and two stages against 0.865 with 14 and three.)

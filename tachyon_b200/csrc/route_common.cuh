@@ -270,6 +270,47 @@ __device__ __forceinline__ void route_topk_gates(const float* slog, int experts,
     }
 }
 
+// Top-k of one token by a whole CTA, a thread per expert: each counts the experts that come before its
+// own in the order (larger key first, lower index first among equals) by reading all of them, four
+// at a time, from shared memory; the thread of rank j < topk has the j-th pick, its id into id_out[j] and
+// s_id[j], its score into s_val[j]. The picks of route_topk_gates without a chain of dependent rounds.
+// slog must be 16-byte aligned; the caller puts a CTA barrier before and after.
+__device__ __forceinline__ void route_rank_picks(const float* slog, int experts, int topk, uint32_t* id_out,
+                                                 uint32_t* s_id, float* s_val, int tid) {
+    if (tid >= experts) return;
+    const float mine = slog[tid];
+    const int key = total_key(mine);
+    int rank = 0;
+    auto before = [&](float v, int j) {
+        const int k = total_key(v);
+        rank += (k > key || (k == key && j < tid)) ? 1 : 0;
+    };
+    int j = 0;
+#pragma unroll 4
+    for (; j + 4 <= experts; j += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(slog + j);
+        before(v.x, j), before(v.y, j + 1), before(v.z, j + 2), before(v.w, j + 3);
+    }
+    for (; j < experts; j++) before(slog[j], j);
+    if (rank < topk) {
+        if (id_out) id_out[rank] = uint32_t(tid);
+        s_id[rank] = uint32_t(tid);
+        s_val[rank] = mine;
+    }
+}
+
+// The gates of those picks by ONE warp (lane j the j-th): softmax over the scores with the top score
+// as the maximum, the sum taken in score order.
+__device__ __forceinline__ float route_pick_gate(const float* s_val, int topk, int lane) {
+    const float my_val = lane < topk ? s_val[lane] : 0.0f;
+    const float mx = __shfl_sync(0xffffffffu, my_val, 0);
+    float ej = 0.0f;
+    if (lane < topk) ej = exp_nonpositive_f64(my_val - mx);
+    float sum = 0.0f;
+    for (int j = 0; j < topk; j++) sum = sum + __shfl_sync(0xffffffffu, ej, j);
+    return __fdiv_rn(ej, sum);
+}
+
 // 8-bit quantization of one token's row, a warp per 32-block: warps first_warp ..
 // first_warp + nq - 1 of the CTA take the blocks (and the zero padding up to whole
 // super-blocks of the scale rows) in turn.
