@@ -19,7 +19,7 @@
 // memory:
 //  - Weights are re-tiled once, when a layer is created, into records of one
 //    unit (16 rows) x one 256-column chunk: 16 rows of [weights | that row's
-//    block scales], row stride 272 bytes (8-bit) or 144 bytes (4-bit). One
+//    block scales], row stride 272 bytes (8-bit) or 144 bytes (4-bit; scales and offsets as f32). One
 //    record is one bulk async copy and lands in shared memory already padded
 //    so that ldmatrix reads hit 32 distinct banks.
 //  - Persistent CTAs, one per SM; the units of experts that have tokens are
@@ -504,13 +504,18 @@ __global__ void tile_weights_kernel(const uint8_t* __restrict__ wdata, const voi
                 reinterpret_cast<uint16_t*>(rec + r * R::ROW_STRIDE + F_KC)[b] = sp[b];
         } else {
             for (int i = threadIdx.x; i < cols_c / 2; i += blockDim.x)
-                rec[r * R::ROW_STRIDE + i] = wdata[(size_t(row) * cols + col0) / 2 + i];
+                rec[r * R::ROW_STRIDE + i] = wdata[(size_t(row) * cols + col0) / 2 + i] ^ 0x88u;  // q -> q - 8
             const int words_per_row = (nb + SUPER - 1) / SUPER * SUPER_WORDS;
             const uint32_t* wp = reinterpret_cast<const uint32_t*>(wscales) + size_t(row) * words_per_row +
                                  c * SUPER_WORDS;
-            if (threadIdx.x < 4)
-                reinterpret_cast<uint32_t*>(rec + r * R::ROW_STRIDE + F_KC / 2)[threadIdx.x] = wp[threadIdx.x];
-            if (threadIdx.x == 4) reinterpret_cast<uint32_t*>(rec + F_ROWS * R::ROW_STRIDE)[r] = wp[4];
+            for (int j = threadIdx.x; j < nblk; j += blockDim.x) {
+                const float d = f16_bits_to_f32(uint16_t(wp[0])) * float((wp[1 + j / 4] >> (8 * (j % 4))) & 0xFFu);
+                const float o = f16_bits_to_f32(uint16_t(wp[0] >> 16)) * float(int(int8_t(uint8_t(wp[3 + j / 4] >> (8 * (j % 4))))));
+                float* tail = reinterpret_cast<float*>(rec + R::TAIL + r * R::TAIL_STRIDE);
+                float* scale = j < 4 ? reinterpret_cast<float*>(rec + r * R::ROW_STRIDE + F_KC / 2) + j : tail + j - 4;
+                *scale = d * 0.0625f;
+                tail[4 + j] = o;
+            }
         }
     }
 }

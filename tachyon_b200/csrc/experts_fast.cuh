@@ -19,13 +19,19 @@ constexpr int F_KC = 256;         // columns per record
 constexpr int F_NBC = F_KC / QK;  // blocks per record
 constexpr int F_ROWS = 16;        // weight rows per unit (one m16 tile)
 
+// 8-bit: 16 rows x (256 weights + 8 f16 scales).
+// 4-bit: 16 rows x (128 nibble bytes + the f32 scales of blocks 0-3), then per row the scales of blocks
+// 4-7 and the f32 offsets of blocks 0-7. The nibbles are q - 8 in two's complement and the scales
+// are divided by 16: a nibble in the upper half of a byte is 16 (q - 8) as it stands, so two bytes cost
+// one mask and one shift, and the sums come out 16 times too large. (With q and the packed 16- and
+// 8-bit scales as stored, unpacking a record was a third of the expert phases: a block of the 3b
+// shape at 4 / 16 / 32 tokens 38.1 / 53.7 / 61.8 -> 33.3 / 45.4 / 53.1 us, for 30 % more bytes of
+// a stream that HBM is far from bounding.)
 template <int KIND>
 struct Rec {
-    // 8-bit: 16 rows x (256 weights + 8 f16 scales).
-    // 4-bit: 16 rows x (128 nibble bytes + words 0..3 of the super-block), then
-    //        word 4 of each row.
     static constexpr int ROW_STRIDE = KIND == 1 ? F_KC + 16 : F_KC / 2 + 16;
-    static constexpr int BYTES = KIND == 1 ? F_ROWS * ROW_STRIDE : F_ROWS * ROW_STRIDE + F_ROWS * 4;
+    static constexpr int TAIL = F_ROWS * ROW_STRIDE, TAIL_STRIDE = 48;  // (4-bit)
+    static constexpr int BYTES = KIND == 1 ? TAIL : TAIL + F_ROWS * TAIL_STRIDE;
 };
 
 // Shared-memory reads below are plain (non-volatile) asm so the compiler may
@@ -54,6 +60,11 @@ __device__ __forceinline__ void mma_s8(int (&d)[4], int a0, int a1, int a2, int 
 __device__ __forceinline__ uint32_t lds32(uint32_t addr, uint32_t token) {
     uint32_t v;
     asm("ld.shared.u32 %0, [%1]; // %2" : "=r"(v) : "r"(addr), "r"(token));
+    return v;
+}
+__device__ __forceinline__ uint2 lds64(uint32_t addr, uint32_t token) {
+    uint2 v;
+    asm("ld.shared.v2.u32 {%0,%1}, [%2]; // %3" : "=r"(v.x), "=r"(v.y) : "r"(addr), "r"(token));
     return v;
 }
 __device__ __forceinline__ uint4 lds128(uint32_t addr, uint32_t token) {
@@ -85,33 +96,6 @@ __device__ __forceinline__ void fast_chunk(uint32_t rec, uint32_t xq_s, uint32_t
     using R = Rec<KIND>;
     const int g = lane >> 2, t = lane & 3;
     const int mat = lane >> 3, mr = lane & 7;
-    // This thread's two rows' scales for the record's eight blocks.
-    float wd[2][F_NBC], wc[2][F_NBC];
-    if (KIND == 1) {
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const uint4 s = lds128(rec + (g + 8 * h) * R::ROW_STRIDE + F_KC, wtok);
-            const uint32_t hw[4] = {s.x, s.y, s.z, s.w};
-#pragma unroll
-            for (int b = 0; b < F_NBC; b += 2) {
-                const uint32_t word = hw[b >> 1];
-                wd[h][b] = f16_scale_to_f32(word & 0xFFFFu);
-                wd[h][b + 1] = f16_scale_to_f32(word >> 16);
-            }
-        }
-    } else {
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const uint4 s = lds128(rec + (g + 8 * h) * R::ROW_STRIDE + F_KC / 2, wtok);
-            const uint32_t o23 = lds32(rec + F_ROWS * R::ROW_STRIDE + (g + 8 * h) * 4, wtok);
-            const float step_d = f16_bits_to_f32(uint16_t(s.x)), step_c = f16_bits_to_f32(uint16_t(s.x >> 16));
-#pragma unroll
-            for (int b = 0; b < F_NBC; b++) {
-                wd[h][b] = step_d * float(((b < 4 ? s.y : s.z) >> (8 * (b & 3))) & 0xFFu);
-                wc[h][b] = step_c * float(int(int8_t(uint8_t((b < 4 ? s.w : o23) >> (8 * (b & 3))))));
-            }
-        }
-    }
     uint32_t a_addr;
     if (KIND == 1)
         a_addr = rec + (mr + (mat & 1) * 8) * R::ROW_STRIDE + (mat >> 1) * 16;
@@ -122,9 +106,29 @@ __device__ __forceinline__ void fast_chunk(uint32_t rec, uint32_t xq_s, uint32_t
     // Four blocks at a time, in three phases so that the loads, the matrix
     // instructions and the float chains of different blocks overlap: all
     // operand loads, then all matrix instructions, then the scaling.
-#pragma unroll
+    // (Rolled: the code of a record is half as long. In a kernel that runs once every few tens of
+    // microseconds the instructions come from far away, and the four instances of this loop are most of them.)
+#pragma unroll 1
     for (int h4 = 0; h4 < F_NBC; h4 += 4) {
         if (h4 < nblk) {
+            // This thread's two rows' scales for the four blocks.
+            float wd[2][4], wc[2][4];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                if (KIND == 1) {
+                    const uint2 s = lds64(rec + (g + 8 * h) * R::ROW_STRIDE + F_KC + h4 * 2, wtok);
+                    wd[h][0] = f16_scale_to_f32(s.x & 0xFFFFu), wd[h][1] = f16_scale_to_f32(s.x >> 16);
+                    wd[h][2] = f16_scale_to_f32(s.y & 0xFFFFu), wd[h][3] = f16_scale_to_f32(s.y >> 16);
+                } else {
+                    const uint32_t tail = rec + R::TAIL + (g + 8 * h) * R::TAIL_STRIDE;
+                    const uint4 sc = lds128(h4 ? tail : rec + (g + 8 * h) * R::ROW_STRIDE + F_KC / 2, wtok);
+                    const uint4 of = lds128(tail + 16 + h4 * 4, wtok);
+                    wd[h][0] = __uint_as_float(sc.x), wd[h][1] = __uint_as_float(sc.y);
+                    wd[h][2] = __uint_as_float(sc.z), wd[h][3] = __uint_as_float(sc.w);
+                    wc[h][0] = __uint_as_float(of.x), wc[h][1] = __uint_as_float(of.y);
+                    wc[h][2] = __uint_as_float(of.z), wc[h][3] = __uint_as_float(of.w);
+                }
+            }
             int A[4][4];
 #pragma unroll
             for (int k = 0; k < 4; k++) {
@@ -135,10 +139,10 @@ __device__ __forceinline__ void fast_chunk(uint32_t rec, uint32_t xq_s, uint32_t
                     // high nibbles elements 16+4t..16+4t+3.
                     int w0, w1;
                     ldmatrix_x2(a_addr + (h4 + k) * 16, wtok, w0, w1);
-                    A[k][0] = nibbles_minus8(uint32_t(w0) & 0x0F0F0F0Fu);
-                    A[k][2] = nibbles_minus8((uint32_t(w0) >> 4) & 0x0F0F0F0Fu);
-                    A[k][1] = nibbles_minus8(uint32_t(w1) & 0x0F0F0F0Fu);
-                    A[k][3] = nibbles_minus8((uint32_t(w1) >> 4) & 0x0F0F0F0Fu);
+                    A[k][0] = (w0 << 4) & 0xF0F0F0F0;
+                    A[k][2] = w0 & 0xF0F0F0F0;
+                    A[k][1] = (w1 << 4) & 0xF0F0F0F0;
+                    A[k][3] = w1 & 0xF0F0F0F0;
                 }
             }
 #pragma unroll
@@ -175,18 +179,17 @@ __device__ __forceinline__ void fast_chunk(uint32_t rec, uint32_t xq_s, uint32_t
 #pragma unroll
                         for (int k = 0; k < 4; k++) {
                             if (h4 + k < nblk) {
-                                const int b = h4 + k;
                                 const float2 magic = make_float2(MAGIC_F, MAGIC_F);
 #pragma unroll
                                 for (int h = 0; h < 2; h++) {  // rows g and g+8; tokens 2t, 2t+1 side by side
                                     const float2 sum = sub2(make_float2(__int_as_float(D[p][k][2 * h]),
                                                                         __int_as_float(D[p][k][2 * h + 1])), magic);
-                                    const float2 d = mul2(make_float2(wd[h][b], wd[h][b]), XS[p][k]);
+                                    const float2 d = mul2(make_float2(wd[h][k], wd[h][k]), XS[p][k]);
                                     const float2 r = fma2(sum, d, make_float2(acc[nt][2 * h], acc[nt][2 * h + 1]));
                                     acc[nt][2 * h] = r.x;
                                     acc[nt][2 * h + 1] = r.y;
                                     if (KIND == 2) {
-                                        const float2 o = fma2(make_float2(wc[h][b], wc[h][b]), SU[p][k],
+                                        const float2 o = fma2(make_float2(wc[h][k], wc[h][k]), SU[p][k],
                                                               make_float2(off[nt][2 * h], off[nt][2 * h + 1]));
                                         off[nt][2 * h] = o.x;
                                         off[nt][2 * h + 1] = o.y;
