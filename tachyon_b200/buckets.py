@@ -27,7 +27,9 @@ class GraphBuckets:
     ``layers`` are ``MoeLayer``-like objects with ``block(norm_weight, eps, y, t)`` and
     ``max_tokens``; ``norm_weights`` their RMSNorm weights on the device. ``ctx`` needs
     ``empty``, ``upload``, ``download``, ``memset``, ``copy_bytes``, ``capture_begin``,
-    ``capture_end`` and ``sync`` (``tachyon_b200.cuda.Context`` has them).
+    ``capture_end`` and ``sync`` (``tachyon_b200.cuda.Context`` has them). With ``host_empty``
+    (page-locked memory) a step is one graph launch and one wait: the rows' copies in and out are
+    nodes of the graph. Without it they are calls of their own.
     """
 
     def __init__(self, ctx, layers, norm_weights, eps: float, hidden: int, buckets=DEFAULT_BUCKETS):
@@ -40,8 +42,11 @@ class GraphBuckets:
         self.ctx, self.layers, self.norm_weights = ctx, list(layers), list(norm_weights)
         self.eps, self.hidden = float(eps), int(hidden)
         rows = self.buckets[-1]
-        self.x_in = ctx.empty((rows, hidden), np.float32)  # the step's rows, then zeros up to the bucket
+        self.pinned = hasattr(ctx, "host_empty")
+        make = ctx.host_empty if self.pinned else ctx.empty
+        self.x_in = make((rows, hidden), np.float32)       # the step's rows, then zeros up to the bucket
         self.x = ctx.empty((rows, hidden), np.float32)     # the residual stream the graph works on
+        self.x_out = make((rows, hidden), np.float32) if self.pinned else self.x
         self.graphs = {}
         self.launches = {b: 0 for b in self.buckets}
 
@@ -58,6 +63,8 @@ class GraphBuckets:
         self.ctx.copy_bytes(self.x.ptr, self.x_in.ptr, b * self.hidden * 4)
         for layer, w in zip(self.layers, self.norm_weights):
             layer.block(w, self.eps, self.x, t=b)  # x += moe(rmsnorm(x)): src/model.rs:662-681
+        if self.pinned:
+            self.ctx.copy_bytes(self.x_out.ptr, self.x.ptr, b * self.hidden * 4)
 
     def graph(self, b: int):
         """The bucket's graph, captured on first use (after one eager pass of the same work)."""
@@ -77,6 +84,13 @@ class GraphBuckets:
             raise ValueError(f"expected [t, {self.hidden}] rows")
         b = self.bucket_for(t)
         g = self.graph(b)
+        if self.pinned:
+            self.x_in.array[:t] = x_host
+            self.x_in.array[t:b] = 0.0
+            g.launch()
+            self.ctx.sync()
+            self.launches[b] += 1
+            return self.x_out.array[:t].copy()
         row = self.hidden * 4
         self.ctx.upload(self.x_in.ptr, x_host)
         if b > t:
@@ -92,5 +106,5 @@ class GraphBuckets:
         for g in self.graphs.values():
             g.free()
         self.graphs.clear()
-        for d in (self.x_in, self.x):
+        for d in {id(d): d for d in (self.x_in, self.x, self.x_out)}.values():
             d.free()

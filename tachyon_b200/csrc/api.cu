@@ -34,9 +34,12 @@ struct tc_ctx {
     tc::PrefillScratch pre;   // token tiles of the tcgen05 path
     std::vector<void*> pre_allocs;
     int prefill_min_avg = 32; // tokens per expert (on average) from which the tcgen05 kernels take over
-    float* host_x = nullptr;  // device staging for the host-buffer entry point
+    float* host_x = nullptr;  // device staging for the host-buffer entry point (large batches)
     float* host_y = nullptr;
     size_t host_elems = 0;
+    float* pinned_xy = nullptr;  // the same for small batches: page-locked memory that the kernels read and write in place
+    size_t pinned_elems = 0;
+    int* status = nullptr;       // the kernels' status word, in page-locked memory: read here without a copy
     bool decode_block = true;      // decode-size blocks as one kernel (moe_decode.cu)
     int decode_block_tokens = 128; // ... up to this many tokens (above 32: through the window below)
     // Batches of 33 tokens and more take the one-kernel path in its expert-parallel form with
@@ -251,13 +254,13 @@ bool ws_reserve(tc_ctx* ctx, const tc::MoeDims& d, int max_tokens) {
               ws_alloc(ctx, w.hidden_f, slots * n.inter) && ws_alloc(ctx, w.hq, slots * n.inter) &&
               ws_alloc(ctx, w.hs, slots * pad8(n.inter / 32)) &&
               ws_alloc(ctx, w.hsum, slots * pad8(n.inter / 32)) &&
-              ws_alloc(ctx, w.out, slots * n.hidden) && ws_alloc(ctx, w.status, size_t(1)) &&
+              ws_alloc(ctx, w.out, slots * n.hidden) &&
               ws_alloc(ctx, w.ticket, size_t(1)) && ws_alloc(ctx, w.grid_sync, size_t(tc::GRID_SYNC_WORDS));
     if (!ok) {
         ws_release(ctx);
         return false;
     }
-    cudaMemset(w.status, 0, sizeof(int));
+    w.status = ctx->status;
     cudaMemset(w.ticket, 0, sizeof(int));
     cudaMemset(w.grid_sync, 0, tc::GRID_SYNC_WORDS * sizeof(uint32_t));
     w.max_tokens = T;
@@ -304,10 +307,12 @@ tc_ctx* tc_create(int device_ordinal, char* err, size_t errlen) {
     tc::init_kernels_decode();
     if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreate(&ctx->ev_start) != cudaSuccess ||
-        cudaEventCreate(&ctx->ev_stop) != cudaSuccess) {
+        cudaEventCreate(&ctx->ev_stop) != cudaSuccess ||
+        cudaHostAlloc(reinterpret_cast<void**>(&ctx->status), sizeof(int), cudaHostAllocMapped) != cudaSuccess) {
         delete ctx;
-        return bail("could not create the stream or events");
+        return bail("could not create the stream, its events or the status word");
     }
+    *ctx->status = 0;
     return ctx;
 }
 
@@ -319,6 +324,8 @@ void tc_destroy(tc_ctx* ctx) {
     for (void* q : ctx->pre_allocs) cudaFree(q);
     if (ctx->host_x) cudaFree(ctx->host_x);
     if (ctx->host_y) cudaFree(ctx->host_y);
+    if (ctx->pinned_xy) cudaFreeHost(ctx->pinned_xy);
+    if (ctx->status) cudaFreeHost(ctx->status);
     if (ctx->phase_stamps) cudaFree(ctx->phase_stamps);
     if (ctx->self_window) cudaFree(ctx->self_window);
     if (ctx->self_epoch) cudaFree(ctx->self_epoch);
@@ -353,17 +360,18 @@ const char* status_text(int status) {
 
 int tc_sync(tc_ctx* ctx) {
     if (!cuda_ok(ctx, cudaStreamSynchronize(ctx->stream), "cudaStreamSynchronize")) return -1;
-    int* words[2] = {ctx->ws.status, ctx->static_status};
     int worst = 0;
-    for (int* w : words) {
-        if (!w) continue;
+    if (ctx->static_status) {
         int status = 0;
-        if (!cuda_ok(ctx, cudaMemcpy(&status, w, sizeof status, cudaMemcpyDeviceToHost), "status readback"))
+        if (!cuda_ok(ctx, cudaMemcpy(&status, ctx->static_status, sizeof status, cudaMemcpyDeviceToHost), "status readback"))
             return -1;
-        if (status != 0) {
-            cudaMemset(w, 0, sizeof(int));
-            worst = status;
-        }
+        if (status != 0) cudaMemset(ctx->static_status, 0, sizeof(int));
+        worst = status;
+    }
+    volatile int* own = ctx->status;  // (kernels wrote it, if they did, before the stream drained)
+    if (*own != 0) {
+        if (!worst) worst = *own;
+        *own = 0;
     }
     if (worst) {
         // A kernel that gave up may have left its arrival counters part-way: start clean.
@@ -409,7 +417,7 @@ int tc_memset(tc_ctx* ctx, void* dst, int value, size_t bytes) {
 }
 
 int tc_copy(tc_ctx* ctx, void* dst, const void* src, size_t bytes) {
-    return cuda_ok(ctx, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, ctx->stream), "copy") ? 0 : -1;
+    return cuda_ok(ctx, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, ctx->stream), "copy") ? 0 : -1;
 }
 
 void* tc_host_alloc(tc_ctx* ctx, size_t bytes) {
@@ -949,6 +957,27 @@ int tc_moe_forward_host(tc_moe_layer* layer, const float* x_host, int t, float* 
     tc_ctx* ctx = layer->ctx;
     if (t <= 0) return fail(ctx, "empty batch");
     size_t elems = size_t(t) * layer->dims.hidden;
+    if (t <= SELF_WINDOW_TOKENS) {
+        // Small batches: the kernels read x and update y in page-locked memory. Every path reads a row of
+        // x once (router) and reads and writes a row of y once (combine), so going over PCIe in
+        // place costs a trip each, where copies cost a trip, an engine's start and a gap in the stream
+        // each (4 tokens of the 1b shape: 69 us with three copies and a status read).
+        if (2 * elems > ctx->pinned_elems) {
+            cudaStreamSynchronize(ctx->stream);
+            if (ctx->pinned_xy) cudaFreeHost(ctx->pinned_xy);
+            ctx->pinned_xy = nullptr, ctx->pinned_elems = 0;
+            if (!cuda_ok(ctx, cudaHostAlloc(reinterpret_cast<void**>(&ctx->pinned_xy), 2 * elems * 4, cudaHostAllocMapped),
+                         "cudaHostAlloc(staging)"))
+                return -1;
+            ctx->pinned_elems = 2 * elems;
+        }
+        float *x = ctx->pinned_xy, *y = x + elems;
+        memcpy(x, x_host, elems * 4);
+        memcpy(y, y_host, elems * 4);
+        if (tc_moe_forward(layer, x, t, y) != 0 || tc_sync(ctx) != 0) return -1;
+        memcpy(y_host, y, elems * 4);
+        return 0;
+    }
     if (elems > ctx->host_elems) {
         cudaStreamSynchronize(ctx->stream);
         if (ctx->host_x) cudaFree(ctx->host_x);

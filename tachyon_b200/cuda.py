@@ -212,7 +212,7 @@ class Context:
         self._check(self.lib.tc_copy(self.handle, dst.ptr, src.ptr, src.nbytes), "tc_copy")
 
     def copy_bytes(self, dst: int, src: int, nbytes: int):
-        """Device to device on the context's stream (can be captured)."""
+        """Device to device, or to or from page-locked memory, on the context's stream (can be captured)."""
         self._check(self.lib.tc_copy(self.handle, dst, src, nbytes), "tc_copy")
 
     def pinned(self, shape, dtype=np.float32) -> np.ndarray:
@@ -224,6 +224,9 @@ class Context:
             raise TachyonCudaError(f"tc_host_alloc: {self.last_error()}")
         buf = (C.c_byte * (n * dtype.itemsize)).from_address(p)
         return np.frombuffer(buf, dtype=dtype).reshape(shape)
+
+    def host_empty(self, shape, dtype=np.float32) -> "HostArray":
+        return HostArray(self, shape, dtype)
 
     PROFILE_STAGES = ("route", "dispatch", "gate_up", "quant_hidden", "down", "combine", "rmsnorm", "decode_block")
 
@@ -325,6 +328,30 @@ class DeviceArray:
         if self.ptr and self.ctx.handle:
             self.ctx.free(self.ptr)
         self.ptr = 0
+
+    def __del__(self):
+        try:
+            self.free()
+        except Exception:
+            pass
+
+
+class HostArray:
+    """A typed buffer in page-locked host memory (``tc_host_alloc``), freed with its owner: ``array``
+    is it as numpy sees it, ``ptr`` what copies on the context's stream take."""
+
+    def __init__(self, ctx: Context, shape, dtype):
+        self.ctx, dtype = ctx, np.dtype(dtype)
+        n = int(np.prod(shape)) * dtype.itemsize
+        self.ptr = ctx.lib.tc_host_alloc(ctx.handle, max(n, 1))
+        if not self.ptr:
+            raise TachyonCudaError(f"tc_host_alloc({n}): {ctx.last_error()}")
+        self.array = np.frombuffer((C.c_byte * n).from_address(self.ptr), dtype=dtype).reshape(shape)
+
+    def free(self):
+        if self.ptr and self.ctx.handle:
+            self.ctx.lib.tc_host_free(self.ctx.handle, self.ptr)
+        self.ptr, self.array = 0, None
 
     def __del__(self):
         try:
