@@ -92,6 +92,7 @@ struct DecodeArgs {
     const uint8_t* dn_tiled;
     float* hidden_f;          // [t * k, inter] SwiGLU rows by slot
     float* out;               // [t * k, hidden] expert outputs by slot
+    int unit_warps;           // warps with a ring: as many as a CTA can have units, all of them if it can have more
     int stages, xcap;         // ring depth per warp; staged rows at a time (a multiple of 8, at most D_TOK)
     int route_rows;           // rows of the router matrix staged at a time in the router phase
     int l2_all;               // ask all of this GPU's expert records into L2 before the router phase
@@ -115,9 +116,9 @@ struct DLayout {
         return xcap * (cols + 16) + nbp * D_TOK * 4 * (KIND == 2 ? 2 : 1);
     }
     __host__ __device__ static int route_base(int hidden, int experts) { return ((hidden + experts) * 4 + 127) / 128 * 128; }
-    __host__ __device__ DLayout(int nwarps, int stages, int xcap, int route_rows, int hidden, int inter, int experts,
+    __host__ __device__ DLayout(int unit_warps, int stages, int xcap, int route_rows, int hidden, int inter, int experts,
                                 int topk, int ids_slots) {
-        int o = nwarps * stages * Rec<KIND>::BYTES;
+        int o = unit_warps * stages * Rec<KIND>::BYTES;
         ring = 0;
         o = (o + 127) / 128 * 128;
         x0 = o;
@@ -182,6 +183,13 @@ __device__ __forceinline__ void grid_arrive(uint32_t* ctr) {
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(ctr) : "memory");
 }
 
+// a / b for a < 2^20, through the float unit: (a + 1/2) / b is at least 1 / (2 b) away from every integer,
+// and the approximate quotient's error is below that. (An integer division is some 25 instructions in a
+// dependent chain; a block's partition takes a dozen of them on its critical path.)
+__device__ __forceinline__ unsigned div_small(unsigned a, unsigned b) {
+    return unsigned(__fdividef(float(a) + 0.5f, float(b)));
+}
+
 // What one of the two expert phases needs to know about its matrix and this warp's share.
 struct Phase {
     const uint8_t* tiled;
@@ -226,6 +234,7 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nwarps = blockDim.x >> 5, nthreads = blockDim.x;
     const int bid = blockIdx.x, nctas = gridDim.x;
+    const int uwarps = a.unit_warps;  // warps that take units (the first ones)
     const int STAGES = a.stages;
     const int t = a.t, hidden = a.hidden, experts = a.experts, topk = a.topk, inter = a.inter;
     // Expert parallel: the expert phases see every rank's tokens (gathered in this rank's window).
@@ -240,8 +249,8 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
     const uint32_t* flags = EP ? reinterpret_cast<const uint32_t*>(window + a.ep.off_flags) : nullptr;
     uint32_t epoch0 = 0;  // EP: blocks completed before this one
     uint32_t routed0 = 0; // EP: router-phase arrivals of those blocks (ranks x tokens each; the batch size may change)
-    const DLayout<KIND> L(nwarps, STAGES, a.xcap, a.route_rows, hidden, inter, experts, topk, a.ids_slots);
-    uint8_t* ring = smem + L.ring + size_t(warp) * STAGES * R::BYTES;
+    const DLayout<KIND> L(uwarps, STAGES, a.xcap, a.route_rows, hidden, inter, experts, topk, a.ids_slots);
+    uint8_t* ring = smem + L.ring + size_t(min(warp, uwarps - 1)) * STAGES * R::BYTES;  // (a warp without units uses none)
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L.bars) + warp * D_MAX_STAGES;
     uint32_t* s_ids = reinterpret_cast<uint32_t*>(smem + L.ids);
     uint16_t* s_slot = reinterpret_cast<uint16_t*>(smem + L.lists);  // [D_NSEG][D_TOK] slots that named the segment's expert
@@ -278,16 +287,15 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
         // units on every SM.)
         bool inside = walk_experts > 0 && walk_experts <= unsigned(nctas);
         if (inside && !EP) {
-            const unsigned per_run = unsigned(nctas) / walk_experts;
-            const unsigned mine = (unsigned(P.upe) + per_run - 1) / per_run, even = (total + nctas - 1) / unsigned(nctas);
-            inside = (mine + nwarps - 1) / nwarps <= (even + nwarps - 1) / nwarps;
+            const unsigned per_run = div_small(nctas, walk_experts);
+            const unsigned mine = div_small(P.upe + per_run - 1, per_run), even = div_small(total + nctas - 1, nctas);
+            inside = div_small(mine + uwarps - 1, uwarps) <= div_small(even + uwarps - 1, uwarps);
         }
         if (inside) {
-            const unsigned per_run = unsigned(nctas) / walk_experts, run = unsigned(bid) / per_run,
-                           part = unsigned(bid) % per_run;
+            const unsigned per_run = div_small(nctas, walk_experts), run = div_small(bid, per_run), part = bid - run * per_run;
             if (run < walk_experts) {
-                P.lo = int(run * unsigned(P.upe) + part * unsigned(P.upe) / per_run);
-                P.hi = int(run * unsigned(P.upe) + (part + 1) * unsigned(P.upe) / per_run);
+                P.lo = int(run * unsigned(P.upe) + div_small(part * unsigned(P.upe), per_run));
+                P.hi = int(run * unsigned(P.upe) + div_small((part + 1) * unsigned(P.upe), per_run));
             } else {
                 P.lo = P.hi = 0;
             }
@@ -296,13 +304,16 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
             P.hi = int(unsigned(bid + 1) * total / unsigned(nctas));
         }
         P.first = P.lo + warp;
-        P.n = P.first < P.hi ? (P.hi - P.first + nwarps - 1) / nwarps : 0;
+        P.n = warp < uwarps && P.first < P.hi ? int(div_small(P.hi - P.first + uwarps - 1, uwarps)) : 0;
     };
     // Where a unit's records start. Walk space counts the units of all experts (dense) or of
     // the picked ones (then the expert comes from the list made after the router phase).
     auto unit_ptr = [&](const Phase& P, int wu) {
         size_t flat = size_t(wu);
-        if (!a.dense) flat = size_t(s_active[wu / P.upe] - (EP ? a.ep.first : 0)) * P.upe + wu % P.upe;
+        if (!a.dense) {
+            const int walk = int(div_small(wu, P.upe));
+            flat = size_t(s_active[walk] - (EP ? a.ep.first : 0)) * P.upe + (wu - walk * P.upe);
+        }
         return P.tiled + flat * P.nchunks * R::BYTES;
     };
     // Producer state: the next record's address, and what is left of its unit and phase.
@@ -330,9 +341,9 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
             if (--pchunks == 0) {
                 const Phase& P = pphase ? P1 : P0;
                 if (--punits > 0) {
-                    pwu += nwarps;
+                    pwu += uwarps;
                     pchunks = P.nchunks;
-                    pptr = a.dense ? pptr + size_t(nwarps - 1) * P.nchunks * R::BYTES : unit_ptr(P, pwu);
+                    pptr = a.dense ? pptr + size_t(uwarps - 1) * P.nchunks * R::BYTES : unit_ptr(P, pwu);
                 } else if (pphase == 0) {
                     start_phase(1);
                 }
@@ -380,16 +391,18 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
     // (dense walk): the ring fills before this grid waits for the kernel in front of it, and
     // through the router phase. Otherwise after the router phase, once the picked experts are known.
     bool streaming = false;
+    auto start_stream = [&](unsigned walk) {
+        share(P0, walk), share(P1, walk);
+        nrec = uint32_t(P0.n * P0.nchunks + P1.n * P1.nchunks);
+        start_phase(P0.n > 0 ? 0 : 1);
+        top_up();
+        streaming = true;
+    };
 #pragma unroll 1
     for (int pass = 0; pass < 2; pass++) {
         if (pass == 0 ? bool(a.dense) : !streaming) {
             if (pass == 1 && s_abort) break;
-            const unsigned walk = a.dense ? unsigned(experts) : unsigned(s_nactive);
-            share(P0, walk), share(P1, walk);
-            nrec = uint32_t(P0.n * P0.nchunks + P1.n * P1.nchunks);
-            start_phase(P0.n > 0 ? 0 : 1);
-            top_up();
-            streaming = true;
+            start_stream(a.dense ? unsigned(experts) : unsigned(s_nactive));
         }
         if (pass == 1) break;
         if (a.l2_all) {
@@ -526,8 +539,39 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
 
         // ---- the batch's expert ids; for small batches the experts that were picked
         if (!s_abort) {
+            // A sparse walk over few experts: every warp finds the picked experts by itself, from the ids as
+            // they arrive, and starts its stream without another barrier.
+            const bool by_warp = !EP && !a.dense && experts <= 64;
+            if (by_warp) {
+                constexpr int HELD = 4;
+                uint32_t m0 = 0, m1 = 0;
 #pragma unroll 1
-            for (int i = tid; i < slots; i += nthreads) s_ids[i] = __ldcg(ids_all + i);
+                for (int i0 = 0; i0 < slots; i0 += 32 * HELD) {
+                    uint32_t id[HELD];
+#pragma unroll
+                    for (int u = 0; u < HELD; u++) {
+                        const int i = i0 + 32 * u + lane;
+                        id[u] = i < slots ? __ldcg(ids_all + i) : 0xffffffffu;
+                    }
+#pragma unroll
+                    for (int u = 0; u < HELD; u++) {
+                        const int i = i0 + 32 * u + lane;
+                        if (warp == 0 && i < slots) s_ids[i] = id[u];
+                        if (id[u] < 32u) m0 |= 1u << id[u];
+                        else if (id[u] < 64u) m1 |= 1u << (id[u] - 32u);
+                    }
+                }
+                m0 = __reduce_or_sync(0xffffffffu, m0), m1 = __reduce_or_sync(0xffffffffu, m1);
+                // (All warps write the same list.)
+                const uint32_t below = (1u << lane) - 1u;
+                if ((m0 >> lane) & 1u) s_active[__popc(m0 & below)] = uint16_t(lane);
+                if ((m1 >> lane) & 1u) s_active[__popc(m0) + __popc(m1 & below)] = uint16_t(lane + 32);
+                __syncwarp();
+                start_stream(unsigned(__popc(m0) + __popc(m1)));
+            } else {
+#pragma unroll 1
+                for (int i = tid; i < slots; i += nthreads) s_ids[i] = __ldcg(ids_all + i);
+            }
             if (EP) {
                 // Runs: each local expert's slots in pieces of up to D_TOK; (run, unit) pairs are what the
                 // CTAs and warps share out, so an expert with many tokens spreads over many warps.
@@ -560,8 +604,9 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
 #pragma unroll
                         for (int o = 16; o > 0; o >>= 1) runs[k] += __shfl_xor_sync(0xffffffffu, runs[k], o);
                         const int len = D_TOK >> k, r = max(1, runs[k]);
-                        const int per_cta = r <= nctas ? (P0.upe + nctas / r - 1) / (nctas / r) : (r * P0.upe + nctas - 1) / nctas;
-                        const int cost = (per_cta + nwarps - 1) / nwarps * (3 + (min(len, most) + 7) / 8);
+                        const unsigned ctas = r <= nctas ? div_small(nctas, r) : 1u;
+                        const int per_cta = int(r <= nctas ? div_small(P0.upe + ctas - 1, ctas) : div_small(r * P0.upe + nctas - 1, nctas));
+                        const int cost = int(div_small(per_cta + uwarps - 1, uwarps)) * (3 + (min(len, most) + 7) / 8);
                         if (cost < best) best = cost, run_len = len;
                     }
                     // A lane per local expert, 32 at a time: the expert's runs after those before it.
@@ -589,7 +634,7 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
                         s_run_len = run_len;
                     }
                 }
-            } else if (!a.dense) {
+            } else if (!a.dense && !by_warp) {
 #pragma unroll 1
                 for (int e = tid; e < experts; e += nthreads) s_picked[e] = 0;
                 __syncthreads();
@@ -630,8 +675,8 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
         const int xsum_off = xs_off + P.nbp * D_TOK * 4;
         float* xsT = reinterpret_cast<float*>(smem + L.x0 + xs_off);
         float* xsumT = reinterpret_cast<float*>(smem + L.x0 + xsum_off);
-        const int seg_first = P.lo < P.hi ? P.lo / P.upe : 0;
-        const int seg_last = P.lo < P.hi ? (P.hi - 1) / P.upe : -1;
+        const int seg_first = P.lo < P.hi ? int(div_small(P.lo, P.upe)) : 0;
+        const int seg_last = P.lo < P.hi ? int(div_small(P.hi - 1, P.upe)) : -1;
 #pragma unroll 1
         for (int sb = seg_first; sb <= seg_last && ok; sb += D_NSEG) {
             const int nseg = min(D_NSEG, seg_last - sb + 1);
@@ -664,7 +709,7 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
                         before += __shfl_xor_sync(0xffffffffu, before, o);
                         total += __shfl_xor_sync(0xffffffffu, total, o);
                     }
-                    int count = before, token = (lo + lane) / topk, pick = (lo + lane) - token * topk;
+                    int count = before, token = int(div_small(lo + lane, topk)), pick = (lo + lane) - token * topk;
 #pragma unroll 1
                     for (int base = lo; base < hi; base += 32) {
                         const bool hit = base + lane < hi && s_ids[base + lane] == e;
@@ -769,41 +814,25 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
                 } else {
                     // The down projection's inputs are the SwiGLU rows in f32: quantized here exactly as
                     // quantize_q8 does (src/kernels.rs:84-98, applied per gathered row by
-                    // src/weights.rs:652-664), straight into the staged layout. A thread per
-                    // (row, 32-block).
+                    // src/weights.rs:652-664), straight into the staged layout. Four lanes per
+                    // (row, 32-block), eight values each.
 #pragma unroll 1
-                    for (int task = tid; task < rows * P.nb; task += nthreads) {
-                        const int r = task / P.nb, b = task - r * P.nb;
-                        const size_t row = s_slot[entry_of_row(r)];
-                        const float4* src = reinterpret_cast<const float4*>(a.hidden_f + row * P.cols + b * QK);
-                        float4 v[8];
-#pragma unroll
-                        for (int i = 0; i < 8; i++) v[i] = __ldcg(src + i);
-                        float amax = 0.0f;
-#pragma unroll
-                        for (int i = 0; i < 8; i++)
-                            amax = fmaxf(fmaxf(fmaxf(fmaxf(amax, fabsf(v[i].x)), fabsf(v[i].y)), fabsf(v[i].z)),
-                                         fabsf(v[i].w));
-                        const float d = __fdiv_rn(amax, 127.0f);
-                        const float id = d > 0.0f ? __fdiv_rn(1.0f, d) : 0.0f;
-                        auto q8 = [&](float x) {
-                            const float rr = roundf(x * id);
-                            return (rr != rr) ? 0 : int(fminf(127.0f, fmaxf(-128.0f, rr)));
-                        };
-                        uint32_t packed[8];
-                        int qsum = 0;
-#pragma unroll
-                        for (int i = 0; i < 8; i++) {
-                            const int q0 = q8(v[i].x), q1 = q8(v[i].y), q2 = q8(v[i].z), q3 = q8(v[i].w);
-                            qsum += q0 + q1 + q2 + q3;
-                            packed[i] = uint32_t(q0 & 0xFF) | (uint32_t(q1 & 0xFF) << 8) |
-                                        (uint32_t(q2 & 0xFF) << 16) | (uint32_t(q3 & 0xFF) << 24);
+                    for (int base = 0; base < rows * P.nb * 4; base += nthreads) {
+                        const int task = (base + tid) >> 2, q = tid & 3;
+                        const bool on = task < rows * P.nb;
+                        const int r = on ? int(div_small(task, P.nb)) : 0, b = on ? task - r * P.nb : 0;
+                        const float4* src = reinterpret_cast<const float4*>(
+                            a.hidden_f + size_t(s_slot[entry_of_row(r)]) * P.cols + b * QK + q * 8);
+                        const float4 lo = __ldcg(src), hi = __ldcg(src + 1);
+                        float d, su;
+                        const uint2 w = quantize_block_quad(lo, hi, d, su);
+                        if (on) {
+                            *reinterpret_cast<uint2*>(smem + L.x0 + r * P.x_stride + b * QK + q * 8) = w;
+                            if (q == 0) {
+                                xsT[b * D_TOK + r] = d;
+                                if (KIND == 2) xsumT[b * D_TOK + r] = su;
+                            }
                         }
-                        uint4* dst = reinterpret_cast<uint4*>(smem + L.x0 + r * P.x_stride + b * QK);
-                        dst[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-                        dst[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
-                        xsT[b * D_TOK + r] = d;
-                        if (KIND == 2) xsumT[b * D_TOK + r] = d * float(qsum);
                     }
                 }
                 __syncthreads();
@@ -813,8 +842,8 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
                 // ---- this warp's units of the group's segments, a unit (all its chunks) at a time
 #pragma unroll 1
                 while (ok && cu < P.n) {
-                    const int wu = P.first + cu * nwarps;
-                    const int seg = wu / P.upe;
+                    const int wu = P.first + cu * uwarps;
+                    const int seg = int(div_small(wu, P.upe));
                     const int sx = seg - sb;  // segment of the unit within this batch
                     if (sx >= sj) break;
                     const int u = wu - seg * P.upe;
@@ -871,7 +900,8 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
                                     const int r0 = u * F_ROWS + g;
                                     float* dst = a.out + slot * hidden;
                                     if (EP) {  // the row's place in its home rank's window, over NVLink
-                                        const size_t per_rank = size_t(t) * topk, home = slot / per_rank;
+                                        const size_t per_rank = size_t(t) * topk;
+                                        const size_t home = ranks == 1 ? 0 : uint32_t(slot) / uint32_t(per_rank);
                                         dst = reinterpret_cast<float*>(a.ep.base[home] + a.ep.off_out) + (slot - home * per_rank) * hidden;
                                     }
                                     if (r0 < hidden) dst[r0] = y0;
@@ -962,40 +992,54 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
     }
 }
 
-// Warps per CTA, ring depth and staged rows: as many warps as possible while each still
-// gets a ring of at least two stages; then the deepest ring that fits.
+// Warps per CTA, how many of them take units, ring depth, staged rows and rows of the router staged at a time:
+// as many warps as possible while each still gets a ring of at least two stages; then the deepest
+// ring that fits.
+struct DecodeConfig {
+    int nwarps = 0, unit_warps = 0, stages = 0, xcap = 0, route_rows = 0;
+};
+
+// The most units of either phase that a CTA can get when at most `walk` experts are walked (see share()
+// in the kernel: an expert's units over the CTAs per expert).
+inline int most_units(const MoeDims& d, int walk, int sms) {
+    if (walk < 1 || walk > sms) return 1 << 20;
+    const int per_run = sms / walk, g = (d.inter + 7) / 8, dn = (d.hidden + 15) / 16;
+    return (max(g, dn) + per_run - 1) / per_run;
+}
+
 template <int KIND>
-bool decode_config(const MoeDims& d, int t, int ids_slots, int& nwarps, int& stages, int& xcap, int& route_rows) {
+bool decode_config(const MoeDims& d, int t, int ids_slots, int sms, bool ep, DecodeConfig& c) {
     // Rows staged at a time: an expert's tokens, up to D_TOK of them, out of all the tokens the expert
     // phases see (every rank's when expert-parallel: ids_slots / topk).
-    xcap = min(D_TOK, (ids_slots / d.topk + 7) / 8 * 8);
+    c.xcap = min(D_TOK, (ids_slots / d.topk + 7) / 8 * 8);
     auto deepest = [&](int w, int rr) {
         for (int k = D_MAX_STAGES; k >= 2; k--)
-            if (size_t(DLayout<KIND>(w, k, xcap, rr, d.hidden, d.inter, d.experts, d.topk, ids_slots).total) <= D_SMEM_LIMIT)
+            if (size_t(DLayout<KIND>(w, k, c.xcap, rr, d.hidden, d.inter, d.experts, d.topk, ids_slots).total) <= D_SMEM_LIMIT)
                 return k;
         return 0;
     };
-    int best_w = 0, best_s = 0, best_r = 0;
+    int best_w = 0, best_u = 0, best_s = 0, best_r = 0;
     for (int w = D_MAX_WARPS; w >= 8; w -= 2) {
+        // One or two tokens: a CTA gets fewer units than it has warps. Only those warps have rings, deep ones:
+        // a unit's records are all on their way at once instead of two at a time.
+        const int units = !ep && !dense_walk(d, t) ? most_units(d, min(d.experts, t * d.topk), sms) : w;
+        const int u = max(1, min(w, units));
         // Rows of the router matrix staged at a time: the whole matrix or the fewest equal parts that
         // leave the ring two stages (each part is a pass of the logits: 1.6 us at 16 rows of 1024).
         const int held = D_ROUTE_VEC * w * 32 / (d.hidden / 8);  // rows the CTA's registers hold at a time
         int rr = 0, s = 0;
         for (int parts = 1; parts <= 8 && s < 2; parts++) {
             rr = (d.experts + parts - 1) / parts;
-            if (rr <= held) s = deepest(w, rr);
+            if (rr <= held) s = deepest(u, rr);
         }
-        if (s < 2) rr = 0, s = deepest(w, 0);  // (the logits read global memory)
+        if (s < 2) rr = 0, s = deepest(u, 0);  // (the logits read global memory)
         // (More warps matter more than a third stage: an expert's units are cut into parts of 16
         // where they can be, one per warp. Measured at granite-1b-a400m, batch 32: 0.83 ms per
         // step with 16 warps and two stages against 0.865 with 14 and three.)
-        if (s >= 2) {
-            nwarps = w, stages = s, route_rows = rr;
-            return true;
-        }
-        if (s > best_s) best_s = s, best_w = w, best_r = rr;
+        if (s > best_s) best_w = w, best_u = u, best_s = s, best_r = rr;
+        if (s >= 2) break;
     }
-    nwarps = best_w, stages = best_s, route_rows = best_r;
+    c.nwarps = best_w, c.unit_warps = best_u, c.stages = best_s, c.route_rows = best_r;
     return best_s >= 2;
 }
 
@@ -1018,8 +1062,8 @@ bool decode_block_applies(const MoeDims& d, int kind_gate_up, int kind_down, int
         return false;
     const int slots = (ranks > 0 ? ranks : 1) * t * d.topk;
     if (slots > 65535 / 16 || d.experts > MAX_EXPERTS) return false;  // (slot lists are 16-bit; ids live in shared memory)
-    int w, s, x, r;
-    return kind_gate_up == 1 ? decode_config<1>(d, t, slots, w, s, x, r) : decode_config<2>(d, t, slots, w, s, x, r);
+    DecodeConfig c;
+    return kind_gate_up == 1 ? decode_config<1>(d, t, slots, 148, ranks > 0, c) : decode_config<2>(d, t, slots, 148, ranks > 0, c);
 }
 
 int launch_decode_block(const MoeDims& d, int kind, const uint16_t* router, const float* bias, const float* x,
@@ -1043,16 +1087,17 @@ int launch_decode_block(const MoeDims& d, int kind, const uint16_t* router, cons
     a.sync = ws.grid_sync;
     a.spin_limit = spin_limit;
     a.status = ws.status;
-    int nwarps = 0;
-    const bool fits = kind == 1 ? decode_config<1>(d, t, a.ids_slots, nwarps, a.stages, a.xcap, a.route_rows)
-                                : decode_config<2>(d, t, a.ids_slots, nwarps, a.stages, a.xcap, a.route_rows);
+    DecodeConfig c;
+    const bool fits = kind == 1 ? decode_config<1>(d, t, a.ids_slots, sms, ep != nullptr, c)
+                                : decode_config<2>(d, t, a.ids_slots, sms, ep != nullptr, c);
     if (!fits) return -1;
+    a.unit_warps = c.unit_warps, a.stages = c.stages, a.xcap = c.xcap, a.route_rows = c.route_rows;
     // One CTA per SM, all resident at once (they wait for one another): never more CTAs than SMs.
-    const int grid = sms;
-    const size_t smem = kind == 1 ? size_t(DLayout<1>(nwarps, a.stages, a.xcap, a.route_rows, d.hidden, d.inter, d.experts,
-                                                      d.topk, a.ids_slots).total)
-                                  : size_t(DLayout<2>(nwarps, a.stages, a.xcap, a.route_rows, d.hidden, d.inter, d.experts,
-                                                      d.topk, a.ids_slots).total);
+    const int grid = sms, nwarps = c.nwarps;
+    const size_t smem = kind == 1 ? size_t(DLayout<1>(c.unit_warps, c.stages, c.xcap, c.route_rows, d.hidden, d.inter,
+                                                      d.experts, d.topk, a.ids_slots).total)
+                                  : size_t(DLayout<2>(c.unit_warps, c.stages, c.xcap, c.route_rows, d.hidden, d.inter,
+                                                      d.experts, d.topk, a.ids_slots).total);
     auto kernel = kind == 1 ? (ep ? moe_decode_kernel<1, true> : moe_decode_kernel<1, false>)
                             : (ep ? moe_decode_kernel<2, true> : moe_decode_kernel<2, false>);
     launch_overlapped(kernel, dim3(grid), dim3(nwarps * 32), smem, stream, a);

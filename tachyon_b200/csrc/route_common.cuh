@@ -51,7 +51,7 @@ __device__ __forceinline__ float hsum8(float v, unsigned mask) {
 __device__ __forceinline__ float sum_squares_avx_order(const float* xr, int n, int lane) {
     float acc = 0.0f;
     int i = 0;
-#pragma unroll 8
+#pragma unroll 16
     for (; i + 32 <= n; i += 32) {
         const float v = xr[i + lane];
         acc = fmaf(v, v, acc);
@@ -311,38 +311,60 @@ __device__ __forceinline__ float route_pick_gate(const float* s_val, int topk, i
     return __fdiv_rn(ej, sum);
 }
 
-// 8-bit quantization of one token's row, a warp per 32-block: warps first_warp ..
-// first_warp + nq - 1 of the CTA take the blocks (and the zero padding up to whole
-// super-blocks of the scale rows) in turn.
+// Eight values of a 32-block as quantize_q8 rounds them (src/kernels.rs:84-98), packed: half away from
+// zero (truncation after adding the float below one half with the value's sign: exact for every
+// |v| < 2^22), NaN to 0, the packing saturates. Returns their sum in `qsum`.
+__device__ __forceinline__ uint2 quantize_eight(const float4& a, const float4& b, float id, int& qsum) {
+    auto q4 = [&](const float4& f) {
+        auto q = [&](float x) {
+            const float v = x * id;
+            return __float2int_rz(v + copysignf(0.49999997f, v));
+        };
+        uint32_t w = 0;
+        asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(w) : "r"(q(f.w)), "r"(q(f.z)), "r"(0));
+        asm("cvt.pack.sat.s8.s32.b32 %0, %1, %2, %3;" : "=r"(w) : "r"(q(f.y)), "r"(q(f.x)), "r"(w));
+        return w;
+    };
+    const uint2 w = make_uint2(q4(a), q4(b));
+    qsum = __dp4a(int(w.x), 0x01010101, __dp4a(int(w.y), 0x01010101, 0));
+    return w;
+}
+
+// A 32-block by four neighbouring lanes, eight values each: every lane gets the block's scale and scaled
+// sum of quants, and its own eight bytes. All lanes of the warp take part.
+__device__ __forceinline__ uint2 quantize_block_quad(const float4& a, const float4& b, float& scale, float& sum) {
+    float amax = fmaxf(fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(a.z), fabsf(a.w))),
+                       fmaxf(fmaxf(fabsf(b.x), fabsf(b.y)), fmaxf(fabsf(b.z), fabsf(b.w))));  // (fmaxf drops NaNs, as f32::max)
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+    const float d = __fdiv_rn(amax, 127.0f);
+    int qsum;
+    const uint2 w = quantize_eight(a, b, d > 0.0f ? __fdiv_rn(1.0f, d) : 0.0f, qsum);
+    qsum += __shfl_xor_sync(0xffffffffu, qsum, 1);
+    qsum += __shfl_xor_sync(0xffffffffu, qsum, 2);
+    scale = d;
+    sum = d * float(qsum);
+    return w;
+}
+
+// 8-bit quantization of one token's row (16-byte aligned, in shared memory), four lanes per 32-block: warps
+// first_warp .. first_warp + nq - 1 of the CTA take eight blocks at a time (and the zero padding up
+// to whole super-blocks of the scale rows).
 __device__ __forceinline__ void route_quantize_row(const float* xrow, int hidden, int8_t* xq_row, float* xs_row,
-                                                   float* xsum_row, int warp, int lane, int first_warp, int nq) {
+                                                         float* xsum_row, int warp, int lane, int first_warp, int nq) {
     const int nb = hidden / QK;
     const int padded = (nb + SUPER - 1) / SUPER * SUPER;
-    for (int b = warp - first_warp; warp >= first_warp && b < padded; b += nq) {
-        if (b >= nb) {
-            if (lane == 0) {
-                xs_row[b] = 0.0f;
-                xsum_row[b] = 0.0f;
-            }
-            continue;
+    for (int b0 = (warp - first_warp) * 8; warp >= first_warp && b0 < padded; b0 += nq * 8) {
+        const int b = b0 + (lane >> 2), q = lane & 3;
+        float4 lo = make_float4(0.0f, 0.0f, 0.0f, 0.0f), hi = lo;
+        if (b < nb) {
+            lo = *reinterpret_cast<const float4*>(xrow + b * QK + q * 8);
+            hi = *reinterpret_cast<const float4*>(xrow + b * QK + q * 8 + 4);
         }
-        const float v = xrow[b * QK + lane];
-        float amax = fabsf(v);
-        // f32::max drops NaN operands, as fmaxf does.
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-        const float d = __fdiv_rn(amax, 127.0f);
-        const float id = d > 0.0f ? __fdiv_rn(1.0f, d) : 0.0f;
-        float r = roundf(v * id);
-        int q = (r != r) ? 0 : int(fminf(127.0f, fmaxf(-128.0f, r)));
-        xq_row[b * QK + lane] = int8_t(q);
-        int qsum = q;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) qsum += __shfl_xor_sync(0xffffffffu, qsum, o);
-        if (lane == 0) {
-            xs_row[b] = d;
-            xsum_row[b] = d * float(qsum);
-        }
+        float d, su;
+        const uint2 w = quantize_block_quad(lo, hi, d, su);
+        if (b < nb) *reinterpret_cast<uint2*>(xq_row + b * QK + q * 8) = w;
+        if (b < padded && q == 0) xs_row[b] = d, xsum_row[b] = su;
     }
 }
 
