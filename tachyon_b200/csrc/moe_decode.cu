@@ -115,7 +115,9 @@ struct DLayout {
         const int nbp = (cols / QK + 7) / 8 * 8;
         return xcap * (cols + 16) + nbp * D_TOK * 4 * (KIND == 2 ? 2 : 1);
     }
-    __host__ __device__ static int route_base(int hidden, int experts) { return ((hidden + experts) * 4 + 127) / 128 * 128; }
+    __host__ __device__ static int route_base(int hidden, int experts) {  // the row, its logits and their order keys
+        return (hidden + 2 * ((experts + 3) / 4 * 4)) * 4 / 128 * 128 + 128;
+    }
     __host__ __device__ DLayout(int unit_warps, int stages, int xcap, int route_rows, int hidden, int inter, int experts,
                                 int topk, int ids_slots) {
         int o = unit_warps * stages * Rec<KIND>::BYTES;
@@ -360,6 +362,7 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
     // registers the same way.
     float* xrow = reinterpret_cast<float*>(smem + L.x0);
     float* slog = xrow + hidden;
+    int* skey = reinterpret_cast<int*>(slog + (experts + 3) / 4 * 4);
     const int wstride = 2 * hidden + 32;
     uint8_t* wsm = smem + L.x0 + DLayout<KIND>::route_base(hidden, experts);
     const int pass_rows = a.route_rows > 0 ? a.route_rows : experts;  // (0: the logits read global memory)
@@ -472,11 +475,11 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
                     __syncthreads();
                 }
                 route_logits(a.router, a.route_rows > 0 ? wsm : nullptr, wstride, xrow, a.bias, hidden, e_lo,
-                             min(experts, e_lo + pass_rows), slog, logits_row, tid, nthreads);
+                             min(experts, e_lo + pass_rows), slog, logits_row, tid, nthreads, skey);
                 __syncthreads();  // the staged rows are no longer read; slog is complete up to here
             }
             // The picks by the first warps (a thread per expert), the row's quantization by the others.
-            route_rank_picks(slog, experts, topk, EP ? nullptr : a.ids + size_t(bid) * topk, s_rids, s_rval, tid);
+            route_rank_picks(skey, slog, experts, topk, EP ? nullptr : a.ids + size_t(bid) * topk, s_rids, s_rval, tid);
             const int rank_warps = (experts + 31) >> 5, qfirst = rank_warps < nwarps ? rank_warps : 0;
             if (!EP) {
                 route_quantize_row(xrow, hidden, a.xq + size_t(bid) * hidden, a.xs + size_t(bid) * P0.nbp,
@@ -663,6 +666,7 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
     float acc[D_GMAX][4], off[D_GMAX][4];
     uint32_t xphase = 0, xtok = 0;
     int arrived = 0;  // expert phases this CTA has announced
+    int listed_first = -1, listed_last = -1;  // the segments whose lists are in shared memory
     int cslot = 0;    // consumer's ring slot and the parity of its barrier
     uint32_t cpar = 0;
 
@@ -675,6 +679,8 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
         const int xsum_off = xs_off + P.nbp * D_TOK * 4;
         float* xsT = reinterpret_cast<float*>(smem + L.x0 + xs_off);
         float* xsumT = reinterpret_cast<float*>(smem + L.x0 + xsum_off);
+        // (Both phases cut the walk the same way wherever a CTA stays inside one expert or run: the lists
+        // made for gate_up then serve down as well.)
         const int seg_first = P.lo < P.hi ? int(div_small(P.lo, P.upe)) : 0;
         const int seg_last = P.lo < P.hi ? int(div_small(P.hi - 1, P.upe)) : -1;
 #pragma unroll 1
@@ -682,7 +688,10 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
             const int nseg = min(D_NSEG, seg_last - sb + 1);
             if (sb != seg_first) __syncthreads();  // the previous lists and staged rows are no longer read
             // ---- the slots that named each expert of this batch of segments, ascending
-            if (EP && slots > 8 * 32) {
+            const bool listed = sb == listed_first && sb + nseg - 1 == listed_last;
+            listed_first = sb, listed_last = sb + nseg - 1;
+            if (listed) {
+            } else if (EP && slots > 8 * 32) {
                 // Many slots (every rank's): all warps scan, each a slice of the ids. First the hits per
                 // slice and segment, then, from the counts of the slices before it, where each hit goes.
                 const int slice = ((slots + nwarps - 1) / nwarps + 31) & ~31;
@@ -732,22 +741,27 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
                 const uint32_t e = uint32_t(a.dense ? walk : int(s_active[walk]));
                 const int skip = EP ? int(s_skip[walk]) : 0;  // the expert's slots that earlier runs took
                 const int run_len = EP ? s_run_len : D_TOK;
-                int count = 0, token = 0, pick = lane;  // slot base + lane = token * topk + pick
-                while (pick >= topk) pick -= topk, token++;
+                int count = 0;
 #pragma unroll 1
-                for (int base = 0; base < slots; base += 32) {
-                    const bool hit = base + lane < slots && s_ids[base + lane] == e;
-                    const unsigned ballot = __ballot_sync(0xffffffffu, hit);
-                    if (hit) {
-                        const int ord = count + __popc(ballot & ((1u << lane) - 1u)) - skip;
-                        if (ord >= 0 && ord < run_len) {
-                            s_slot[warp * D_TOK + ord] = uint16_t(base + lane);
-                            s_tok[warp * D_TOK + ord] = uint16_t(token);
-                        }
+                for (int base0 = 0; base0 < slots; base0 += 8 * 32) {
+                    uint32_t id[8];
+#pragma unroll
+                    for (int u = 0; u < 8; u++) {
+                        const int i = base0 + u * 32 + lane;
+                        id[u] = i < slots ? s_ids[i] : 0xffffffffu;
                     }
-                    count += __popc(ballot);
-                    pick += 32;
-                    while (pick >= topk) pick -= topk, token++;
+#pragma unroll
+                    for (int u = 0; u < 8; u++) {
+                        const bool hit = id[u] == e;
+                        const unsigned ballot = __ballot_sync(0xffffffffu, hit);
+                        const int ord = count + __popc(ballot & ((1u << lane) - 1u)) - skip;
+                        if (hit && ord >= 0 && ord < run_len) {
+                            const int i = base0 + u * 32 + lane;
+                            s_slot[warp * D_TOK + ord] = uint16_t(i);
+                            s_tok[warp * D_TOK + ord] = uint16_t(div_small(i, topk));
+                        }
+                        count += __popc(ballot);
+                    }
                 }
                 if (lane == 0) s_seg_count[warp] = min(run_len, max(0, count - skip));
             }

@@ -104,7 +104,7 @@ __device__ __forceinline__ float route_dot_quad(const uint16_t* router, const ui
     if (!busy) {
     } else if (staged) {
         const uint8_t* ws = staged + size_t(e_staged >= 0 ? e_staged : e) * wstride + q * 8;
-#pragma unroll 8
+#pragma unroll 16
         for (int c = 0; c < hidden; c += 16) {
             const uint2 wv = *reinterpret_cast<const uint2*>(ws + 2 * c);
             const float4 xv = *reinterpret_cast<const float4*>(xr + c);
@@ -147,12 +147,13 @@ __device__ __forceinline__ float route_dot_quad(const uint16_t* router, const ui
     return y + 0.0f;
 }
 
-// Router logits of one token, experts e_lo..e_hi-1, into slog[e] (and, when given, a global
-// row), by every thread of the CTA, four per expert. `staged`: rows e_lo.. of the router
+// Router logits of one token, experts e_lo..e_hi-1, into slog[e] (and, when given, their order keys into
+// skey[e] and the logits into a global row), by every thread of the CTA, four per expert. `staged`: rows e_lo.. of the router
 // matrix in shared memory, or null. The caller puts a CTA barrier after it.
 __device__ __forceinline__ void route_logits(const uint16_t* router, const uint8_t* staged, int wstride,
                                              const float* xrow, const float* bias, int hidden, int e_lo, int e_hi,
-                                             float* slog, float* logits_row, int tid, int nthreads) {
+                                             float* slog, float* logits_row, int tid, int nthreads,
+                                             int* skey = nullptr) {
     for (int e0 = e_lo; e0 < e_hi; e0 += nthreads / 4) {
         const int e = e0 + (tid >> 2);
         const bool valid = e < e_hi;
@@ -161,6 +162,7 @@ __device__ __forceinline__ void route_logits(const uint16_t* router, const uint8
         if (valid && (tid & 3) == 0) {
             if (bias) y = y + bias[e];
             slog[e] = y;
+            if (skey) skey[e] = total_key(y);
             if (logits_row) logits_row[e] = y;
         }
     }
@@ -271,31 +273,38 @@ __device__ __forceinline__ void route_topk_gates(const float* slog, int experts,
 }
 
 // Top-k of one token by a whole CTA, a thread per expert: each counts the experts that come before its
-// own in the order (larger key first, lower index first among equals) by reading all of them, four
+// own in the order (larger key first, lower index first among equals) by reading all keys, four
 // at a time, from shared memory; the thread of rank j < topk has the j-th pick, its id into id_out[j] and
 // s_id[j], its score into s_val[j]. The picks of route_topk_gates without a chain of dependent rounds.
-// slog must be 16-byte aligned; the caller puts a CTA barrier before and after.
-__device__ __forceinline__ void route_rank_picks(const float* slog, int experts, int topk, uint32_t* id_out,
-                                                 uint32_t* s_id, float* s_val, int tid) {
-    if (tid >= experts) return;
-    const float mine = slog[tid];
-    const int key = total_key(mine);
-    int rank = 0;
-    auto before = [&](float v, int j) {
-        const int k = total_key(v);
-        rank += (k > key || (k == key && j < tid)) ? 1 : 0;
-    };
-    int j = 0;
-#pragma unroll 4
-    for (; j + 4 <= experts; j += 4) {
-        const float4 v = *reinterpret_cast<const float4*>(slog + j);
-        before(v.x, j), before(v.y, j + 1), before(v.z, j + 2), before(v.w, j + 3);
+// skey[e] = total_key of expert e's logit, 16-byte aligned, readable up to a multiple of 4 experts; the
+// caller puts a CTA barrier before and after. Whole warps take part.
+__device__ __forceinline__ void route_rank_picks(const int* skey, const float* slog, int experts, int topk,
+                                                 uint32_t* id_out, uint32_t* s_id, float* s_val, int tid) {
+    const int warp = tid >> 5, lane = tid & 31;
+    if (warp * 32 >= experts) return;
+    const bool on = tid < experts;
+    const int key = on ? skey[tid] : 0;
+    // Experts of warps before this one come first among equals, those of warps behind it do not; within the
+    // warp the lower lanes do.
+    int rank = __popc(__match_any_sync(0xffffffffu, key) & __ballot_sync(0xffffffffu, on) & ((1u << lane) - 1u));
+#pragma unroll 1
+    for (int j0 = 0; j0 < experts; j0 += 32) {
+        const bool before = (j0 >> 5) < warp;
+#pragma unroll
+        for (int u = 0; u < 32; u += 4) {
+            if (j0 + u < experts) {
+                const int4 k = *reinterpret_cast<const int4*>(skey + j0 + u);
+                const int kk[4] = {k.x, k.y, k.z, k.w};
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+                    if (j0 + u + i < experts && (before ? kk[i] >= key : kk[i] > key)) rank++;
+            }
+        }
     }
-    for (; j < experts; j++) before(slog[j], j);
-    if (rank < topk) {
+    if (on && rank < topk) {
         if (id_out) id_out[rank] = uint32_t(tid);
         s_id[rank] = uint32_t(tid);
-        s_val[rank] = mine;
+        s_val[rank] = slog[tid];
     }
 }
 
