@@ -242,7 +242,6 @@ bool ws_reserve(tc_ctx* ctx, const tc::MoeDims& d, int max_tokens) {
     cudaStreamSynchronize(ctx->stream);
     ws_release(ctx);
     size_t slots = size_t(T) * n.topk;
-    size_t blocks = (size_t(T) + 255) / 256;
     bool ok = ws_alloc(ctx, w.logits, size_t(T) * n.experts) && ws_alloc(ctx, w.ids, slots) &&
               ws_alloc(ctx, w.gates, slots) && ws_alloc(ctx, w.xq, size_t(T) * n.hidden) &&
               ws_alloc(ctx, w.xs, size_t(T) * pad8(n.hidden / 32)) &&
@@ -250,7 +249,7 @@ bool ws_reserve(tc_ctx* ctx, const tc::MoeDims& d, int max_tokens) {
               ws_alloc(ctx, w.counts, size_t(n.experts)) &&
               ws_alloc(ctx, w.offsets, size_t(n.experts) + 1) && ws_alloc(ctx, w.perm, slots) &&
               ws_alloc(ctx, w.pos, slots) && ws_alloc(ctx, w.slot_token, slots) &&
-              ws_alloc(ctx, w.active, size_t(n.experts) + 1) && ws_alloc(ctx, w.block_hist, blocks * n.experts) &&
+              ws_alloc(ctx, w.active, size_t(n.experts) + 1) &&
               ws_alloc(ctx, w.hidden_f, slots * n.inter) && ws_alloc(ctx, w.hq, slots * n.inter) &&
               ws_alloc(ctx, w.hs, slots * pad8(n.inter / 32)) &&
               ws_alloc(ctx, w.hsum, slots * pad8(n.inter / 32)) &&
@@ -904,14 +903,16 @@ int moe_enqueue(tc_moe_layer* layer, const float* x, const float* norm_w, float 
         if (!ctx->capturing && !cuda_ok(ctx, cudaGetLastError(), "MoE launch")) return -1;
         return 0;
     }
+    tc::Workspace wr = ws;  // (the router and dispatch also cut the token tiles of a prefill-size block)
+    if (prefill) wr.tiles = ctx->pre.tiles, wr.tile_count = ctx->pre.tile_count, wr.tile_cols = tc::prefill_tile_columns(layer->pw);
     n += staged(ctx, 0, [&] {
         return tc::launch_route(d, static_cast<const uint16_t*>(layer->router->dev.data), layer->bias,
-                                x, norm_w, eps, t, ws, s);
+                                x, norm_w, eps, t, wr, s);
     });
     if (prefill) {
         const int slots = t * d.topk;
         n += staged(ctx, 2, [&] {
-            return tc::launch_prefill(d, true, layer->gu.kind == TC_Q4, layer->pw, ctx->pre, ws, slots,
+            return tc::launch_prefill(d, true, layer->gu.kind == TC_Q4, layer->pw, ctx->pre, wr, slots,
                                       nullptr, nullptr, s);
         });
         n += staged(ctx, 4, [&] {

@@ -71,6 +71,14 @@ struct RunList {
     int* n = nullptr;             // number of runs
 };
 
+// A tile of one expert's tokens: n of them (sorted slots p0, p0 + 1, ...) in `cols` columns (32, 64
+// or 128); row0 counts the columns of the tiles before it (where its rows start in the tile buffers).
+struct TokenTile {
+    int expert;
+    uint32_t p0, row0;
+    uint16_t n, cols;
+};
+
 struct Workspace {
     int max_tokens = 0, hidden = 0, experts = 0, topk = 0, inter = 0;
     int sms = 0;                  // multiprocessors of the context's device
@@ -86,7 +94,6 @@ struct Workspace {
     uint32_t* pos = nullptr;      // [T*k] token*k + j -> sorted slot
     uint32_t* slot_token = nullptr;  // [T*k] sorted slot -> token
     int* active = nullptr;        // [E+1] experts with tokens, ascending; [E] = how many
-    uint32_t* block_hist = nullptr;  // [blocks, E] dispatch: per-block histograms / bases
     float* hidden_f = nullptr;    // [T*k, I] silu(gate)*up, sorted order
     int8_t* hq = nullptr;         // [T*k, I]
     float* hs = nullptr;          // [T*k, pad8(I/32)]
@@ -95,6 +102,9 @@ struct Workspace {
     int* status = nullptr;        // device status word
     int* ticket = nullptr;        // arrival counter of the router CTAs (zero between launches)
     uint32_t* grid_sync = nullptr;  // [GRID_SYNC_WORDS] arrival counters of the one-kernel decode block (zero between launches)
+    TokenTile* tiles = nullptr;   // when set: the dispatch also cuts the experts' tokens into tiles of up to
+    int* tile_count = nullptr;    // tile_cols columns for the tensor-core kernels
+    int tile_cols = 0;
     RunList runs;                 // when set: the expert kernels walk these instead of counts/offsets/active
     PeerWait combine_wait;        // set for the peer-memory exchange only
     PeerWait dispatch_wait;       // the same, before the dispatch over every rank's tokens
@@ -263,13 +273,6 @@ struct PrefillWeights {  // per layer: the 8-bit values as f16 tiles + f32 block
     uint16_t *gu_t = nullptr, *dn_t = nullptr;
     float *gu_d = nullptr, *gu_c = nullptr, *dn_d = nullptr, *dn_c = nullptr;
 };
-// A tile of one expert's tokens: n of them (sorted slots p0, p0 + 1, ...) in `cols` columns (32, 64
-// or 128); row0 counts the columns of the tiles before it (where its rows start in the tile buffers).
-struct TokenTile {
-    int expert;
-    uint32_t p0, row0;
-    uint16_t n, cols;
-};
 struct PrefillScratch {  // per context
     TokenTile* tiles = nullptr;
     int* tile_count = nullptr;
@@ -281,6 +284,7 @@ struct PrefillScratch {  // per context
 void init_kernels_prefill();
 size_t prefill_weight_bytes(const MoeDims& d, bool gate_up);
 size_t prefill_scale_elems(const MoeDims& d, bool gate_up);
+int prefill_tile_columns(const PrefillWeights& w);  // the largest token tile of a layer with these weights
 int prefill_max_token_tiles(int slots, int experts, bool q4);
 size_t prefill_max_rows(int slots, int experts);  // columns of all the tiles of a batch, at most
 void tile_prefill_weights(const MoeDims& d, const MatrixDev& m, bool gate_up, uint16_t* wt, float* wd, float* wc,

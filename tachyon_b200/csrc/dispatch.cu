@@ -12,6 +12,9 @@
 // base, and a warp-shuffle exclusive scan over experts gives each expert's
 // first slot.
 //
+// (Batches above 256 tokens of a layer take the one-kernel form further down; the three passes serve the entry
+// point that may be handed ids from anywhere.)
+//
 // Outputs: counts[E], offsets[E+1], perm[sorted slot] = token*k + j,
 // slot_token[sorted slot] = token, pos[token*k + j] = sorted slot, and the
 // ascending list of experts that have tokens (active[0..n), active[E] = n),
@@ -34,25 +37,22 @@ dispatch_small_kernel(const uint32_t* ids, int t, int experts, int topk,
                       uint32_t* __restrict__ counts, uint32_t* __restrict__ offsets,
                       uint32_t* __restrict__ perm, uint32_t* __restrict__ pos,
                       uint32_t* __restrict__ slot_token, int* __restrict__ active, const PeerWait pw,
-                      int* status) {
+                      int* status, TokenTile* tiles, int* tile_count, int tile_cols) {
     __shared__ DispatchSmem sm;
     if (pw.flags) {  // the ids come from other ranks: all of them have signalled this block
         if (int(threadIdx.x) < pw.ranks) peer_wait(pw, threadIdx.x);
         __syncthreads();
     }
     dispatch_small_body(sm, ids, t, experts, topk, counts, offsets, perm, pos, slot_token, active, status);
+    if (tiles) token_tiles_body(sm.scount, sm.soff, experts, tile_cols, tiles, tile_count, sm.stiles, sm.srows);
 }
 
-// Large batches, pass 1: each CTA's histogram of its DISPATCH_THREADS tokens.
+// The entry point without allocation, pass 1: each CTA's histogram of its DISPATCH_THREADS tokens.
 __global__ void __launch_bounds__(DISPATCH_THREADS)
 dispatch_count_kernel(const uint32_t* ids, int t, int experts, int topk,
-                      uint32_t* __restrict__ block_hist, const PeerWait pw, int* status) {
+                      uint32_t* __restrict__ block_hist, int* status) {
     __shared__ uint32_t bits[MAX_EXPERTS][DISPATCH_WARPS];
     const int tid = threadIdx.x;
-    if (pw.flags) {
-        if (tid < pw.ranks) peer_wait(pw, tid);
-        __syncthreads();
-    }
     mark_picks(bits, ids, blockIdx.x * DISPATCH_THREADS + tid, t, experts, topk, status);
     for (int e = tid; e < experts; e += DISPATCH_THREADS)
         block_hist[size_t(blockIdx.x) * experts + e] = row_count(bits, e);
@@ -110,32 +110,123 @@ dispatch_permute_kernel(const uint32_t* __restrict__ ids, int t, int experts, in
 
 }  // namespace
 
+namespace {
+
+// Large batches in one kernel, a CTA per expert: expert e's slots start after all the slots of lower
+// experts, so a CTA that counts the ids below e and those equal to e as it reads them needs nothing from the
+// others. A warp owns a contiguous range of the slots (read twice: count, then place), which keeps the
+// order. The last CTA to finish lists the experts that have tokens and, when asked, cuts the token tiles.
+// (Three passes with a histogram per 256 tokens took 26 us for 4096 tokens of 8 picks, most of it
+// launches and a serial scan; every CTA reading all ids, 128 KB from L2, takes 6.)
+constexpr int DISPATCH_E_THREADS = 1024;
+constexpr int DISPATCH_E_WARPS = DISPATCH_E_THREADS / 32;
+
+struct DispatchArgs {
+    const uint32_t* ids;
+    int slots, experts, topk;
+    uint32_t *counts, *offsets, *perm, *pos, *slot_token;
+    int* active;
+    TokenTile* tiles;
+    int* tile_count;
+    int tile_cols;
+    int *ticket, *status;
+};
+
+__global__ void __launch_bounds__(DISPATCH_E_THREADS) dispatch_experts_kernel(const DispatchArgs a, const PeerWait pw) {
+    __shared__ uint32_t s_hits[DISPATCH_E_WARPS], s_below[DISPATCH_E_WARPS];
+    __shared__ int s_last;
+    __shared__ int s_tiles[MAX_EXPERTS / 32], s_rows[MAX_EXPERTS / 32];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t e = blockIdx.x;
+    grid_launch_dependents();
+    grid_dependency_wait();
+    if (pw.flags) {  // the ids come from other ranks: all of them have signalled this block
+        if (tid < pw.ranks) peer_wait(pw, tid);
+        __syncthreads();
+    }
+    const int per_warp = ((a.slots + DISPATCH_E_WARPS - 1) / DISPATCH_E_WARPS + 31) & ~31;
+    const int lo = min(a.slots, warp * per_warp), hi = min(a.slots, lo + per_warp);
+    constexpr int HELD = 8;
+    auto walk = [&](auto use) {
+#pragma unroll 1
+        for (int i0 = lo; i0 < hi; i0 += 32 * HELD) {
+            uint32_t id[HELD];
+#pragma unroll
+            for (int u = 0; u < HELD; u++) {
+                const int i = i0 + 32 * u + lane;
+                id[u] = i < hi ? __ldcg(a.ids + i) : 0xffffffffu;
+            }
+#pragma unroll
+            for (int u = 0; u < HELD; u++) use(i0 + 32 * u + lane, id[u]);
+        }
+    };
+    uint32_t hits = 0, below = 0;
+    bool bad = false;
+    walk([&](int i, uint32_t id) {
+        hits += id == e, below += id < e;
+        bad |= i < hi && id >= uint32_t(a.experts);
+    });
+    hits = __reduce_add_sync(0xffffffffu, hits), below = __reduce_add_sync(0xffffffffu, below);
+    if (e == 0 && bad) atomicExch(a.status, ERR_BAD_EXPERT_ID);
+    if (lane == 0) s_hits[warp] = hits, s_below[warp] = below;
+    __syncthreads();
+    const uint32_t h = s_hits[lane], first = __reduce_add_sync(0xffffffffu, s_below[lane]);
+    uint32_t at = first + __reduce_add_sync(0xffffffffu, lane < warp ? h : 0u);
+    const uint32_t total = __reduce_add_sync(0xffffffffu, h);
+    if (hits) {
+        walk([&](int i, uint32_t id) {
+            const unsigned ballot = __ballot_sync(0xffffffffu, id == e);
+            if (id == e) {
+                const uint32_t p = at + __popc(ballot & ((1u << lane) - 1u));
+                a.perm[p] = uint32_t(i);
+                a.slot_token[p] = uint32_t(i) / uint32_t(a.topk);
+                a.pos[i] = p;
+            }
+            at += __popc(ballot);
+        });
+    }
+    if (tid == 0) {
+        a.counts[e] = total;
+        a.offsets[e] = first;
+        if (int(e) == a.experts - 1) a.offsets[a.experts] = first + total;
+        __threadfence();
+        s_last = atomicAdd(a.ticket, 1) == a.experts - 1;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    if (tid == 0) *a.ticket = 0;  // ready for the next launch on this stream
+    if (a.tiles) token_tiles_body(a.counts, a.offsets, a.experts, a.tile_cols, a.tiles, a.tile_count, s_tiles, s_rows);
+    if (warp == DISPATCH_E_WARPS - 1) list_active(a.counts, a.experts, a.active, lane);
+}
+
+}  // namespace
+
 int launch_dispatch(const MoeDims& d, int t, Workspace& ws, cudaStream_t stream) {
     if (t <= DISPATCH_THREADS) {
         dispatch_small_kernel<<<1, DISPATCH_THREADS, 0, stream>>>(ws.ids, t, d.experts, d.topk,
                                                                   ws.counts, ws.offsets, ws.perm,
                                                                   ws.pos, ws.slot_token, ws.active,
-                                                                  ws.dispatch_wait, ws.status);
+                                                                  ws.dispatch_wait, ws.status, ws.tiles, ws.tile_count,
+                                                                  ws.tile_cols);
         return 1;
     }
-    const int blocks = (t + DISPATCH_THREADS - 1) / DISPATCH_THREADS;
-    dispatch_count_kernel<<<blocks, DISPATCH_THREADS, 0, stream>>>(ws.ids, t, d.experts, d.topk,
-                                                                   ws.block_hist, ws.dispatch_wait,
-                                                                   ws.status);
-    dispatch_scan_kernel<<<1, DISPATCH_THREADS, 0, stream>>>(ws.block_hist, blocks, d.experts,
-                                                             ws.counts, ws.offsets, ws.active);
-    dispatch_permute_kernel<<<blocks, DISPATCH_THREADS, 0, stream>>>(
-        ws.ids, t, d.experts, d.topk, ws.block_hist, ws.offsets, ws.perm, ws.pos, ws.slot_token);
-    return 3;
+    DispatchArgs a{};
+    a.ids = ws.ids, a.slots = t * d.topk, a.experts = d.experts, a.topk = d.topk;
+    a.counts = ws.counts, a.offsets = ws.offsets, a.perm = ws.perm, a.pos = ws.pos, a.slot_token = ws.slot_token;
+    a.active = ws.active;
+    a.tiles = ws.tiles, a.tile_count = ws.tile_count, a.tile_cols = ws.tile_cols;
+    a.ticket = ws.ticket, a.status = ws.status;
+    launch_overlapped(dispatch_experts_kernel, dim3(d.experts), dim3(DISPATCH_E_THREADS), size_t(0), stream, a, ws.dispatch_wait);
+    return 1;
 }
 
 // ---------------------------------------------------------------------------
 // Dispatch for callers that must not allocate.
 //
 // The three-pass dispatch above needs one piece of scratch besides its inputs
-// and outputs: the per-CTA histograms (block_hist). launch_dispatch() takes it
-// from the workspace a layer allocates when it is created. The entry point
-// below instead keeps it in the array that follows, which lives in the
+// and outputs: the per-CTA histograms (block_hist). The entry point
+// below keeps it in the array that follows, which lives in the
 // library's image: every GPU that loads the library holds these 64 KiB until
 // the process exits, and no call ever allocates or frees anything.
 //
@@ -200,8 +291,7 @@ const char* dispatch_static(int device, const uint32_t* ids, int t, int experts,
     }
     if (status_word) *status_word = status;
     const int blocks = (t + DISPATCH_THREADS - 1) / DISPATCH_THREADS;
-    dispatch_count_kernel<<<blocks, DISPATCH_THREADS, 0, stream>>>(ids, t, experts, topk, block_hist, PeerWait{},
-                                                                   status);
+    dispatch_count_kernel<<<blocks, DISPATCH_THREADS, 0, stream>>>(ids, t, experts, topk, block_hist, status);
     dispatch_scan_kernel<<<1, DISPATCH_THREADS, 0, stream>>>(block_hist, blocks, experts, counts, offsets, active);
     dispatch_permute_kernel<<<blocks, DISPATCH_THREADS, 0, stream>>>(ids, t, experts, topk, block_hist, offsets,
                                                                      perm, pos, slot_token);

@@ -97,11 +97,46 @@ __device__ __forceinline__ void list_active(const uint32_t* counts, int experts,
     if (lane == 0) active[experts] = n;
 }
 
+// The token tiles of the experts, by one CTA of at least MAX_EXPERTS threads. Expert e's m tokens: whole
+// tiles of most_cols (128 or 64), then the remainder as one tile of 32, 64 or 128 columns. A thread per
+// expert; s_tiles / s_rows: MAX_EXPERTS / 32 words each.
+__device__ __forceinline__ void token_tiles_body(const uint32_t* counts, const uint32_t* offsets, int experts, int most_cols,
+                                                 TokenTile* tiles, int* tile_count, int* s_tiles, int* s_rows) {
+    const int e = threadIdx.x, lane = e & 31, warp = e >> 5;
+    const bool mine_on = e < MAX_EXPERTS;
+    const int m = e < experts ? int(counts[e]) : 0;
+    const int whole = m / most_cols, rest = m - whole * most_cols;
+    const int mine = whole + (rest ? 1 : 0);
+    const int rows = whole * most_cols + (rest == 0 ? 0 : rest > 64 ? 128 : rest > 32 ? 64 : 32);
+    int t_in = mine, r_in = rows;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t_up = __shfl_up_sync(0xffffffffu, t_in, o), r_up = __shfl_up_sync(0xffffffffu, r_in, o);
+        if (lane >= o) t_in += t_up, r_in += r_up;
+    }
+    if (mine_on && lane == 31) s_tiles[warp] = t_in, s_rows[warp] = r_in;
+    __syncthreads();
+    if (!mine_on) return;
+    int tt = t_in - mine, row0 = r_in - rows;
+    for (int k = 0; k < warp; k++) tt += s_tiles[k], row0 += s_rows[k];
+    if (e == MAX_EXPERTS - 1) *tile_count = tt + mine;
+    if (e >= experts) return;
+    uint32_t p0 = offsets[e];
+    int left = m;
+    for (int i = 0; i < mine; i++) {
+        const int cols = left > 64 ? most_cols : left > 32 ? 64 : 32;
+        const int n = min(left, cols);
+        tiles[tt + i] = TokenTile{e, p0, uint32_t(row0), uint16_t(n), uint16_t(cols)};
+        p0 += n, row0 += cols, left -= n;
+    }
+}
+
 // Shared memory of the single-CTA dispatch.
 struct DispatchSmem {
     uint32_t bits[MAX_EXPERTS][DISPATCH_WARPS];
     uint32_t scount[MAX_EXPERTS];
     uint32_t soff[MAX_EXPERTS + 1];
+    int stiles[MAX_EXPERTS / 32], srows[MAX_EXPERTS / 32];
 };
 
 // Small batches (t <= DISPATCH_THREADS): the whole dispatch by one CTA of

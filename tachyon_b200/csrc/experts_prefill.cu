@@ -37,6 +37,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "dispatch_common.cuh"
 #include "experts_common.cuh"
 #include "umma.cuh"
 
@@ -634,39 +635,14 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// The token tiles of the experts. Expert e's m tokens: whole tiles of most_cols (128 or 64), then the
-// remainder as one tile of 32, 64 or 128 columns. One CTA, a thread per expert.
+// (A dispatch that was given the tile list has built it already.)
 __global__ void __launch_bounds__(MAX_EXPERTS)
     build_token_tiles_kernel(const uint32_t* counts, const uint32_t* offsets, int experts, int most_cols,
                              TokenTile* tiles, int* tile_count) {
     __shared__ int s_tiles[MAX_EXPERTS / 32], s_rows[MAX_EXPERTS / 32];
     grid_launch_dependents();
     grid_dependency_wait();
-    const int e = threadIdx.x, lane = e & 31, warp = e >> 5;
-    const int m = e < experts ? int(counts[e]) : 0;
-    const int whole = m / most_cols, rest = m - whole * most_cols;
-    const int mine = whole + (rest ? 1 : 0);
-    const int rows = whole * most_cols + (rest == 0 ? 0 : rest > 64 ? 128 : rest > 32 ? 64 : 32);
-    int t_in = mine, r_in = rows;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int t_up = __shfl_up_sync(0xffffffffu, t_in, o), r_up = __shfl_up_sync(0xffffffffu, r_in, o);
-        if (lane >= o) t_in += t_up, r_in += r_up;
-    }
-    if (lane == 31) s_tiles[warp] = t_in, s_rows[warp] = r_in;
-    __syncthreads();
-    int tt = t_in - mine, row0 = r_in - rows;
-    for (int k = 0; k < warp; k++) tt += s_tiles[k], row0 += s_rows[k];
-    if (e == MAX_EXPERTS - 1) *tile_count = tt + mine;
-    if (e >= experts) return;
-    uint32_t p0 = offsets[e];
-    int left = m;
-    for (int i = 0; i < mine; i++) {
-        const int cols = left > 64 ? most_cols : left > 32 ? 64 : 32;
-        const int n = min(left, cols);
-        tiles[tt + i] = TokenTile{e, p0, uint32_t(row0), uint16_t(n), uint16_t(cols)};
-        p0 += n, row0 += cols, left -= n;
-    }
+    token_tiles_body(counts, offsets, experts, most_cols, tiles, tile_count, s_tiles, s_rows);
 }
 
 // The 8-bit rows of the block's input (xq/xs/xsum through row_of_slot) as f16 into canonical
@@ -730,6 +706,8 @@ size_t prefill_scale_elems(const MoeDims& d, bool gate_up) {
     return size_t(d.experts) * prefill_row_tiles(d, gate_up) * P_ROWS * (cols / QK);
 }
 
+int prefill_tile_columns(const PrefillWeights& w) { return prefill_columns(w.gu_c || w.dn_c); }
+
 // Bounds over every routing: an expert adds at most one tile beyond its whole ones, and pads by up to 63 rows.
 int prefill_max_token_tiles(int slots, int experts, bool q4) {
     return slots / prefill_columns(q4) + std::min(slots, experts);
@@ -763,16 +741,19 @@ int launch_prefill(const MoeDims& d, bool gate_up, bool q4, const PrefillWeights
     const int max_tiles = prefill_max_token_tiles(slots, d.experts, narrow);
     int launched = 0;
     if (gate_up) {
-        launch_overlapped(build_token_tiles_kernel, dim3(1), dim3(MAX_EXPERTS), size_t(0), stream,
-                          static_cast<const uint32_t*>(ws.counts), static_cast<const uint32_t*>(ws.offsets), d.experts,
-                          prefill_columns(narrow), s.tiles, s.tile_count);
+        if (!ws.tiles) {
+            launch_overlapped(build_token_tiles_kernel, dim3(1), dim3(MAX_EXPERTS), size_t(0), stream,
+                              static_cast<const uint32_t*>(ws.counts), static_cast<const uint32_t*>(ws.offsets), d.experts,
+                              prefill_columns(narrow), s.tiles, s.tile_count);
+            launched++;
+        }
         launch_overlapped(q4 ? tile_activations_kernel<true> : tile_activations_kernel<false>,
                           dim3(max_tiles, (nb + P_ACT_BLOCKS - 1) / P_ACT_BLOCKS), dim3(256), size_t(0), stream,
                           static_cast<const int8_t*>(ws.xq), static_cast<const float*>(ws.xs),
                           static_cast<const float*>(ws.xsum), static_cast<const uint32_t*>(ws.slot_token), cols, nbp,
                           static_cast<const TokenTile*>(s.tiles), static_cast<const int*>(s.tile_count), s.xt, s.xst,
                           s.xsumt);
-        launched += 2;
+        launched++;
     }
     PrefillArgs a{};
     a.wt = gate_up ? w.gu_t : w.dn_t;

@@ -51,6 +51,8 @@ struct RouteArgs {
     int* status;
     uint32_t *counts, *offsets, *perm, *pos, *slot_token;
     int* active;
+    TokenTile* tiles;      // when set: token tiles of up to tile_cols columns are cut as well
+    int *tile_count, tile_cols;
     PeerPlan scatter;      // ranks > 0: the last CTA sends the rows to every rank instead of dispatching
 };
 
@@ -153,24 +155,29 @@ __global__ void __launch_bounds__(ROUTE_THREADS) route_kernel(const RouteArgs a)
                 DispatchSmem& sm = *reinterpret_cast<DispatchSmem*>(smem);
                 dispatch_small_body(sm, a.ids, a.t, experts, topk, a.counts, a.offsets, a.perm, a.pos,
                                     a.slot_token, a.active, a.status);
+                if (a.tiles)
+                    token_tiles_body(sm.scount, sm.soff, experts, a.tile_cols, a.tiles, a.tile_count, sm.stiles, sm.srows);
             }
             if (tid == 0) *a.ticket = 0;  // ready for the next launch on this stream
         }
     }
 }
 
-// Prefill-size batches: a CTA takes ROUTE_TILE tokens at a time (walking tiles blockIdx.x,
-// blockIdx.x + gridDim.x, ...), so that every warp has work in every step: a warp per token for
-// the norm, the ranking and the quantization, four threads per (token, expert) pair for the
-// logits, with the router matrix staged once per CTA. Same arithmetic per token as route_kernel.
-constexpr int ROUTE_TILE = 8;
+// Prefill-size batches: a CTA takes a tile of 2 * TG tokens at a time (walking tiles blockIdx.x,
+// blockIdx.x + gridDim.x, ...): a warp per token for the norm, the ranking and the quantization,
+// four threads per (expert, group of TG tokens) for the logits, with the router matrix staged once
+// per CTA. Same arithmetic per token as route_kernel. TG = 4 keeps every warp busy and reads the router
+// matrix least; batches that would then leave SMs without a tile take TG = 2 or 1 (333 tokens of the 1b
+// shape: 42 tiles of 8, 167 of 2).
 
 // Shared memory of the tile kernel before the staged router matrix: padded rows, logits, norm weight.
-__host__ __device__ inline size_t route_tile_bytes(int hidden, int experts) {
-    return (size_t(ROUTE_TILE) * (hidden / QK * ROW_PAD_BLOCK + experts) * 4 + size_t(hidden) * 4 + 127) / 128 * 128;
+__host__ __device__ inline size_t route_tile_bytes(int hidden, int experts, int tile) {
+    return (size_t(tile) * (hidden / QK * ROW_PAD_BLOCK + experts) * 4 + size_t(hidden) * 4 + 127) / 128 * 128;
 }
 
+template <int TG>
 __global__ void __launch_bounds__(ROUTE_THREADS) route_tile_kernel(const RouteArgs a) {
+    constexpr int ROUTE_TILE = 2 * TG;
     extern __shared__ __align__(128) float smem[];
     const int hidden = a.hidden, experts = a.experts, topk = a.topk;
     const int rstride = hidden / QK * ROW_PAD_BLOCK;  // floats per padded row
@@ -181,7 +188,7 @@ __global__ void __launch_bounds__(ROUTE_THREADS) route_tile_kernel(const RouteAr
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     grid_launch_dependents();
     const int wstride = 2 * hidden + 32;
-    uint8_t* wsm = reinterpret_cast<uint8_t*>(smem) + route_tile_bytes(hidden, experts);
+    uint8_t* wsm = reinterpret_cast<uint8_t*>(smem) + route_tile_bytes(hidden, experts, ROUTE_TILE);
     if (a.norm_w)
         for (int c = tid; c < hidden; c += ROUTE_THREADS) snw[c] = a.norm_w[c];  // (a constant: before the wait)
     if (a.stage_router) {
@@ -204,10 +211,23 @@ __global__ void __launch_bounds__(ROUTE_THREADS) route_tile_kernel(const RouteAr
         const int t0 = tile * ROUTE_TILE, nt = min(ROUTE_TILE, a.t - t0);
         __syncthreads();  // the previous tile's rows and logits are no longer read
         const int vec_per_row = hidden / 4;
-        for (int k = 0; k < nt; k++) {
-            const float4* src = reinterpret_cast<const float4*>(a.x + size_t(t0 + k) * hidden);
-            for (int i = tid; i < vec_per_row; i += ROUTE_THREADS)
-                *reinterpret_cast<float4*>(xrows + k * rstride + padded_at(4 * i)) = src[i];
+        const float4* src = reinterpret_cast<const float4*>(a.x + size_t(t0) * hidden);  // (the tile's rows are one run)
+        const int vecs = nt * vec_per_row;
+        for (int i0 = 0; i0 < vecs; i0 += ROUTE_THREADS * ROUTE_TILE) {  // all requests of a pass before the first store
+            float4 v[ROUTE_TILE];
+#pragma unroll
+            for (int u = 0; u < ROUTE_TILE; u++) {
+                const int i = i0 + u * ROUTE_THREADS + tid;
+                if (i < vecs) v[u] = src[i];
+            }
+#pragma unroll
+            for (int u = 0; u < ROUTE_TILE; u++) {
+                const int i = i0 + u * ROUTE_THREADS + tid;
+                if (i < vecs) {
+                    const int k = i / vec_per_row, c = 4 * (i - k * vec_per_row);
+                    *reinterpret_cast<float4*>(xrows + k * rstride + padded_at(c)) = v[u];
+                }
+            }
         }
         __syncthreads();
         if (a.norm_w && warp < nt) {  // a warp per token
@@ -224,11 +244,11 @@ __global__ void __launch_bounds__(ROUTE_THREADS) route_tile_kernel(const RouteAr
             w_waited = true;
         }
         __syncthreads();
-        // Logits: four threads per (expert, group of ROUTE_TG tokens): the expert's row is read from
+        // Logits: four threads per (expert, group of TG tokens): the expert's row is read from
         // shared memory once for the group's tokens (the row reads, distinct per expert, are what
         // the shared-memory pipe is busy with; the tokens' reads are broadcasts). Each (token,
         // expert) logit keeps its own accumulators: the same sums as one token at a time.
-        constexpr int ROUTE_TG = 4;
+        constexpr int ROUTE_TG = TG;
         const int groups = (nt + ROUTE_TG - 1) / ROUTE_TG, tasks = groups * experts;
         for (int p0 = 0; p0 < tasks; p0 += ROUTE_THREADS / 4) {
             const int p = p0 + (tid >> 2), q = tid & 3;
@@ -312,7 +332,9 @@ __global__ void rmsnorm_kernel(const float* x, const float* __restrict__ w, floa
 
 void init_kernels_route() {
     cudaFuncSetAttribute(route_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ROUTE_SMEM_LIMIT));
-    cudaFuncSetAttribute(route_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ROUTE_SMEM_LIMIT));
+    cudaFuncSetAttribute(route_tile_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ROUTE_SMEM_LIMIT));
+    cudaFuncSetAttribute(route_tile_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ROUTE_SMEM_LIMIT));
+    cudaFuncSetAttribute(route_tile_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ROUTE_SMEM_LIMIT));
 }
 
 int launch_route(const MoeDims& d, const uint16_t* router, const float* bias, const float* x,
@@ -342,6 +364,7 @@ int launch_route(const MoeDims& d, const uint16_t* router, const float* bias, co
     a.pos = ws.pos;
     a.slot_token = ws.slot_token;
     a.active = ws.active;
+    a.tiles = ws.tiles, a.tile_count = ws.tile_count, a.tile_cols = ws.tile_cols;
     if (a.fuse_dispatch) a.scatter = ws.route_scatter;
     size_t smem = (size_t(d.hidden + d.experts) * sizeof(float) + 127) / 128 * 128;
     const size_t staged = smem + size_t(d.experts) * (2 * size_t(d.hidden) + 32);
@@ -353,15 +376,17 @@ int launch_route(const MoeDims& d, const uint16_t* router, const float* bias, co
         // Up to one CTA's worth of tokens: a CTA per token; the last one to finish runs the dispatch.
         launch_overlapped(route_kernel, dim3(t), dim3(ROUTE_THREADS), smem, stream, a);
     } else {
-        // Larger batches: CTAs that walk tiles of ROUTE_TILE tokens with every warp busy, as many as
-        // stay resident (the staged router matrix is then read a few hundred times, not once per token).
-        size_t tsmem = route_tile_bytes(d.hidden, d.experts);
+        // Larger batches: CTAs that walk tiles, as many as stay resident (the staged router matrix is then
+        // read a few hundred times, not once per token).
+        const int tg = t >= 8 * sms ? 4 : t >= 4 * sms ? 2 : 1, tile = 2 * tg;
+        size_t tsmem = route_tile_bytes(d.hidden, d.experts, tile);
         const size_t tstaged = tsmem + size_t(d.experts) * (2 * size_t(d.hidden) + 32);
         a.stage_router = tstaged <= ROUTE_SMEM_LIMIT;
         if (a.stage_router) tsmem = tstaged;
         const int per_sm = int(std::max<size_t>(1, std::min<size_t>(4, (220 * 1024) / (tsmem + 1024))));
-        const int tiles = (t + ROUTE_TILE - 1) / ROUTE_TILE;
-        launch_overlapped(route_tile_kernel, dim3(std::min(tiles, per_sm * sms)), dim3(ROUTE_THREADS), tsmem, stream, a);
+        const int tiles = (t + tile - 1) / tile;
+        launch_overlapped(tg == 4 ? route_tile_kernel<4> : tg == 2 ? route_tile_kernel<2> : route_tile_kernel<1>,
+                          dim3(std::min(tiles, per_sm * sms)), dim3(ROUTE_THREADS), tsmem, stream, a);
     }
     int launched = 1;
     // (Expert parallel over peer windows: the dispatch runs later, over every rank's tokens.)
