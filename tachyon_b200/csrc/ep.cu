@@ -273,7 +273,7 @@ bool ep_uniform_reserve(EpState& st, const MoeDims& d, int max_tokens) {
     const bool ok = get(u.xq, size_t(T) * H) && get(u.xs, size_t(T) * nbp) && get(u.xsum, size_t(T) * nbp) &&
                     get(u.ids, slots) && get(u.counts, size_t(E) + 1) && get(u.offsets, size_t(E) + 2) &&
                     get(u.perm, slots) && get(u.pos, slots) && get(u.slot_token, slots) &&
-                    get(u.active, size_t(E) + 2) && get(u.block_hist, size_t((T + 255) / 256) * E) &&
+                    get(u.active, size_t(E) + 2) &&
                     get(u.hidden_f, slots * I) && get(u.identity, slots) &&
                     // (the reduce-scatter buffer of the exchange over NCCL; the peer windows do without it)
                     (slots * H * 4 > UNIFORM_MAX_BYTES ? (u.big = nullptr, true) : get(u.big, slots * H)) &&
@@ -324,7 +324,6 @@ const char* ep_forward_uniform(EpState& st, EpLayerBuffers& b, const MoeDims& d,
     gw.pos = u.pos;
     gw.slot_token = u.slot_token;
     gw.active = u.active;
-    gw.block_hist = u.block_hist;
     *launches += launch_dispatch(d, G, gw, stream);
     if (gate_up.kind == 2) {
         const size_t want_blocks = (size_t(G) * nbp + 7) / 8;
@@ -553,7 +552,6 @@ const char* ep_forward_peer(EpState& st, EpLayerBuffers& b, const MoeDims& d, co
     gw.pos = u.pos;
     gw.slot_token = u.slot_token;
     gw.active = u.active;
-    gw.block_hist = u.block_hist;
     gw.dispatch_wait.flags = reinterpret_cast<const uint32_t*>(p.window + p.off_flags);
     gw.dispatch_wait.epoch = p.epoch;
     gw.dispatch_wait.ranks = R;
