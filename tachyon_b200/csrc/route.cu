@@ -46,6 +46,7 @@ struct RouteArgs {
     float* xsum;
     // dispatch outputs, used when fused
     int fuse_dispatch;
+    int stage_rows;        // tile kernel: rows of the router matrix in shared memory at a time
     int stage_router;      // the router matrix fits in shared memory beside the row: stage it with bulk copies
     int* ticket;
     int* status;
@@ -172,61 +173,70 @@ __global__ void __launch_bounds__(ROUTE_THREADS) route_kernel(const RouteArgs a)
 
 // Shared memory of the tile kernel before the staged router matrix: padded rows, logits, norm weight.
 __host__ __device__ inline size_t route_tile_bytes(int hidden, int experts, int tile) {
-    return (size_t(tile) * (hidden / QK * ROW_PAD_BLOCK + experts) * 4 + size_t(hidden) * 4 + 127) / 128 * 128;
+    return (size_t(tile) * (hidden / QK * ROW_PAD_BLOCK + (experts + 3) / 4 * 4) * 4 + size_t(hidden) * 4 + 127) / 128 * 128;
 }
 
 template <int TG>
 __global__ void __launch_bounds__(ROUTE_THREADS) route_tile_kernel(const RouteArgs a) {
-    constexpr int ROUTE_TILE = 2 * TG;
+    constexpr int TILE = 2 * TG;
     extern __shared__ __align__(128) float smem[];
     const int hidden = a.hidden, experts = a.experts, topk = a.topk;
     const int rstride = hidden / QK * ROW_PAD_BLOCK;  // floats per padded row
-    float* xrows = smem;                              // [ROUTE_TILE] padded rows
-    float* slog = xrows + ROUTE_TILE * rstride;       // [ROUTE_TILE][experts]
-    float* snw = slog + ROUTE_TILE * experts;         // [hidden] the norm's weight
+    const int lstride = (experts + 3) / 4 * 4;
+    float* xrows = smem;                        // [TILE] padded rows
+    float* slog = xrows + TILE * rstride;       // [TILE][lstride]
+    float* snw = slog + TILE * lstride;         // [hidden] the norm's weight
     __shared__ __align__(8) uint64_t s_wbar;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     grid_launch_dependents();
-    const int wstride = 2 * hidden + 32;
-    uint8_t* wsm = reinterpret_cast<uint8_t*>(smem) + route_tile_bytes(hidden, experts, ROUTE_TILE);
+    // The router matrix by bulk copies, one per row, into rows padded by 32 bytes: all of it, once, or (a
+    // matrix larger than the space left) stage_rows experts at a time, again for every tile.
+    const int wstride = 2 * hidden + 32, stage_rows = a.stage_rows;
+    uint8_t* wsm = reinterpret_cast<uint8_t*>(smem) + route_tile_bytes(hidden, experts, TILE);
+    auto stage = [&](int e_lo) {
+        const int n = min(stage_rows, experts - e_lo);
+        if (warp == 0) {
+            if (lane == 0) mbar_expect_tx(&s_wbar, uint32_t(n) * 2u * uint32_t(hidden));
+            __syncwarp();
+            for (int e = lane; e < n; e += 32)
+                bulk_copy(wsm + size_t(e) * wstride, a.router + size_t(e_lo + e) * hidden, 2 * hidden, &s_wbar);
+        }
+    };
+    if (tid == 0) {
+        mbar_init(&s_wbar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
     if (a.norm_w)
         for (int c = tid; c < hidden; c += ROUTE_THREADS) snw[c] = a.norm_w[c];  // (a constant: before the wait)
-    if (a.stage_router) {
-        if (tid == 0) {
-            mbar_init(&s_wbar, 1);
-            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            mbar_expect_tx(&s_wbar, uint32_t(experts) * 2u * uint32_t(hidden));
-        }
-        __syncthreads();
-        if (warp == 0)
-            for (int e = lane; e < experts; e += 32)
-                bulk_copy(wsm + size_t(e) * wstride, a.router + size_t(e) * hidden, 2 * hidden, &s_wbar);
-    }
+    __syncthreads();
+    stage(0);  // (constants as well)
     grid_dependency_wait();
-    bool w_landed = true, w_waited = false;
+    bool landed = true;
+    uint32_t stagings = 0;  // waited for
+    const bool once = stage_rows >= experts;
     const int padded = (hidden / QK + SUPER - 1) / SUPER * SUPER;
-    const int tiles = (a.t + ROUTE_TILE - 1) / ROUTE_TILE;
+    const int tiles = (a.t + TILE - 1) / TILE, vec_per_row = hidden / 4;
+    const int dk = ROUTE_THREADS / vec_per_row, dv = ROUTE_THREADS - dk * vec_per_row;
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        const int t0 = tile * ROUTE_TILE, nt = min(ROUTE_TILE, a.t - t0);
+        const int t0 = tile * TILE, nt = min(TILE, a.t - t0);
         __syncthreads();  // the previous tile's rows and logits are no longer read
-        const int vec_per_row = hidden / 4;
         const float4* src = reinterpret_cast<const float4*>(a.x + size_t(t0) * hidden);  // (the tile's rows are one run)
         const int vecs = nt * vec_per_row;
-        for (int i0 = 0; i0 < vecs; i0 += ROUTE_THREADS * ROUTE_TILE) {  // all requests of a pass before the first store
-            float4 v[ROUTE_TILE];
+        int k = tid / vec_per_row, vc = tid - k * vec_per_row;  // piece i of the run is piece vc of row k
+        for (int i0 = 0; i0 < vecs; i0 += ROUTE_THREADS * TILE) {  // all requests of a pass before the first store
+            float4 v[TILE];
 #pragma unroll
-            for (int u = 0; u < ROUTE_TILE; u++) {
+            for (int u = 0; u < TILE; u++) {
                 const int i = i0 + u * ROUTE_THREADS + tid;
                 if (i < vecs) v[u] = src[i];
             }
 #pragma unroll
-            for (int u = 0; u < ROUTE_TILE; u++) {
-                const int i = i0 + u * ROUTE_THREADS + tid;
-                if (i < vecs) {
-                    const int k = i / vec_per_row, c = 4 * (i - k * vec_per_row);
-                    *reinterpret_cast<float4*>(xrows + k * rstride + padded_at(c)) = v[u];
-                }
+            for (int u = 0; u < TILE; u++) {
+                if (i0 + u * ROUTE_THREADS + tid < vecs)
+                    *reinterpret_cast<float4*>(xrows + k * rstride + padded_at(4 * vc)) = v[u];
+                k += dk, vc += dv;
+                if (vc >= vec_per_row) vc -= vec_per_row, k++;
             }
         }
         __syncthreads();
@@ -235,82 +245,84 @@ __global__ void __launch_bounds__(ROUTE_THREADS) route_tile_kernel(const RouteAr
             const float ss = __fdiv_rn(sum_squares_padded_row(xr, hidden, lane), float(hidden));
             const float inv = __fdiv_rn(1.0f, __fsqrt_rn(ss + a.eps));
             __syncwarp();
-#pragma unroll 4
-            for (int k = 0; k < hidden / QK; k++)
-                xr[k * ROW_PAD_BLOCK + lane] = xr[k * ROW_PAD_BLOCK + lane] * inv * snw[k * QK + lane];
+#pragma unroll 8
+            for (int c = 0; c < hidden / QK; c++)
+                xr[c * ROW_PAD_BLOCK + lane] = xr[c * ROW_PAD_BLOCK + lane] * inv * snw[c * QK + lane];
         }
-        if (a.stage_router && !w_waited) {
-            w_landed = mbar_wait_bounded(&s_wbar, 0);
-            w_waited = true;
-        }
-        __syncthreads();
-        // Logits: four threads per (expert, group of TG tokens): the expert's row is read from
-        // shared memory once for the group's tokens (the row reads, distinct per expert, are what
-        // the shared-memory pipe is busy with; the tokens' reads are broadcasts). Each (token,
-        // expert) logit keeps its own accumulators: the same sums as one token at a time.
-        constexpr int ROUTE_TG = TG;
-        const int groups = (nt + ROUTE_TG - 1) / ROUTE_TG, tasks = groups * experts;
-        for (int p0 = 0; p0 < tasks; p0 += ROUTE_THREADS / 4) {
-            const int p = p0 + (tid >> 2), q = tid & 3;
-            const bool valid = p < tasks;
-            const int grp = valid ? p / experts : 0, e = valid ? p - grp * experts : 0;
-            float acc[ROUTE_TG][4];
+        for (int e_lo = 0; e_lo < experts; e_lo += stage_rows) {
+            if (!once || stagings == 0) {
+                landed = mbar_wait_bounded(&s_wbar, stagings & 1) && landed;
+                stagings++;
+            }
+            if (e_lo == 0) __syncthreads();  // the normed rows are complete
+            // Logits: four threads per (expert, group of TG tokens): the expert's row is read from
+            // shared memory once for the group's tokens (the row reads, distinct per expert, are what
+            // the shared-memory pipe is busy with; the tokens' reads are broadcasts). Each (token,
+            // expert) logit keeps its own accumulators, as route_dot_quad: thread q of a quad has elements
+            // 16 j + 4 q .. + 3. (Rows past the tile's tokens hold anything; their logits are not stored.)
+            const int n_e = min(stage_rows, experts - e_lo);
+            const int groups = (nt + TG - 1) / TG, tasks = groups * n_e;
+            for (int p0 = 0; p0 < tasks; p0 += ROUTE_THREADS / 4) {
+                const int p = p0 + (tid >> 2), q = tid & 3;
+                const bool valid = p < tasks;
+                const int grp = valid ? p / n_e : 0, e = valid ? p - grp * n_e : 0;
+                float2 acc[TG][2];
 #pragma unroll
-            for (int k = 0; k < ROUTE_TG; k++) acc[k][0] = acc[k][1] = acc[k][2] = acc[k][3] = 0.0f;
-            if (p0 + ((tid >> 5) << 3) < tasks) {  // (a warp without work skips the loop)
-                const bool staged = a.stage_router && w_landed;
-                const uint8_t* ws = wsm + size_t(e) * wstride + q * 8;
-                const uint16_t* wg = a.router + size_t(e) * hidden + q * 4;
-                const float* xr = xrows + size_t(grp * ROUTE_TG) * rstride + q * 4;
+                for (int i = 0; i < TG; i++) acc[i][0] = acc[i][1] = make_float2(0.0f, 0.0f);
+                if (p0 + ((tid >> 5) << 3) < tasks) {  // (a warp without work skips the loop)
+                    const uint8_t* ws = wsm + size_t(e) * wstride + q * 8;
+                    const float* xr = xrows + size_t(grp * TG) * rstride + q * 4;
 #pragma unroll 2
-                for (int c = 0; c < hidden; c += 16) {
-                    const uint2 wv = staged ? *reinterpret_cast<const uint2*>(ws + 2 * c)
-                                            : __ldg(reinterpret_cast<const uint2*>(wg + c));
-                    const float w0 = bf16_lo(wv.x), w1 = bf16_hi(wv.x), w2 = bf16_lo(wv.y), w3 = bf16_hi(wv.y);
+                    for (int blk = 0; blk < hidden / QK; blk++, ws += 2 * QK, xr += ROW_PAD_BLOCK) {
 #pragma unroll
-                    for (int k = 0; k < ROUTE_TG; k++) {
-                        if (grp * ROUTE_TG + k < nt) {
-                            const float4 xv = *reinterpret_cast<const float4*>(xr + k * rstride + padded_at(c));
-                            acc[k][0] = fmaf(w0, xv.x, acc[k][0]);
-                            acc[k][1] = fmaf(w1, xv.y, acc[k][1]);
-                            acc[k][2] = fmaf(w2, xv.z, acc[k][2]);
-                            acc[k][3] = fmaf(w3, xv.w, acc[k][3]);
+                        for (int h = 0; h < 2; h++) {
+                            const uint2 wv = *reinterpret_cast<const uint2*>(ws + 32 * h);
+                            const float2 w01 = make_float2(bf16_lo(wv.x), bf16_hi(wv.x)), w23 = make_float2(bf16_lo(wv.y), bf16_hi(wv.y));
+#pragma unroll
+                            for (int i = 0; i < TG; i++) {
+                                const float4 xv = *reinterpret_cast<const float4*>(xr + i * rstride + 16 * h);
+                                acc[i][0] = fma2(w01, make_float2(xv.x, xv.y), acc[i][0]);
+                                acc[i][1] = fma2(w23, make_float2(xv.z, xv.w), acc[i][1]);
+                            }
                         }
                     }
                 }
-            }
 #pragma unroll
-            for (int k = 0; k < ROUTE_TG; k++) {
-                // As route_dot_quad: the two 8-lane accumulators added lane-wise, then the hsum tree.
-                float v[4], sv[4];
+                for (int i = 0; i < TG; i++) {
+                    // The two 8-lane accumulators added lane-wise, then the hsum tree.
+                    const float lanes[4] = {acc[i][0].x, acc[i][0].y, acc[i][1].x, acc[i][1].y};
+                    float v[4], sv[4];
 #pragma unroll
-                for (int l = 0; l < 4; l++) v[l] = acc[k][l] + __shfl_xor_sync(0xffffffffu, acc[k][l], 2);
+                    for (int l = 0; l < 4; l++) v[l] = lanes[l] + __shfl_xor_sync(0xffffffffu, lanes[l], 2);
 #pragma unroll
-                for (int l = 0; l < 4; l++) sv[l] = v[l] + __shfl_xor_sync(0xffffffffu, v[l], 1);
-                float y = (sv[0] + sv[2]) + (sv[1] + sv[3]);
-                y = y + 0.0f;  // the dot's scalar tail is an empty sum
-                const int token = grp * ROUTE_TG + k;
-                if (valid && q == 0 && token < nt) {
-                    if (a.bias) y = y + a.bias[e];
-                    slog[token * experts + e] = y;
-                    if (a.logits) a.logits[size_t(t0 + token) * experts + e] = y;
+                    for (int l = 0; l < 4; l++) sv[l] = v[l] + __shfl_xor_sync(0xffffffffu, v[l], 1);
+                    float y = (sv[0] + sv[2]) + (sv[1] + sv[3]);
+                    y = y + 0.0f;  // the dot's scalar tail is an empty sum
+                    const int token = grp * TG + i;
+                    if (valid && q == 0 && token < nt) {
+                        if (a.bias) y = y + a.bias[e_lo + e];
+                        slog[token * lstride + e_lo + e] = y;
+                        if (a.logits) a.logits[size_t(t0 + token) * experts + e_lo + e] = y;
+                    }
                 }
             }
+            __syncthreads();
+            // The next part of the matrix, for this tile or the next one.
+            if (!once && (e_lo + stage_rows < experts || tile + int(gridDim.x) < tiles))
+                stage(e_lo + stage_rows < experts ? e_lo + stage_rows : 0);
         }
-        __syncthreads();
         if (warp < nt) {  // a warp per token: ranking and gates, then the row's 8-bit blocks
             const size_t token = size_t(t0 + warp);
-            route_topk_gates(slog + warp * experts, experts, topk, a.ids + token * topk, a.gates + token * topk, lane);
+            route_topk_gates(slog + warp * lstride, experts, topk, a.ids + token * topk, a.gates + token * topk, lane);
             route_quantize_padded_row(xrows + warp * rstride, hidden, a.xq + token * hidden, a.xs + token * padded,
                                       a.xsum + token * padded, lane);
         }
     }
-    if (a.stage_router && (!w_waited || !w_landed)) {
-        // Not waited for (a CTA without tiles) or not arrived in time: a last bounded chance for the
-        // copy to land before this shared memory is released; a late copy is reported.
-        const bool late = w_waited && !w_landed;
-        mbar_wait_bounded(&s_wbar, 0);
-        if (late && tid == 0) atomicExch(a.status, ERR_COPY_WAIT_TIMEOUT);
+    if (stagings == 0) mbar_wait_bounded(&s_wbar, 0);  // (a CTA without tiles: the copy lands before the memory is released)
+    if (!landed) {
+        // A copy was late: reported, with a last bounded chance to land.
+        mbar_wait_bounded(&s_wbar, (stagings - 1) & 1);
+        if (tid == 0) atomicExch(a.status, ERR_COPY_WAIT_TIMEOUT);
     }
 }
 
@@ -378,11 +390,14 @@ int launch_route(const MoeDims& d, const uint16_t* router, const float* bias, co
     } else {
         // Larger batches: CTAs that walk tiles, as many as stay resident (the staged router matrix is then
         // read a few hundred times, not once per token).
-        const int tg = t >= 8 * sms ? 4 : t >= 4 * sms ? 2 : 1, tile = 2 * tg;
+        int tg = t >= 8 * sms ? 4 : t >= 4 * sms ? 2 : 1;
+        const size_t wrow = 2 * size_t(d.hidden) + 32;
+        while (tg > 1 && route_tile_bytes(d.hidden, d.experts, 2 * tg) + 8 * wrow > ROUTE_SMEM_LIMIT) tg /= 2;
+        const int tile = 2 * tg;
         size_t tsmem = route_tile_bytes(d.hidden, d.experts, tile);
-        const size_t tstaged = tsmem + size_t(d.experts) * (2 * size_t(d.hidden) + 32);
-        a.stage_router = tstaged <= ROUTE_SMEM_LIMIT;
-        if (a.stage_router) tsmem = tstaged;
+        const int fit = int((ROUTE_SMEM_LIMIT - tsmem) / wrow), parts = (d.experts + fit - 1) / fit;
+        a.stage_rows = (d.experts + parts - 1) / parts;
+        tsmem += size_t(a.stage_rows) * wrow;
         const int per_sm = int(std::max<size_t>(1, std::min<size_t>(4, (220 * 1024) / (tsmem + 1024))));
         const int tiles = (t + tile - 1) / tile;
         launch_overlapped(tg == 4 ? route_tile_kernel<4> : tg == 2 ? route_tile_kernel<2> : route_tile_kernel<1>,

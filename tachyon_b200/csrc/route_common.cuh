@@ -198,67 +198,89 @@ __device__ __forceinline__ float exp_nonpositive_f64(float xf) {
     return float(__longlong_as_double(bits));
 }
 
-// Top-k and gates of one token, by ONE warp: lane l holds experts l, l+32, ...; after the
-// k rounds lane j < k holds the j-th pick and writes ids_row[j] / gates_row[j].
-__device__ __forceinline__ void route_topk_gates(const float* slog, int experts, int topk, uint32_t* ids_row,
+// Top-k and gates of one token, by ONE warp: lane l holds experts l, l+32, .... Up to 64 experts: each
+// lane ranks its experts against all keys (written over the logits, which are given up) and the picks are
+// scattered to their ranks; above, k rounds of taking the largest. Lane j < k ends with the j-th pick and
+// writes ids_row[j] / gates_row[j]. slog is 16-byte aligned and readable up to a multiple of 4 experts.
+__device__ __forceinline__ void route_topk_gates(float* slog, int experts, int topk, uint32_t* ids_row,
                                                  float* gates_row, int lane) {
-    constexpr int SLOTS = MAX_EXPERTS / 32;
-    const int nslots = (experts + 31) >> 5;
-    unsigned ukeys[SLOTS];  // order-preserving unsigned keys; 0 = not a candidate
-    unsigned taken = 0;
-#pragma unroll
-    for (int s = 0; s < SLOTS; s++) {
-        const int e = lane + 32 * s;
-        // total_key is a signed order; flipping the sign bit makes it unsigned. +1 keeps 0 free
-        // (the all-ones key, -NaN's neighbour in this order, cannot occur: it would be key 2^32).
-        ukeys[s] = (s < nslots && e < experts) ? (unsigned(total_key(slog[e])) ^ 0x80000000u) : 0u;
-        if (!(s < nslots && e < experts)) taken |= 1u << s;
-    }
     int my_id = 0;
     float my_val = 0.0f;
-    if (experts <= 32) {
-        // One expert per lane: each lane counts the experts that come before its own in the
-        // order (larger key first, lower index first among equals), all 32 comparisons
-        // independent of one another; the lane of rank j is the j-th pick. Same picks as the
-        // rounds below, without their chain of dependent steps.
-        const unsigned key = ukeys[0];
-        int rank = 0;
+    if (experts <= 64) {
+        // Larger key first, lower index first among equals: lane's experts `lane` and `lane + 32`.
+        int* skey = reinterpret_cast<int*>(slog);
+        const bool on0 = lane < experts, on1 = lane + 32 < experts;
+        const float val0 = on0 ? slog[lane] : 0.0f, val1 = on1 ? slog[lane + 32] : 0.0f;
+        const int key0 = total_key(val0), key1 = total_key(val1);
+        __syncwarp();
+        if (on0) skey[lane] = key0;
+        if (on1) skey[lane + 32] = key1;
+        __syncwarp();
+        const unsigned below = (1u << lane) - 1u;
+        int rank0 = __popc(__match_any_sync(0xffffffffu, key0) & __ballot_sync(0xffffffffu, on0) & below);
+        int rank1 = __popc(__match_any_sync(0xffffffffu, key1) & __ballot_sync(0xffffffffu, on1) & below);
 #pragma unroll
-        for (int j = 0; j < 32; j++) {
-            const unsigned kj = __shfl_sync(0xffffffffu, key, j);
-            rank += (j < experts && (kj > key || (kj == key && j < lane))) ? 1 : 0;
+        for (int j = 0; j < 64; j += 4) {
+            if (j < experts) {
+                const int4 k4 = *reinterpret_cast<const int4*>(skey + j);
+                const int kk[4] = {k4.x, k4.y, k4.z, k4.w};
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    if (j + i < experts) {
+                        rank0 += kk[i] > key0 ? 1 : 0;                           // (equals among 0..31: counted above; 32.. come after)
+                        if (experts > 32) rank1 += (j + i < 32 ? kk[i] >= key1 : kk[i] > key1) ? 1 : 0;
+                    }
+                }
+            }
         }
-        if (lane >= experts) rank = 0x7fffffff;
+        __syncwarp();
+        // The picks to their ranks: ids over the first words, scores behind them (topk <= 32, and the row
+        // has experts >= topk words; with fewer than 2 topk words the scores follow in a second step).
+        if (on0 && rank0 < topk) skey[rank0] = lane;
+        if (on1 && rank1 < topk) skey[rank1] = lane + 32;
+        __syncwarp();
+        if (lane < topk) my_id = skey[lane];
+        __syncwarp();
+        if (on0 && rank0 < topk) slog[rank0] = val0;
+        if (on1 && rank1 < topk) slog[rank1] = val1;
+        __syncwarp();
+        if (lane < topk) my_val = slog[lane];
+    } else {
+        constexpr int SLOTS = MAX_EXPERTS / 32;
+        const int nslots = (experts + 31) >> 5;
+        unsigned ukeys[SLOTS];  // order-preserving unsigned keys; 0 = not a candidate
+        unsigned taken = 0;
+    #pragma unroll
+        for (int s = 0; s < SLOTS; s++) {
+            const int e = lane + 32 * s;
+            // total_key is a signed order; flipping the sign bit makes it unsigned. +1 keeps 0 free
+            // (the all-ones key, -NaN's neighbour in this order, cannot occur: it would be key 2^32).
+            ukeys[s] = (s < nslots && e < experts) ? (unsigned(total_key(slog[e])) ^ 0x80000000u) : 0u;
+            if (!(s < nslots && e < experts)) taken |= 1u << s;
+        }
         for (int j = 0; j < topk; j++) {
-            const int win = __ffs(__ballot_sync(0xffffffffu, rank == j)) - 1;
+            unsigned best_key = 0;
+            int best_idx = 0x7fffffff;
+    #pragma unroll
+            for (int s = 0; s < SLOTS; s++) {
+                if (s < nslots && !((taken >> s) & 1u)) {
+                    if (best_idx == 0x7fffffff || ukeys[s] > best_key) {
+                        best_key = ukeys[s];
+                        best_idx = lane + 32 * s;
+                    }
+                }
+            }
+            // The largest key in the warp, then the lowest expert index among its holders.
+            const bool have = best_idx != 0x7fffffff;
+            const unsigned wmax = __reduce_max_sync(0xffffffffu, have ? best_key : 0u);
+            const bool tie = have && best_key == wmax;
+            const unsigned widx = __reduce_min_sync(0xffffffffu, tie ? unsigned(best_idx) : 0xffffffffu);
+            const int win = int(widx);
+            if ((win & 31) == lane) taken |= 1u << (win >> 5);
             if (lane == j) {
                 my_id = win;
                 my_val = slog[win];
             }
-        }
-    } else
-    for (int j = 0; j < topk; j++) {
-        unsigned best_key = 0;
-        int best_idx = 0x7fffffff;
-#pragma unroll
-        for (int s = 0; s < SLOTS; s++) {
-            if (s < nslots && !((taken >> s) & 1u)) {
-                if (best_idx == 0x7fffffff || ukeys[s] > best_key) {
-                    best_key = ukeys[s];
-                    best_idx = lane + 32 * s;
-                }
-            }
-        }
-        // The largest key in the warp, then the lowest expert index among its holders.
-        const bool have = best_idx != 0x7fffffff;
-        const unsigned wmax = __reduce_max_sync(0xffffffffu, have ? best_key : 0u);
-        const bool tie = have && best_key == wmax;
-        const unsigned widx = __reduce_min_sync(0xffffffffu, tie ? unsigned(best_idx) : 0xffffffffu);
-        const int win = int(widx);
-        if ((win & 31) == lane) taken |= 1u << (win >> 5);
-        if (lane == j) {
-            my_id = win;
-            my_val = slog[win];
         }
     }
     const float mx = __shfl_sync(0xffffffffu, my_val, 0);
