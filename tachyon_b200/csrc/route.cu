@@ -164,21 +164,27 @@ __global__ void __launch_bounds__(ROUTE_THREADS) route_kernel(const RouteArgs a)
     }
 }
 
-// Prefill-size batches: a CTA takes a tile of 2 * TG tokens at a time (walking tiles blockIdx.x,
+// Prefill-size batches: a CTA takes a tile of TILE tokens at a time (walking tiles blockIdx.x,
 // blockIdx.x + gridDim.x, ...): a warp per token for the norm, the ranking and the quantization,
-// four threads per (expert, group of TG tokens) for the logits, with the router matrix staged once
-// per CTA. Same arithmetic per token as route_kernel. TG = 4 keeps every warp busy and reads the router
-// matrix least; batches that would then leave SMs without a tile take TG = 2 or 1 (333 tokens of the 1b
-// shape: 42 tiles of 8, 167 of 2).
+// four threads per (TG tokens, ROUTE_TE experts) for the logits, with the router matrix staged once
+// per CTA. Same arithmetic per token as route_kernel.
+//
+// Bound by the shared-memory reads and the latency of a tile's chain (load, norm, logits, ranking). A
+// thread's 2 tokens x 2 experts take four reads for four products and keep all eight warps of a CTA busy;
+// measured for the whole stage at 4096 tokens of the 1b shape / of 2048 columns and 64 experts: 4 x 1 54 us /
+// 154 us, 2 x 2 52 / 148, 4 x 2 52 / 166, 2 x 4 57 / 153 (half the warps idle); 4 x 1 with 512 threads 70 /
+// 158. TILE = 8 lets two CTAs share an SM; batches that would then leave SMs without a tile take 4 or 2 (333
+// tokens of the 1b shape: 42 tiles of 8, 167 of 2).
+constexpr int ROUTE_TE = 2;
 
 // Shared memory of the tile kernel before the staged router matrix: padded rows, logits, norm weight.
 __host__ __device__ inline size_t route_tile_bytes(int hidden, int experts, int tile) {
     return (size_t(tile) * (hidden / QK * ROW_PAD_BLOCK + (experts + 3) / 4 * 4) * 4 + size_t(hidden) * 4 + 127) / 128 * 128;
 }
 
-template <int TG>
+template <int TILE>
 __global__ void __launch_bounds__(ROUTE_THREADS) route_tile_kernel(const RouteArgs a) {
-    constexpr int TILE = 2 * TG;
+    constexpr int TG = TILE > 2 ? 2 : 1, TE = ROUTE_TE;
     extern __shared__ __align__(128) float smem[];
     const int hidden = a.hidden, experts = a.experts, topk = a.topk;
     const int rstride = hidden / QK * ROW_PAD_BLOCK;  // floats per padded row
@@ -255,56 +261,65 @@ __global__ void __launch_bounds__(ROUTE_THREADS) route_tile_kernel(const RouteAr
                 stagings++;
             }
             if (e_lo == 0) __syncthreads();  // the normed rows are complete
-            // Logits: four threads per (expert, group of TG tokens): the expert's row is read from
-            // shared memory once for the group's tokens (the row reads, distinct per expert, are what
-            // the shared-memory pipe is busy with; the tokens' reads are broadcasts). Each (token,
-            // expert) logit keeps its own accumulators, as route_dot_quad: thread q of a quad has elements
-            // 16 j + 4 q .. + 3. (Rows past the tile's tokens hold anything; their logits are not stored.)
-            const int n_e = min(stage_rows, experts - e_lo);
-            const int groups = (nt + TG - 1) / TG, tasks = groups * n_e;
+            // Logits. Each (token, expert) keeps its own accumulators, as route_dot_quad: thread q of a quad has
+            // elements 16 j + 4 q .. + 3. (Rows past the tile's tokens hold anything and experts past the
+            // last repeat it; those logits are not stored.)
+            const int n_e = min(stage_rows, experts - e_lo), egroups = (n_e + TE - 1) / TE;
+            const int tasks = (nt + TG - 1) / TG * egroups;
             for (int p0 = 0; p0 < tasks; p0 += ROUTE_THREADS / 4) {
                 const int p = p0 + (tid >> 2), q = tid & 3;
+                if (p0 + ((tid >> 5) << 3) >= tasks) continue;  // (a warp without work)
                 const bool valid = p < tasks;
-                const int grp = valid ? p / n_e : 0, e = valid ? p - grp * n_e : 0;
-                float2 acc[TG][2];
+                const int grp = valid ? p / egroups : 0, e0 = valid ? (p - grp * egroups) * TE : 0;
+                float2 acc[TG][TE][2];
 #pragma unroll
-                for (int i = 0; i < TG; i++) acc[i][0] = acc[i][1] = make_float2(0.0f, 0.0f);
-                if (p0 + ((tid >> 5) << 3) < tasks) {  // (a warp without work skips the loop)
-                    const uint8_t* ws = wsm + size_t(e) * wstride + q * 8;
-                    const float* xr = xrows + size_t(grp * TG) * rstride + q * 4;
+                for (int i = 0; i < TG; i++)
+#pragma unroll
+                    for (int j = 0; j < TE; j++) acc[i][j][0] = acc[i][j][1] = make_float2(0.0f, 0.0f);
+                const uint8_t* ws[TE];
+#pragma unroll
+                for (int j = 0; j < TE; j++) ws[j] = wsm + size_t(min(e0 + j, n_e - 1)) * wstride + q * 8;
+                const float* xr = xrows + size_t(grp * TG) * rstride + q * 4;
 #pragma unroll 2
-                    for (int blk = 0; blk < hidden / QK; blk++, ws += 2 * QK, xr += ROW_PAD_BLOCK) {
+                for (int blk = 0; blk < hidden / QK; blk++) {
 #pragma unroll
-                        for (int h = 0; h < 2; h++) {
-                            const uint2 wv = *reinterpret_cast<const uint2*>(ws + 32 * h);
+                    for (int h = 0; h < 2; h++) {
+                        float4 xv[TG];
+#pragma unroll
+                        for (int i = 0; i < TG; i++)
+                            xv[i] = *reinterpret_cast<const float4*>(xr + i * rstride + blk * ROW_PAD_BLOCK + 16 * h);
+#pragma unroll
+                        for (int j = 0; j < TE; j++) {
+                            const uint2 wv = *reinterpret_cast<const uint2*>(ws[j] + blk * 2 * QK + 32 * h);
                             const float2 w01 = make_float2(bf16_lo(wv.x), bf16_hi(wv.x)), w23 = make_float2(bf16_lo(wv.y), bf16_hi(wv.y));
 #pragma unroll
                             for (int i = 0; i < TG; i++) {
-                                const float4 xv = *reinterpret_cast<const float4*>(xr + i * rstride + 16 * h);
-                                acc[i][0] = fma2(w01, make_float2(xv.x, xv.y), acc[i][0]);
-                                acc[i][1] = fma2(w23, make_float2(xv.z, xv.w), acc[i][1]);
+                                acc[i][j][0] = fma2(w01, make_float2(xv[i].x, xv[i].y), acc[i][j][0]);
+                                acc[i][j][1] = fma2(w23, make_float2(xv[i].z, xv[i].w), acc[i][j][1]);
                             }
                         }
                     }
                 }
 #pragma unroll
-                for (int i = 0; i < TG; i++) {
-                    // The two 8-lane accumulators added lane-wise, then the hsum tree.
-                    const float lanes[4] = {acc[i][0].x, acc[i][0].y, acc[i][1].x, acc[i][1].y};
-                    float v[4], sv[4];
+                for (int i = 0; i < TG; i++)
 #pragma unroll
-                    for (int l = 0; l < 4; l++) v[l] = lanes[l] + __shfl_xor_sync(0xffffffffu, lanes[l], 2);
+                    for (int j = 0; j < TE; j++) {
+                        // The two 8-lane accumulators added lane-wise, then the hsum tree.
+                        const float lanes[4] = {acc[i][j][0].x, acc[i][j][0].y, acc[i][j][1].x, acc[i][j][1].y};
+                        float v[4], sv[4];
 #pragma unroll
-                    for (int l = 0; l < 4; l++) sv[l] = v[l] + __shfl_xor_sync(0xffffffffu, v[l], 1);
-                    float y = (sv[0] + sv[2]) + (sv[1] + sv[3]);
-                    y = y + 0.0f;  // the dot's scalar tail is an empty sum
-                    const int token = grp * TG + i;
-                    if (valid && q == 0 && token < nt) {
-                        if (a.bias) y = y + a.bias[e_lo + e];
-                        slog[token * lstride + e_lo + e] = y;
-                        if (a.logits) a.logits[size_t(t0 + token) * experts + e_lo + e] = y;
+                        for (int l = 0; l < 4; l++) v[l] = lanes[l] + __shfl_xor_sync(0xffffffffu, lanes[l], 2);
+#pragma unroll
+                        for (int l = 0; l < 4; l++) sv[l] = v[l] + __shfl_xor_sync(0xffffffffu, v[l], 1);
+                        float y = (sv[0] + sv[2]) + (sv[1] + sv[3]);
+                        y = y + 0.0f;  // the dot's scalar tail is an empty sum
+                        const int token = grp * TG + i, e = e_lo + e0 + j;
+                        if (valid && q == 0 && token < nt && e0 + j < n_e) {
+                            if (a.bias) y = y + a.bias[e];
+                            slog[token * lstride + e] = y;
+                            if (a.logits) a.logits[size_t(t0 + token) * experts + e] = y;
+                        }
                     }
-                }
             }
             __syncthreads();
             // The next part of the matrix, for this tile or the next one.
@@ -344,9 +359,9 @@ __global__ void rmsnorm_kernel(const float* x, const float* __restrict__ w, floa
 
 void init_kernels_route() {
     cudaFuncSetAttribute(route_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ROUTE_SMEM_LIMIT));
+    cudaFuncSetAttribute(route_tile_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ROUTE_SMEM_LIMIT));
     cudaFuncSetAttribute(route_tile_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ROUTE_SMEM_LIMIT));
     cudaFuncSetAttribute(route_tile_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ROUTE_SMEM_LIMIT));
-    cudaFuncSetAttribute(route_tile_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ROUTE_SMEM_LIMIT));
 }
 
 int launch_route(const MoeDims& d, const uint16_t* router, const float* bias, const float* x,
@@ -390,17 +405,16 @@ int launch_route(const MoeDims& d, const uint16_t* router, const float* bias, co
     } else {
         // Larger batches: CTAs that walk tiles, as many as stay resident (the staged router matrix is then
         // read a few hundred times, not once per token).
-        int tg = t >= 8 * sms ? 4 : t >= 4 * sms ? 2 : 1;
         const size_t wrow = 2 * size_t(d.hidden) + 32;
-        while (tg > 1 && route_tile_bytes(d.hidden, d.experts, 2 * tg) + 8 * wrow > ROUTE_SMEM_LIMIT) tg /= 2;
-        const int tile = 2 * tg;
+        int tile = t >= 8 * sms ? 8 : t >= 4 * sms ? 4 : 2;
+        while (tile > 2 && route_tile_bytes(d.hidden, d.experts, tile) + 8 * wrow > ROUTE_SMEM_LIMIT) tile /= 2;
         size_t tsmem = route_tile_bytes(d.hidden, d.experts, tile);
         const int fit = int((ROUTE_SMEM_LIMIT - tsmem) / wrow), parts = (d.experts + fit - 1) / fit;
         a.stage_rows = (d.experts + parts - 1) / parts;
         tsmem += size_t(a.stage_rows) * wrow;
         const int per_sm = int(std::max<size_t>(1, std::min<size_t>(4, (220 * 1024) / (tsmem + 1024))));
         const int tiles = (t + tile - 1) / tile;
-        launch_overlapped(tg == 4 ? route_tile_kernel<4> : tg == 2 ? route_tile_kernel<2> : route_tile_kernel<1>,
+        launch_overlapped(tile == 8 ? route_tile_kernel<8> : tile == 4 ? route_tile_kernel<4> : route_tile_kernel<2>,
                           dim3(std::min(tiles, per_sm * sms)), dim3(ROUTE_THREADS), tsmem, stream, a);
     }
     int launched = 1;
