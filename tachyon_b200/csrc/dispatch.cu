@@ -21,8 +21,6 @@
 // which the expert kernels cut into equal shares.
 #include <atomic>
 
-#include <atomic>
-
 #include "dispatch_common.cuh"
 
 namespace tc {
@@ -116,8 +114,8 @@ namespace {
 // experts, so a CTA that counts the ids below e and those equal to e as it reads them needs nothing from the
 // others. A warp owns a contiguous range of the slots (read twice: count, then place), which keeps the
 // order. The last CTA to finish lists the experts that have tokens and, when asked, cuts the token tiles.
-// (Three passes with a histogram per 256 tokens took 26 us for 4096 tokens of 8 picks, most of it
-// launches and a serial scan; every CTA reading all ids, 128 KB from L2, takes 6.)
+// (Three passes with a histogram per 256 tokens, most of it launches and a serial scan, against every CTA
+// reading all ids, 128 KB from L2: router and dispatch of 4096 tokens of the 1b shape 68 to 58 us.)
 constexpr int DISPATCH_E_THREADS = 1024;
 constexpr int DISPATCH_E_WARPS = DISPATCH_E_THREADS / 32;
 

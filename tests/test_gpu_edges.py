@@ -1,0 +1,49 @@
+"""The edges of the kernels' tiles and of the rules that choose a variant: one token more or less than a tile, an
+odd number of 32-value blocks per row, router matrices that fit on chip or not, more experts than a warp ranks at
+once, experts without a token; a call over host buffers on both sides of its rule. Against the oracle."""
+import numpy as np
+import pytest
+
+from tachyon_b200 import synth, workloads
+from tachyon_b200.workloads import MoeShape
+from test_gpu_parity import check_block, ctx, layer_weights, make_layer, oracle_moe  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+ODD_Q8 = MoeShape("odd-q8", 288, 8, 2, 160, fmt="q8")        # 9 and 5 blocks per row; rows end inside a tile of 128
+ODD_Q4 = MoeShape("odd-q4", 288, 8, 2, 160, fmt="q4")
+ONE_BLOCK = MoeShape("one-block", 32, 3, 1, 32, fmt="q8")    # one block per row, one pick
+ODD_EXPERTS = MoeShape("experts-37", 96, 37, 5, 32, fmt="q8")
+PAST_64 = MoeShape("experts-65", 64, 65, 8, 32, fmt="q8")    # one expert more than two per lane
+WIDE = MoeShape("wide-router", 2048, 64, 8, 32, fmt="q4")    # 256 KB of router matrix: staged in parts
+
+
+@pytest.mark.parametrize("shape,t,skewed", [
+    # One kernel per block: a token, an odd few, and both sides of 32 tokens and of the largest batch.
+    (ODD_Q4, 1, False), (ODD_EXPERTS, 3, False), (PAST_64, 31, True), (ONE_BLOCK, 33, False), (WIDE, 127, True),
+    (ODD_Q8, 129, False),
+    # Tensor-core tiles: whole ones, one token past them, experts with hardly any.
+    (ODD_Q8, 256, False), (ODD_Q4, 257, False), (ODD_Q8, 1025, True), (ODD_Q4, 770, True), (ONE_BLOCK, 193, False),
+    # Router tiles of 2, 4 and 8 tokens, each with a remainder; the dispatch past one CTA's batch.
+    (ODD_EXPERTS, 257, False), (ODD_EXPERTS, 595, False), (ODD_EXPERTS, 1187, True), (PAST_64, 1191, True),
+    (WIDE, 259, False), (WIDE, 597, True), (WIDE, 1189, False), (ONE_BLOCK, 2049, False),
+], ids=lambda v: v.name if isinstance(v, MoeShape) else str(v))
+def test_blocks_at_the_edges(oracle, ctx, shape, t, skewed):
+    lw = layer_weights(oracle, shape, 17)
+    bias = synth.zipf_router_bias(17, shape.experts) if skewed else None
+    check_block(oracle, ctx, shape, lw, workloads.hidden_states(shape, t, seed=t), bias=bias, arith="fast")
+
+
+@pytest.mark.parametrize("t", [1, 128, 129])
+def test_host_buffers_at_the_edges(oracle, ctx, t):
+    lw = layer_weights(oracle, ODD_Q8, 17)
+    x = workloads.hidden_states(ODD_Q8, t, seed=t)
+    y = np.ones_like(x)
+    ctx.set_arithmetic(ctx.ARITH_FAST)
+    layer = make_layer(ctx, lw, ODD_Q8.topk, t)
+    try:
+        layer.forward_host(x, y)
+    finally:
+        layer.free()
+    want = 1.0 + oracle_moe(oracle, lw, x, ODD_Q8.topk).proj
+    assert np.abs(y - want).max() <= 2e-3
