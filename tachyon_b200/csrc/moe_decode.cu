@@ -409,9 +409,8 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
         }
         if (pass == 1) break;
         if (a.l2_all) {
-            // Which records a warp needs is only known after the router phase (expert parallel, or a
-            // batch small enough to walk only the picked experts), but most experts will be picked:
-            // all of this GPU's share of the layer is asked into L2 now (every CTA a slice), and the
+            // Which records a warp needs is only known after the router phase, but most experts will be
+            // picked: all of this GPU's share of the layer is asked into L2 now (every CTA a slice), and the
             // copies into shared memory that follow the router phase find it there.
             const Phase* Ps[2] = {&P0, &P1};
 #pragma unroll
@@ -1092,10 +1091,11 @@ int launch_decode_block(const MoeDims& d, int kind, const uint16_t* router, cons
     a.gu_tiled = gate_up_tiled, a.dn_tiled = down_tiled;
     a.hidden_f = ep ? hidden_f_all : ws.hidden_f, a.out = ws.out;
     a.dense = !ep && dense_walk(d, t) ? 1 : 0;
-    // (For a sparse walk on one GPU, batches of 3 to 15 tokens, the same request made the step
-    // slower, 1.06 ms against 0.86 at 8 tokens: 53 MB of requests are still in the way of the
-    // picked experts' records when the router phase ends.)
-    a.l2_all = ep && (long long)ep->ranks * t * d.topk >= 4LL * d.experts;
+    // Between GPUs the exchange of the rows takes long enough to bring a rank's share of the layer into L2.
+    // On one GPU the requests are in the way of the router matrix and the rows: a block of 64 tokens of
+    // the 1b shape took 44.8 us with them and 41.4 without, 100 tokens of the 3b shape 74.6 and 60.5.
+    // (A sparse walk, too: the 1b model's step at 8 tokens 1.06 ms against 0.86.)
+    a.l2_all = ep && ep->ranks > 1 && (long long)ep->ranks * t * d.topk >= 4LL * d.experts;
     if (ep) a.ep = *ep;
     a.ids_slots = (ep ? ep->ranks : 1) * t * d.topk;
     a.sync = ws.grid_sync;
