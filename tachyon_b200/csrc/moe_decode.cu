@@ -200,14 +200,17 @@ struct Phase {
     int first, n;      // this warp's first unit and how many it owns (stride nwarps)
 };
 
-__device__ __forceinline__ void arrive_on_peer(uint32_t* flag) {
-    asm volatile("red.release.sys.global.add.u32 [%0], 1;" ::"l"(flag) : "memory");
+// (With one rank every counter is this GPU's own, and its scope is enough.)
+__device__ __forceinline__ void arrive_on_peer(uint32_t* flag, bool alone) {
+    if (alone) grid_arrive(flag);
+    else asm volatile("red.release.sys.global.add.u32 [%0], 1;" ::"l"(flag) : "memory");
 }
 // One thread: waits until the counter (written by other GPUs) has reached target, wrap-safe.
-__device__ __forceinline__ bool peer_count_wait(const uint32_t* ctr, uint32_t target, uint32_t limit) {
+__device__ __forceinline__ bool peer_count_wait(const uint32_t* ctr, uint32_t target, uint32_t limit, bool alone) {
     for (uint32_t i = 0; i < limit; i++) {
         uint32_t seen;
-        asm volatile("ld.acquire.sys.global.u32 %0, [%1];" : "=r"(seen) : "l"(ctr) : "memory");
+        if (alone) seen = ld_acquire(ctr);
+        else asm volatile("ld.acquire.sys.global.u32 %0, [%1];" : "=r"(seen) : "l"(ctr) : "memory");
         if (int32_t(seen - target) >= 0) return true;
         __nanosleep(i < 64 ? 32 : 256);
     }
@@ -241,6 +244,7 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
     const int t = a.t, hidden = a.hidden, experts = a.experts, topk = a.topk, inter = a.inter;
     // Expert parallel: the expert phases see every rank's tokens (gathered in this rank's window).
     const int ranks = EP ? a.ep.ranks : 1, own = EP ? a.ep.me * t : 0;  // own: this rank's first token among all
+    const bool alone = ranks == 1;  // nothing crosses a link
     const int slots = ranks * t * topk;
     uint8_t* window = EP ? a.ep.base[a.ep.me] : nullptr;
     const int8_t* xq_all = EP ? reinterpret_cast<const int8_t*>(window + a.ep.off_xq) : a.xq;
@@ -441,6 +445,11 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
         }
         grid_dependency_wait();  // everything below reads or writes what other kernels touch
         if (stamping) a.stamps[1] = wall_clock_ns();
+        if (EP) {
+            epoch0 = a.ep.epoch[0];
+            routed0 = a.ep.epoch[1];
+            for (int e = tid; e < a.ep.local; e += nthreads) s_cnt[e] = 0;
+        }
 
         // ---- router phase, part two
         if (routing) {
@@ -478,13 +487,15 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
                 __syncthreads();  // the staged rows are no longer read; slog is complete up to here
             }
             // The picks by the first warps (a thread per expert), the row's quantization by the others.
-            route_rank_picks(skey, slog, experts, topk, EP ? nullptr : a.ids + size_t(bid) * topk, s_rids, s_rval, tid);
+            route_rank_picks(skey, slog, experts, topk, alone ? const_cast<uint32_t*>(ids_all) + size_t(bid) * topk : nullptr, s_rids, s_rval, tid);
             const int rank_warps = (experts + 31) >> 5, qfirst = rank_warps < nwarps ? rank_warps : 0;
-            if (!EP) {
-                route_quantize_row(xrow, hidden, a.xq + size_t(bid) * hidden, a.xs + size_t(bid) * P0.nbp,
-                                   a.xsum + size_t(bid) * P0.nbp, warp, lane, qfirst, nwarps - qfirst);
+            if (alone) {
+                route_quantize_row(xrow, hidden, const_cast<int8_t*>(xq_all) + size_t(bid) * hidden,
+                                   const_cast<float*>(xs_all) + size_t(bid) * P0.nbp,
+                                   const_cast<float*>(xsum_all) + size_t(bid) * P0.nbp, warp, lane, qfirst, nwarps - qfirst);
                 __syncthreads();
-                if (tid == 0) grid_arrive(a.sync + 0);
+                if (tid == 0 && !(EP && a.ep.mute))
+                    grid_arrive(EP ? reinterpret_cast<uint32_t*>(window + a.ep.off_flags) + DECODE_EP_FLAG_ROUTE : a.sync + 0);
             } else {
                 // The row is quantized into shared memory (where the router matrix was), then stored
                 // into every rank's window, this rank's included, and announced there.
@@ -509,10 +520,9 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
                     else
                         reinterpret_cast<uint32_t*>(w + a.ep.off_ids)[g * topk + (j - vq - 2 * vs)] = s_rids[j - vq - 2 * vs];
                 }
-                if (tid < topk) a.ids[size_t(bid) * topk + tid] = s_rids[tid];  // (the routing taps read these)
                 __syncthreads();
                 if (tid < ranks && !a.ep.mute)
-                    arrive_on_peer(reinterpret_cast<uint32_t*>(a.ep.base[tid] + a.ep.off_flags) + DECODE_EP_FLAG_ROUTE);
+                    arrive_on_peer(reinterpret_cast<uint32_t*>(a.ep.base[tid] + a.ep.off_flags) + DECODE_EP_FLAG_ROUTE, false);
             }
             // The gates, and the order the combine adds the picks in (ascending expert): wanted by this
             // CTA's combine only, so they are worked out behind the arrival.
@@ -523,15 +533,14 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
                     const uint32_t mine = s_rids[lane];
                     int rank = 0;
                     for (int j = 0; j < topk; j++) rank += s_rids[j] < mine ? 1 : 0;
+                    if (EP) a.ids[size_t(bid) * topk + lane] = mine;  // (the routing taps read these)
                     s_cpos[rank] = uint32_t(bid * topk + lane);
                     s_cgate[rank] = gate;
                 }
             }
         }
         if (EP) {
-            epoch0 = a.ep.epoch[0];
-            routed0 = a.ep.epoch[1];
-            if (tid == 0 && !peer_count_wait(flags + DECODE_EP_FLAG_ROUTE, routed0 + uint32_t(ranks * t), a.spin_limit))
+            if (tid == 0 && !peer_count_wait(flags + DECODE_EP_FLAG_ROUTE, routed0 + uint32_t(ranks * t), a.spin_limit, alone))
                 s_abort = 4;
         } else if (tid == 0 && !grid_wait(a.sync + 0, uint32_t(t), a.spin_limit)) {
             s_abort = 1;
@@ -572,19 +581,15 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
                 start_stream(unsigned(__popc(m0) + __popc(m1)));
             } else {
 #pragma unroll 1
-                for (int i = tid; i < slots; i += nthreads) s_ids[i] = __ldcg(ids_all + i);
+                for (int i = tid; i < slots; i += nthreads) {
+                    const uint32_t id = __ldcg(ids_all + i);
+                    s_ids[i] = id;
+                    if (EP && id - uint32_t(a.ep.first) < uint32_t(a.ep.local)) atomicAdd(&s_cnt[id - uint32_t(a.ep.first)], 1u);
+                }
             }
             if (EP) {
                 // Runs: each local expert's slots in pieces of up to D_TOK; (run, unit) pairs are what the
                 // CTAs and warps share out, so an expert with many tokens spreads over many warps.
-#pragma unroll 1
-                for (int e = tid; e < a.ep.local; e += nthreads) s_cnt[e] = 0;
-                __syncthreads();
-#pragma unroll 1
-                for (int i = tid; i < slots; i += nthreads) {
-                    const uint32_t e = s_ids[i] - uint32_t(a.ep.first);
-                    if (e < uint32_t(a.ep.local)) atomicAdd(&s_cnt[e], 1u);
-                }
                 __syncthreads();
                 if (warp == 0) {
                     // Run length 32, 16 or 8: the one with the least work on the busiest warp. A run's
@@ -598,14 +603,11 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
 #pragma unroll
                         for (int k = 0; k < 3; k++) runs[k] += (c + (D_TOK >> k) - 1) / (D_TOK >> k);
                     }
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
+                    most = __reduce_max_sync(0xffffffffu, most);
                     int run_len = D_TOK, best = 0x7fffffff;
 #pragma unroll
                     for (int k = 0; k < 3; k++) {
-#pragma unroll
-                        for (int o = 16; o > 0; o >>= 1) runs[k] += __shfl_xor_sync(0xffffffffu, runs[k], o);
-                        const int len = D_TOK >> k, r = max(1, runs[k]);
+                        const int len = D_TOK >> k, r = max(1, __reduce_add_sync(0xffffffffu, runs[k]));
                         const unsigned ctas = r <= nctas ? div_small(nctas, r) : 1u;
                         const int per_cta = int(r <= nctas ? div_small(P0.upe + ctas - 1, ctas) : div_small(r * P0.upe + nctas - 1, nctas));
                         const int cost = int(div_small(per_cta + uwarps - 1, uwarps)) * (3 + (min(len, most) + 7) / 8);
@@ -616,7 +618,7 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
 #pragma unroll 1
                     for (int e0 = 0; e0 < a.ep.local; e0 += 32) {
                         const int e = e0 + lane;
-                        const int mine = e < a.ep.local ? (int(s_cnt[e]) + run_len - 1) / run_len : 0;
+                        const int mine = e < a.ep.local ? int(div_small(s_cnt[e] + run_len - 1, run_len)) : 0;
                         int before = mine;
 #pragma unroll
                         for (int o = 1; o < 32; o <<= 1) {
@@ -938,7 +940,7 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
         arrived = p + 1;
         if (EP && p == 1) {
             if (tid < ranks)
-                arrive_on_peer(reinterpret_cast<uint32_t*>(a.ep.base[tid] + a.ep.off_flags) + DECODE_EP_FLAG_DOWN);
+                arrive_on_peer(reinterpret_cast<uint32_t*>(a.ep.base[tid] + a.ep.off_flags) + DECODE_EP_FLAG_DOWN, alone);
         } else if (tid == 0) {
             grid_arrive(a.sync + 1 + p);
         }
@@ -952,7 +954,7 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
         if (tid * 4 < hidden) y_ahead = *reinterpret_cast<const float4*>(a.y + size_t(bid) * hidden + tid * 4);
         if (tid == 0) {
             const bool came = EP ? peer_count_wait(flags + DECODE_EP_FLAG_DOWN, (epoch0 + 1u) * uint32_t(ranks * nctas),
-                                                   a.spin_limit)
+                                                   a.spin_limit, alone)
                                  : grid_wait(a.sync + 2, uint32_t(nctas), a.spin_limit);
             if (!came) s_abort = EP ? 4 : 2;
         }
