@@ -68,7 +68,8 @@ constexpr int D_TOK = 8 * D_GMAX;  // tokens per block this kernel takes; rows s
 constexpr int D_NORM_HELD = 8;     // elements of the norm's weight a thread holds (rows of up to 8 x 256 floats)
 constexpr int D_ROUTE_VEC = 10;    // 16-byte pieces of the router matrix a thread holds at a time
 constexpr int D_NSEG = 4;          // experts of a CTA's range whose slot lists are held at a time
-constexpr size_t D_SMEM_LIMIT = 227 * 1024 - 3584;  // dynamic part: the kernel also has up to 3.2 KB of static shared memory
+// Dynamic part: the kernel also has 1.4 KB of static shared memory, 3.2 KB in the expert-parallel form.
+__host__ __device__ constexpr size_t decode_smem_limit(bool ep) { return 227 * 1024 - (ep ? 3584 : 1536); }
 
 constexpr int DECODE_EP_FLAG_ROUTE = 16, DECODE_EP_FLAG_DOWN = 17;  // words of the window's flag area
 
@@ -95,6 +96,7 @@ struct DecodeArgs {
     int unit_warps;           // warps with a ring: as many as a CTA can have units, all of them if it can have more
     int stages, xcap;         // ring depth per warp; staged rows at a time (a multiple of 8, at most D_TOK)
     int route_rows;           // rows of the router matrix staged at a time in the router phase
+    int route_in_ring;        // ... all of them, where the ring will be: nothing streams before the picks are known
     int l2_all;               // ask all of this GPU's expert records into L2 before the router phase
     int dense;
     uint32_t* sync;           // [GRID_SYNC_WORDS], zero between launches
@@ -139,7 +141,7 @@ struct DLayout {
         o += D_NSEG * D_TOK * 2 * 2;
         o = (o + 15) / 16 * 16;
         bars = o;
-        o += D_MAX_WARPS * D_MAX_STAGES * 8;
+        o += D_MAX_WARPS * stages * 8;
         total = o;
     }
 };
@@ -255,9 +257,9 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
     const uint32_t* flags = EP ? reinterpret_cast<const uint32_t*>(window + a.ep.off_flags) : nullptr;
     uint32_t epoch0 = 0;  // EP: blocks completed before this one
     uint32_t routed0 = 0; // EP: router-phase arrivals of those blocks (ranks x tokens each; the batch size may change)
-    const DLayout<KIND> L(uwarps, STAGES, a.xcap, a.route_rows, hidden, inter, experts, topk, a.ids_slots);
+    const DLayout<KIND> L(uwarps, STAGES, a.xcap, a.route_in_ring ? 0 : a.route_rows, hidden, inter, experts, topk, a.ids_slots);
     uint8_t* ring = smem + L.ring + size_t(min(warp, uwarps - 1)) * STAGES * R::BYTES;  // (a warp without units uses none)
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L.bars) + warp * D_MAX_STAGES;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L.bars) + warp * STAGES;
     uint32_t* s_ids = reinterpret_cast<uint32_t*>(smem + L.ids);
     uint16_t* s_slot = reinterpret_cast<uint16_t*>(smem + L.lists);  // [D_NSEG][D_TOK] slots that named the segment's expert
     uint16_t* s_tok = s_slot + D_NSEG * D_TOK;                        // the same slots' tokens
@@ -368,13 +370,14 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
     float* slog = xrow + hidden;
     int* skey = reinterpret_cast<int*>(slog + (experts + 3) / 4 * 4);
     const int wstride = 2 * hidden + 32;
-    uint8_t* wsm = smem + L.x0 + DLayout<KIND>::route_base(hidden, experts);
+    uint8_t* wsm = a.route_in_ring ? smem + L.ring : smem + L.x0 + DLayout<KIND>::route_base(hidden, experts);
     const int pass_rows = a.route_rows > 0 ? a.route_rows : experts;  // (0: the logits read global memory)
     const int vec_per_wrow = hidden / 8;  // 16-byte pieces of a router row
     float nw[D_NORM_HELD];
     uint4 rv[D_ROUTE_VEC];
+    const int trip_rows = min(pass_rows, int(div_small(D_ROUTE_VEC * nthreads, vec_per_wrow)));  // rows the registers hold
     auto request_router_rows = [&](int e_lo) {
-        const int n = a.route_rows > 0 ? min(pass_rows, experts - e_lo) * vec_per_wrow : 0;
+        const int n = a.route_rows > 0 ? min(trip_rows, experts - e_lo) * vec_per_wrow : 0;
         const uint4* src = reinterpret_cast<const uint4*>(a.router + size_t(e_lo) * hidden);
 #pragma unroll
         for (int k = 0; k < D_ROUTE_VEC; k++) {
@@ -382,13 +385,13 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
             if (i < n) rv[k] = load_now_v4(src + i);
         }
     };
-    auto store_router_rows = [&](int e_lo) {
-        const int n = min(pass_rows, experts - e_lo) * vec_per_wrow;
+    auto store_router_rows = [&](int e_lo, int row0) {
+        const int n = min(trip_rows, experts - e_lo) * vec_per_wrow;
         int r = tid / vec_per_wrow, v = tid - r * vec_per_wrow;  // piece tid + k * nthreads = (row r, piece v)
         const int dr = nthreads / vec_per_wrow, dv = nthreads - dr * vec_per_wrow;
 #pragma unroll
         for (int k = 0; k < D_ROUTE_VEC; k++) {
-            if (tid + k * nthreads < n) *reinterpret_cast<uint4*>(wsm + size_t(r) * wstride + v * 16) = rv[k];
+            if (tid + k * nthreads < n) *reinterpret_cast<uint4*>(wsm + size_t(row0 + r) * wstride + v * 16) = rv[k];
             r += dr, v += dv;
             if (v >= vec_per_wrow) v -= vec_per_wrow, r++;
         }
@@ -400,6 +403,7 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
     bool streaming = false;
     auto start_stream = [&](unsigned walk) {
         share(P0, walk), share(P1, walk);
+        if (a.route_in_ring) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // (read as plain memory so far)
         nrec = uint32_t(P0.n * P0.nchunks + P1.n * P1.nchunks);
         start_phase(P0.n > 0 ? 0 : 1);
         top_up();
@@ -432,8 +436,14 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
         if (routing) {
             // Part 0 of the router matrix goes all the way into shared memory before the wait,
             // part 1 (if any) into registers.
+            // (A whole matrix of more rows than the registers hold: in several trips, all before the wait.)
             request_router_rows(0);
-            if (a.route_rows > 0) store_router_rows(0);
+            if (a.route_rows > 0) store_router_rows(0, 0);
+#pragma unroll 1
+            for (int e = trip_rows; e < experts && a.route_rows >= experts; e += trip_rows) {
+                request_router_rows(e);
+                store_router_rows(e, e);
+            }
             if (a.route_rows > 0 && pass_rows < experts) request_router_rows(pass_rows);
             if (a.norm_w) {
 #pragma unroll
@@ -477,7 +487,7 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
             for (int e_lo = 0; e_lo < experts; e_lo += pass_rows) {
                 if (a.route_rows > 0) {
                     if (e_lo > 0) {  // (part 0 was stored before the wait above; the registers hold part 1)
-                        store_router_rows(e_lo);
+                        store_router_rows(e_lo, 0);
                         if (e_lo + pass_rows < experts) request_router_rows(e_lo + pass_rows);
                     }
                     __syncthreads();
@@ -1011,7 +1021,7 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
 // as many warps as possible while each still gets a ring of at least two stages; then the deepest
 // ring that fits.
 struct DecodeConfig {
-    int nwarps = 0, unit_warps = 0, stages = 0, xcap = 0, route_rows = 0;
+    int nwarps = 0, unit_warps = 0, stages = 0, xcap = 0, route_rows = 0, route_in_ring = 0;
 };
 
 // The most units of either phase that a CTA can get when at most `walk` experts are walked (see share()
@@ -1029,43 +1039,47 @@ bool decode_config(const MoeDims& d, int t, int ids_slots, int sms, bool ep, Dec
     c.xcap = min(D_TOK, (ids_slots / d.topk + 7) / 8 * 8);
     auto deepest = [&](int w, int rr) {
         for (int k = D_MAX_STAGES; k >= 2; k--)
-            if (size_t(DLayout<KIND>(w, k, c.xcap, rr, d.hidden, d.inter, d.experts, d.topk, ids_slots).total) <= D_SMEM_LIMIT)
+            if (size_t(DLayout<KIND>(w, k, c.xcap, rr, d.hidden, d.inter, d.experts, d.topk, ids_slots).total) <= decode_smem_limit(ep))
                 return k;
         return 0;
     };
-    int best_w = 0, best_u = 0, best_s = 0, best_r = 0;
+    int best_w = 0, best_u = 0, best_s = 0, best_r = 0, best_in = 0;
+    const bool dense = !ep && dense_walk(d, t);
     for (int w = D_MAX_WARPS; w >= 8; w -= 2) {
         // One or two tokens: a CTA gets fewer units than it has warps. Only those warps have rings, deep ones:
         // a unit's records are all on their way at once instead of two at a time.
-        const int units = !ep && !dense_walk(d, t) ? most_units(d, min(d.experts, t * d.topk), sms) : w;
+        const int units = !ep && !dense ? most_units(d, min(d.experts, t * d.topk), sms) : w;
         const int u = max(1, min(w, units));
         // Rows of the router matrix staged at a time: the whole matrix or the fewest equal parts that
-        // leave the ring two stages (each part is a pass of the logits: 1.6 us at 16 rows of 1024).
+        // leave the ring two stages (each part is a pass of the logits: 1.6 us at 16 rows of 1024). Parts go
+        // through the registers one ahead. Walks that stream only once the picks are known stage it in the
+        // ring, if it holds all of it.
         const int held = D_ROUTE_VEC * w * 32 / (d.hidden / 8);  // rows the CTA's registers hold at a time
-        int rr = 0, s = 0;
+        int rr = d.experts, s = dense ? 0 : deepest(u, 0);
+        const int in = s >= 2 && size_t(u) * s * Rec<KIND>::BYTES >= size_t(d.experts) * (2 * size_t(d.hidden) + 32);
+        if (!in) s = 0;
         for (int parts = 1; parts <= 8 && s < 2; parts++) {
             rr = (d.experts + parts - 1) / parts;
-            if (rr <= held) s = deepest(u, rr);
+            if (rr <= held || parts == 1) s = deepest(u, rr);
         }
         if (s < 2) rr = 0, s = deepest(u, 0);  // (the logits read global memory)
         // (More warps matter more than a third stage: an expert's units are cut into parts of 16
         // where they can be, one per warp. Measured at granite-1b-a400m, batch 32: 0.83 ms per
         // step with 16 warps and two stages against 0.865 with 14 and three.)
-        if (s > best_s) best_w = w, best_u = u, best_s = s, best_r = rr;
+        if (s > best_s) best_w = w, best_u = u, best_s = s, best_r = rr, best_in = in;
         if (s >= 2) break;
     }
-    c.nwarps = best_w, c.unit_warps = best_u, c.stages = best_s, c.route_rows = best_r;
+    c.nwarps = best_w, c.unit_warps = best_u, c.stages = best_s, c.route_rows = best_r, c.route_in_ring = best_in;
     return best_s >= 2;
 }
 
 }  // namespace
 
 void init_kernels_decode() {
-    const int lim = int(D_SMEM_LIMIT);
-    cudaFuncSetAttribute(moe_decode_kernel<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    cudaFuncSetAttribute(moe_decode_kernel<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    cudaFuncSetAttribute(moe_decode_kernel<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    cudaFuncSetAttribute(moe_decode_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+    cudaFuncSetAttribute(moe_decode_kernel<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(decode_smem_limit(false)));
+    cudaFuncSetAttribute(moe_decode_kernel<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(decode_smem_limit(false)));
+    cudaFuncSetAttribute(moe_decode_kernel<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(decode_smem_limit(true)));
+    cudaFuncSetAttribute(moe_decode_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(decode_smem_limit(true)));
 }
 
 // `ranks` > 1 (or an expert-parallel layer of one rank): t is the tokens per rank. A token's router
@@ -1107,12 +1121,14 @@ int launch_decode_block(const MoeDims& d, int kind, const uint16_t* router, cons
     const bool fits = kind == 1 ? decode_config<1>(d, t, a.ids_slots, sms, ep != nullptr, c)
                                 : decode_config<2>(d, t, a.ids_slots, sms, ep != nullptr, c);
     if (!fits) return -1;
-    a.unit_warps = c.unit_warps, a.stages = c.stages, a.xcap = c.xcap, a.route_rows = c.route_rows;
+    a.unit_warps = c.unit_warps, a.stages = c.stages, a.xcap = c.xcap;
+    a.route_rows = c.route_rows, a.route_in_ring = c.route_in_ring;
+    const int beside = c.route_in_ring ? 0 : c.route_rows;  // rows in the token area
     // One CTA per SM, all resident at once (they wait for one another): never more CTAs than SMs.
     const int grid = sms, nwarps = c.nwarps;
-    const size_t smem = kind == 1 ? size_t(DLayout<1>(c.unit_warps, c.stages, c.xcap, c.route_rows, d.hidden, d.inter,
+    const size_t smem = kind == 1 ? size_t(DLayout<1>(c.unit_warps, c.stages, c.xcap, beside, d.hidden, d.inter,
                                                       d.experts, d.topk, a.ids_slots).total)
-                                  : size_t(DLayout<2>(c.unit_warps, c.stages, c.xcap, c.route_rows, d.hidden, d.inter,
+                                  : size_t(DLayout<2>(c.unit_warps, c.stages, c.xcap, beside, d.hidden, d.inter,
                                                       d.experts, d.topk, a.ids_slots).total);
     auto kernel = kind == 1 ? (ep ? moe_decode_kernel<1, true> : moe_decode_kernel<1, false>)
                             : (ep ? moe_decode_kernel<2, true> : moe_decode_kernel<2, false>);
