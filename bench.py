@@ -306,7 +306,7 @@ def decode_point(ctx, shape, layers, batch, target_ms, repeats, peak):
 
 def block_point(ctx, cuda, shape, lw, tokens, bias, int8_pops, target_ms, repeats):
     """One MoE block at `tokens` tokens (prefill-size: the tcgen05 kernels when the batch averages
-    32 tokens per expert): time per block, per-kernel shares, and the expert kernels' rate."""
+    16 tokens per expert): time per block, per-kernel shares, and the expert kernels' rate."""
     layer = cuda.MoeLayer(ctx, lw.router, lw.gate_up, lw.down, shape.topk, tokens)
     if bias is not None:
         layer.set_router_bias(bias)

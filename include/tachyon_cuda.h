@@ -58,7 +58,7 @@ int tc_set_launch_overlap(tc_ctx *ctx, int on);
 
 /* From how many tokens per expert (batch tokens x experts per token / experts,
  * on average) a block's expert products run on the tcgen05 tensor-core kernels
- * instead of the bandwidth-oriented ones. Default 32; 0 = always; a huge value
+ * instead of the bandwidth-oriented ones. Default 16; 0 = always; a huge value
  * = never. Both give the same values (same fma chain per output). */
 int tc_set_prefill_threshold(tc_ctx *ctx, int avg_tokens_per_expert);
 

@@ -177,7 +177,7 @@ class Context:
         return {name: float(v) for name, v in zip(self.PHASES, d)}
 
     def set_prefill_threshold(self, avg_tokens_per_expert: int):
-        """Average tokens per expert from which the tcgen05 kernels take over (default 32; 0 = always)."""
+        """Average tokens per expert from which the tcgen05 kernels take over (default 16; 0 = always)."""
         self._check(self.lib.tc_set_prefill_threshold(self.handle, avg_tokens_per_expert),
                     "tc_set_prefill_threshold")
 

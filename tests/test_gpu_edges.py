@@ -24,6 +24,8 @@ WIDE = MoeShape("wide-router", 2048, 64, 8, 32, fmt="q4")    # 256 KB of router 
     (ODD_Q8, 129, False),
     # Tensor-core tiles: whole ones, one token past them, experts with hardly any.
     (ODD_Q8, 256, False), (ODD_Q4, 257, False), (ODD_Q8, 1025, True), (ODD_Q4, 770, True), (ONE_BLOCK, 193, False),
+    # Both sides of the switch to the tensor cores past 128 tokens.
+    (PAST_64, 129, True), (WIDE, 129, True),
     # Router tiles of 2, 4 and 8 tokens, each with a remainder; the dispatch past one CTA's batch.
     (ODD_EXPERTS, 257, False), (ODD_EXPERTS, 595, False), (ODD_EXPERTS, 1187, True), (PAST_64, 1191, True),
     (WIDE, 259, False), (WIDE, 597, True), (WIDE, 1189, False), (ONE_BLOCK, 2049, False),
