@@ -59,14 +59,20 @@ int tc_set_launch_overlap(tc_ctx *ctx, int on);
 /* From how many tokens per expert (batch tokens x experts per token / experts,
  * on average) a block's expert products run on the tcgen05 tensor-core kernels
  * instead of the bandwidth-oriented ones. Default 16; 0 = always; a huge value
- * = never. Both give the same values (same fma chain per output). */
+ * = never. Both give the same values (same fma chain per output).
+ * A layer holds the tcgen05 kernels' copy of its experts only if some batch of up to its
+ * max_tokens can reach those kernels. This call and tc_set_decode_block make the
+ * copies that have become reachable: they may allocate and wait then. While capturing, and for
+ * layers whose uploaded matrices were detached, none is made; such blocks run on the
+ * bandwidth-oriented kernels. */
 int tc_set_prefill_threshold(tc_ctx *ctx, int avg_tokens_per_expert);
 
 /* Decode-size blocks (8-bit or 4-bit experts, default arithmetic) run as ONE kernel whose
  * CTAs meet at grid-wide counters (no counterpart in the reference, whose Metal backend
  * encodes a dispatch per step: src/gpu/mod.rs:651-702): up to 32 tokens directly, and up to
  * 128 tokens with an expert's tokens walked in runs of up to 32. on = 1: the default; on = 0: the four-kernel path;
- * on > 1: one kernel up to that many tokens (at most 128). All give the same values. */
+ * on > 1: one kernel up to that many tokens (at most 128). All give the same values. (Like
+ * tc_set_prefill_threshold, it may make copies of layers' experts.) */
 int tc_set_decode_block(tc_ctx *ctx, int on);
 
 /* ---- device buffers: replace tm_buffer / tm_buffer_contents / tm_buffer_free
@@ -112,7 +118,8 @@ tc_moe_layer *tc_moe_layer_create(tc_ctx *ctx, int hidden, int experts, int expe
                                   const tc_matrix *down, int max_tokens);
 void tc_moe_layer_free(tc_moe_layer *layer);
 /* A layer keeps its own re-tiled copies of the expert matrices; the matrices as uploaded are
- * only read again by TC_ARITH_CPU_LANES. After this call the layer no longer refers to them, so
+ * only read again by TC_ARITH_CPU_LANES, and by the two switches above when they make another
+ * copy. After this call the layer no longer refers to them, so
  * the caller may tc_matrix_free gate_up and down (a third of the layer's expert memory); blocks
  * in TC_ARITH_CPU_LANES are then refused for this layer. (The Metal backend keeps one copy,
  * src/gpu/mod.rs:222-251; no counterpart there.) */

@@ -3,6 +3,7 @@
 // files of this directory.
 #include "../../include/tachyon_cuda.h"
 
+#include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -55,6 +56,7 @@ struct tc_ctx {
     uint32_t grid_spin_limit = 1u << 22;
     unsigned long long* phase_stamps = nullptr;  // device [8], while phase profiling is on
     int* static_status = nullptr;  // status word of tc_dispatch_static on this device, once it has been used
+    std::vector<tc_moe_layer*> layers;  // living ones, for make_reachable_prefill_tiles
 };
 
 struct tc_matrix {
@@ -74,8 +76,9 @@ struct tc_moe_layer {
     bool dispatch_stale = false;       // the last forward built no dispatch (one-kernel block): built on demand
     uint8_t* gate_up_tiled = nullptr;  // the fast kernels' record layout of the two expert matrices
     uint8_t* down_tiled = nullptr;
-    tc::PrefillWeights pw;             // the tcgen05 kernels' tiles of the two expert matrices
+    tc::PrefillWeights pw;             // the tcgen05 kernels' tiles of the two expert matrices (see reaches_prefill)
     std::vector<void*> pw_allocs;
+    bool prefill_scratch = false;      // the context's token tiles were reserved for this layer's max_tokens
     bool ep = false;                   // expert-parallel layer: gate_up/down hold this rank's experts only
     tc::EpLayerBuffers epb;
     tc::MatrixDev gu, dn;              // the expert matrices as uploaded (pointers null once detached)
@@ -234,6 +237,72 @@ bool self_window_reserve(tc_ctx* ctx, const tc::MoeDims& d, int max_tokens) {
     return true;
 }
 
+// Which one-kernel form takes a block of t tokens in the default arithmetic: 0 none, 1 the direct one (up to 32
+// tokens), 2 the run-walking one through the local window (up to 128), whose layout then is in *self.
+int decode_form(const tc_ctx* ctx, const tc_moe_layer* l, int t, tc::DecodeEp* self) {
+    if (!ctx->decode_block || l->ep) return 0;
+    if (tc::decode_block_applies(l->dims, l->gu.kind, l->dn.kind, t)) return 1;
+    return t > 32 && t <= ctx->decode_block_tokens && t <= ctx->sms && ctx->self_window &&
+           self_window_layout(l->dims, t, self) <= ctx->self_bytes &&
+           tc::decode_block_applies(l->dims, l->gu.kind, l->dn.kind, t, 1) ? 2 : 0;
+}
+
+bool prefill_sized(const tc_ctx* ctx, const tc_moe_layer* l, int t) {
+    return (long long)t * l->dims.topk >= (long long)ctx->prefill_min_avg * l->dims.experts;
+}
+
+// Whether any block of the layer can run on the tcgen05 kernels as the context's switches stand. A layer of up to
+// 128 tokens whose blocks all run as one kernel never does, and does without their copy of the experts
+// (2.125 bytes per 8-bit weight, twice the matrix as uploaded).
+bool reaches_prefill(const tc_ctx* ctx, const tc_moe_layer* l) {
+    if (!l->prefill_scratch) return false;
+    if (l->ep) return true;
+    tc::DecodeEp self;
+    for (int t = l->max_tokens; t > 0 && prefill_sized(ctx, l, t); t--)
+        if (t > SELF_WINDOW_TOKENS || !decode_form(ctx, l, t, &self)) return true;
+    return false;
+}
+
+// The third copy of a layer's experts, for prefill-size groups: the values as f16 tiles in the tensor core's
+// canonical order and f32 block scales. `held`: the shape of the matrices held here. Enqueued, not waited for.
+bool make_prefill_tiles(tc_ctx* ctx, tc_moe_layer* l, const tc::MoeDims& held) {
+    auto get = [&](auto*& dst, size_t bytes) {
+        void* raw = nullptr;
+        if (!cuda_ok(ctx, cudaMalloc(&raw, bytes + 256), "cudaMalloc(prefill weights)")) return false;
+        l->pw_allocs.push_back(raw);
+        dst = static_cast<std::remove_reference_t<decltype(dst)>>(raw);
+        return true;
+    };
+    tc::PrefillWeights w;
+    bool ok = get(w.gu_t, tc::prefill_weight_bytes(held, true)) && get(w.gu_d, tc::prefill_scale_elems(held, true) * 4) &&
+              get(w.dn_t, tc::prefill_weight_bytes(held, false)) && get(w.dn_d, tc::prefill_scale_elems(held, false) * 4);
+    if (ok && l->gu.kind == TC_Q4) ok = get(w.gu_c, tc::prefill_scale_elems(held, true) * 4);
+    if (ok && l->dn.kind == TC_Q4) ok = get(w.dn_c, tc::prefill_scale_elems(held, false) * 4);
+    if (!ok) {
+        for (void* q : l->pw_allocs) cudaFree(q);
+        l->pw_allocs.clear();
+        return false;
+    }
+    l->pw = w;
+    tc::tile_prefill_weights(held, l->gu, true, w.gu_t, w.gu_d, w.gu_c, ctx->stream);
+    tc::tile_prefill_weights(held, l->dn, false, w.dn_t, w.dn_d, w.dn_c, ctx->stream);
+    return true;
+}
+
+// After a switch has moved: the tcgen05 kernels' copies that blocks can reach now. (Not while capturing, when nothing
+// can be allocated, and not for a layer whose uploaded matrices are gone: without the copy such a block runs
+// on the bandwidth-oriented kernels, which give the same values.)
+int make_reachable_prefill_tiles(tc_ctx* ctx) {
+    bool made = false;
+    for (tc_moe_layer* l : ctx->layers) {
+        if (ctx->capturing || l->pw.gu_t || !l->gu.data || !reaches_prefill(ctx, l)) continue;
+        cudaSetDevice(ctx->device);
+        if (!make_prefill_tiles(ctx, l, l->dims)) return -1;
+        made = true;
+    }
+    return !made || cuda_ok(ctx, cudaStreamSynchronize(ctx->stream), "weight tiling") ? 0 : -1;
+}
+
 // Grows the context's scratch so a layer of these dimensions fits.
 bool ws_reserve(tc_ctx* ctx, const tc::MoeDims& d, int max_tokens) {
     tc::Workspace& w = ctx->ws;
@@ -323,6 +392,7 @@ void tc_destroy(tc_ctx* ctx) {
     if (!ctx) return;
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
+    for (tc_moe_layer* l : ctx->layers) l->ctx = nullptr;
     ws_release(ctx);
     for (void* q : ctx->pre_allocs) cudaFree(q);
     if (ctx->host_x) cudaFree(ctx->host_x);
@@ -449,7 +519,7 @@ int tc_set_launch_overlap(tc_ctx* ctx, int on) {
 int tc_set_decode_block(tc_ctx* ctx, int on) {
     ctx->decode_block = on != 0;
     ctx->decode_block_tokens = on > 1 ? std::min(on, SELF_WINDOW_TOKENS) : SELF_WINDOW_TOKENS;
-    return 0;
+    return make_reachable_prefill_tiles(ctx);
 }
 
 int tc_profile_phases(tc_ctx* ctx, int on) {
@@ -477,7 +547,7 @@ int tc_profile_read_phases(tc_ctx* ctx, uint64_t* ns6) {
 int tc_set_prefill_threshold(tc_ctx* ctx, int avg_tokens_per_expert) {
     if (avg_tokens_per_expert < 0) return fail(ctx, "the threshold cannot be negative");
     ctx->prefill_min_avg = avg_tokens_per_expert;
-    return 0;
+    return make_reachable_prefill_tiles(ctx);
 }
 
 int tc_profile_enable(tc_ctx* ctx, int on) {
@@ -744,33 +814,16 @@ tc_moe_layer* layer_create(tc_ctx* ctx, int hidden, int experts, int k, int inte
     tc::tile_weights(dl, gate_up->dev, true, l->gate_up_tiled, ctx->stream);
     tc::tile_weights(dl, down->dev, false, l->down_tiled, ctx->stream);
     // (Expert-parallel layers: tiles of this rank's experts; scratch for every rank's tokens.)
-    const tc::MoeDims& dp = ep ? dl : d;
-    if (prefill_reserve(ctx, d, ep ? max_tokens * ctx->ep.size : max_tokens)) {
-        // Third copy of the experts, for prefill-size groups: the values as f16 tiles in the tensor
-        // core's canonical order and f32 block scales.
-        auto get = [&](auto*& dst, size_t bytes) {
-            void* raw = nullptr;
-            if (!cuda_ok(ctx, cudaMalloc(&raw, bytes + 256), "cudaMalloc(prefill weights)")) return false;
-            l->pw_allocs.push_back(raw);
-            dst = static_cast<std::remove_reference_t<decltype(dst)>>(raw);
-            return true;
-        };
-        const bool q4g = gate_up->dev.kind == TC_Q4, q4d = down->dev.kind == TC_Q4;
-        bool okp = get(l->pw.gu_t, tc::prefill_weight_bytes(dp, true)) && get(l->pw.gu_d, tc::prefill_scale_elems(dp, true) * 4) &&
-                   get(l->pw.dn_t, tc::prefill_weight_bytes(dp, false)) && get(l->pw.dn_d, tc::prefill_scale_elems(dp, false) * 4);
-        if (okp && q4g) okp = get(l->pw.gu_c, tc::prefill_scale_elems(dp, true) * 4);
-        if (okp && q4d) okp = get(l->pw.dn_c, tc::prefill_scale_elems(dp, false) * 4);
-        if (!okp) {
-            tc_moe_layer_free(l);
-            return nullptr;
-        }
-        tc::tile_prefill_weights(dp, gate_up->dev, true, l->pw.gu_t, l->pw.gu_d, l->pw.gu_c, ctx->stream);
-        tc::tile_prefill_weights(dp, down->dev, false, l->pw.dn_t, l->pw.dn_d, l->pw.dn_c, ctx->stream);
+    l->prefill_scratch = prefill_reserve(ctx, d, ep ? max_tokens * ctx->ep.size : max_tokens);
+    if (reaches_prefill(ctx, l) && !make_prefill_tiles(ctx, l, dl)) {
+        tc_moe_layer_free(l);
+        return nullptr;
     }
     if (!cuda_ok(ctx, cudaStreamSynchronize(ctx->stream), "weight tiling")) {
         tc_moe_layer_free(l);
         return nullptr;
     }
+    ctx->layers.push_back(l);
     return l;
 }
 }  // namespace
@@ -779,6 +832,10 @@ extern "C" {
 
 void tc_moe_layer_free(tc_moe_layer* layer) {
     if (!layer) return;
+    if (layer->ctx) {  // (null: the context went first)
+        std::vector<tc_moe_layer*>& all = layer->ctx->layers;
+        all.erase(std::remove(all.begin(), all.end(), layer), all.end());
+    }
     if (layer->bias) cudaFree(layer->bias);
     for (void* q : layer->pw_allocs) cudaFree(q);
     if (layer->ep) tc::ep_layer_free(layer->epb);
@@ -866,8 +923,9 @@ int moe_enqueue(tc_moe_layer* layer, const float* x, const float* norm_w, float 
     }
     const bool lanes = ctx->arith == tc::ARITH_CPU_LANES;
     layer->dispatch_stale = false;
-    if (!lanes && ctx->decode_block &&
-        tc::decode_block_applies(d, layer->gu.kind, layer->dn.kind, t)) {
+    tc::DecodeEp self;
+    const int form = lanes ? 0 : decode_form(ctx, layer, t, &self);
+    if (form == 1) {
         // Decode-size batch: the whole block is one kernel (no dispatch is built).
         n += staged(ctx, 7, [&] {
             return tc::launch_decode_block(d, layer->gu.kind,
@@ -881,13 +939,8 @@ int moe_enqueue(tc_moe_layer* layer, const float* x, const float* norm_w, float 
         if (!ctx->capturing && !cuda_ok(ctx, cudaGetLastError(), "MoE launch")) return -1;
         return 0;
     }
-    const bool prefill = !lanes && layer->pw.gu_t &&
-                         (long long)t * d.topk >= (long long)ctx->prefill_min_avg * d.experts;
-    tc::DecodeEp self;
-    if (!lanes && ctx->decode_block && t > 32 && t <= ctx->decode_block_tokens && t <= ctx->sms &&
-        ctx->self_window &&
-        self_window_layout(d, t, &self) <= ctx->self_bytes &&
-        tc::decode_block_applies(d, layer->gu.kind, layer->dn.kind, t, 1)) {
+    const bool prefill = !lanes && layer->pw.gu_t && prefill_sized(ctx, layer, t);
+    if (form == 2) {
         // Up to 128 tokens: still one kernel, in its expert-parallel form with this GPU as the only
         // rank (an expert's tokens in runs of up to 32; rows and outputs through the local window).
         // Measured at the 1b-a400m shape, 24 blocks: 0.81 ms at 64 tokens (1.82 as separate kernels), 1.12 at

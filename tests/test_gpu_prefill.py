@@ -110,3 +110,50 @@ def test_scratch_shared_by_layers_only_grows(oracle, ctx):
         ctx.set_prefill_threshold(32)
         la.free()
         lb.free()
+
+
+@pytest.mark.parametrize("fmt", ["q8", "q4"])
+def test_decode_only_layers_hold_no_tensor_core_copy(oracle, ctx, fmt):
+    """A layer whose every block runs as one kernel does without the tensor-core kernels' copy of its experts
+    (2.125 bytes per 8-bit weight, 2.25 with 4-bit offsets). Once a switch makes those kernels reachable the
+    copy is there and they run; a layer whose uploaded matrices are gone runs on the bandwidth-oriented
+    kernels instead. The same bits every time."""
+    import torch
+
+    shape = MoeShape("1b", 1024, 32, 8, 512, fmt=fmt)
+    copy = shape.experts * 3 * shape.inter * shape.hidden * (2.125 if fmt == "q8" else 2.25)
+    pages = 16 << 20  # (allocations take whole pages of 2 MB)
+    lw = layer_weights(oracle, shape, 0)
+    x = workloads.hidden_states(shape, 128, seed=31)
+    y0 = np.zeros_like(x)
+    ctx.set_arithmetic(ctx.ARITH_FAST)
+
+    def launches_of(layer):
+        before = ctx.launch_count()
+        return forward(ctx, layer, x, y0), ctx.launch_count() - before
+
+    layers = [make_layer(ctx, lw, shape.topk, 129)]  # (the context's scratch has its size from here on)
+    try:
+        free = [torch.cuda.mem_get_info(ctx.device)[0]]
+        for most in (128, 129):  # 129 tokens: one past the one-kernel block
+            layers.append(make_layer(ctx, lw, shape.topk, most))
+            free.append(torch.cuda.mem_get_info(ctx.device)[0])
+        small, large = free[0] - free[1], free[1] - free[2]
+        assert abs(large - small - copy) < pages
+        one, n = launches_of(layers[1])
+        assert n == 1
+        detached = make_layer(ctx, lw, shape.topk, 128)
+        layers.append(detached)
+        detached.detach_experts()
+        before = torch.cuda.mem_get_info(ctx.device)[0]
+        ctx.set_decode_block(False)  # 32 tokens per expert: the tensor-core kernels, for the layers that can have the copy
+        assert abs(before - torch.cuda.mem_get_info(ctx.device)[0] - copy) < pages
+        layers.append(make_layer(ctx, lw, shape.topk, 128))
+        for layer, kernels in [(layers[1], 5), (layers[2], 5), (detached, 4), (layers[4], 5)]:
+            y, n = launches_of(layer)
+            assert n == kernels
+            assert np.array_equal(y, one)
+    finally:
+        ctx.set_decode_block(True)
+        for layer in layers:
+            layer.free()
