@@ -83,7 +83,7 @@ int tc_upload(tc_ctx *ctx, void *dst_dev, const void *src_host, size_t bytes);
 int tc_download(tc_ctx *ctx, void *dst_host, const void *src_dev, size_t bytes);
 int tc_memset(tc_ctx *ctx, void *dst_dev, int value, size_t bytes);
 /* Copy on the context's stream (not waited for): device to device, or to or from
- * page-locked memory (tc_host_alloc). */
+ * page-locked memory (tc_host_alloc). Pageable memory is refused. */
 int tc_copy(tc_ctx *ctx, void *dst_dev, const void *src_dev, size_t bytes);
 /* Page-locked host memory, so uploads and downloads run at full PCIe rate. */
 void *tc_host_alloc(tc_ctx *ctx, size_t bytes);

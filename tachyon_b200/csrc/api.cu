@@ -490,6 +490,14 @@ int tc_memset(tc_ctx* ctx, void* dst, int value, size_t bytes) {
 }
 
 int tc_copy(tc_ctx* ctx, void* dst, const void* src, size_t bytes) {
+    // Pageable memory is refused here: the copy would be taken, and a capture would keep its address.
+    for (const void* p : {static_cast<const void*>(dst), src}) {
+        cudaPointerAttributes at{};
+        if (bytes == 0) break;
+        if (!cuda_ok(ctx, cudaPointerGetAttributes(&at, p), "copy")) return -1;
+        if (at.type == cudaMemoryTypeUnregistered)
+            return fail(ctx, "copy: %p is neither device memory nor page-locked", p);
+    }
     return cuda_ok(ctx, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, ctx->stream), "copy") ? 0 : -1;
 }
 

@@ -49,3 +49,31 @@ def test_host_buffers_at_the_edges(oracle, ctx, t):
         layer.free()
     want = 1.0 + oracle_moe(oracle, lw, x, ODD_Q8.topk).proj
     assert np.abs(y - want).max() <= 2e-3
+
+
+def test_copies_take_device_and_page_locked_memory_only(ctx):
+    """Pageable memory is refused either way round, also inside a capture, which stays usable."""
+    from tachyon_b200 import cuda
+
+    n = 1024
+    host, plain = ctx.host_empty(n), np.full(n, 7.0, np.float32)
+    a, b = ctx.to_device(np.arange(n, dtype=np.float32)), ctx.to_device(np.zeros(n, np.float32))
+
+    def refused(dst, src):
+        with pytest.raises(cuda.TachyonCudaError, match="page-locked"):
+            ctx.copy_bytes(dst, src, 4 * n)
+
+    refused(a.ptr, plain.ctypes.data)
+    refused(plain.ctypes.data, a.ptr)
+    ctx.capture_begin()
+    refused(a.ptr, plain.ctypes.data)
+    refused(plain.ctypes.data, a.ptr)
+    ctx.copy_bytes(b.ptr + 4, a.ptr + 4, 4 * n - 4)
+    ctx.copy_bytes(host.ptr, b.ptr, 4 * n)
+    g = ctx.capture_end()
+    g.launch()
+    ctx.sync()
+    assert np.array_equal(a.get(), np.arange(n)) and np.array_equal(host.array, np.arange(n)) and np.all(plain == 7.0)
+    g.free()
+    for d in (host, a, b):
+        d.free()
