@@ -26,10 +26,9 @@ class GraphBuckets:
 
     ``layers`` are ``MoeLayer``-like objects with ``block(norm_weight, eps, y, t)`` and
     ``max_tokens``; ``norm_weights`` their RMSNorm weights on the device. ``ctx`` needs
-    ``empty``, ``upload``, ``download``, ``memset``, ``copy_bytes``, ``capture_begin``,
-    ``capture_end`` and ``sync`` (``tachyon_b200.cuda.Context`` has them). With ``host_empty``
-    (page-locked memory) a step is one graph launch and one wait: the rows' copies in and out are
-    nodes of the graph. Without it they are calls of their own.
+    ``empty``, ``host_empty`` (page-locked memory), ``copy_bytes``, ``capture_begin``,
+    ``capture_end`` and ``sync`` (``tachyon_b200.cuda.Context`` has them). A step is one graph
+    launch and one wait: the rows' copies in and out are nodes of the graph.
     """
 
     def __init__(self, ctx, layers, norm_weights, eps: float, hidden: int, buckets=DEFAULT_BUCKETS):
@@ -42,11 +41,9 @@ class GraphBuckets:
         self.ctx, self.layers, self.norm_weights = ctx, list(layers), list(norm_weights)
         self.eps, self.hidden = float(eps), int(hidden)
         rows = self.buckets[-1]
-        self.pinned = hasattr(ctx, "host_empty")
-        make = ctx.host_empty if self.pinned else ctx.empty
-        self.x_in = make((rows, hidden), np.float32)       # the step's rows, then zeros up to the bucket
-        self.x = ctx.empty((rows, hidden), np.float32)     # the residual stream the graph works on
-        self.x_out = make((rows, hidden), np.float32) if self.pinned else self.x
+        self.x_in = ctx.host_empty((rows, hidden), np.float32)  # the step's rows, then zeros up to the bucket
+        self.x = ctx.empty((rows, hidden), np.float32)          # the residual stream the graph works on
+        self.x_out = ctx.host_empty((rows, hidden), np.float32)
         self.graphs = {}
         self.launches = {b: 0 for b in self.buckets}
 
@@ -63,8 +60,7 @@ class GraphBuckets:
         self.ctx.copy_bytes(self.x.ptr, self.x_in.ptr, b * self.hidden * 4)
         for layer, w in zip(self.layers, self.norm_weights):
             layer.block(w, self.eps, self.x, t=b)  # x += moe(rmsnorm(x)): src/model.rs:662-681
-        if self.pinned:
-            self.ctx.copy_bytes(self.x_out.ptr, self.x.ptr, b * self.hidden * 4)
+        self.ctx.copy_bytes(self.x_out.ptr, self.x.ptr, b * self.hidden * 4)
 
     def graph(self, b: int):
         """The bucket's graph, captured on first use (after one eager pass of the same work)."""
@@ -84,27 +80,16 @@ class GraphBuckets:
             raise ValueError(f"expected [t, {self.hidden}] rows")
         b = self.bucket_for(t)
         g = self.graph(b)
-        if self.pinned:
-            self.x_in.array[:t] = x_host
-            self.x_in.array[t:b] = 0.0
-            g.launch()
-            self.ctx.sync()
-            self.launches[b] += 1
-            return self.x_out.array[:t].copy()
-        row = self.hidden * 4
-        self.ctx.upload(self.x_in.ptr, x_host)
-        if b > t:
-            self.ctx.memset(self.x_in.ptr + t * row, 0, (b - t) * row)
+        self.x_in.array[:t] = x_host
+        self.x_in.array[t:b] = 0.0
         g.launch()
         self.ctx.sync()
         self.launches[b] += 1
-        out = np.empty((t, self.hidden), np.float32)
-        self.ctx.download(out, self.x.ptr)
-        return out
+        return self.x_out.array[:t].copy()
 
     def free(self):
         for g in self.graphs.values():
             g.free()
         self.graphs.clear()
-        for d in {id(d): d for d in (self.x_in, self.x, self.x_out)}.values():
+        for d in (self.x_in, self.x, self.x_out):
             d.free()

@@ -6,11 +6,15 @@ from tachyon_b200.buckets import GraphBuckets
 
 
 class FakeArray:
-    def __init__(self, mem, ptr, shape):
-        self.mem, self.ptr, self.shape = mem, ptr, shape
+    def __init__(self, mem, ptr, shape, dtype, on_host):
+        self.ptr, self.shape, self.freed = ptr, shape, False
+        if on_host:
+            n = int(np.prod(shape)) * np.dtype(dtype).itemsize
+            self.array = mem[ptr:ptr + n].view(dtype).reshape(shape)
 
     def free(self):
-        pass
+        assert not self.freed
+        self.freed = True
 
 
 class FakeGraph:
@@ -27,19 +31,25 @@ class FakeGraph:
 
 
 class FakeContext:
-    """Device memory is one byte array; work enqueued while capturing is recorded, not run."""
+    """Device and page-locked memory are one byte array, seen from the host where page-locked; work
+    enqueued while capturing is recorded, not run."""
 
     def __init__(self):
         self.mem = np.zeros(1 << 20, np.uint8)
         self.top = 256
         self.capturing = None
         self.captures = 0
+        self.arrays = []
 
-    def empty(self, shape, dtype=np.float32):
+    def empty(self, shape, dtype=np.float32, on_host=False):
         n = int(np.prod(shape)) * np.dtype(dtype).itemsize
-        a = FakeArray(self.mem, self.top, tuple(shape))
+        a = FakeArray(self.mem, self.top, tuple(shape), dtype, on_host)
         self.top += (n + 255) // 256 * 256
+        self.arrays.append(a)
         return a
+
+    def host_empty(self, shape, dtype=np.float32):
+        return self.empty(shape, dtype, on_host=True)
 
     def _do(self, op):
         if self.capturing is not None:
@@ -49,18 +59,6 @@ class FakeContext:
 
     def copy_bytes(self, dst, src, n):
         self._do(lambda: self.mem.__setitem__(slice(dst, dst + n), self.mem[src:src + n].copy()))
-
-    def memset(self, dst, value, n):
-        assert self.capturing is None
-        self.mem[dst:dst + n] = value
-
-    def upload(self, dst, host):
-        assert self.capturing is None
-        b = np.ascontiguousarray(host).view(np.uint8).ravel()
-        self.mem[dst:dst + b.size] = b
-
-    def download(self, host, src):
-        host.view(np.uint8).ravel()[:] = self.mem[src:src + host.nbytes]
 
     def sync(self):
         pass
@@ -117,12 +115,15 @@ def test_buckets_above_the_layers_limit_are_dropped():
 def test_step_pads_with_zeros_and_returns_the_real_rows():
     ctx, layers, gb = make()
     x = np.arange(3 * 8, dtype=np.float32).reshape(3, 8)
+    gb.step(np.full((4, 8), 9.0, np.float32))  # (fills the bucket: its last row must not stay)
     y = gb.step(x)
     assert np.array_equal(y, x + 2 * (1.0 + np.arange(3, dtype=np.float32)[:, None]))  # two layers
     assert np.array_equal(ctx.rows(gb.x_in, 4, 8)[3], np.zeros(8, np.float32))         # the pad row went in as zeros
     # A smaller step into the same bucket must not see the previous step's rows.
     y1 = gb.step(x[:1] + 100)
     assert y1.shape == (1, 8) and np.array_equal(y1, x[:1] + 100 + 2.0)
+    # A result is the caller's own: later steps leave it as it is.
+    assert np.array_equal(y, x + 2 * (1.0 + np.arange(3, dtype=np.float32)[:, None]))
 
 
 def test_one_capture_per_bucket_and_replays_after_that():
@@ -138,4 +139,4 @@ def test_one_capture_per_bucket_and_replays_after_that():
     assert layers[0].calls.count(8) == 2 and layers[0].calls.count(2) == 2
     graphs = list(gb.graphs.values())
     gb.free()
-    assert all(g.freed for g in graphs)
+    assert all(g.freed for g in graphs) and all(a.freed for a in ctx.arrays)
