@@ -68,6 +68,10 @@ constexpr int D_TOK = 8 * D_GMAX;  // tokens per block this kernel takes; rows s
 constexpr int D_NORM_HELD = 8;     // elements of the norm's weight a thread holds (rows of up to 8 x 256 floats)
 constexpr int D_ROUTE_VEC = 10;    // 16-byte pieces of the router matrix a thread holds at a time
 constexpr int D_NSEG = 4;          // experts of a CTA's range whose slot lists are held at a time
+constexpr int D_MAX_SLOTS = 4095;  // (token, pick) slots of a block: their ids live in shared memory
+// Runs of the run-walking form. Cut into the longest, D_TOK slots, an expert has at most one more than slots / D_TOK,
+// so those always fit; shorter ones are only taken where theirs do.
+constexpr int D_MAX_RUNS = MAX_EXPERTS + (D_MAX_SLOTS + D_TOK) / D_TOK;
 // Dynamic part: the kernel also has 1.4 KB of static shared memory, 3.2 KB in the expert-parallel form.
 __host__ __device__ constexpr size_t decode_smem_limit(bool ep) { return 227 * 1024 - (ep ? 3584 : 1536); }
 
@@ -228,7 +232,7 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
     __shared__ int s_nactive;
     __shared__ int s_seg_count[D_NSEG];
     __shared__ uint8_t s_picked[MAX_EXPERTS];
-    constexpr int MAX_RUNS = EP ? MAX_EXPERTS + 4096 / 8 / 8 : MAX_EXPERTS;  // (experts + slots / shortest run)
+    constexpr int MAX_RUNS = EP ? D_MAX_RUNS : MAX_EXPERTS;
     __shared__ uint16_t s_active[MAX_RUNS];     // walk index -> expert (sparse walk); EP: -> the run's expert
     __shared__ uint16_t s_skip[EP ? MAX_RUNS : 1];      // EP: slots of that expert in earlier runs
     __shared__ int s_run_len;                           // EP: slots per run (32, 16 or 8)
@@ -621,7 +625,7 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
                         const unsigned ctas = r <= nctas ? div_small(nctas, r) : 1u;
                         const int per_cta = int(r <= nctas ? div_small(P0.upe + ctas - 1, ctas) : div_small(r * P0.upe + nctas - 1, nctas));
                         const int cost = int(div_small(per_cta + uwarps - 1, uwarps)) * (3 + (min(len, most) + 7) / 8);
-                        if (cost < best) best = cost, run_len = len;
+                        if (cost < best && r <= MAX_RUNS) best = cost, run_len = len;
                     }
                     // A lane per local expert, 32 at a time: the expert's runs after those before it.
                     int n = 0;
@@ -637,6 +641,8 @@ __global__ void __launch_bounds__(D_MAX_WARPS * 32, 1) moe_decode_kernel(const D
                         }
                         const int total = __shfl_sync(0xffffffffu, before, 31);
                         before -= mine;
+                        // (The runs fit; with the bound in the loop its code is the shorter: 100 tokens of the 3b
+                        // shape 53 us a block against 54.)
                         for (int j = 0; j < mine && n + before + j < MAX_RUNS; j++) {
                             s_active[n + before + j] = uint16_t(a.ep.first + e);
                             s_skip[n + before + j] = uint16_t(j * run_len);
@@ -1090,7 +1096,7 @@ bool decode_block_applies(const MoeDims& d, int kind_gate_up, int kind_down, int
     if (t < 1 || t > most || kind_gate_up != kind_down || d.topk > MAX_TOPK || d.hidden > D_NORM_HELD * 256)
         return false;
     const int slots = (ranks > 0 ? ranks : 1) * t * d.topk;
-    if (slots > 65535 / 16 || d.experts > MAX_EXPERTS) return false;  // (slot lists are 16-bit; ids live in shared memory)
+    if (slots > D_MAX_SLOTS || d.experts > MAX_EXPERTS) return false;
     DecodeConfig c;
     return kind_gate_up == 1 ? decode_config<1>(d, t, slots, 148, ranks > 0, c) : decode_config<2>(d, t, slots, 148, ranks > 0, c);
 }

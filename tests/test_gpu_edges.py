@@ -4,7 +4,7 @@ once, experts without a token; a call over host buffers on both sides of its rul
 import numpy as np
 import pytest
 
-from tachyon_b200 import synth, workloads
+from tachyon_b200 import synth, weights, workloads
 from tachyon_b200.workloads import MoeShape
 from test_gpu_parity import check_block, ctx, layer_weights, make_layer, oracle_moe  # noqa: F401
 
@@ -15,13 +15,14 @@ ODD_Q4 = MoeShape("odd-q4", 288, 8, 2, 160, fmt="q4")
 ONE_BLOCK = MoeShape("one-block", 32, 3, 1, 32, fmt="q8")    # one block per row, one pick
 ODD_EXPERTS = MoeShape("experts-37", 96, 37, 5, 32, fmt="q8")
 PAST_64 = MoeShape("experts-65", 64, 65, 8, 32, fmt="q8")    # one expert more than two per lane
+MANY_PICKS = MoeShape("picks-31", 96, 31, 31, 32, fmt="q8")  # every expert by every token: 496 runs of 8 at 128 tokens
 WIDE = MoeShape("wide-router", 2048, 64, 8, 32, fmt="q4")    # 256 KB of router matrix: staged in parts
 
 
 @pytest.mark.parametrize("shape,t,skewed", [
     # One kernel per block: a token, an odd few, and both sides of 32 tokens and of the largest batch.
     (ODD_Q4, 1, False), (ODD_EXPERTS, 3, False), (PAST_64, 31, True), (ONE_BLOCK, 33, False), (WIDE, 127, True),
-    (ODD_Q8, 129, False),
+    (ODD_Q8, 129, False), (MANY_PICKS, 128, False), (MANY_PICKS, 90, True),
     # Tensor-core tiles: whole ones, one token past them, experts with hardly any.
     (ODD_Q8, 256, False), (ODD_Q4, 257, False), (ODD_Q8, 1025, True), (ODD_Q4, 770, True), (ONE_BLOCK, 193, False),
     # Both sides of the switch to the tensor cores past 128 tokens.
@@ -77,3 +78,17 @@ def test_copies_take_device_and_page_locked_memory_only(ctx):
     g.free()
     for d in (host, a, b):
         d.free()
+
+
+def test_more_short_runs_than_the_kernel_lists(oracle, ctx):
+    """The run-walking form where runs of 8 tokens look cheapest and there would be 336 of them, 16 more than its tables
+    once held: the runs past the end were left out. The router is the identity, so a row's largest elements
+    are its picks and every expert gets the tokens asked for."""
+    counts = [1] * 230 + [30] * 25 + [44]
+    shape = MoeShape("runs", 256, len(counts), 8, 32, fmt="q8")
+    t = sum(counts) // shape.topk
+    lw = layer_weights(oracle, shape, 17)
+    lw = workloads.LayerWeights(weights.Matrix.from_f32(np.eye(256, dtype=np.float32).ravel(), 256, 256, "bf16"), lw.gate_up, lw.down)
+    x = 0.1 * workloads.hidden_states(shape, t, seed=3)
+    x[np.arange(sum(counts)) % t, np.repeat(np.arange(len(counts)), counts)] += 4.0
+    check_block(oracle, ctx, shape, lw, x, arith="fast")
