@@ -105,6 +105,7 @@ int fail(tc_ctx* ctx, const char* fmt, ...) {
 
 bool cuda_ok(tc_ctx* ctx, cudaError_t e, const char* what) {
     if (e == cudaSuccess) return true;
+    cudaGetLastError();  // (reported here: the check after the next launch must not find it again)
     fail(ctx, "%s: %s", what, cudaGetErrorString(e));
     return false;
 }
@@ -163,7 +164,8 @@ void ws_release(tc_ctx* ctx) {
 // Scratch of the tcgen05 path: token tiles for up to max_tokens * topk slots. Shared by
 // the context's layers, so it only ever grows: every dimension is the largest any
 // layer has asked for. Growing it frees the old buffers, which invalidates graphs
-// captured earlier; create every layer before capturing.
+// captured earlier; create every layer before capturing. (They are freed once the new ones are
+// there: a scratch that cannot grow stays as it is, for the layers and graphs that run on it.)
 bool prefill_reserve(tc_ctx* ctx, const tc::MoeDims& d, int max_tokens) {
     const int slots = max_tokens * d.topk;
     const size_t rows = tc::prefill_max_rows(slots, d.experts);
@@ -172,28 +174,26 @@ bool prefill_reserve(tc_ctx* ctx, const tc::MoeDims& d, int max_tokens) {
     if (p.max_tiles >= tiles && p.xt_elems >= rows * d.hidden && p.ht_elems >= rows * d.inter) return true;
     const size_t T = std::max(tiles, p.max_tiles), xt = std::max(rows * d.hidden, p.xt_elems),
                  ht = std::max(rows * d.inter, p.ht_elems);
-    cudaStreamSynchronize(ctx->stream);
-    for (void* q : ctx->pre_allocs) cudaFree(q);
-    ctx->pre_allocs.clear();
-    p = tc::PrefillScratch{};
+    tc::PrefillScratch grown;
+    std::vector<void*> allocs;
     auto get = [&](auto*& dst, size_t bytes) {
         void* raw = nullptr;
         if (!cuda_ok(ctx, cudaMalloc(&raw, bytes + 256), "cudaMalloc(prefill scratch)")) return false;
-        ctx->pre_allocs.push_back(raw);
+        allocs.push_back(raw);
         dst = static_cast<std::remove_reference_t<decltype(dst)>>(raw);
         return true;
     };
-    if (!(get(p.tiles, T * sizeof(tc::TokenTile)) && get(p.tile_count, 4) && get(p.xt, xt * 2) && get(p.xst, xt / 8) &&
-          get(p.xsumt, xt / 8) && get(p.ht, ht * 2) && get(p.hst, ht / 8) && get(p.hsumt, ht / 8))) {
-        for (void* q : ctx->pre_allocs) cudaFree(q);
-        ctx->pre_allocs.clear();
-        p = tc::PrefillScratch{};
-        return false;
+    const bool ok = get(grown.tiles, T * sizeof(tc::TokenTile)) && get(grown.tile_count, 4) && get(grown.xt, xt * 2) &&
+                    get(grown.xst, xt / 8) && get(grown.xsumt, xt / 8) && get(grown.ht, ht * 2) && get(grown.hst, ht / 8) &&
+                    get(grown.hsumt, ht / 8);
+    if (ok) {
+        cudaStreamSynchronize(ctx->stream);
+        grown.max_tiles = T, grown.xt_elems = xt, grown.ht_elems = ht;
+        p = grown;
+        allocs.swap(ctx->pre_allocs);
     }
-    p.max_tiles = T;
-    p.xt_elems = xt;
-    p.ht_elems = ht;
-    return true;
+    for (void* q : allocs) cudaFree(q);
+    return ok;
 }
 
 constexpr size_t SELF_FLAG_BYTES = 256;
@@ -224,13 +224,14 @@ bool self_window_reserve(tc_ctx* ctx, const tc::MoeDims& d, int max_tokens) {
     if (max_tokens <= 32) return true;  // those blocks need no window
     const size_t need = self_window_layout(d, std::min(max_tokens, SELF_WINDOW_TOKENS), nullptr);
     if (need <= ctx->self_bytes) return true;
-    cudaStreamSynchronize(ctx->stream);
-    if (ctx->self_window) cudaFree(ctx->self_window);
-    ctx->self_window = nullptr, ctx->self_bytes = 0;
     if (!ctx->self_epoch) {
         if (!cuda_ok(ctx, cudaMalloc(reinterpret_cast<void**>(&ctx->self_epoch), 32), "cudaMalloc(window)")) return false;
     }
-    if (!cuda_ok(ctx, cudaMalloc(reinterpret_cast<void**>(&ctx->self_window), need), "cudaMalloc(window)")) return false;
+    void* grown = nullptr;
+    if (!cuda_ok(ctx, cudaMalloc(&grown, need), "cudaMalloc(window)")) return false;
+    cudaStreamSynchronize(ctx->stream);
+    if (ctx->self_window) cudaFree(ctx->self_window);
+    ctx->self_window = static_cast<uint8_t*>(grown);
     cudaMemset(ctx->self_window, 0, SELF_FLAG_BYTES);
     cudaMemset(ctx->self_epoch, 0, 32);
     ctx->self_bytes = need;
@@ -312,8 +313,9 @@ bool ws_reserve(tc_ctx* ctx, const tc::MoeDims& d, int max_tokens) {
     tc::MoeDims n{std::max(w.hidden, d.hidden), std::max(w.experts, d.experts),
                   std::max(w.topk, d.topk), std::max(w.inter, d.inter)};
     int T = std::max(w.max_tokens, max_tokens);
-    cudaStreamSynchronize(ctx->stream);
-    ws_release(ctx);
+    const tc::Workspace before = w;  // (kept until the new one is whole, as in prefill_reserve)
+    std::vector<void*> before_allocs;
+    before_allocs.swap(ctx->ws_allocs);
     size_t slots = size_t(T) * n.topk;
     bool ok = ws_alloc(ctx, w.logits, size_t(T) * n.experts) && ws_alloc(ctx, w.ids, slots) &&
               ws_alloc(ctx, w.gates, slots) && ws_alloc(ctx, w.xq, size_t(T) * n.hidden) &&
@@ -330,8 +332,12 @@ bool ws_reserve(tc_ctx* ctx, const tc::MoeDims& d, int max_tokens) {
               ws_alloc(ctx, w.ticket, size_t(1)) && ws_alloc(ctx, w.grid_sync, size_t(tc::GRID_SYNC_WORDS));
     if (!ok) {
         ws_release(ctx);
+        w = before;
+        before_allocs.swap(ctx->ws_allocs);
         return false;
     }
+    cudaStreamSynchronize(ctx->stream);
+    for (void* p : before_allocs) cudaFree(p);
     w.status = ctx->status;
     cudaMemset(w.ticket, 0, sizeof(int));
     cudaMemset(w.grid_sync, 0, tc::GRID_SYNC_WORDS * sizeof(uint32_t));

@@ -92,3 +92,32 @@ def test_more_short_runs_than_the_kernel_lists(oracle, ctx):
     x = 0.1 * workloads.hidden_states(shape, t, seed=3)
     x[np.arange(sum(counts)) % t, np.repeat(np.arange(len(counts)), counts)] += 4.0
     check_block(oracle, ctx, shape, lw, x, arith="fast")
+
+
+@pytest.mark.parametrize("t", [20, 100, 300])
+def test_a_layer_that_cannot_be_had_leaves_the_others_working(oracle, ctx, t):
+    """Scratch is shared by a context's layers and grows with them. A layer whose scratch is more than the device has
+    is refused; the layers that are there, and graphs captured on them, go on as before."""
+    from tachyon_b200 import cuda
+
+    many = MoeShape("many", 32, 256, 1, 32, fmt="q8")
+    lw, other = layer_weights(oracle, ODD_Q8, 17), layer_weights(oracle, many, 17)
+    x = workloads.hidden_states(ODD_Q8, t, seed=t)
+    ctx.set_arithmetic(ctx.ARITH_FAST)
+    layer = make_layer(ctx, lw, ODD_Q8.topk, t)
+    xd, yd = ctx.to_device(x), ctx.to_device(np.zeros_like(x))
+    ctx.capture_begin()
+    layer.forward(xd, yd)
+    g = ctx.capture_end()
+    with pytest.raises(cuda.TachyonCudaError, match="memory"):
+        make_layer(ctx, other, many.topk, 1 << 28)  # 256 GB of logits
+    g.launch()
+    ctx.sync()
+    first = yd.get()
+    yd.set(np.zeros_like(x))
+    layer.forward(xd, yd)
+    ctx.sync()
+    assert np.array_equal(yd.get(), first)
+    assert np.abs(first - oracle_moe(oracle, lw, x, ODD_Q8.topk).proj).max() <= 2e-3
+    g.free()
+    layer.free()
