@@ -224,6 +224,12 @@ tc_moe_layer *tc_moe_ep_layer_create(tc_ctx *ctx, int hidden, int experts, int e
 int tc_umma_selftest(tc_ctx *ctx, const int8_t *a_rows_host, const int8_t *b_rows_host, int n,
                      int32_t *d_out_host);
 
+/* Self-check of two pieces of kernel arithmetic (no counterpart in the reference): the packed
+ * SwiGLU division against the IEEE one for every float, and the partition's small integer
+ * division for every dividend below 2^20 and divisor up to 4096. counts3: SwiGLU values
+ * compared, those that differ in a bit, quotients that differ (the last two must be 0). */
+int tc_arith_selftest(tc_ctx *ctx, uint64_t *counts3);
+
 /* The dense int8 rate of the tensor cores, measured (no counterpart in the reference):
  * every SM issues `batches` batches of 32 tcgen05 MMAs (128 x 256 x 32, int8 -> int32,
  * accumulating in tensor memory) from operands resident in shared memory. Returns the

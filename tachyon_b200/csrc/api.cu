@@ -1164,6 +1164,18 @@ int tc_umma_selftest(tc_ctx* ctx, const int8_t* a_rows, const int8_t* b_rows, in
     return 0;
 }
 
+int tc_arith_selftest(tc_ctx* ctx, uint64_t* counts3) {
+    cudaSetDevice(ctx->device);
+    unsigned long long* dev = nullptr;
+    if (!cuda_ok(ctx, cudaMalloc(reinterpret_cast<void**>(&dev), 3 * sizeof *dev), "cudaMalloc")) return -1;
+    cudaMemsetAsync(dev, 0, 3 * sizeof *dev, ctx->stream);
+    ctx->launches += tc::launch_arith_selftest(ctx->sms, dev, ctx->stream);
+    const bool ok = cuda_ok(ctx, cudaStreamSynchronize(ctx->stream), "arithmetic self-test") &&
+                    cuda_ok(ctx, cudaMemcpy(counts3, dev, 3 * sizeof *dev, cudaMemcpyDeviceToHost), "count readback");
+    cudaFree(dev);
+    return ok ? 0 : -1;
+}
+
 int tc_int8_peak(tc_ctx* ctx, int batches, double* ops_out, float* ms_out) {
     if (batches < 1) return fail(ctx, "tc_int8_peak: at least one batch");
     cudaSetDevice(ctx->device);

@@ -299,6 +299,10 @@ int launch_prefill(const MoeDims& d, bool gate_up, bool q4, const PrefillWeights
 int launch_umma_selftest(const int8_t* a_tile, const int8_t* b_tile, int n, int* d_out, int* status,
                       cudaStream_t stream);
 
+// silu2 over every float and div_small over every small pair against the exact forms (arith_selftest.cu); out:
+// device, three zeroed counts.
+int launch_arith_selftest(int sms, unsigned long long* out, cudaStream_t stream);
+
 int launch_combine(const MoeDims& d, int t, Workspace& ws, float* y, cudaStream_t stream);
 
 // The dense int8 tensor-core rate: `batches` batches of MMAs on each of `sms` SMs; returns the

@@ -174,6 +174,15 @@ __device__ __forceinline__ void bulk_copy_once(void* dst_smem, const void* src_g
         : "memory");
 }
 
+// a / b for a < DIV_SMALL, through the float unit: (a + 1/2) / b is at least 1 / (2 b) away from every integer,
+// and the approximate quotient's error is below that. (An integer division is some 25 instructions in a
+// dependent chain; a block's partition takes a dozen of them on its critical path. tc_arith_selftest
+// compares it with that division for every a and every b up to 4096.)
+constexpr unsigned DIV_SMALL = 1u << 20;
+__device__ __forceinline__ unsigned div_small(unsigned a, unsigned b) {
+    return unsigned(__fdividef(float(a) + 0.5f, float(b)));
+}
+
 // Exact int -> float for |v| < 2^22: the dp4a accumulates onto the bit pattern
 // of 1.5*2^23, whose float value is then 1.5*2^23 + v.
 __device__ __forceinline__ float lane_sum(int w, int x) {
@@ -258,6 +267,56 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
         : "=f"(r.x), "=f"(r.y)
         : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
     return r;
+}
+
+__device__ __forceinline__ float2 splat(float v) { return make_float2(v, v); }
+
+// a + b in one packed operation: fma(a, 1, b) with a 1 the compiler cannot see. (It fuses a packed
+// product into a packed addition that follows it, even where fusing is turned off for the scalar
+// forms, and also when the addition is written as an fma by a constant 1.)
+__device__ __forceinline__ float2 add2_exact(float2 a, float2 b, float2 one) { return fma2(a, one, b); }
+
+// exp_poly on two values: the same operations, packed. Rounding half away from
+// zero is truncation after adding the float below one half with the value's sign, which is exact
+// for the arguments that reach it (|x * log2 e| < 129).
+__device__ __forceinline__ float2 exp_poly2(float2 x, float2 one) {
+    auto clamp = [](float v) {
+        float r;
+        asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(v), "f"(-87.33655f));
+        asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(r), "f"(88.7f));
+        return r;
+    };
+    x.x = clamp(x.x), x.y = clamp(x.y);
+    const float2 z = mul2(x, splat(1.44269504088896340736f));
+    const int n0 = __float2int_rz(z.x + copysignf(0.49999997f, z.x)), n1 = __float2int_rz(z.y + copysignf(0.49999997f, z.y));
+    const float2 n = make_float2(__int2float_rn(n0), __int2float_rn(n1));
+    // x - n * c1 - n * c2, each product rounded first (negating a factor negates the product exactly)
+    const float2 r = add2_exact(mul2(n, splat(2.1219444e-4f)), add2_exact(mul2(n, splat(-0.6933594f)), x, one), one);
+    float2 y = splat(1.9875692e-4f);
+    y = add2_exact(mul2(y, r), splat(1.3981999e-3f), one);
+    y = add2_exact(mul2(y, r), splat(8.333452e-3f), one);
+    y = add2_exact(mul2(y, r), splat(4.1665796e-2f), one);
+    y = add2_exact(mul2(y, r), splat(0.16666665f), one);
+    y = add2_exact(mul2(y, r), splat(0.5f), one);
+    y = add2_exact(add2_exact(mul2(y, mul2(r, r)), r, one), one, one);
+    return make_float2(__int_as_float(__float_as_int(y.x) + (n0 << 23)), __int_as_float(__float_as_int(y.y) + (n1 << 23)));
+}
+
+// silu(g) = g / (1 + exp(-g)) on two values, correctly rounded as the IEEE division is: Markstein's
+// scheme (IBM J. Res. Dev. 34, 1990: a reciprocal refined once, a quotient, one correction by its exact
+// remainder), packed. Not for arguments whose quotient or remainder could leave the normal range:
+// `usable` becomes false for those. (tc_arith_selftest compares it with the division for every float g.)
+__device__ __forceinline__ float2 silu2(float2 g, float2 one, bool& usable) {
+    const float2 den = add2_exact(exp_poly2(make_float2(-g.x, -g.y), one), one, one);
+    float2 y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y.x) : "f"(den.x));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y.y) : "f"(den.y));
+    const float2 nden = make_float2(-den.x, -den.y);
+    y = fma2(y, fma2(nden, y, splat(1.0f)), y);
+    const float2 q = mul2(g, y);
+    usable = usable && fmaxf(den.x, den.y) < 1e18f && fminf(fabsf(g.x), fabsf(g.y)) > 1e-18f &&
+             fmaxf(fabsf(g.x), fabsf(g.y)) < 1e18f;
+    return fma2(fma2(nden, q, g), y, q);
 }
 
 }  // namespace tc

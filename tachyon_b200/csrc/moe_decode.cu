@@ -191,13 +191,6 @@ __device__ __forceinline__ void grid_arrive(uint32_t* ctr) {
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(ctr) : "memory");
 }
 
-// a / b for a < 2^20, through the float unit: (a + 1/2) / b is at least 1 / (2 b) away from every integer,
-// and the approximate quotient's error is below that. (An integer division is some 25 instructions in a
-// dependent chain; a block's partition takes a dozen of them on its critical path.)
-__device__ __forceinline__ unsigned div_small(unsigned a, unsigned b) {
-    return unsigned(__fdividef(float(a) + 0.5f, float(b)));
-}
-
 // What one of the two expert phases needs to know about its matrix and this warp's share.
 struct Phase {
     const uint8_t* tiled;
@@ -1043,6 +1036,12 @@ bool decode_config(const MoeDims& d, int t, int ids_slots, int sms, bool ep, Dec
     // Rows staged at a time: an expert's tokens, up to D_TOK of them, out of all the tokens the expert
     // phases see (every rank's when expert-parallel: ids_slots / topk).
     c.xcap = min(D_TOK, (ids_slots / d.topk + 7) / 8 * 8);
+    // The kernel divides with div_small: unit counts (of the experts walked or of the runs listed, plus the grid) and
+    // positions in a run's rows must stay below its limit, an expert's units below the divisors it is checked for.
+    // (They do wherever the rows fit in shared memory: 12 bytes a column at the least, so 2421 units an expert and,
+    // with 383 runs, 930 thousand in all.)
+    const int units = max((d.inter + 7) / 8, (d.hidden + 15) / 16);
+    if (units > 4096 || (long long)(ep ? D_MAX_RUNS : d.experts) * units + sms >= (long long)DIV_SMALL) return false;
     auto deepest = [&](int w, int rr) {
         for (int k = D_MAX_STAGES; k >= 2; k--)
             if (size_t(DLayout<KIND>(w, k, c.xcap, rr, d.hidden, d.inter, d.experts, d.topk, ids_slots).total) <= decode_smem_limit(ep))

@@ -66,6 +66,7 @@ SYMBOLS = {
     "tc_ep_barrier": (_i, [_vp]),
     "tc_moe_ep_layer_create": (_vp, [_vp, _i, _i, _i, _i, _vp, _vp, _vp, _i]),
     "tc_umma_selftest": (_i, [_vp, _vp, _vp, _i, _vp]),
+    "tc_arith_selftest": (_i, [_vp, _vp]),
     "tc_int8_peak": (_i, [_vp, _i, C.POINTER(C.c_double), C.POINTER(C.c_float)]),
     "tc_dispatch_static": (_i, [_vp, _vp, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp]),
     "tc_rmsnorm": (_i, [_vp, _vp, _vp, _f, _i, _i, _vp]),
@@ -280,6 +281,13 @@ class Context:
         self._check(self.lib.tc_umma_selftest(self.handle, _ptr(a_rows), _ptr(b_rows), n, _ptr(out)),
                     "tc_umma_selftest")
         return out
+
+    def arith_selftest(self) -> dict:
+        """The packed SwiGLU division over every float, and the small integer division over every small pair,
+        against the exact forms."""
+        n = np.zeros(3, np.uint64)
+        self._check(self.lib.tc_arith_selftest(self.handle, _ptr(n)), "tc_arith_selftest")
+        return {"silu_compared": int(n[0]), "silu_different": int(n[1]), "quotients_different": int(n[2])}
 
     def capture_begin(self):
         self._check(self.lib.tc_capture_begin(self.handle), "tc_capture_begin")

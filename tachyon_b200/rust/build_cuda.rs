@@ -30,6 +30,7 @@ const SOURCES: &[&str] = &[
     "int8_peak",
     "quantize",
     "umma_selftest",
+    "arith_selftest",
     "combine",
     "ep",
 ];

@@ -18,3 +18,18 @@ def test_one_tcgen05_int8_mma_is_exact(n):
     want = a.astype(np.int32) @ b.astype(np.int32).T
     assert np.array_equal(got, want)
     ctx.close()
+
+
+def test_packed_and_float_unit_divisions_are_exact():
+    """The packed SwiGLU division has the IEEE division's bits for every float it is used for (1e-18 to 1e18 in
+    magnitude, not below -41: 1.55e9 floats and the NaNs, in either half of a pair), and the partition's division
+    is the integer one."""
+    from tachyon_b200 import build, cuda
+
+    build.build()
+    ctx = cuda.Context(0)
+    n = ctx.arith_selftest()
+    assert n["silu_compared"] > 2 * 1_500_000_000
+    assert n["silu_different"] == 0
+    assert n["quotients_different"] == 0
+    ctx.close()
