@@ -295,8 +295,8 @@ int launch_prefill(const MoeDims& d, bool gate_up, bool q4, const PrefillWeights
                    const Workspace& ws, int slots, float* out, const uint32_t* out_rows, cudaStream_t stream,
                    float* const* peer_out = nullptr, int peer_ranks = 0, uint32_t peer_rows = 0);
 
-// One 128 x n x 32 int8 tcgen05 MMA (n = 64 or 128) through TMEM: a self-check of the encodings.
-int launch_umma_selftest(const int8_t* a_tile, const int8_t* b_tile, int n, int* d_out, int* status,
+// One 128 x n x 32 block (n = 64 or 128) of f16 values by tcgen05 through TMEM: a self-check of the encodings.
+int launch_umma_selftest(const uint16_t* a_tile, const uint16_t* b_tile, int n, float* d_out, int* status,
                       cudaStream_t stream);
 
 // silu2 over every float and div_small over every small pair against the exact forms (arith_selftest.cu); out:

@@ -80,10 +80,7 @@ struct Stage {
     static_assert(SMEM <= P_SMEM_LIMIT, "stages fit");
 };
 
-// Byte offset of (row, k) in a block's operand tile of `rows` rows x 32 f16: 8-row x 16-byte core matrices.
-__host__ __device__ constexpr uint32_t f16_tile_offset(uint32_t rows, uint32_t row, uint32_t k) {
-    return (k / 8) * (rows * 16) + (row / 8) * 128 + (row % 8) * 16 + (k % 8) * 2;
-}
+using umma::f16_tile_offset;
 
 struct PrefillArgs {
     const uint16_t* wt;      // weight tiles, f16 [expert][row tile][block][128 x 32 canonical]

@@ -1,16 +1,15 @@
 // tcgen05 (5th-generation tensor core) building blocks for sm_100a: shared-memory
-// matrix descriptors, the instruction descriptor for int8 x int8 -> int32,
+// matrix descriptors, the instruction descriptors (f16 x f16 -> f32, int8 x int8 -> int32),
 // TMEM allocation, MMA issue, commit, and TMEM loads. One thread issues an MMA
 // for the whole CTA; accumulators live in tensor memory (128 lanes x 512
 // 32-bit columns per SM) and come back to registers with tcgen05.ld.
 //
 // Operand tiles sit in shared memory in the K-major "no swizzle" canonical
-// layout: 8-row x 16-byte core matrices, each 128 contiguous bytes. For a tile
-// of R rows x 32 bytes of K (one quantization block of int8):
-//     offset(row, kbyte) = (kbyte / 16) * (R / 8) * 128 + (row / 8) * 128 + (row % 8) * 16 + kbyte % 16
-// so SBO (stride between 8-row groups) = 128 bytes and LBO (stride between the
-// two 16-byte K halves) = R * 16 bytes. Global memory holds the tiles in
-// exactly this order, so one bulk copy brings a tile in ready for the MMA.
+// layout: 8-row x 16-byte core matrices, each 128 contiguous bytes, those of 16 bytes of K
+// (8 f16 or 16 int8) one after another, R / 8 of them for R rows. So SBO (stride between
+// 8-row groups) = 128 bytes and LBO (stride between 16-byte pieces of K) = R * 16 bytes.
+// Global memory holds the tiles in exactly this order (f16_tile_offset), so one bulk copy
+// brings a tile in ready for the MMA.
 #pragma once
 
 #include <stdint.h>
@@ -82,23 +81,8 @@ __device__ __forceinline__ void commit(uint64_t* bar) {
 
 __device__ __forceinline__ void fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// 32 lanes (this warp's quadrant) x 32 consecutive 32-bit columns: thread i gets lane i's 32 values.
-__device__ __forceinline__ void ld_32x32(uint32_t taddr, int (&v)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
-          "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
-          "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-        : "r"(taddr)
-        : "memory");
-}
-
-// The same for 16 columns of f32 values.
+// 32 lanes (this warp's quadrant) x 16 consecutive columns of f32 values: thread i gets lane i's.
 __device__ __forceinline__ void ld_f32(uint32_t taddr, float (&v)[16]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
@@ -120,9 +104,9 @@ __device__ __forceinline__ void wait_ld(float (&v)[16]) {
                  : "memory");
 }
 
-// Byte offset of (row, kbyte) inside a tile of `rows` rows x 32 K-bytes.
-__host__ __device__ constexpr uint32_t tile_offset(uint32_t rows, uint32_t row, uint32_t kbyte) {
-    return (kbyte / 16) * (rows / 8) * 128 + (row / 8) * 128 + (row % 8) * 16 + kbyte % 16;
+// Byte offset of (row, k) in a block's operand tile of `rows` rows x 32 f16.
+__host__ __device__ constexpr uint32_t f16_tile_offset(uint32_t rows, uint32_t row, uint32_t k) {
+    return (k / 8) * (rows * 16) + (row / 8) * 128 + (row % 8) * 16 + (k % 8) * 2;
 }
 
 }  // namespace umma

@@ -273,7 +273,7 @@ class Context:
                 "shape": "tcgen05.mma kind::i8 m128 n256 k32, cta_group::1, operands resident in shared memory"}
 
     def umma_selftest(self, a_rows: np.ndarray, b_rows: np.ndarray) -> np.ndarray:
-        """a_rows i8[128, 32] x b_rows i8[n, 32]^T through one tcgen05 MMA; returns i32[128, n]."""
+        """a_rows i8[128, 32] x b_rows i8[n, 32]^T, as f16 through tcgen05 like a block of the expert kernels; returns i32[128, n]."""
         a_rows = np.ascontiguousarray(a_rows, np.int8)
         b_rows = np.ascontiguousarray(b_rows, np.int8)
         n = b_rows.shape[0]

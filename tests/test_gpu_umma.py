@@ -1,4 +1,5 @@
-"""The tcgen05 (tensor memory) building blocks: one int8 MMA must give the exact integer product."""
+"""The tcgen05 (tensor memory) building blocks as the expert kernels use them: a block of 8-bit values, as f16, must
+give the exact integer product. And the arithmetic that stands in for exact divisions."""
 import numpy as np
 import pytest
 
@@ -6,7 +7,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("n", [64, 128])
-def test_one_tcgen05_int8_mma_is_exact(n):
+def test_one_tcgen05_block_is_exact(n):
     from tachyon_b200 import build, cuda
 
     build.build()
@@ -14,8 +15,10 @@ def test_one_tcgen05_int8_mma_is_exact(n):
     rng = np.random.default_rng(n)
     a = rng.integers(-127, 128, size=(128, 32), dtype=np.int8)
     b = rng.integers(-127, 128, size=(n, 32), dtype=np.int8)
+    a[:2], b[:2] = -128, -128  # (the largest sums: 32 * 2^14)
     got = ctx.umma_selftest(a, b)
     want = a.astype(np.int32) @ b.astype(np.int32).T
+    assert want.max() == 1 << 19
     assert np.array_equal(got, want)
     ctx.close()
 
