@@ -102,7 +102,7 @@ def test_one_kernel_block_from_33_to_128_tokens(oracle, ctx, shape):
                 one, four = both_paths(ctx, layer, x, y0)
                 assert np.array_equal(one, four), (shape.name, t, b is not None, np.abs(one - four).max())
     finally:
-        ctx.set_prefill_threshold(32)
+        ctx.set_prefill_threshold(16)
         layer.free()
 
 

@@ -1,8 +1,9 @@
 """The tcgen05 (tensor memory) expert kernels against the oracle and against the
 bandwidth-oriented kernels: same fma chain per output, so the same bits.
 
-The library picks the tensor-core kernels from an average of 32 tokens per
-expert; the tests force either path with the threshold."""
+Past the one-kernel block's 128 tokens the library picks the tensor-core kernels from an
+average of 16 tokens per expert; the tests force either path with the threshold, and
+below 129 tokens with the one-kernel block off."""
 import numpy as np
 import pytest
 
@@ -12,7 +13,7 @@ from test_gpu_parity import check_block, ctx, layer_weights, make_layer  # noqa:
 
 pytestmark = pytest.mark.gpu
 
-NEVER = 1 << 30
+NEVER, DEFAULT = 1 << 30, 16
 
 
 def forward(ctx, layer, x, y0):
@@ -29,7 +30,7 @@ def forward(ctx, layer, x, y0):
 def always_prefill(ctx):
     ctx.set_prefill_threshold(0)
     yield ctx
-    ctx.set_prefill_threshold(32)
+    ctx.set_prefill_threshold(DEFAULT)
 
 
 @pytest.mark.parametrize("shape,t", [
@@ -57,31 +58,51 @@ def test_both_kernel_families_give_the_same_bits(oracle, ctx, fmt):
         layer = make_layer(ctx, lw, shape.topk, t)
         layer.set_router_bias(bias)
         try:
+            default = forward(ctx, layer, x, y0)  # up to 128 tokens: the one-kernel block
+            ctx.set_decode_block(False)
             ctx.set_prefill_threshold(NEVER)
             a = forward(ctx, layer, x, y0)
             ctx.set_prefill_threshold(0)
+            before = ctx.launch_count()
             b = forward(ctx, layer, x, y0)
+            assert ctx.launch_count() - before >= 5  # (the tensor-core kernels tile the activations first)
             b2 = forward(ctx, layer, x, y0)
         finally:
-            ctx.set_prefill_threshold(32)
+            ctx.set_decode_block(True)
+            ctx.set_prefill_threshold(DEFAULT)
             layer.free()
+        assert np.array_equal(a, default)
         assert np.array_equal(a, b)
         assert np.array_equal(b, b2)
 
 
 def test_default_threshold_switches_by_batch_size(oracle, ctx):
-    """Crossing the threshold must not change a token's output."""
+    """Crossing the threshold, or the end of the one-kernel block, must not change a token's output."""
     shape = MoeShape("small-q8", 256, 8, 2, 96, fmt="q8")
     lw = layer_weights(oracle, shape, 11)
     ctx.set_arithmetic(ctx.ARITH_FAST)
-    ctx.set_prefill_threshold(32)
-    x = workloads.hidden_states(shape, 256, seed=3)  # 256 * 2 / 8 = 64 per expert: tensor-core path
+    ctx.set_prefill_threshold(DEFAULT)
+    x = workloads.hidden_states(shape, 256, seed=3)
     y0 = np.zeros_like(x)
     layer = make_layer(ctx, lw, shape.topk, 256)
-    big = forward(ctx, layer, x, y0)
-    small = forward(ctx, layer, x[:40], y0[:40])     # 10 per expert: bandwidth path
-    layer.free()
-    assert np.array_equal(big[:40], small)
+
+    def run(t, launches):
+        before = ctx.launch_count()
+        y = forward(ctx, layer, x[:t], y0[:t])
+        assert ctx.launch_count() - before == launches
+        return y
+
+    try:
+        big = run(256, 5)      # 64 per expert: tensor-core path
+        one = run(40, 1)       # the one-kernel block
+        ctx.set_decode_block(False)
+        at = run(64, 5)        # 16 per expert: tensor-core path
+        below = run(63, 4)     # bandwidth path
+    finally:
+        ctx.set_decode_block(True)
+        layer.free()
+    for y in (one, at, below):
+        assert np.array_equal(big[:len(y)], y)
 
 
 def test_scratch_shared_by_layers_only_grows(oracle, ctx):
@@ -107,7 +128,7 @@ def test_scratch_shared_by_layers_only_grows(oracle, ctx):
             assert np.abs(got - want).max() <= 2e-3
             assert np.mean(np.all(got == want, axis=1)) > 0.5
     finally:
-        ctx.set_prefill_threshold(32)
+        ctx.set_prefill_threshold(DEFAULT)
         la.free()
         lb.free()
 

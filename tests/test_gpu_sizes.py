@@ -1,6 +1,6 @@
 """Parity at the sizes the workloads name, not only at toy token counts: the
 routing-skew shape at 256, 4096 and 16384 tokens, the 3b-a800m shape in 4 bits at a
-prefill of 4 x 1024 tokens, and the 1b-a400m shape at the batch where the library
+prefill of 4 x 1024 tokens, and the 1b-a400m shape at the batches where the library
 switches kernel families. Both families (the bandwidth-oriented kernels and the
 tcgen05 ones) against the oracle, and against each other bit for bit."""
 import numpy as np
@@ -12,14 +12,14 @@ from test_gpu_parity import check_block, ctx, layer_weights, make_layer, oracle_
 
 pytestmark = pytest.mark.gpu
 
-NEVER = 1 << 30
+NEVER, DEFAULT = 1 << 30, 16
 SKEW = MoeShape("skew", 2048, 64, 8, 1024, fmt="q8")
 
 
 @pytest.fixture
 def thresholds(ctx):
     yield ctx
-    ctx.set_prefill_threshold(32)
+    ctx.set_prefill_threshold(DEFAULT)
     ctx.set_arithmetic(ctx.ARITH_FAST)
 
 
@@ -89,20 +89,26 @@ def test_granite_3b_shape_4bit_prefill_of_4096_tokens(oracle, thresholds):
     shape = MoeShape("3b-q4", 1536, 40, 8, 512, fmt="q4")
     lw = layer_weights(oracle, shape, 1)
     x = workloads.hidden_states(shape, 4096, seed=23)
-    ctx.set_prefill_threshold(32)  # the library's own choice at this size: the tcgen05 kernels
+    ctx.set_prefill_threshold(DEFAULT)  # the library's own choice at this size: the tcgen05 kernels
     check_block(oracle, ctx, shape, lw, x, arith="fast")
 
 
 @pytest.mark.parametrize("fmt", ["q8", "q4"])
 def test_granite_1b_shape_at_the_switch_between_kernel_families(oracle, thresholds, fmt):
-    """Batch 128 of the 1b-a400m shape averages exactly 32 tokens per expert, the default
-    threshold; 127 tokens stay on the other side. Both against the CPU path, and the shared
-    tokens bit for bit against each other."""
+    """128 tokens are the one-kernel block's last batch, 129 the tensor-core kernels' first. Without the one-kernel
+    block 64 tokens average exactly 16 per expert, the default threshold, and 63 stay on the bandwidth side.
+    All against the CPU path, and the shared tokens bit for bit against one another."""
     ctx = thresholds
     shape = MoeShape("1b", 1024, 32, 8, 512, fmt=fmt)
     lw = layer_weights(oracle, shape, 0)
-    x = workloads.hidden_states(shape, 128, seed=24)
-    ctx.set_prefill_threshold(32)
-    a = check_block(oracle, ctx, shape, lw, x, arith="fast")
-    b = check_block(oracle, ctx, shape, lw, x[:127], arith="fast")
-    assert np.array_equal(a[:127], b)
+    x = workloads.hidden_states(shape, 129, seed=24)
+    ctx.set_prefill_threshold(DEFAULT)
+    outs = []
+    try:
+        for t, one_kernel in [(129, True), (128, True), (64, False), (63, False)]:
+            ctx.set_decode_block(one_kernel)
+            outs.append(check_block(oracle, ctx, shape, lw, x[:t], arith="fast"))
+    finally:
+        ctx.set_decode_block(True)
+    for y in outs[1:]:
+        assert np.array_equal(outs[0][:len(y)], y)
