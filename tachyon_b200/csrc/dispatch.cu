@@ -174,8 +174,9 @@ __global__ void __launch_bounds__(DISPATCH_E_THREADS) dispatch_experts_kernel(co
     if (hits) {
         walk([&](int i, uint32_t id) {
             const unsigned ballot = __ballot_sync(0xffffffffu, id == e);
-            if (id == e) {
-                const uint32_t p = at + __popc(ballot & ((1u << lane) - 1u));
+            const uint32_t p = at + __popc(ballot & ((1u << lane) - 1u));
+            // (The bound: after a wait for another rank has run out, its ids may still arrive between the two reads.)
+            if (id == e && p < first + total) {
                 a.perm[p] = uint32_t(i);
                 a.slot_token[p] = uint32_t(i) / uint32_t(a.topk);
                 a.pos[i] = p;
