@@ -37,10 +37,14 @@ struct tc_ctx {
     tc::EpState ep;           // expert parallelism (size 1 until tc_ep_init)
     tc::PrefillScratch pre;   // token tiles of the tcgen05 path
     std::vector<void*> pre_allocs;
-    // Tokens per expert (on average) from which the tcgen05 kernels take over. Below the one-kernel block's 128
-    // tokens it does not matter; at the first sizes past it they are ahead from 16 on: 64 experts of 2048
-    // columns, 8 picks, 130 tokens 240 against 246 us per block, 180 tokens 253 against 304, with a router that
-    // prefers a few experts 257 against 1062; the 3b shape at 159 tokens 124 against 159.
+    // Tokens per expert (on average) from which the tcgen05 kernels take over, past the one-kernel block's 128 tokens.
+    // 16 is about where they cross the bandwidth-oriented ones under an even router (us per block, tcgen05 / the
+    // others, 8-bit, 8 picks): 64 experts of 2048 x 1024 at 129 tokens, an average of 16.1: 239 / 250; 128 experts of
+    // 1024 x 512 at 14: 166 / 156, 16: 169 / 163, 20: 171 / 172; 256 of them at 14: 293 / 266, 16: 295 / 281, 20: 303 / 312;
+    // 96 of 2048 x 768, 4 picks, at 13: 283 / 271, 16: 285 / 274, 20: 289 / 330. 4-bit weights cross at the same place;
+    // 32 to 40 experts are past it at 129 tokens (80 / 104, 110 / 135). A router that prefers a few experts puts the
+    // tcgen05 kernels far ahead below the line too: 128 experts at 144 tokens, an average of 9, with a Zipf bias 110 / 447.
+    // But the counts are on the device and the choice is made on the host, from the average.
     int prefill_min_avg = 16;
     float* host_x = nullptr;  // device staging for the host-buffer entry point (large batches)
     float* host_y = nullptr;
@@ -960,8 +964,12 @@ int moe_enqueue(tc_moe_layer* layer, const float* x, const float* norm_w, float 
     if (form == 2) {
         // Up to 128 tokens: still one kernel, in its expert-parallel form with this GPU as the only
         // rank (an expert's tokens in runs of up to 32; rows and outputs through the local window).
-        // Measured at the 1b-a400m shape, 24 blocks: 0.81 ms at 64 tokens (1.82 as separate kernels), 1.12 at
-        // 128 (the tcgen05 kernels 1.8 when they were last compared there).
+        // It is ahead of the separate kernels up to its end (us per block at 128 tokens, one kernel / tcgen05 /
+        // bandwidth-oriented, even router): 1b shape 48 / 80 / 102, 3b 60 / 110 / 130, 64 experts of 2048 x 1024
+        // 129 / 239 / 249, 128 of 1024 x 512 71 / 161 / 109, 256 of them 112 / 262 / 161; in 4 bits 56 / 84 / 106,
+        // 73 / 117 / 134, 176 / 248 / 254, 81 / 163 / 112, 111 / 272 / 162; with a Zipf bias on the router 52 / 92 / 227,
+        // 69 / 115 / 267, 146 / 250 / 786. At 129 tokens the first three take 80, 110 and 239. (The end is not where the
+        // sides cross: a token takes a CTA of its own in the router phase and the combine, and there are 148.)
         self.ranks = 1, self.me = 0, self.first = 0, self.local = d.experts;
         self.base[0] = ctx->self_window;
         self.epoch = ctx->self_epoch + 4;

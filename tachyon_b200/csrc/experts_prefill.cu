@@ -27,11 +27,16 @@
 // remainder of 128, 64 or 32 columns (4-bit: 64 at most, since each output keeps a second chain).
 // Every wait is bounded; TMEM is freed on every path.
 //
-// Measured (granite-1b-a400m, 4096 tokens, int8): gate_up 352 -> 234 us, down 220 -> 103 us against the
+// Measured (granite-1b-a400m, 4096 tokens, int8): gate_up 352 -> 233 us, down 220 -> 110 us against the
 // form with 64-column tiles, kind::i8, one tile per CTA, f32 SwiGLU rows in memory and a
-// kernel that tiled them for down. That is 375-410 cycles per unit: two float warps per scheduler do not
-// cover each other's waits for tensor memory, shared memory (which the products read at
-// 128 bytes a clock a third of the time) and the hand-over. Tried: 16 float warps of 32 columns (as
+// kernel that tiled them for down. Where gate_up's 233 go: 24 tile the activations; the kernel's busiest CTA
+// works off 960 units in 364 thousand cycles, 203 us at the 1.79 GHz the SMs hold under it. (An average CTA has
+// 905 units, 886 without the tiles' padding; the last of 15 rounds of tiles is two thirds full.) A unit takes 375
+// cycles of a float warp: 334 its chains, 12 waiting for a tile's first sums, 9 for later ones, 13 parking the tile
+// and waiting for the space. down, with half as many blocks per tile: 430, of which chains 355, waits 34, parking 26.
+// (64 experts of 2048 x 1024: 355 and 395.) The chains take 334 instead of 180 because two float warps per
+// scheduler do not cover each other's waits for tensor memory and shared memory (which the products read at
+// 128 bytes a clock a third of the time). Tried: 16 float warps of 32 columns (as
 // fast, a third more instructions), hand-over block by block (5 % slower), polling instead of suspended
 // waits (no change), mma.sync with the sums in registers (8 % slower), kind::i8 (10 % slower).
 #include <algorithm>

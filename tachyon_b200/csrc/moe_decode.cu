@@ -33,10 +33,11 @@
 // (the length with the least work on the busiest warp), the (run, unit) pairs are what CTAs and
 // warps share out, every CTA stays inside one run, and the run's slot list is built by all
 // warps of the CTA. Rows, ids and expert outputs travel through per-rank windows (peer memory
-// over NVLink, or local memory when there is one rank) and the rendezvous are system-scope
-// counters in those windows that only grow. Which records a warp needs depends on the routing
-// there, so nothing is copied into shared memory before the router phase; the rank's share of
-// the layer is asked into L2 instead.
+// over NVLink, or local memory when there is one rank) and the rendezvous are counters in those
+// windows that only grow: at system scope between GPUs, at GPU scope when there is one rank.
+// Which records a warp needs depends on the routing there, so nothing is copied into shared memory
+// before the router phase. Between GPUs the rank's share of the layer is asked into L2
+// meanwhile; on one GPU nothing is, because the requests delay the router phase (see l2_all).
 //
 // No token -> expert permutation is built: with at most 32 tokens every CTA keeps
 // the batch's expert ids in shared memory and lists, per expert of its range, the
