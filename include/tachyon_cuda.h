@@ -129,8 +129,8 @@ int tc_moe_layer_detach_experts(tc_moe_layer *layer);
  * adds one on both the CPU and the GPU side. bias_host: f32[experts]. */
 int tc_moe_set_router_bias(tc_moe_layer *layer, const float *bias_host);
 /* y[t,hidden] += moe(x[t,hidden]); x is the normed input (`s.xb`), y the
- * residual stream (`s.x`): src/model.rs:671-681. Device pointers; enqueued on
- * the context's stream, returns without waiting. */
+ * residual stream (`s.x`): src/model.rs:671-681. Device pointers, 16-byte aligned;
+ * enqueued on the context's stream, returns without waiting. */
 int tc_moe_forward(tc_moe_layer *layer, const float *x_dev, int t, float *y_dev);
 /* The whole MLP block of a MoE layer on the residual stream, as
  * src/model.rs:662-681 runs it: y[t,hidden] += moe(rmsnorm(y, norm_weight, eps)).

@@ -898,6 +898,8 @@ int moe_enqueue(tc_moe_layer* layer, const float* x, const float* norm_w, float 
     tc_ctx* ctx = layer->ctx;
     if (t <= 0) return fail(ctx, "empty batch");
     if (t > layer->max_tokens) return fail(ctx, "%d tokens, layer was created for %d", t, layer->max_tokens);
+    if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) % 16)
+        return fail(ctx, "x and y must be 16-byte aligned: their rows are read 16 bytes at a time");
     if (ctx->arith == tc::ARITH_CPU_LANES && !layer->gu.data)
         return fail(ctx, "TC_ARITH_CPU_LANES reads the expert matrices as uploaded, and this layer's were detached");
     const tc::MoeDims& d = layer->dims;

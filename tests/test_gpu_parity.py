@@ -308,6 +308,12 @@ def test_bad_arguments_are_refused(ctx):
         layer.forward(x, x)
     with pytest.raises(cuda.TachyonCudaError):  # empty batch (src/model.rs:565)
         layer.forward(x, x, t=0)
+    one = ctx.to_device(np.ones(64, np.float32))
+    for xo, yo in [(4, 0), (0, 8), (12, 12)]:  # rows that 16-byte loads cannot read
+        assert ctx.lib.tc_moe_forward(layer.handle, x.ptr + xo, 1, x.ptr + 256 + yo) != 0
+        assert "aligned" in ctx.last_error()
+    assert ctx.lib.tc_moe_block(layer.handle, one.ptr, 1e-6, 1, x.ptr + 4) != 0
+    ctx.sync()
     layer.free()
 
 
