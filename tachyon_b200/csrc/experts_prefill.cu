@@ -7,9 +7,14 @@
 // One block of 32 columns is one product of its own into its own tensor-memory buffer: the block's
 // sums must leave the tensor core to be scaled before they can be added.
 //
-// What bounds it: that float work, two packed FP32 operations per output pair and block: 139 cycles
-// per 128 x 64 x 32 unit and SM, 180 with the tensor-memory loads. So everything else is kept off the
-// float warps' issue slots and off the FP32 pipe:
+// What bounds it, in cycles per 128 x 64 x 32 unit and SM: that float work, two packed FP32 operations per output pair
+// and block, 128 (and 34 of the finishing warps); the reads of tensor memory, 128 (the 16-lane shape moves half of what
+// the 32-lane one does) beside the products' own 37; and shared memory at 128 bytes a clock: 64 for the products'
+// operands, 66 for the copies that bring them, 80 for the scales. So:
+//  - A lane has 4 rows x 16 tokens (the 16x256b shape), 20 words of scales per 64 outputs. With a row of 64 tokens
+//    (32x32b) they were 65 words: 272 cycles of shared memory a unit beside the other 130, in units of 365 to 430.
+//  - The float loop's code is 4 blocks long with constant addresses, a barrier test and an arrival per 2 blocks;
+//    the finishing code is rolled. (Unrolled as far as 16 KB it cost the float warps 20 % in instruction fetches.)
 //  - The operands are the 8-bit values as f16 (kind::f16). Products and sums of a block are
 //    integers below 2^20, exact in the f32 accumulator, so the sums arrive as floats. With kind::i8
 //    every sum costs a conversion besides (238 cycles per unit); with mma.sync, which would leave the
@@ -27,18 +32,13 @@
 // remainder of 128, 64 or 32 columns (4-bit: 64 at most, since each output keeps a second chain).
 // Every wait is bounded; TMEM is freed on every path.
 //
-// Measured (granite-1b-a400m, 4096 tokens, int8): gate_up 352 -> 233 us, down 220 -> 110 us against the
-// form with 64-column tiles, kind::i8, one tile per CTA, f32 SwiGLU rows in memory and a
-// kernel that tiled them for down. Where gate_up's 233 go: 24 tile the activations; the kernel's busiest CTA
-// works off 960 units in 364 thousand cycles, 203 us at the 1.79 GHz the SMs hold under it. (An average CTA has
-// 905 units, 886 without the tiles' padding; the last of 15 rounds of tiles is two thirds full.) A unit takes 375
-// cycles of a float warp: 334 its chains, 12 waiting for a tile's first sums, 9 for later ones, 13 parking the tile
-// and waiting for the space. down, with half as many blocks per tile: 430, of which chains 355, waits 34, parking 26.
-// (64 experts of 2048 x 1024: 355 and 395.) The chains take 334 instead of 180 because two float warps per
-// scheduler do not cover each other's waits for tensor memory and shared memory (which the products read at
-// 128 bytes a clock a third of the time). Tried: 16 float warps of 32 columns (as
-// fast, a third more instructions), hand-over block by block (5 % slower), polling instead of suspended
-// waits (no change), mma.sync with the sums in registers (8 % slower), kind::i8 (10 % slower).
+// Measured (granite-1b-a400m, 4096 tokens, int8; 24 us of gate_up tile the activations): gate_up 234 -> 195 us, down 109
+// -> 92; 64 experts of 2048 x 1024: 812 -> 664, 383 -> 314; 40 of 1536 x 512 in 4 bits at 2047 tokens: 276 -> 230, 138 ->
+// 115. A unit takes 330 cycles now (365 to 430 before); nothing in it is saturated, two float warps per scheduler share its
+// issue slots with a finishing warp. Tried: 16 float warps of 32 columns (as before or slower), the loop rolled to a
+// block (4 warps' bookkeeping: 342 instructions a unit against 177) or to a chunk (211 / 99 us), pieces of 32 values a
+// lane (spills), a block's scales read a block ahead (spills), polling instead of suspended waits (no change), kind::i8
+// (conversions: 10 % slower), mma.sync with the sums in registers (8 % slower).
 #include <algorithm>
 #include <type_traits>
 
@@ -64,7 +64,7 @@ constexpr size_t P_SMEM_LIMIT = 227 * 1024 - 256;  // the kernel also has a few 
 constexpr int P_HSTRIDE = P_ROWS + 4;   // floats per parked token (the pad keeps 16-byte reads conflict-free)
 
 // Registers: 128 a thread at launch (ptxas gives a 512-thread block that many), then split.
-constexpr int P_REGS_LAUNCH = 128, P_REGS_FLOAT = 168, P_REGS_ISSUE = 64, P_REGS_FINISH = 112;
+constexpr int P_REGS_LAUNCH = 128, P_REGS_FLOAT = 176, P_REGS_ISSUE = 56, P_REGS_FINISH = 104;
 static_assert((P_EW * P_REGS_FLOAT + P_IW * P_REGS_ISSUE + P_FW * P_REGS_FINISH) * 32 <= P_THREADS * P_REGS_LAUNCH, "register split");
 
 __host__ __device__ constexpr int prefill_columns(bool q4) { return q4 ? 64 : 128; }  // the largest token tile
@@ -171,157 +171,211 @@ __device__ __forceinline__ uint32_t half_of(uint32_t c) { return c % P_NGRP; }
 __device__ __forceinline__ uint32_t half_par(uint32_t c) { return (c / P_NGRP) & 1; }
 
 struct Bars {
-    uint64_t *full, *empty;    // [stages] operands landed; left by every float warp (and, before them, by the MMAs)
-    uint64_t *tfull, *tempty;  // [P_NGRP] a chunk's sums are in TMEM; read out by every float warp
+    uint64_t *full, *empty;    // [stages] operands landed; left by the MMAs and every float warp (the issuer passes it on)
+    uint64_t *tfull, *tempty;  // [P_NGRP] a chunk's sums are in TMEM, its scales in shared memory; read by every float warp
     uint64_t *pfull, *pempty;  // a tile has been parked by every float warp; taken by every finishing warp
     uint64_t* drain;           // after a failure only: the issuer's MMAs so far are done
     volatile int* abort_flag;
 };
+
+// The token tile of a CTA's work item, read one item ahead by every role: the trip to L2 would otherwise stand at the
+// start of each tile, in every warp.
+__device__ __forceinline__ TokenTile tile_of(const PrefillArgs& a, int w, int work) {
+    return a.tiles[w < work ? w / a.row_tiles : 0];
+}
 
 __device__ __forceinline__ float4 staged_f4(uint32_t addr) {
     float4 v;
     asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
     return v;
 }
-__device__ __forceinline__ float staged_f1(uint32_t addr) {
-    float v;
-    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+__device__ __forceinline__ float2 staged_f2(uint32_t addr) {
+    float2 v;
+    asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr));
     return v;
 }
+// Where a tile's logical row sits in the product, so that a lane's four rows are neighbours (see float_chains).
+__host__ __device__ constexpr int product_row(int r) { return (r & ~31) + (r & 3) * 8 + ((r & 31) >> 2); }
+// Where a token's scale sits among its tile's: a lane's four columns of every sixteen are neighbours.
+__host__ __device__ constexpr int scale_place(int n) { return (n & ~15) + ((n & 7) >> 1) * 4 + ((n & 8) >> 2) + (n & 1); }
 
-// One tile's float work for this warp's 32 rows x CW tokens: reads each block's sums from TMEM (a piece
-// ahead of the arithmetic: the load is asynchronous until wait_ld, and two register pieces
-// alternate) and keeps the chains in registers. A barrier is tested one piece of arithmetic before the
-// answer is needed.
+// One tile's float work for this warp's 32 rows x CW tokens: reads each block's sums from TMEM half a block (the lower
+// or upper 16 rows) ahead of the arithmetic (the load is asynchronous until wait_ld, and two register pieces
+// alternate) and keeps the chains in registers. A lane has 4 rows x CW / 4 tokens (the order of an m16n8
+// accumulator in each half of the quadrant), so a block's scales are CW / 4 + 4 values a lane; the next block's
+// replace them as they are used up. Four blocks, one turn of the TMEM halves, are a pass of the loop: its addresses are
+// constants but for the stages', and a chunk costs one test of a barrier and one arrival. `turn`: turns so far.
 template <bool Q4, int CW>
-__device__ __forceinline__ void float_chains(float (&acc)[64], float (&off)[Q4 ? 32 : 1], uint32_t& c, uint32_t smem,
-                                             const Bars& bars, uint32_t tbase, int nb, int col0, int row, int lane) {
+__device__ __forceinline__ void float_chains(float (&acc)[64], float (&off)[Q4 ? 32 : 1], uint32_t& turn, uint32_t smem,
+                                             const Bars& bars, uint32_t tbase, int nb, int col0, int row0, int lane) {
     using S = Stage<Q4>;
-    constexpr int N = CW * 2, PC = 16, PIECES = CW / PC;
+    // A piece: half of the rows x up to 32 columns.
+    constexpr int N = CW * 2, CC = CW < 32 ? CW : 32, PC = CC / 2, PIECES = CW / CC * 2;
     float v[2][PC];
+    float2 w[2], wc[Q4 ? 2 : 1];
+    float4 x[CW / 16], u[Q4 ? CW / 16 : 1];
+    const uint32_t wat = S::WD + (row0 + (lane >> 2) * 4) * 4, xat = S::XS + (col0 + (lane & 3) * 4) * 4;
+    auto row_scales = [&](uint32_t st, int k, int h) {  // of the lane's two rows in half h
+        w[h] = staged_f2(st + wat + (k * P_ROWS + 2 * h) * 4);
+        if (Q4) wc[Q4 ? h : 0] = staged_f2(st + wat + (S::WC - S::WD) + (k * P_ROWS + 2 * h) * 4);
+    };
+    auto column_scales = [&](uint32_t st, int k, int j) {  // of the lane's columns among sixteen
+        x[j] = staged_f4(st + xat + (k * N + j * 16) * 4);
+        if (Q4) u[Q4 ? j : 0] = staged_f4(st + xat + (S::XSUM - S::XS) + (k * N + j * 16) * 4);
+    };
+    auto chains = [&](const float (&cur)[PC], int p, int j) {  // columns 16 j .. of piece p
+        const int h = p & 1;
+        const float w2[2] = {w[h].x, w[h].y}, c2[2] = {wc[Q4 ? h : 0].x, wc[Q4 ? h : 0].y};
+        const float4 xj = x[j], uj = u[Q4 ? j : 0];
+#pragma unroll
+        for (int q = 0; q < 2; q++) {  // 8 columns: two rows x two neighbouring tokens
+            const float2 x2 = q ? make_float2(xj.z, xj.w) : make_float2(xj.x, xj.y);
+            const float2 u2 = q ? make_float2(uj.z, uj.w) : make_float2(uj.x, uj.y);
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+                const int i = 8 * (j - p / 2 * (CC / 16)) + 4 * q + 2 * r, o = p * PC + i;
+                const float2 s = fma2(make_float2(cur[i], cur[i + 1]), mul2(splat(w2[r]), x2), make_float2(acc[o], acc[o + 1]));
+                acc[o] = s.x, acc[o + 1] = s.y;
+                if (Q4) {
+                    const float2 f = fma2(splat(c2[r]), u2, make_float2(off[o], off[o + 1]));
+                    off[o] = f.x, off[o + 1] = f.y;
+                }
+            }
+        }
+    };
 #pragma unroll
     for (int j = 0; j < CW; j++) {
         acc[j] = 0.0f;
         if (Q4) off[j] = 0.0f;
     }
-    auto fetch = [&](uint32_t half, int k, int p, float (&dst)[PC]) {
-        umma::ld_f32(tbase + (half * P_CHUNK + k) * P_TBUF + col0 + p * PC, dst);
-    };
-    // A piece's scales: one of its row, PC of its tokens (4-bit: and the offsets').
-    struct Scales {
-        float w, c;
-        float4 x[PC / 4], u[Q4 ? PC / 4 : 1];
-    };
-    auto chains = [&](const float (&cur)[PC], int p, const Scales& sc) {
-        const float2 w = make_float2(sc.w, sc.w), cc = make_float2(sc.c, sc.c);
+    const uint32_t sums = tbase + col0;
+    auto fetch = [&](uint32_t at, int p) { umma::ld_half_f32(at + p / 2 * 32 + (uint32_t(p & 1) << 20), v[p & 1]); };
+    auto first_scales = [&](uint32_t st, int k) {
+        row_scales(st, k, 0);
+        row_scales(st, k, 1);
 #pragma unroll
-        for (int j = 0; j < PC / 4; j++) {
-            const float4 x = sc.x[j];
-            const int i = 4 * j, o = p * PC + i;
-            const float2 r0 = fma2(make_float2(cur[i], cur[i + 1]), mul2(w, make_float2(x.x, x.y)), make_float2(acc[o], acc[o + 1]));
-            const float2 r1 = fma2(make_float2(cur[i + 2], cur[i + 3]), mul2(w, make_float2(x.z, x.w)), make_float2(acc[o + 2], acc[o + 3]));
-            acc[o] = r0.x, acc[o + 1] = r0.y, acc[o + 2] = r1.x, acc[o + 3] = r1.y;
-            if (Q4) {
-                const float4 u = sc.u[Q4 ? j : 0];
-                const float2 o0 = fma2(cc, make_float2(u.x, u.y), make_float2(off[o], off[o + 1]));
-                const float2 o1 = fma2(cc, make_float2(u.z, u.w), make_float2(off[o + 2], off[o + 3]));
-                off[o] = o0.x, off[o + 1] = o0.y, off[o + 2] = o1.x, off[o + 3] = o1.y;
+        for (int j = 0; j < CW / 16; j++) column_scales(st, k, j);
+    };
+    // A half's chunk has been read, sums and scales: the issuer may overwrite them.
+    auto release = [&](int half) {
+        umma::fence_before_sync();
+        __syncwarp();
+        mbar_arrive_if(bars.tempty + half, lane == 0);
+    };
+    const int whole = nb / (P_NGRP * P_CHUNK);
+    if (whole > 0) {
+        wait_or_abort(bars.tfull, turn & 1, bars.abort_flag);
+        umma::fence_after_sync();
+        fetch(sums, 0);
+        first_scales(smem + (turn & 1) * P_NGRP * S::BYTES, 0);
+    }
+#pragma unroll 1
+    for (int t = 1; t <= whole; t++, turn++) {
+        const uint32_t par = turn & 1, st = smem + par * P_NGRP * S::BYTES, other = smem + (par ^ 1) * P_NGRP * S::BYTES;
+        const bool again = t < whole;
+#pragma unroll
+        for (int i = 0; i < P_NGRP * P_CHUNK; i++) {
+            const int half = i / P_CHUNK, kn = (i + 1) % P_CHUNK;
+            const bool ends = kn == 0, last = i + 1 == P_NGRP * P_CHUNK, more = !last || again;
+            const uint32_t next = last ? other : st + (i + 1) / P_CHUNK * S::BYTES;  // the next block's stage
+            bool ready = true;
+#pragma unroll
+            for (int p = 0; p < PIECES; p++) {
+                const bool final = p + 1 == PIECES;
+                umma::wait_ld(v[p & 1]);
+                if (final && ends) release(half);
+                if (final && ends && more) {
+                    if (!ready) wait_or_abort(bars.tfull + (half ^ 1), last ? par ^ 1 : par, bars.abort_flag);
+                    umma::fence_after_sync();
+                }
+                if (!final) fetch(sums + i * P_TBUF, p + 1);
+                else if (more) fetch(sums + (last ? 0 : i + 1) * P_TBUF, 0);
+                if (p + 2 == PIECES && ends && more) ready = mbar_test(bars.tfull + (half ^ 1), last ? par ^ 1 : par);
+                // The next block's scales, as this one's are used up (another chunk's once it is known to be there).
+                if (final && ends && more) {
+                    row_scales(next, kn, 0);
+#pragma unroll
+                    for (int j = 0; j < p / 2 * (CC / 16); j++) column_scales(next, kn, j);
+                }
+#pragma unroll
+                for (int j = p / 2 * (CC / 16); j < (p / 2 + 1) * (CC / 16); j++) {
+                    chains(v[p & 1], p, j);
+                    if ((p & 1) && more && (final || !ends)) column_scales(next, kn, j);
+                }
+                if (p + 2 == PIECES && !ends) row_scales(next, kn, 0);
+                if (final && more) row_scales(next, kn, 1);
             }
         }
-    };
-    // A chunk of NBLK blocks in TMEM half HALF (constants keep the addresses out of the loop's
-    // arithmetic); its first piece is already on its way into v[0].
-    auto chunk = [&](bool more, auto nblk_c, auto half_c) {
-        constexpr int NBLK = decltype(nblk_c)::value, ITEMS = NBLK * PIECES;
-        constexpr uint32_t HALF = decltype(half_c)::value;
-        const uint32_t st = smem + stage_of<Q4>(c) * S::BYTES;
-        const uint32_t ws = st + S::WD + row * 4, xs = st + S::XS + col0 * 4;
-        const uint32_t wcs = st + S::WC + row * 4, su = st + S::XSUM + col0 * 4;
-        bool ready = false;
+    }
+    // What is left of a number of blocks that is no multiple of four (a turn all the same, of fewer blocks).
+    if (const int rest = nb - whole * P_NGRP * P_CHUNK) {
+        const uint32_t st = smem + (turn & 1) * P_NGRP * S::BYTES;
+#pragma unroll 1
+        for (int half = 0; half < P_NGRP; half++) {
+            wait_or_abort(bars.tfull + half, turn & 1, bars.abort_flag);
+            umma::fence_after_sync();
+#pragma unroll 1
+            for (int k = 0; k < P_CHUNK && half * P_CHUNK + k < rest; k++) {
+                first_scales(st + half * S::BYTES, k);
 #pragma unroll
-        for (int i = 0; i < ITEMS; i++) {
-            const int k = i / PIECES, p = i % PIECES;
-            Scales sc;
-            sc.w = staged_f1(ws + k * P_ROWS * 4);
-            sc.c = Q4 ? staged_f1(wcs + k * P_ROWS * 4) : 0.0f;
+                for (int p = 0; p < PIECES; p++) {
+                    fetch(sums + (half * P_CHUNK + k) * P_TBUF, p);
+                    umma::wait_ld(v[p & 1]);
 #pragma unroll
-            for (int j = 0; j < PC / 4; j++) {
-                sc.x[j] = staged_f4(xs + (k * N + p * PC + 4 * j) * 4);
-                if (Q4) sc.u[j] = staged_f4(su + (k * N + p * PC + 4 * j) * 4);
-            }
-            umma::wait_ld(v[i & 1]);
-            if (i + 1 < ITEMS) {
-                fetch(HALF, (i + 1) / PIECES, (i + 1) % PIECES, v[(i + 1) & 1]);
-                if (i + 2 == ITEMS && more)  // the next chunk's sums, and its scales, which its own copies wrote
-                    ready = mbar_test(bars.tfull + (HALF ^ 1), half_par(c + 1)) &&
-                            mbar_test(bars.full + stage_of<Q4>(c + 1), stage_par<Q4>(c + 1));
-            } else {
-                // The chunk's sums and scales have been read: the issuer may overwrite this half, the
-                // producer this stage (whose MMAs were done before the sums could be read).
-                umma::fence_before_sync();
-                __syncwarp();
-                mbar_arrive_if(bars.tempty + HALF, lane == 0);
-                mbar_arrive_if(bars.empty + stage_of<Q4>(c), lane == 0);
-                if (more) {
-                    if (!ready) {
-                        wait_or_abort(bars.full + stage_of<Q4>(c + 1), stage_par<Q4>(c + 1), bars.abort_flag);
-                        wait_or_abort(bars.tfull + (HALF ^ 1), half_par(c + 1), bars.abort_flag);
-                    }
-                    umma::fence_after_sync();
-                    fetch(HALF ^ 1, 0, 0, v[(i + 1) & 1]);
+                    for (int j = p / 2 * (CC / 16); j < (p / 2 + 1) * (CC / 16); j++) chains(v[p & 1], p, j);
                 }
             }
-            chains(v[i & 1], p, sc);
+            release(half);
         }
-        c++;
-    };
-    auto any_half = [&](bool more, auto nblk_c) {
-        if (half_of(c)) chunk(more, nblk_c, std::integral_constant<uint32_t, 1>{});
-        else chunk(more, nblk_c, std::integral_constant<uint32_t, 0>{});
-    };
-    wait_or_abort(bars.full + stage_of<Q4>(c), stage_par<Q4>(c), bars.abort_flag);
-    wait_or_abort(bars.tfull + half_of(c), half_par(c), bars.abort_flag);
-    umma::fence_after_sync();
-    fetch(half_of(c), 0, 0, v[0]);
-#pragma unroll 1
-    for (int b = 0; b + 1 < nb; b += 2) any_half(b + 2 < nb, std::integral_constant<int, 2>{});
-    if (nb & 1) any_half(false, std::integral_constant<int, 1>{});
+        turn++;
+    }
 }
 
 // silu(gate) * up of 32 hidden columns of one token (the parked row holds gate and up side by side),
-// then quantize_q8 (src/kernels.rs:84-98) of that block, as f16 into the token's row of the tile.
-__device__ __forceinline__ void finish_block(const float4* parked, float2 one, uint8_t* dst, int N, float& scale, float& sum) {
-    float2 h[16];
-    bool usable = true;
-#pragma unroll
-    for (int i = 0; i < 16; i++) {
-        const float4 v = parked[i];  // gate, up, gate, up
-        h[i] = mul2(silu2(make_float2(v.x, v.z), one, usable), make_float2(v.y, v.w));
-    }
-    if (!usable) {  // (one test for the block: a branch at every pair would keep them from overlapping)
-#pragma unroll
-        for (int i = 0; i < 16; i++) {
-            const float4 v = parked[i];
-            h[i].x = __fdiv_rn(v.x, 1.0f + exp_poly(-v.x)) * v.y;
-            h[i].y = __fdiv_rn(v.z, 1.0f + exp_poly(-v.z)) * v.w;
-        }
-    }
+// then quantize_q8 (src/kernels.rs:84-98) of that block, as f16 into the token's row of the tile. The products go back
+// over the gates and ups on the way, and both loops stay short: a straight run of all 32 columns is 16 KB of
+// instructions, fetched past the float warps' own.
+__device__ __forceinline__ void finish_block(float4* parked, float2 one, uint8_t* dst, int N, float& scale, float& sum) {
     float amax = 0.0f;
+#pragma unroll 1
+    for (int i = 0; i < 4; i++) {  // 8 columns
+        float4 v[4];
+        float2 h[4];
+        bool usable = true;
 #pragma unroll
-    for (int i = 0; i < 16; i++) amax = fmaxf(fmaxf(amax, fabsf(h[i].x)), fabsf(h[i].y));
+        for (int j = 0; j < 4; j++) {
+            v[j] = parked[4 * i + j];  // gate, up, gate, up
+            h[j] = mul2(silu2(make_float2(v[j].x, v[j].z), one, usable), make_float2(v[j].y, v[j].w));
+        }
+        if (!usable) {  // (one test for the lot: a branch at every pair would keep them from overlapping)
+#pragma unroll 1
+            for (int j = 0; j < 4; j++) {
+                const float4 u = parked[4 * i + j];
+                const float2 t = make_float2(__fdiv_rn(u.x, 1.0f + exp_poly(-u.x)) * u.y, __fdiv_rn(u.z, 1.0f + exp_poly(-u.z)) * u.w);
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+                    if (k == j) h[k] = t;
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++) amax = fmaxf(fmaxf(amax, fabsf(h[j].x)), fabsf(h[j].y));
+        parked[2 * i] = make_float4(h[0].x, h[0].y, h[1].x, h[1].y);
+        parked[2 * i + 1] = make_float4(h[2].x, h[2].y, h[3].x, h[3].y);
+    }
     const float d = __fdiv_rn(amax, 127.0f);
     const float id = d > 0.0f ? __fdiv_rn(1.0f, d) : 0.0f;
     int qsum = 0;
-#pragma unroll
+#pragma unroll 1
     for (int i = 0; i < 4; i++) {  // 8 columns: 16 bytes of f16
         uint2 f[2];
 #pragma unroll
         for (int u = 0; u < 2; u++) {
             // Rounds half away from zero as exp_poly2 does; NaN becomes 0; the packing saturates.
+            const float4 h = parked[2 * i + u];
             int q[4];
 #pragma unroll
             for (int k = 0; k < 2; k++) {
-                const float2 t = mul2(h[4 * i + 2 * u + k], make_float2(id, id));
+                const float2 t = mul2(k ? make_float2(h.z, h.w) : make_float2(h.x, h.y), make_float2(id, id));
                 q[2 * k] = __float2int_rz(t.x + copysignf(0.49999997f, t.x));
                 q[2 * k + 1] = __float2int_rz(t.y + copysignf(0.49999997f, t.y));
             }
@@ -361,10 +415,10 @@ __global__ void __launch_bounds__(P_THREADS, 1)
     if (tid == 0) {
         for (int s = 0; s < S::N; s++) {
             mbar_init(bars.full + s, 1);
-            mbar_init(bars.empty + s, P_EW);
+            mbar_init(bars.empty + s, 1);
         }
         for (int g = 0; g < P_NGRP; g++) {
-            mbar_init(bars.tfull + g, 1);
+            mbar_init(bars.tfull + g, 2);
             mbar_init(bars.tempty + g, P_EW);
         }
         mbar_init(bars.pfull, P_EW);
@@ -383,29 +437,43 @@ __global__ void __launch_bounds__(P_THREADS, 1)
     umma::fence_after_sync();
     const uint32_t tmem = s_tmem;
     grid_dependency_wait();  // everything below reads what earlier kernels wrote
-    const int nb = a.nb;
+    const int nb = a.nb, turn_blocks = (nb + P_NGRP * P_CHUNK - 1) / (P_NGRP * P_CHUNK) * (P_NGRP * P_CHUNK);
     const int work = int(warp_uniform(uint32_t(*a.tile_count * a.row_tiles)));
     if (warp < P_EW) {
         // ---- float warps
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(P_REGS_FLOAT));
         const int quad = warp & 3, slice = warp >> 2;
-        const int row = quad * 32 + lane;  // row of the tile = TMEM lane
         const uint32_t tbase = tmem + (uint32_t(quad * 32) << 16);
-        uint32_t c = 0;
+        uint32_t c = 0;  // turns of the TMEM halves
         uint32_t parity = 1;  // of pempty: the first tile finds the parking space free
+        TokenTile ahead = tile_of(a, blockIdx.x, work);
         for (int w = blockIdx.x; w < work; w += gridDim.x) {
-            const int N = int(warp_uniform(a.tiles[w / a.row_tiles].cols));
+            const int N = int(warp_uniform(ahead.cols));
+            ahead = tile_of(a, w + gridDim.x, work);
             const int col0 = slice * (N / 2);  // this warp's first token of the tile
             float acc[64], off[Q4 ? 32 : 1];
-            if (!Q4 && N == 128) float_chains<Q4, Q4 ? 32 : 64>(acc, off, c, smem_addr(smem), bars, tbase, nb, col0, row, lane);
-            else if (N == 64) float_chains<Q4, 32>(acc, off, c, smem_addr(smem), bars, tbase, nb, col0, row, lane);
-            else float_chains<Q4, 16>(acc, off, c, smem_addr(smem), bars, tbase, nb, col0, row, lane);
+            if (!Q4 && N == 128) float_chains<Q4, Q4 ? 32 : 64>(acc, off, c, smem_addr(smem), bars, tbase, nb, col0, quad * 32, lane);
+            else if (N == 64) float_chains<Q4, 32>(acc, off, c, smem_addr(smem), bars, tbase, nb, col0, quad * 32, lane);
+            else float_chains<Q4, 16>(acc, off, c, smem_addr(smem), bars, tbase, nb, col0, quad * 32, lane);
             wait_or_abort(bars.pempty, parity, bars.abort_flag);
             parity ^= 1;
-            float* dst = parked + col0 * P_HSTRIDE + row;
+            // A lane's four rows of a token side by side (the 132-float stride spreads the lanes over the banks).
+            float* dst = parked + (col0 + 2 * (lane & 3)) * P_HSTRIDE + quad * 32 + (lane >> 2) * 4;
+            auto value = [&](int i) { return Q4 ? acc[i] + off[Q4 ? i : 0] : acc[i]; };
+            auto park = [&](auto cw) {
+                constexpr int CW = decltype(cw)::value, CC = CW < 32 ? CW : 32, H = CC / 2;  // (the order of float_chains)
 #pragma unroll
-            for (int j = 0; j < (Q4 ? 32 : 64); j++)
-                if (j < N / 2) dst[j * P_HSTRIDE] = Q4 ? acc[j] + off[Q4 ? j : 0] : acc[j];
+                for (int j = 0; j < CW / 8; j++)
+#pragma unroll
+                    for (int i = 0; i < 2; i++) {
+                        const int lo = j / (CC / 8) * CC + j % (CC / 8) * 4 + i;
+                        *reinterpret_cast<float4*>(dst + (8 * j + i) * P_HSTRIDE) =
+                            make_float4(value(lo), value(lo + 2), value(H + lo), value(H + lo + 2));
+                    }
+            };
+            if (!Q4 && N == 128) park(std::integral_constant<int, Q4 ? 32 : 64>{});
+            else if (N == 64) park(std::integral_constant<int, 32>{});
+            else park(std::integral_constant<int, 16>{});
             __syncwarp();
             mbar_arrive_if(bars.pfull, lane == 0);
         }
@@ -415,18 +483,21 @@ __global__ void __launch_bounds__(P_THREADS, 1)
             // ---- producer: operand chunks, each once its stage is free again
             asm volatile("fence.proxy.async;" ::: "memory");  // the tiles were written by plain stores
             uint32_t c = 0;
+            TokenTile ahead = tile_of(a, blockIdx.x, work);
             for (int w = blockIdx.x; w < work; w += gridDim.x) {
-                const TokenTile tile = a.tiles[w / a.row_tiles];
+                const TokenTile tile = ahead;
+                ahead = tile_of(a, w + gridDim.x, work);
                 const size_t wtile = size_t(tile.expert) * a.row_tiles + w % a.row_tiles;
                 const uint32_t N = tile.cols;
-                for (int b0 = 0; b0 < nb; b0 += P_CHUNK, c++) {
-                    const uint32_t nblk = min(P_CHUNK, nb - b0);
+                for (int b0 = 0; b0 < turn_blocks; b0 += P_CHUNK, c++) {
+                    const uint32_t nblk = max(0, min(P_CHUNK, nb - b0));  // (none in the chunks that fill up a turn)
                     uint64_t* full = bars.full + stage_of<Q4>(c);
                     if (c >= uint32_t(S::N)) wait_or_abort(bars.empty + stage_of<Q4>(c), stage_par<Q4>(c) ^ 1, bars.abort_flag);
                     uint8_t* st = smem + stage_of<Q4>(c) * S::BYTES;
                     const uint32_t wb = nblk * P_A_BLOCK, xb = nblk * N * 64, wf = nblk * P_ROWS * 4, xf = nblk * N * 4;
                     const size_t wo = wtile * nb + b0, xo = size_t(tile.row0) * nb + size_t(b0) * N;
                     mbar_expect_tx(full, wb + xb + (wf + xf) * (Q4 ? 2 : 1));
+                    if (nblk == 0) continue;
                     bulk_copy(st, a.wt + wo * (P_A_BLOCK / 2), wb, full);
                     bulk_copy(st + S::B, a.xt + xo * 32, xb, full);
                     bulk_copy(st + S::WD, a.wd + wo * P_ROWS, wf, full);
@@ -445,12 +516,17 @@ __global__ void __launch_bounds__(P_THREADS, 1)
         } else if (warp == P_EW + 1 && lane == 0) {
             // ---- MMA issuer: a block = two K = 16 products into its own TMEM buffer, a commit per chunk
             uint32_t c = 0;
+            TokenTile ahead = tile_of(a, blockIdx.x, work);
             for (int w = blockIdx.x; w < work; w += gridDim.x) {
-                const uint32_t N = a.tiles[w / a.row_tiles].cols, idesc = umma::idesc_f16(P_ROWS, int(N));
-                for (int b0 = 0; b0 < nb; b0 += P_CHUNK, c++) {
+                const uint32_t N = ahead.cols, idesc = umma::idesc_f16(P_ROWS, int(N));
+                ahead = tile_of(a, w + gridDim.x, work);
+                for (int b0 = 0; b0 < turn_blocks; b0 += P_CHUNK, c++) {
                     const int nblk = min(P_CHUNK, nb - b0);
+                    if (c >= uint32_t(P_NGRP)) {
+                        wait_or_abort(bars.tempty + half_of(c), half_par(c) ^ 1, bars.abort_flag);
+                        mbar_arrive_if(bars.empty + stage_of<Q4>(c - P_NGRP), true);
+                    }
                     wait_or_abort(bars.full + stage_of<Q4>(c), stage_par<Q4>(c), bars.abort_flag);
-                    if (c >= uint32_t(P_NGRP)) wait_or_abort(bars.tempty + half_of(c), half_par(c) ^ 1, bars.abort_flag);
                     umma::fence_after_sync();
                     const uint32_t sa = smem_addr(smem + stage_of<Q4>(c) * S::BYTES), sb = sa + S::B;
 #pragma unroll
@@ -464,6 +540,7 @@ __global__ void __launch_bounds__(P_THREADS, 1)
                         }
                     }
                     umma::commit(bars.tfull + half_of(c));
+                    mbar_arrive_if(bars.tfull + half_of(c), true);  // (what this thread saw land, the float warps may read)
                 }
             }
             if (s_abort) {
@@ -478,8 +555,10 @@ __global__ void __launch_bounds__(P_THREADS, 1)
         const int ftid = tid - (P_EW + P_IW) * 32;
         const float2 one = make_float2(a.one, a.one);
         uint32_t parity = 0;  // of pfull
+        TokenTile ahead = tile_of(a, blockIdx.x, work);
         for (int w = blockIdx.x; w < work; w += gridDim.x, parity ^= 1) {
-            const TokenTile tile = a.tiles[w / a.row_tiles];
+            const TokenTile tile = ahead;
+            ahead = tile_of(a, w + gridDim.x, work);
             const int rt = w % a.row_tiles, N = int(tile.cols), tile_n = int(tile.n);
             wait_or_abort(bars.pfull, parity, bars.abort_flag);
             if (GATE_UP) {
@@ -493,8 +572,8 @@ __global__ void __launch_bounds__(P_THREADS, 1)
                     uint8_t* dst = reinterpret_cast<uint8_t*>(a.xt_out + size_t(tile.row0) * a.out_cols + size_t(b) * N * 32) +
                                    f16_tile_offset(N, n, 0);
                     float d, su;
-                    finish_block(reinterpret_cast<const float4*>(parked + n * P_HSTRIDE + q * 64), one, dst, N, d, su);
-                    const size_t so = size_t(tile.row0) * nb_out + size_t(b) * N + n;
+                    finish_block(reinterpret_cast<float4*>(parked + n * P_HSTRIDE + q * 64), one, dst, N, d, su);
+                    const size_t so = size_t(tile.row0) * nb_out + size_t(b) * N + scale_place(n);
                     a.xst_out[so] = d;
                     a.xsumt_out[so] = su;
                 }
@@ -576,7 +655,7 @@ __global__ void __launch_bounds__(256)
             }
         }
         const size_t at = (size_t(e) * row_tiles + rt) * nb + b;
-        uint8_t* dst = reinterpret_cast<uint8_t*>(wt) + at * P_A_BLOCK + f16_tile_offset(P_ROWS, r, 0);
+        uint8_t* dst = reinterpret_cast<uint8_t*>(wt) + at * P_A_BLOCK + f16_tile_offset(P_ROWS, product_row(r), 0);
 #pragma unroll
         for (int i = 0; i < 4; i++) {
             const uint2 f0 = f16_from_s8(w[2 * i]), f1 = f16_from_s8(w[2 * i + 1]);
@@ -624,7 +703,7 @@ __global__ void __launch_bounds__(256)
             const uint2 f0 = f16_from_s8(i & 1 ? in[i / 2].z : in[i / 2].x), f1 = f16_from_s8(i & 1 ? in[i / 2].w : in[i / 2].y);
             *reinterpret_cast<uint4*>(dst + i * N * 16) = make_uint4(f0.x, f0.y, f1.x, f1.y);
         }
-        const size_t so = size_t(tile.row0) * nb + size_t(b) * N + n;
+        const size_t so = size_t(tile.row0) * nb + size_t(b) * N + scale_place(n);
         xst[so] = d;
         if (Q4) xsumt[so] = xsum[row * nbp + b];
     }

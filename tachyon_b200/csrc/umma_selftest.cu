@@ -49,13 +49,33 @@ umma_selftest_kernel(const uint16_t* __restrict__ a_tile, const uint16_t* __rest
     const bool landed = mbar_wait_bounded(&s_bar, 0);
     umma::fence_after_sync();
     if (landed) {
-#pragma unroll
-        for (int c0 = 0; c0 < N; c0 += 16) {
-            float v[16];
-            umma::ld_f32(tmem + (uint32_t(warp * 32) << 16) + c0, v);
+        // As the prefill kernels read them: a half of the rows at a time, here once 32 and twice 16 of every 64 columns.
+        const uint32_t base = tmem + (uint32_t(warp * 32) << 16);
+        auto read = [&](int c0, int h, auto& v) {
+            constexpr int n = sizeof(v) / sizeof(float);
+            umma::ld_half_f32(base + (uint32_t(h) << 20) + c0, v);
             umma::wait_ld(v);
 #pragma unroll
-            for (int j = 0; j < 16; j++) d_out[(warp * 32 + lane) * N + c0 + j] = v[j];
+            for (int j = 0; j < n / 4; j++)
+#pragma unroll
+                for (int r = 0; r < 2; r++)
+                    *reinterpret_cast<float2*>(d_out + (warp * 32 + h * 16 + r * 8 + (lane >> 2)) * N + c0 + 8 * j + 2 * (lane & 3)) =
+                        make_float2(v[4 * j + 2 * r], v[4 * j + 2 * r + 1]);
+        };
+#pragma unroll
+        for (int c0 = 0; c0 < N; c0 += 64) {
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                if (c0 > 0) {
+                    float v[32];
+                    read(c0, h, v);
+                } else {
+                    float v[16], lo[8], hi[8];
+                    read(0, h, v);
+                    read(32, h, lo);
+                    read(48, h, hi);
+                }
+            }
         }
     } else if (tid == 0) {
         atomicExch(status, ERR_COPY_WAIT_TIMEOUT);

@@ -76,6 +76,32 @@ def test_both_kernel_families_give_the_same_bits(oracle, ctx, fmt):
         assert np.array_equal(b, b2)
 
 
+@pytest.mark.parametrize("fmt", ["q8", "q4"])
+@pytest.mark.parametrize("hidden,inter", [(32, 64), (64, 160), (96, 32), (160, 96), (192, 288), (224, 256)])
+def test_any_number_of_blocks_gives_the_same_bits(oracle, ctx, fmt, hidden, inter):
+    """Rows of 1 to 9 blocks: whole passes of the float loop (four blocks), what is left after them, and chunks of
+    one block; token tiles of every width, some not full."""
+    shape = MoeShape("blocks", hidden, 6, 2, inter, fmt=fmt)
+    lw = layer_weights(oracle, shape, 7)
+    ctx.set_arithmetic(ctx.ARITH_FAST)
+    layer = make_layer(ctx, lw, shape.topk, 500)
+    layer.set_router_bias(synth.zipf_router_bias(7, 6))
+    try:
+        for t in [33, 130, 500]:
+            x = workloads.hidden_states(shape, t, seed=t)
+            y0 = np.zeros_like(x)
+            ctx.set_decode_block(False)
+            ctx.set_prefill_threshold(NEVER)
+            a = forward(ctx, layer, x, y0)
+            ctx.set_prefill_threshold(0)
+            b = forward(ctx, layer, x, y0)
+            assert np.array_equal(a, b)
+    finally:
+        ctx.set_decode_block(True)
+        ctx.set_prefill_threshold(DEFAULT)
+        layer.free()
+
+
 def test_default_threshold_switches_by_batch_size(oracle, ctx):
     """Crossing the threshold, or the end of the one-kernel block, must not change a token's output."""
     shape = MoeShape("small-q8", 256, 8, 2, 96, fmt="q8")
