@@ -18,7 +18,7 @@
 // The softmax exponential is evaluated in double precision and rounded to
 // float; the CPU path calls libm's expf. The two agree except where expf
 // itself is not correctly rounded, hence the 1e-5 tolerance on gates.
-#include <algorithm>
+#include <type_traits>
 
 #include "dispatch_common.cuh"
 #include "experts_common.cuh"
@@ -46,7 +46,6 @@ struct RouteArgs {
     float* xsum;
     // dispatch outputs, used when fused
     int fuse_dispatch;
-    int stage_rows;        // tile kernel: rows of the router matrix in shared memory at a time
     int stage_router;      // the router matrix fits in shared memory beside the row: stage it with bulk copies
     int* ticket;
     int* status;
@@ -164,180 +163,286 @@ __global__ void __launch_bounds__(ROUTE_THREADS) route_kernel(const RouteArgs a)
     }
 }
 
-// Prefill-size batches: a CTA takes a tile of TILE tokens at a time (walking tiles blockIdx.x,
-// blockIdx.x + gridDim.x, ...): a warp per token for the norm, the ranking and the quantization,
-// four threads per (TG tokens, ROUTE_TE experts) for the logits, with the router matrix staged once
-// per CTA. Same arithmetic per token as route_kernel.
-//
-// Bound by the shared-memory reads and the latency of a tile's chain (load, norm, logits, ranking). A
-// thread's 2 tokens x 2 experts take four reads for four products and keep all eight warps of a CTA busy;
-// measured for the whole stage at 4096 tokens of the 1b shape / of 2048 columns and 64 experts: 4 x 1 54 us /
-// 154 us, 2 x 2 52 / 148, 4 x 2 52 / 166, 2 x 4 57 / 153 (half the warps idle); 4 x 1 with 512 threads 70 /
-// 158. TILE = 8 lets two CTAs share an SM; batches that would then leave SMs without a tile take 4 or 2 (333
-// tokens of the 1b shape: 42 tiles of 8, 167 of 2).
-constexpr int ROUTE_TE = 2;
-
-// Shared memory of the tile kernel before the staged router matrix: padded rows, logits, norm weight.
-__host__ __device__ inline size_t route_tile_bytes(int hidden, int experts, int tile) {
-    return (size_t(tile) * (hidden / QK * ROW_PAD_BLOCK + (experts + 3) / 4 * 4) * 4 + size_t(hidden) * 4 + 127) / 128 * 128;
+__device__ __forceinline__ void cp_async16(void* dst_smem, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst_smem)), "l"(src) : "memory");
 }
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
-template <int TILE>
-__global__ void __launch_bounds__(ROUTE_THREADS) route_tile_kernel(const RouteArgs a) {
-    constexpr int TG = TILE > 2 ? 2 : 1, TE = ROUTE_TE;
-    extern __shared__ __align__(128) float smem[];
-    const int hidden = a.hidden, experts = a.experts, topk = a.topk;
-    const int rstride = hidden / QK * ROW_PAD_BLOCK;  // floats per padded row
-    const int lstride = (experts + 3) / 4 * 4;
-    float* xrows = smem;                        // [TILE] padded rows
-    float* slog = xrows + TILE * rstride;       // [TILE][lstride]
-    float* snw = slog + TILE * lstride;         // [hidden] the norm's weight
-    __shared__ __align__(8) uint64_t s_wbar;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    grid_launch_dependents();
-    // The router matrix by bulk copies, one per row, into rows padded by 32 bytes: all of it, once, or (a
-    // matrix larger than the space left) stage_rows experts at a time, again for every tile.
-    const int wstride = 2 * hidden + 32, stage_rows = a.stage_rows;
-    uint8_t* wsm = reinterpret_cast<uint8_t*>(smem) + route_tile_bytes(hidden, experts, TILE);
-    auto stage = [&](int e_lo) {
-        const int n = min(stage_rows, experts - e_lo);
-        if (warp == 0) {
-            if (lane == 0) mbar_expect_tx(&s_wbar, uint32_t(n) * 2u * uint32_t(hidden));
-            __syncwarp();
-            for (int e = lane; e < n; e += 32)
-                bulk_copy(wsm + size_t(e) * wstride, a.router + size_t(e_lo + e) * hidden, 2 * hidden, &s_wbar);
-        }
-    };
-    if (tid == 0) {
-        mbar_init(&s_wbar, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+// Prefill-size batches: a CTA per tile of NG x TG tokens. The logits are a matrix product whose every output is sixteen
+// chains of its own (the AVX dot's lanes), so it runs on the FP32 pipe: four threads per TG tokens x TE experts, thread
+// q with lanes 4 q .. 4 q + 3, over chunks of KC columns that stand in shared memory twice over. While eight warps work on a
+// chunk, eight others bring the next: the rows through registers, normed and quantized on the way, the router's
+// by asynchronous copies. Then a warp per token ranks the logits, and every pick gets its gate from a thread of its
+// own. Experts beyond the 64 / NG x TE of a pass take another pass over the columns.
+//
+// Bound by shared memory, 16 TG + 8 TE bytes a thread for 2 TG TE packed products: at 4 x 4 a step of sixteen columns is 24
+// cycles of it a warp against 16 of the FP32 pipe, at 4 x 8 32 against 32; with whole rows and the whole matrix staged
+// (2 x 2, a warp per token for norm, ranking and quantization, one after the other) it was 12 against 4. A step
+// takes twice its bound: two warps per scheduler, beside two that bring rows.
+// Measured, the kernel alone (us): 4096 tokens of the 1b shape 37 -> 26; 2047 of the 3b shape 42 -> 26; 4096 of 2048 columns
+// and 64 experts 138 -> 70; 333 of the 1b shape 12.8 -> 9.7. Where the 26 go, in thousands of cycles: 4 the squares, 30
+// the chunks (25 of them products), 6 ranks, 3 gates. Tried: all warps doing both (35), the next step's
+// operands requested a step ahead (no change), quantization by four threads a block as the rows come in (twice the instructions).
+template <int N>
+using Int = std::integral_constant<int, N>;
+constexpr int RT_HALF = 256, RT_THREADS = 2 * RT_HALF;  // the threads of either kind
+
+template <int NG, int TG, int TE, int KC>
+struct RouteTile {
+    static constexpr int TM = NG * TG, EG = RT_HALF / 4 / NG, EP = EG * TE;  // tokens, expert groups, experts of a pass
+    static constexpr int XSTRIDE = KC / QK * ROW_PAD_BLOCK;  // floats per staged row piece
+    static constexpr int WSTRIDE = KC * 2 + 32;  // bytes per staged router row piece: four neighbouring rows on distinct banks
+    static constexpr int X = TM * XSTRIDE * 4, W = EP * WSTRIDE;             // bytes of a buffer
+    // Registers: 128 a thread at launch, then split.
+    static constexpr int REGS_DOTS = TG * TE > 20 ? 176 : 136, REGS_ROWS = 256 - REGS_DOTS;
+    static_assert(KC >= MAX_TOPK, "the exponentials of a tile's picks fit where its rows were");
+    __host__ __device__ static int key_stride(int experts) { return (experts + 31) / 32 * 32; }
+    __host__ __device__ static size_t bytes(int experts, int topk) {
+        return 2 * size_t(X + W) + size_t(TM) * (key_stride(experts) + 2 * topk + 1) * 4;
     }
-    if (a.norm_w)
-        for (int c = tid; c < hidden; c += ROUTE_THREADS) snw[c] = a.norm_w[c];  // (a constant: before the wait)
-    __syncthreads();
-    stage(0);  // (constants as well)
+};
+
+template <int NG, int TG, int TE, int KC>
+__global__ void __launch_bounds__(RT_THREADS, 1) route_tile_kernel(const RouteArgs a) {
+    using L = RouteTile<NG, TG, TE, KC>;
+    constexpr int TM = L::TM, EG = L::EG, KV = KC / 8;
+    constexpr int TASKS = TM * KV, PER = (TASKS + RT_HALF - 1) / RT_HALF;  // eight columns of a row each
+    static_assert(TASKS % 32 == 0 && (TASKS <= RT_HALF || RT_HALF % KV == 0), "whole warps, rows evenly");
+    extern __shared__ __align__(128) uint8_t rt_smem[];
+    const int hidden = a.hidden, experts = a.experts, topk = a.topk, nb = hidden / QK;
+    const int kstride = L::key_stride(experts);
+    float* xbuf = reinterpret_cast<float*>(rt_smem);              // [2][TM][XSTRIDE]
+    uint8_t* wbuf = rt_smem + 2 * L::X;                           // [2][EP][WSTRIDE]
+    int* skey = reinterpret_cast<int*>(wbuf + 2 * L::W);          // [TM][kstride] order keys of the logits
+    uint32_t* sid = reinterpret_cast<uint32_t*>(skey + TM * kstride);  // [TM][topk] picks
+    float* sval = reinterpret_cast<float*>(sid + TM * topk);           // [TM][topk] their scores
+    float* sinv = sval + TM * topk;                                    // [TM] 1 / rms
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int t0 = blockIdx.x * TM, nt = min(TM, a.t - t0);
+    const int padded = (nb + SUPER - 1) / SUPER * SUPER;
+    const int chunks = (hidden + KC - 1) / KC;
+    const bool dots = tid < RT_HALF;
+    const int rid = tid - RT_HALF;  // of the threads that bring the rows
+    grid_launch_dependents();
+    auto stage_router = [&](int e_lo, int c) {
+        const int n = min(L::EP, experts - e_lo), vecs = min(KC, hidden - c * KC) / 8;
+        uint8_t* dst = wbuf + (c & 1) * L::W;
+#pragma unroll 4
+        for (int i = rid; i < n * KV; i += RT_HALF) {
+            const int e = i / KV, v = i % KV;
+            if (v < vecs) cp_async16(dst + e * L::WSTRIDE + v * 16, a.router + size_t(e_lo + e) * hidden + c * KC + v * 8);
+        }
+        cp_async_commit();
+    };
+    if (!dots) stage_router(0, 0);  // (a constant: before the wait)
     grid_dependency_wait();
-    bool landed = true;
-    uint32_t stagings = 0;  // waited for
-    const bool once = stage_rows >= experts;
-    const int padded = (hidden / QK + SUPER - 1) / SUPER * SUPER;
-    const int tiles = (a.t + TILE - 1) / TILE, vec_per_row = hidden / 4;
-    const int dk = ROUTE_THREADS / vec_per_row, dv = ROUTE_THREADS - dk * vec_per_row;
-    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        const int t0 = tile * TILE, nt = min(TILE, a.t - t0);
-        __syncthreads();  // the previous tile's rows and logits are no longer read
-        const float4* src = reinterpret_cast<const float4*>(a.x + size_t(t0) * hidden);  // (the tile's rows are one run)
-        const int vecs = nt * vec_per_row;
-        int k = tid / vec_per_row, vc = tid - k * vec_per_row;  // piece i of the run is piece vc of row k
-        for (int i0 = 0; i0 < vecs; i0 += ROUTE_THREADS * TILE) {  // all requests of a pass before the first store
-            float4 v[TILE];
+
+    // ---- 1 / rms of the rows, a warp per token, several at a time
+    if (a.norm_w) {
+        constexpr int NW = RT_THREADS / 32, AT = TM > NW ? TM / NW : 1;
+        if (warp < TM) {
+            float acc[AT];
+            const float* xr[AT];
 #pragma unroll
-            for (int u = 0; u < TILE; u++) {
-                const int i = i0 + u * ROUTE_THREADS + tid;
-                if (i < vecs) v[u] = src[i];
+            for (int i = 0; i < AT; i++) acc[i] = 0.0f, xr[i] = a.x + size_t(t0 + min(warp + NW * i, nt - 1)) * hidden + lane;
+#pragma unroll 16
+            for (int k = 0; k < nb; k++) {
+                float v[AT];
+#pragma unroll
+                for (int i = 0; i < AT; i++) v[i] = xr[i][k * QK];
+#pragma unroll
+                for (int i = 0; i < AT; i++) acc[i] = fmaf(v[i], v[i], acc[i]);
             }
 #pragma unroll
-            for (int u = 0; u < TILE; u++) {
-                if (i0 + u * ROUTE_THREADS + tid < vecs)
-                    *reinterpret_cast<float4*>(xrows + k * rstride + padded_at(4 * vc)) = v[u];
-                k += dk, vc += dv;
-                if (vc >= vec_per_row) vc -= vec_per_row, k++;
+            for (int i = 0; i < AT; i++) {
+                const float ss = __fdiv_rn(fold_squares(acc[i]) + 0.0f, float(hidden));  // (the scalar tail is an empty sum)
+                if (lane == 0) sinv[warp + NW * i] = __fdiv_rn(1.0f, __fsqrt_rn(ss + a.eps));
             }
         }
         __syncthreads();
-        if (a.norm_w && warp < nt) {  // a warp per token
-            float* xr = xrows + warp * rstride;
-            const float ss = __fdiv_rn(sum_squares_padded_row(xr, hidden, lane), float(hidden));
-            const float inv = __fdiv_rn(1.0f, __fsqrt_rn(ss + a.eps));
-            __syncwarp();
-#pragma unroll 8
-            for (int c = 0; c < hidden / QK; c++)
-                xr[c * ROW_PAD_BLOCK + lane] = xr[c * ROW_PAD_BLOCK + lane] * inv * snw[c * QK + lane];
-        }
-        for (int e_lo = 0; e_lo < experts; e_lo += stage_rows) {
-            if (!once || stagings == 0) {
-                landed = mbar_wait_bounded(&s_wbar, stagings & 1) && landed;
-                stagings++;
+    }
+
+    // ---- logits
+    if (!dots) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(L::REGS_ROWS));
+        // This thread stages columns 8 col8 .. of rows row0, row0 + 256 / KV, ... of every chunk.
+        const int row0 = rid / KV, col8 = rid % KV;
+        const bool stages = rid < TASKS;  // (whole warps)
+        float4 ahead[PER][2], nw[2];
+        auto request = [&](int c) {
+            const int col = c * KC + col8 * 8;
+            const bool on = stages && col < hidden;
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                nw[h] = on && a.norm_w ? *reinterpret_cast<const float4*>(a.norm_w + col + 4 * h) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+                for (int i = 0; i < PER; i++) {
+                    ahead[i][h] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    if (on)
+                        ahead[i][h] = *reinterpret_cast<const float4*>(a.x + size_t(t0 + min(row0 + RT_HALF / KV * i, nt - 1)) * hidden + col + 4 * h);
+                }
             }
-            if (e_lo == 0) __syncthreads();  // the normed rows are complete
-            // Logits. Each (token, expert) keeps its own accumulators, as route_dot_quad: thread q of a quad has
-            // elements 16 j + 4 q .. + 3. (Rows past the tile's tokens hold anything and experts past the
-            // last repeat it; those logits are not stored.)
-            const int n_e = min(stage_rows, experts - e_lo), egroups = (n_e + TE - 1) / TE;
-            const int tasks = (nt + TG - 1) / TG * egroups;
-            for (int p0 = 0; p0 < tasks; p0 += ROUTE_THREADS / 4) {
-                const int p = p0 + (tid >> 2), q = tid & 3;
-                if (p0 + ((tid >> 5) << 3) >= tasks) continue;  // (a warp without work)
-                const bool valid = p < tasks;
-                const int grp = valid ? p / egroups : 0, e0 = valid ? (p - grp * egroups) * TE : 0;
-                float2 acc[TG][TE][2];
+        };
+        auto stage_rows = [&](int c) {
+            float* dst = xbuf + (c & 1) * (L::X / 4) + row0 * L::XSTRIDE + col8 / 4 * ROW_PAD_BLOCK + col8 % 4 * 8;
 #pragma unroll
-                for (int i = 0; i < TG; i++)
-#pragma unroll
-                    for (int j = 0; j < TE; j++) acc[i][j][0] = acc[i][j][1] = make_float2(0.0f, 0.0f);
-                const uint8_t* ws[TE];
-#pragma unroll
-                for (int j = 0; j < TE; j++) ws[j] = wsm + size_t(min(e0 + j, n_e - 1)) * wstride + q * 8;
-                const float* xr = xrows + size_t(grp * TG) * rstride + q * 4;
-#pragma unroll 2
-                for (int blk = 0; blk < hidden / QK; blk++) {
+            for (int i = 0; i < PER; i++) {
+                float4 v[2] = {ahead[i][0], ahead[i][1]};
+                if (a.norm_w) {
+                    const float inv = sinv[row0 + RT_HALF / KV * i];
 #pragma unroll
                     for (int h = 0; h < 2; h++) {
-                        float4 xv[TG];
+                        v[h].x = v[h].x * inv * nw[h].x, v[h].y = v[h].y * inv * nw[h].y;
+                        v[h].z = v[h].z * inv * nw[h].z, v[h].w = v[h].w * inv * nw[h].w;
+                    }
+                }
+                *reinterpret_cast<float4*>(dst + RT_HALF / KV * i * L::XSTRIDE) = v[0];
+                *reinterpret_cast<float4*>(dst + RT_HALF / KV * i * L::XSTRIDE + 4) = v[1];
+            }
+        };
+        // The 8-bit blocks of a chunk that stands in shared memory, a thread per block (with four threads per block, as
+        // the rows come in, the divisions cost as many instructions for a quarter of the values), by
+        // one half of these warps for the even chunks and the other for the odd ones.
+        auto quantize_rows = [&](int c) {
+            constexpr int BLOCKS = KC / QK;
+            for (int i = rid ^ (c & 1 ? RT_HALF / 2 : 0); i < TM * BLOCKS; i += RT_HALF) {
+                const int row = i / BLOCKS, b = c * BLOCKS + i % BLOCKS;
+                if (row >= nt || b >= padded) continue;
+                const size_t token = size_t(t0 + row);
+                float d = 0.0f, su = 0.0f;
+                if (b < nb) {
+                    const float4* src = reinterpret_cast<const float4*>(xbuf + (c & 1) * (L::X / 4) + row * L::XSTRIDE + i % BLOCKS * ROW_PAD_BLOCK);
+                    float4 v[QK / 4];
+                    float amax = 0.0f;
 #pragma unroll
-                        for (int i = 0; i < TG; i++)
-                            xv[i] = *reinterpret_cast<const float4*>(xr + i * rstride + blk * ROW_PAD_BLOCK + 16 * h);
+                    for (int k = 0; k < QK / 4; k++) {
+                        v[k] = src[k];
+                        amax = fmaxf(fmaxf(fmaxf(fmaxf(amax, fabsf(v[k].x)), fabsf(v[k].y)), fabsf(v[k].z)), fabsf(v[k].w));
+                    }
+                    d = __fdiv_rn(amax, 127.0f);
+                    const float id = d > 0.0f ? __fdiv_rn(1.0f, d) : 0.0f;
+                    int qsum = 0;
+                    uint4* dst = reinterpret_cast<uint4*>(a.xq + token * hidden + size_t(b) * QK);
 #pragma unroll
-                        for (int j = 0; j < TE; j++) {
-                            const uint2 wv = *reinterpret_cast<const uint2*>(ws[j] + blk * 2 * QK + 32 * h);
-                            const float2 w01 = make_float2(bf16_lo(wv.x), bf16_hi(wv.x)), w23 = make_float2(bf16_lo(wv.y), bf16_hi(wv.y));
+                    for (int k = 0; k < 2; k++) {
+                        int q0, q1;
+                        const uint2 lo = quantize_eight(v[4 * k], v[4 * k + 1], id, q0), hi = quantize_eight(v[4 * k + 2], v[4 * k + 3], id, q1);
+                        dst[k] = make_uint4(lo.x, lo.y, hi.x, hi.y);
+                        qsum += q0 + q1;
+                    }
+                    su = d * float(qsum);
+                }
+                a.xs[token * padded + b] = d, a.xsum[token * padded + b] = su;  // (zeros up to whole super-blocks)
+            }
+        };
+        for (int e_lo = 0; e_lo < experts; e_lo += L::EP) {
+            if (e_lo > 0) stage_router(e_lo, 0);
+            request(0);
+#pragma unroll 1
+            for (int c = 0; c <= chunks; c++) {  // chunk c goes in while c - 1 is worked on
+                if (c > 0 && c < chunks) stage_router(e_lo, c);
+                if (stages && c < chunks) {
+                    stage_rows(c);
+                    if (c + 1 < chunks) request(c + 1);
+                }
+                if (c > 0 && e_lo == 0) quantize_rows(c - 1);
+                cp_async_wait_all();
+                __syncthreads();
+            }
+        }
+    } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(L::REGS_DOTS));
+        const int quad = tid >> 2, q = tid & 3, tg = quad / EG, eg = quad % EG;  // tokens tg + NG i, experts eg + EG j
+        for (int e_lo = 0; e_lo < experts; e_lo += L::EP) {
+            const int n_e = min(L::EP, experts - e_lo);
+            float2 acc[TG][TE][2];
 #pragma unroll
-                            for (int i = 0; i < TG; i++) {
-                                acc[i][j][0] = fma2(w01, make_float2(xv[i].x, xv[i].y), acc[i][j][0]);
-                                acc[i][j][1] = fma2(w23, make_float2(xv[i].z, xv[i].w), acc[i][j][1]);
-                            }
+            for (int i = 0; i < TG; i++)
+#pragma unroll
+                for (int j = 0; j < TE; j++) acc[i][j][0] = acc[i][j][1] = make_float2(0.0f, 0.0f);
+            __syncthreads();
+#pragma unroll 1
+            for (int c = 0; c < chunks; c++) {
+                const float* xr = xbuf + (c & 1) * (L::X / 4) + tg * L::XSTRIDE + q * 4;
+                const uint8_t* wr = wbuf + (c & 1) * L::W + eg * L::WSTRIDE + q * 8;
+                const int steps = min(KC, hidden - c * KC) / 16;
+#pragma unroll(TG * TE < 16 ? 8 : 2)
+                for (int s = 0; s < steps; s++) {
+                    float4 xv[TG];
+#pragma unroll
+                    for (int i = 0; i < TG; i++)
+                        xv[i] = *reinterpret_cast<const float4*>(xr + i * NG * L::XSTRIDE + s / 2 * ROW_PAD_BLOCK + s % 2 * 16);
+#pragma unroll
+                    for (int j = 0; j < TE; j++) {  // (experts past the last read what the buffer holds; nothing is made of it)
+                        const uint2 w = *reinterpret_cast<const uint2*>(wr + j * EG * L::WSTRIDE + s * 32);
+                        const float2 w01 = make_float2(bf16_lo(w.x), bf16_hi(w.x)), w23 = make_float2(bf16_lo(w.y), bf16_hi(w.y));
+#pragma unroll
+                        for (int i = 0; i < TG; i++) {
+                            acc[i][j][0] = fma2(w01, make_float2(xv[i].x, xv[i].y), acc[i][j][0]);
+                            acc[i][j][1] = fma2(w23, make_float2(xv[i].z, xv[i].w), acc[i][j][1]);
                         }
                     }
                 }
-#pragma unroll
-                for (int i = 0; i < TG; i++)
-#pragma unroll
-                    for (int j = 0; j < TE; j++) {
-                        // The two 8-lane accumulators added lane-wise, then the hsum tree.
-                        const float lanes[4] = {acc[i][j][0].x, acc[i][j][0].y, acc[i][j][1].x, acc[i][j][1].y};
-                        float v[4], sv[4];
-#pragma unroll
-                        for (int l = 0; l < 4; l++) v[l] = lanes[l] + __shfl_xor_sync(0xffffffffu, lanes[l], 2);
-#pragma unroll
-                        for (int l = 0; l < 4; l++) sv[l] = v[l] + __shfl_xor_sync(0xffffffffu, v[l], 1);
-                        float y = (sv[0] + sv[2]) + (sv[1] + sv[3]);
-                        y = y + 0.0f;  // the dot's scalar tail is an empty sum
-                        const int token = grp * TG + i, e = e_lo + e0 + j;
-                        if (valid && q == 0 && token < nt && e0 + j < n_e) {
-                            if (a.bias) y = y + a.bias[e];
-                            slog[token * lstride + e] = y;
-                            if (a.logits) a.logits[size_t(t0 + token) * experts + e] = y;
-                        }
-                    }
+                __syncthreads();
             }
-            __syncthreads();
-            // The next part of the matrix, for this tile or the next one.
-            if (!once && (e_lo + stage_rows < experts || tile + int(gridDim.x) < tiles))
-                stage(e_lo + stage_rows < experts ? e_lo + stage_rows : 0);
-        }
-        if (warp < nt) {  // a warp per token: ranking and gates, then the row's 8-bit blocks
-            const size_t token = size_t(t0 + warp);
-            route_topk_gates(slog + warp * lstride, experts, topk, a.ids + token * topk, a.gates + token * topk, lane);
-            route_quantize_padded_row(xrows + warp * rstride, hidden, a.xq + token * hidden, a.xs + token * padded,
-                                      a.xsum + token * padded, lane);
+#pragma unroll
+            for (int i = 0; i < TG; i++)
+#pragma unroll
+                for (int j = 0; j < TE; j++) {
+                    // The two 8-lane accumulators added lane-wise, then the hsum tree.
+                    const float lanes[4] = {acc[i][j][0].x, acc[i][j][0].y, acc[i][j][1].x, acc[i][j][1].y};
+                    float v[4], sv[4];
+#pragma unroll
+                    for (int l = 0; l < 4; l++) v[l] = lanes[l] + __shfl_xor_sync(0xffffffffu, lanes[l], 2);
+#pragma unroll
+                    for (int l = 0; l < 4; l++) sv[l] = v[l] + __shfl_xor_sync(0xffffffffu, v[l], 1);
+                    float y = (sv[0] + sv[2]) + (sv[1] + sv[3]);
+                    y = y + 0.0f;  // the dot's scalar tail is an empty sum
+                    const int token = tg + NG * i, e = eg + EG * j;
+                    if (q == 0 && token < nt && e < n_e) {
+                        if (a.bias) y = y + a.bias[e_lo + e];
+                        skey[token * kstride + e_lo + e] = total_key(y);
+                        if (a.logits) a.logits[size_t(t0 + token) * experts + e_lo + e] = y;
+                    }
+                }
         }
     }
-    if (stagings == 0) mbar_wait_bounded(&s_wbar, 0);  // (a CTA without tiles: the copy lands before the memory is released)
-    if (!landed) {
-        // A copy was late: reported, with a last bounded chance to land.
-        mbar_wait_bounded(&s_wbar, (stagings - 1) & 1);
-        if (tid == 0) atomicExch(a.status, ERR_COPY_WAIT_TIMEOUT);
+    // Scale rows are padded with zeros to whole super-blocks; those past the last chunk's columns:
+    if (!dots && padded > chunks * (KC / QK)) {
+        const int n = padded - chunks * (KC / QK);
+        for (int i = rid; i < nt * n; i += RT_HALF) {
+            const size_t at = size_t(t0 + i / n) * padded + chunks * (KC / QK) + i % n;
+            a.xs[at] = 0.0f;
+            a.xsum[at] = 0.0f;
+        }
+    }
+    __syncthreads();  // the keys are complete
+
+    // ---- ranks: larger key first, lower expert first among equals; a warp per token and 32 experts
+    const int groups = (experts + 31) / 32;
+#pragma unroll 1
+    for (int i = warp; i < nt * groups; i += RT_THREADS / 32) {
+        const int token = i / groups, g = i - token * groups, e = g * 32 + lane;
+        const int* keys = skey + token * kstride;
+        const int key = keys[e];
+        const int rank = rank_in_order(keys, experts, g, key, e < experts, lane);
+        if (e < experts && rank < topk) {
+            sid[token * topk + rank] = uint32_t(e);
+            sval[token * topk + rank] = __int_as_float(key ^ int(unsigned(key >> 31) >> 1));  // (total_key is its own inverse)
+        }
+    }
+    __syncthreads();
+    // ---- gates: softmax over a token's picks, the top score as the maximum, the sum taken in score order
+    float* sexp = xbuf;  // (no longer read)
+    for (int i = tid; i < nt * topk; i += RT_THREADS) sexp[i] = exp_nonpositive_f64(sval[i] - sval[i / topk * topk]);
+    __syncthreads();
+    for (int i = tid; i < nt * topk; i += RT_THREADS) {
+        const float* ex = sexp + i / topk * topk;
+        float sum = 0.0f;
+        for (int j = 0; j < topk; j++) sum = sum + ex[j];
+        a.ids[size_t(t0) * topk + i] = sid[i];
+        a.gates[size_t(t0) * topk + i] = __fdiv_rn(sexp[i], sum);
     }
 }
 
@@ -359,9 +464,11 @@ __global__ void rmsnorm_kernel(const float* x, const float* __restrict__ w, floa
 
 void init_kernels_route() {
     cudaFuncSetAttribute(route_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ROUTE_SMEM_LIMIT));
-    cudaFuncSetAttribute(route_tile_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ROUTE_SMEM_LIMIT));
-    cudaFuncSetAttribute(route_tile_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ROUTE_SMEM_LIMIT));
-    cudaFuncSetAttribute(route_tile_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ROUTE_SMEM_LIMIT));
+    auto opt_in = [](auto kernel) { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ROUTE_SMEM_LIMIT)); };
+    opt_in(route_tile_kernel<8, 4, 4, 128>), opt_in(route_tile_kernel<8, 4, 5, 128>), opt_in(route_tile_kernel<8, 4, 8, 128>);
+    opt_in(route_tile_kernel<8, 2, 4, 128>), opt_in(route_tile_kernel<8, 2, 5, 128>), opt_in(route_tile_kernel<8, 2, 8, 128>);
+    opt_in(route_tile_kernel<8, 1, 4, 256>), opt_in(route_tile_kernel<8, 1, 5, 256>), opt_in(route_tile_kernel<8, 1, 8, 256>);
+    opt_in(route_tile_kernel<4, 1, 2, 512>), opt_in(route_tile_kernel<4, 1, 3, 512>), opt_in(route_tile_kernel<4, 1, 4, 512>);
 }
 
 int launch_route(const MoeDims& d, const uint16_t* router, const float* bias, const float* x,
@@ -403,19 +510,28 @@ int launch_route(const MoeDims& d, const uint16_t* router, const float* bias, co
         // Up to one CTA's worth of tokens: a CTA per token; the last one to finish runs the dispatch.
         launch_overlapped(route_kernel, dim3(t), dim3(ROUTE_THREADS), smem, stream, a);
     } else {
-        // Larger batches: CTAs that walk tiles, as many as stay resident (the staged router matrix is then
-        // read a few hundred times, not once per token).
-        const size_t wrow = 2 * size_t(d.hidden) + 32;
-        int tile = t >= 8 * sms ? 8 : t >= 4 * sms ? 4 : 2;
-        while (tile > 2 && route_tile_bytes(d.hidden, d.experts, tile) + 8 * wrow > ROUTE_SMEM_LIMIT) tile /= 2;
-        size_t tsmem = route_tile_bytes(d.hidden, d.experts, tile);
-        const int fit = int((ROUTE_SMEM_LIMIT - tsmem) / wrow), parts = (d.experts + fit - 1) / fit;
-        a.stage_rows = (d.experts + parts - 1) / parts;
-        tsmem += size_t(a.stage_rows) * wrow;
-        const int per_sm = int(std::max<size_t>(1, std::min<size_t>(4, (220 * 1024) / (tsmem + 1024))));
-        const int tiles = (t + tile - 1) / tile;
-        launch_overlapped(tile == 8 ? route_tile_kernel<8> : tile == 4 ? route_tile_kernel<4> : route_tile_kernel<2>,
-                          dim3(std::min(tiles, per_sm * sms)), dim3(ROUTE_THREADS), tsmem, stream, a);
+        // Larger batches: a CTA per tile of 32, 16, 8 or 4 tokens, the widest that still gives two thirds of the SMs one.
+        // (The wider the tile, the fewer bytes of shared memory a product costs. 333 tokens of the 1b shape in tiles of 2,
+        // which are more than there are SMs: 14.9 us, of 4: 9.7.)
+        const int tm = t >= 32 * 2 * sms / 3 ? 32 : t >= 16 * 2 * sms / 3 ? 16 : t >= 8 * 2 * sms / 3 ? 8 : 4;
+        auto go = [&](auto kernel, size_t smem_bytes) {
+            launch_overlapped(kernel, dim3((t + tm - 1) / tm), dim3(RT_THREADS), smem_bytes, stream, a);
+        };
+        auto tile = [&](auto ng, auto tg, auto te, auto kc) {
+            constexpr int NG = decltype(ng)::value, TG = decltype(tg)::value, TE = decltype(te)::value, KC = decltype(kc)::value;
+            go(route_tile_kernel<NG, TG, TE, KC>, RouteTile<NG, TG, TE, KC>::bytes(d.experts, d.topk));
+        };
+        auto eight_groups = [&](auto tg, auto kc) {
+            if (d.experts <= 32) tile(Int<8>{}, tg, Int<4>{}, kc);
+            else if (d.experts <= 40) tile(Int<8>{}, tg, Int<5>{}, kc);
+            else tile(Int<8>{}, tg, Int<8>{}, kc);
+        };
+        if (tm == 32) eight_groups(Int<4>{}, Int<128>{});
+        else if (tm == 16) eight_groups(Int<2>{}, Int<128>{});
+        else if (tm == 8) eight_groups(Int<1>{}, Int<256>{});
+        else if (d.experts <= 32) tile(Int<4>{}, Int<1>{}, Int<2>{}, Int<512>{});
+        else if (d.experts <= 48) tile(Int<4>{}, Int<1>{}, Int<3>{}, Int<512>{});
+        else tile(Int<4>{}, Int<1>{}, Int<4>{}, Int<512>{});
     }
     int launched = 1;
     // (Expert parallel over peer windows: the dispatch runs later, over every rank's tokens.)

@@ -44,6 +44,14 @@ __device__ __forceinline__ float hsum8(float v, unsigned mask) {
     return v;
 }
 
+// The end of the sum of squares below: the four 8-lane accumulators that the lanes hold side by side, (acc0+acc1)+(acc2+acc3)
+// lane-wise, then the hsum tree. Lane 0 ends with the sum.
+__device__ __forceinline__ float fold_squares(float acc) {
+    float s = acc + __shfl_down_sync(0xffffffffu, acc, 8);  // lanes 0-7: a0+a1; 16-23: a2+a3
+    s = s + __shfl_down_sync(0xffffffffu, s, 16);           // lanes 0-7: the four summed
+    return hsum8(s, 0xffffffffu);
+}
+
 // Sum of squares of a row in dot_f32's order, by one warp: lane L owns the
 // elements L, L+32, ... (the four 8-lane accumulators of the main loop side by
 // side); leftover groups of eight go to the first accumulator; then
@@ -62,9 +70,7 @@ __device__ __forceinline__ float sum_squares_avx_order(const float* xr, int n, i
             acc = fmaf(v, v, acc);
         }
     }
-    float s = acc + __shfl_down_sync(0xffffffffu, acc, 8);  // lanes 0-7: a0+a1; 16-23: a2+a3
-    s = s + __shfl_down_sync(0xffffffffu, s, 16);           // lanes 0-7: the four summed
-    s = hsum8(s, 0xffffffffu);
+    float s = fold_squares(acc);
     float tail = 0.0f;
     for (int j = i; j < n; j++) tail = tail + xr[j] * xr[j];
     s = s + tail;
@@ -294,6 +300,28 @@ __device__ __forceinline__ void route_topk_gates(float* slog, int experts, int t
     }
 }
 
+// How many of the token's experts come before expert 32 group + lane, whose key is `key` (`on`: there is such an expert).
+// Experts of groups before this one come first among equals, those of groups behind it do not; within the
+// group the lower lanes do. Whole warps; skey 16-byte aligned and readable up to a multiple of 4 experts.
+__device__ __forceinline__ int rank_in_order(const int* skey, int experts, int group, int key, bool on, int lane) {
+    int rank = __popc(__match_any_sync(0xffffffffu, key) & __ballot_sync(0xffffffffu, on) & ((1u << lane) - 1u));
+#pragma unroll 1
+    for (int j0 = 0; j0 < experts; j0 += 32) {
+        const bool before = (j0 >> 5) < group;
+#pragma unroll
+        for (int u = 0; u < 32; u += 4) {
+            if (j0 + u < experts) {
+                const int4 k = *reinterpret_cast<const int4*>(skey + j0 + u);
+                const int kk[4] = {k.x, k.y, k.z, k.w};
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+                    if (j0 + u + i < experts && (before ? kk[i] >= key : kk[i] > key)) rank++;
+            }
+        }
+    }
+    return rank;
+}
+
 // Top-k of one token by a whole CTA, a thread per expert: each counts the experts that come before its
 // own in the order (larger key first, lower index first among equals) by reading all keys, four
 // at a time, from shared memory; the thread of rank j < topk has the j-th pick, its id into id_out[j] and
@@ -306,23 +334,7 @@ __device__ __forceinline__ void route_rank_picks(const int* skey, const float* s
     if (warp * 32 >= experts) return;
     const bool on = tid < experts;
     const int key = on ? skey[tid] : 0;
-    // Experts of warps before this one come first among equals, those of warps behind it do not; within the
-    // warp the lower lanes do.
-    int rank = __popc(__match_any_sync(0xffffffffu, key) & __ballot_sync(0xffffffffu, on) & ((1u << lane) - 1u));
-#pragma unroll 1
-    for (int j0 = 0; j0 < experts; j0 += 32) {
-        const bool before = (j0 >> 5) < warp;
-#pragma unroll
-        for (int u = 0; u < 32; u += 4) {
-            if (j0 + u < experts) {
-                const int4 k = *reinterpret_cast<const int4*>(skey + j0 + u);
-                const int kk[4] = {k.x, k.y, k.z, k.w};
-#pragma unroll
-                for (int i = 0; i < 4; i++)
-                    if (j0 + u + i < experts && (before ? kk[i] >= key : kk[i] > key)) rank++;
-            }
-        }
-    }
+    const int rank = rank_in_order(skey, experts, warp, key, on, lane);
     if (on && rank < topk) {
         if (id_out) id_out[rank] = uint32_t(tid);
         s_id[rank] = uint32_t(tid);
@@ -399,73 +411,8 @@ __device__ __forceinline__ void route_quantize_row(const float* xrow, int hidden
     }
 }
 
-// Rows kept in shared memory with four floats of padding after every 32-element block
-// (element c at c + 4 * (c / 32)): lanes that each walk their own block then spread over the
-// banks instead of all hitting the same one, and 16-byte vector accesses stay aligned.
+// Rows kept in shared memory with four floats of padding after every 32-element block: lanes that each walk a
+// block of their own then spread over the banks, and 16-byte accesses stay aligned.
 constexpr int ROW_PAD_BLOCK = QK + 4;
-__device__ __forceinline__ int padded_at(int c) { return c + ((c >> 5) << 2); }
-
-// sum_squares_avx_order over such a padded row (n a multiple of 32): lane L owns elements
-// L, L + 32, ... as there; the same additions in the same order.
-__device__ __forceinline__ float sum_squares_padded_row(const float* xr, int n, int lane) {
-    float acc = 0.0f;
-#pragma unroll 8
-    for (int k = 0; k < n / QK; k++) {
-        const float v = xr[k * ROW_PAD_BLOCK + lane];
-        acc = fmaf(v, v, acc);
-    }
-    float s = acc + __shfl_down_sync(0xffffffffu, acc, 8);
-    s = s + __shfl_down_sync(0xffffffffu, s, 16);
-    s = hsum8(s, 0xffffffffu);
-    s = s + 0.0f;  // the scalar tail is an empty sum
-    return __shfl_sync(0xffffffffu, s, 0);
-}
-
-// The row quantization by ONE warp with a lane per 32-block (32 blocks at a time) over a
-// padded row: each lane runs its block's 32 elements itself, so the warp spends a few
-// hundred instructions on the row instead of a shuffle reduction per block. Same values:
-// the maximum does not depend on the order, the sum of the quants is an integer.
-__device__ __forceinline__ void route_quantize_padded_row(const float* xrow, int hidden, int8_t* xq_row, float* xs_row,
-                                                          float* xsum_row, int lane) {
-    const int nb = hidden / QK;
-    const int padded = (nb + SUPER - 1) / SUPER * SUPER;
-    for (int b0 = 0; b0 < padded; b0 += 32) {
-        const int b = b0 + lane;
-        if (b >= padded) continue;
-        if (b >= nb) {  // zero padding up to whole super-blocks
-            xs_row[b] = 0.0f;
-            xsum_row[b] = 0.0f;
-            continue;
-        }
-        const float4* xb = reinterpret_cast<const float4*>(xrow + b * ROW_PAD_BLOCK);
-        float4 v[QK / 4];
-        float amax = 0.0f;
-#pragma unroll
-        for (int i = 0; i < QK / 4; i++) {
-            v[i] = xb[i];
-            amax = fmaxf(fmaxf(fmaxf(fmaxf(amax, fabsf(v[i].x)), fabsf(v[i].y)), fabsf(v[i].z)), fabsf(v[i].w));
-        }
-        const float d = __fdiv_rn(amax, 127.0f);
-        const float id = d > 0.0f ? __fdiv_rn(1.0f, d) : 0.0f;
-        auto q8 = [&](float x) {
-            const float r = roundf(x * id);
-            return (r != r) ? 0 : int(fminf(127.0f, fmaxf(-128.0f, r)));
-        };
-        int qsum = 0;
-        uint32_t words[QK / 4];
-#pragma unroll
-        for (int i = 0; i < QK / 4; i++) {
-            const int q0 = q8(v[i].x), q1 = q8(v[i].y), q2 = q8(v[i].z), q3 = q8(v[i].w);
-            qsum += q0 + q1 + q2 + q3;
-            words[i] = uint32_t(q0 & 0xFF) | (uint32_t(q1 & 0xFF) << 8) | (uint32_t(q2 & 0xFF) << 16) |
-                       (uint32_t(q3 & 0xFF) << 24);
-        }
-        uint4* dst = reinterpret_cast<uint4*>(xq_row + b * QK);
-        dst[0] = make_uint4(words[0], words[1], words[2], words[3]);
-        dst[1] = make_uint4(words[4], words[5], words[6], words[7]);
-        xs_row[b] = d;
-        xsum_row[b] = d * float(qsum);
-    }
-}
 
 }  // namespace tc

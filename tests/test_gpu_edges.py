@@ -27,7 +27,7 @@ WIDE = MoeShape("wide-router", 2048, 64, 8, 32, fmt="q4")    # 256 KB of router 
     (ODD_Q8, 256, False), (ODD_Q4, 257, False), (ODD_Q8, 1025, True), (ODD_Q4, 770, True), (ONE_BLOCK, 193, False),
     # Both sides of the switch to the tensor cores past 128 tokens.
     (PAST_64, 129, True), (WIDE, 129, True),
-    # Router tiles of 2, 4 and 8 tokens, each with a remainder; the dispatch past one CTA's batch.
+    # Router tiles of 4 and 8 tokens, each with a remainder; the dispatch past one CTA's batch.
     (ODD_EXPERTS, 257, False), (ODD_EXPERTS, 595, False), (ODD_EXPERTS, 1187, True), (PAST_64, 1191, True),
     (WIDE, 259, False), (WIDE, 597, True), (WIDE, 1189, False), (ONE_BLOCK, 2049, False),
 ], ids=lambda v: v.name if isinstance(v, MoeShape) else str(v))
@@ -35,6 +35,41 @@ def test_blocks_at_the_edges(oracle, ctx, shape, t, skewed):
     lw = layer_weights(oracle, shape, 17)
     bias = synth.zipf_router_bias(17, shape.experts) if skewed else None
     check_block(oracle, ctx, shape, lw, workloads.hidden_states(shape, t, seed=t), bias=bias, arith="fast")
+
+
+@pytest.mark.parametrize("hidden,experts,topk", [(96, 31, 5), (160, 40, 8), (544, 64, 8), (1056, 130, 8), (64, 256, 32)])
+@pytest.mark.parametrize("t", [261, 803, 1601, 3200])
+def test_router_tiles_match_the_router_of_one_token(oracle, ctx, hidden, experts, topk, t):
+    """Every tile size with a remainder, one to four passes over the experts, rows that end inside a chunk, and experts
+    of equal rows (so equal logits): the routing of the same tokens 200 at a time, bit for bit."""
+    router = synth.normal(41, synth.STREAM_ROUTER, experts * hidden).reshape(experts, hidden) * 0.1
+    router[experts // 2] = router[3]
+    router[experts - 1] = router[0]
+    shape = MoeShape("tiles", hidden, experts, topk, 32, fmt="q8")
+    lw = layer_weights(oracle, shape, 3)
+    lw = workloads.LayerWeights(weights.Matrix.from_f32(router.reshape(-1), experts, hidden, "bf16"), lw.gate_up, lw.down)
+    x = workloads.hidden_states(shape, t, seed=t)
+    x[5] = 0.0  # (all logits equal)
+    norm = ctx.to_device((1.0 + 0.1 * synth.normal(7, synth.STREAM_HIDDEN, hidden)).astype(np.float32))
+    ctx.set_arithmetic(ctx.ARITH_FAST)
+    layer = make_layer(ctx, lw, topk, t)
+
+    def routing(rows):
+        y = ctx.to_device(rows)
+        layer.block(norm, 1e-6, y)
+        ids, gates, _, logits = layer.last_routing(len(rows))
+        y.free()
+        return ids, gates, logits
+
+    try:
+        ctx.set_decode_block(False)
+        whole = routing(x)
+        for lo in range(0, t, 200):
+            for a, b in zip(routing(x[lo:lo + 200]), whole):
+                assert np.array_equal(a, b[lo:lo + 200])
+    finally:
+        ctx.set_decode_block(True)
+        layer.free()
 
 
 @pytest.mark.parametrize("t", [1, 128, 129])
