@@ -15,6 +15,8 @@
 //    (32x32b) they were 65 words: 272 cycles of shared memory a unit beside the other 130, in units of 365 to 430.
 //  - The float loop's code is 4 blocks long with constant addresses, a barrier test and an arrival per 2 blocks;
 //    the finishing code is rolled. (Unrolled as far as 16 KB it cost the float warps 20 % in instruction fetches.)
+//  - Products are issued and copies made by converged warps, and an operand stage is free again once its products
+//    are done; the scales have a longer ring of their own.
 //  - The operands are the 8-bit values as f16 (kind::f16). Products and sums of a block are
 //    integers below 2^20, exact in the f32 accumulator, so the sums arrive as floats. With kind::i8
 //    every sum costs a conversion besides (238 cycles per unit); with mma.sync, which would leave the
@@ -32,13 +34,16 @@
 // remainder of 128, 64 or 32 columns (4-bit: 64 at most, since each output keeps a second chain).
 // Every wait is bounded; TMEM is freed on every path.
 //
-// Measured (granite-1b-a400m, 4096 tokens, int8; 24 us of gate_up tile the activations): gate_up 234 -> 195 us, down 109
-// -> 92; 64 experts of 2048 x 1024: 812 -> 664, 383 -> 314; 40 of 1536 x 512 in 4 bits at 2047 tokens: 276 -> 230, 138 ->
-// 115. A unit takes 330 cycles now (365 to 430 before); nothing in it is saturated, two float warps per scheduler share its
-// issue slots with a finishing warp. Tried: 16 float warps of 32 columns (as before or slower), the loop rolled to a
-// block (4 warps' bookkeeping: 342 instructions a unit against 177) or to a chunk (211 / 99 us), pieces of 32 values a
-// lane (spills), a block's scales read a block ahead (spills), polling instead of suspended waits (no change), kind::i8
-// (conversions: 10 % slower), mma.sync with the sums in registers (8 % slower).
+// Measured (granite-1b-a400m, 4096 tokens, int8; 24 us of gate_up tile the activations): gate_up 234 -> 189 us, down 109
+// -> 88; 64 experts of 2048 x 1024: 812 -> 626, 383 -> 293; 40 of 1536 x 512 in 4 bits at 2047 tokens: 276 -> 213, 138 ->
+// 109. A chunk of two blocks takes 750 cycles (188 a unit), a tile 3300 besides, and another 3300 of a scheduler's time go
+// to finishing it in gate_up; 4-bit tiles, of 64 columns, take 480 a unit, where shared memory alone is 395 (192 the
+// scales, 96 operands, 98 copies). Tried: 16 float warps of 32 columns (as before or slower), the loop rolled to a
+// block (bookkeeping: 342 instructions a unit against 177) or to a chunk (211 / 99 us), pieces of 32 values a
+// lane (spills), a block's scales read a block ahead (spills), 4-bit tiles of 128 columns (spills), remainders of 65 to 96
+// tokens as 64 + 32 columns (333 tokens 42 + 25 -> 54 + 31 us: a narrow tile costs nearly as much as a wide one), the widest
+// tiles first (1 %), polling instead of suspended waits (3 % slower), kind::i8 (conversions: 10 % slower), mma.sync with the
+// sums in registers (8 % slower).
 #include <algorithm>
 #include <type_traits>
 
@@ -69,19 +74,27 @@ static_assert((P_EW * P_REGS_FLOAT + P_IW * P_REGS_ISSUE + P_FW * P_REGS_FINISH)
 
 __host__ __device__ constexpr int prefill_columns(bool q4) { return q4 ? 64 : 128; }  // the largest token tile
 
-// A shared-memory stage: P_CHUNK blocks of weights, activations, and their scales.
+// Shared memory: a ring of N operand stages (P_CHUNK blocks of weights and activations), left as soon as their products are
+// done, a ring of SN sets of their scales, read until the float warps are through with the sums, and a parked tile.
+// (Scales in the operands' stages held those back by a chunk, and the copies' latency showed: 4-bit tiles waited 370 of the
+// 980 cycles of a chunk for operands.)
 template <bool Q4>
 struct Stage {
     static constexpr int TOK = prefill_columns(Q4);
     static constexpr int B = P_CHUNK * P_A_BLOCK;
-    static constexpr int WD = B + P_CHUNK * TOK * 64;
-    static constexpr int XS = WD + P_CHUNK * P_ROWS * 4;
-    static constexpr int WC = XS + P_CHUNK * TOK * 4;      // (4-bit only from here)
+    static constexpr int BYTES = B + P_CHUNK * TOK * 64;
+    static constexpr int N = 4;                             // operand stages
+    static constexpr int XS = P_CHUNK * P_ROWS * 4;         // (the weights' scales come first)
+    static constexpr int WC = XS + P_CHUNK * TOK * 4;       // (4-bit only from here)
     static constexpr int XSUM = WC + P_CHUNK * P_ROWS * 4;
-    static constexpr int BYTES = Q4 ? XSUM + P_CHUNK * TOK * 4 : WC;
-    static constexpr int N = 4;                             // ring depth
+    static constexpr int SET = Q4 ? XSUM + P_CHUNK * TOK * 4 : WC;
+    // Sets of scales. Chunk c's go in when the products of chunk c - N are done, and those waited for the float warps to be
+    // through with chunk c - N - P_NGRP.
+    static constexpr int SN = 8;
+    static_assert(SN >= N + P_NGRP, "a set is read before it is overwritten");
     static constexpr int PARK = TOK * P_HSTRIDE * 4;
-    static constexpr size_t SMEM = size_t(N) * BYTES + PARK + (2 * N + 2 * P_NGRP + 3) * 8;
+    static constexpr int SCALES = N * BYTES, PARKED = SCALES + SN * SET, BARS = PARKED + PARK;
+    static constexpr size_t SMEM = size_t(BARS) + (2 * N + 2 * P_NGRP + 3) * 8;
     static_assert(SMEM <= P_SMEM_LIMIT, "stages fit");
 };
 
@@ -161,8 +174,8 @@ __device__ __forceinline__ uint2 f16_from_s8(uint32_t w) {
     return make_uint2(*reinterpret_cast<const uint32_t*>(&l), *reinterpret_cast<const uint32_t*>(&h));
 }
 
-// A role's place in the two rings is one number, the chunks of the CTA's sequence so far, across tiles:
-// chunk c is in operand stage c % 4 and in TMEM half c % 2.
+// A role's place in the rings is one number, the chunks of the CTA's sequence so far, across tiles:
+// chunk c is in operand stage c % 4, scale set c % 8 and TMEM half c % 2.
 template <bool Q4>
 __device__ __forceinline__ uint32_t stage_of(uint32_t c) { return c % Stage<Q4>::N; }
 template <bool Q4>
@@ -171,7 +184,7 @@ __device__ __forceinline__ uint32_t half_of(uint32_t c) { return c % P_NGRP; }
 __device__ __forceinline__ uint32_t half_par(uint32_t c) { return (c / P_NGRP) & 1; }
 
 struct Bars {
-    uint64_t *full, *empty;    // [stages] operands landed; left by the MMAs and every float warp (the issuer passes it on)
+    uint64_t *full, *empty;    // [stages] operands and scales landed; left by the MMAs
     uint64_t *tfull, *tempty;  // [P_NGRP] a chunk's sums are in TMEM, its scales in shared memory; read by every float warp
     uint64_t *pfull, *pempty;  // a tile has been parked by every float warp; taken by every finishing warp
     uint64_t* drain;           // after a failure only: the issuer's MMAs so far are done
@@ -214,10 +227,10 @@ __device__ __forceinline__ void float_chains(float (&acc)[64], float (&off)[Q4 ?
     float v[2][PC];
     float2 w[2], wc[Q4 ? 2 : 1];
     float4 x[CW / 16], u[Q4 ? CW / 16 : 1];
-    const uint32_t wat = S::WD + (row0 + (lane >> 2) * 4) * 4, xat = S::XS + (col0 + (lane & 3) * 4) * 4;
+    const uint32_t wat = S::SCALES + (row0 + (lane >> 2) * 4) * 4, xat = S::SCALES + S::XS + (col0 + (lane & 3) * 4) * 4;
     auto row_scales = [&](uint32_t st, int k, int h) {  // of the lane's two rows in half h
         w[h] = staged_f2(st + wat + (k * P_ROWS + 2 * h) * 4);
-        if (Q4) wc[Q4 ? h : 0] = staged_f2(st + wat + (S::WC - S::WD) + (k * P_ROWS + 2 * h) * 4);
+        if (Q4) wc[Q4 ? h : 0] = staged_f2(st + wat + S::WC + (k * P_ROWS + 2 * h) * 4);
     };
     auto column_scales = [&](uint32_t st, int k, int j) {  // of the lane's columns among sixteen
         x[j] = staged_f4(st + xat + (k * N + j * 16) * 4);
@@ -249,6 +262,7 @@ __device__ __forceinline__ void float_chains(float (&acc)[64], float (&off)[Q4 ?
         if (Q4) off[j] = 0.0f;
     }
     const uint32_t sums = tbase + col0;
+    auto set_of = [](uint32_t turn) { return turn % (S::SN / P_NGRP) * P_NGRP; };  // a turn's first set of scales
     auto fetch = [&](uint32_t at, int p) { umma::ld_half_f32(at + p / 2 * 32 + (uint32_t(p & 1) << 20), v[p & 1]); };
     auto first_scales = [&](uint32_t st, int k) {
         row_scales(st, k, 0);
@@ -267,17 +281,17 @@ __device__ __forceinline__ void float_chains(float (&acc)[64], float (&off)[Q4 ?
         wait_or_abort(bars.tfull, turn & 1, bars.abort_flag);
         umma::fence_after_sync();
         fetch(sums, 0);
-        first_scales(smem + (turn & 1) * P_NGRP * S::BYTES, 0);
+        first_scales(smem + set_of(turn) * S::SET, 0);
     }
 #pragma unroll 1
     for (int t = 1; t <= whole; t++, turn++) {
-        const uint32_t par = turn & 1, st = smem + par * P_NGRP * S::BYTES, other = smem + (par ^ 1) * P_NGRP * S::BYTES;
+        const uint32_t par = turn & 1, st = smem + set_of(turn) * S::SET, other = smem + set_of(turn + 1) * S::SET;
         const bool again = t < whole;
 #pragma unroll
         for (int i = 0; i < P_NGRP * P_CHUNK; i++) {
             const int half = i / P_CHUNK, kn = (i + 1) % P_CHUNK;
             const bool ends = kn == 0, last = i + 1 == P_NGRP * P_CHUNK, more = !last || again;
-            const uint32_t next = last ? other : st + (i + 1) / P_CHUNK * S::BYTES;  // the next block's stage
+            const uint32_t next = last ? other : st + (i + 1) / P_CHUNK * S::SET;  // where the next block's scales are
             bool ready = true;
 #pragma unroll
             for (int p = 0; p < PIECES; p++) {
@@ -309,14 +323,14 @@ __device__ __forceinline__ void float_chains(float (&acc)[64], float (&off)[Q4 ?
     }
     // What is left of a number of blocks that is no multiple of four (a turn all the same, of fewer blocks).
     if (const int rest = nb - whole * P_NGRP * P_CHUNK) {
-        const uint32_t st = smem + (turn & 1) * P_NGRP * S::BYTES;
+        const uint32_t st = smem + set_of(turn) * S::SET;
 #pragma unroll 1
         for (int half = 0; half < P_NGRP; half++) {
             wait_or_abort(bars.tfull + half, turn & 1, bars.abort_flag);
             umma::fence_after_sync();
 #pragma unroll 1
             for (int k = 0; k < P_CHUNK && half * P_CHUNK + k < rest; k++) {
-                first_scales(st + half * S::BYTES, k);
+                first_scales(st + half * S::SET, k);
 #pragma unroll
                 for (int p = 0; p < PIECES; p++) {
                     fetch(sums + (half * P_CHUNK + k) * P_TBUF, p);
@@ -396,11 +410,11 @@ __global__ void __launch_bounds__(P_THREADS, 1)
     expert_prefill_kernel(const PrefillArgs a, const std::conditional_t<PEER, PrefillPeer, NoPeer> peer) {
     using S = Stage<Q4>;
     extern __shared__ __align__(128) uint8_t smem[];
-    float* parked = reinterpret_cast<float*>(smem + S::N * S::BYTES);  // [tokens][P_HSTRIDE] a finished tile
+    float* parked = reinterpret_cast<float*>(smem + S::PARKED);  // [tokens][P_HSTRIDE] a finished tile
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
     Bars bars;
-    bars.full = reinterpret_cast<uint64_t*>(smem + S::N * S::BYTES + S::PARK);
+    bars.full = reinterpret_cast<uint64_t*>(smem + S::BARS);
     bars.empty = bars.full + S::N;
     bars.tfull = bars.empty + S::N;
     bars.tempty = bars.tfull + P_NGRP;
@@ -479,33 +493,47 @@ __global__ void __launch_bounds__(P_THREADS, 1)
         }
     } else if (warp < P_EW + P_IW) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(P_REGS_ISSUE));
-        if (warp == P_EW && lane == 0) {
+        // (Both warps run converged, a lane elected for what only one may do: addresses and descriptors then stay in
+        // uniform registers. By a lone lane the four products and commit of a chunk took 465 cycles of issue, a
+        // chunk 780 of this warp's 1060.)
+        if (warp == P_EW) {
             // ---- producer: operand chunks, each once its stage is free again
             asm volatile("fence.proxy.async;" ::: "memory");  // the tiles were written by plain stores
             uint32_t c = 0;
             TokenTile ahead = tile_of(a, blockIdx.x, work);
             for (int w = blockIdx.x; w < work; w += gridDim.x) {
-                const TokenTile tile = ahead;
+                const uint32_t N = warp_uniform(ahead.cols), expert = warp_uniform(uint32_t(ahead.expert)), row0 = warp_uniform(ahead.row0);
                 ahead = tile_of(a, w + gridDim.x, work);
-                const size_t wtile = size_t(tile.expert) * a.row_tiles + w % a.row_tiles;
-                const uint32_t N = tile.cols;
+                const size_t wo = (size_t(expert) * a.row_tiles + w % a.row_tiles) * nb, xo = size_t(row0) * nb;
+                const uint8_t* wt = reinterpret_cast<const uint8_t*>(a.wt) + wo * P_A_BLOCK;
+                const uint8_t* xt = reinterpret_cast<const uint8_t*>(a.xt) + xo * 64;
+                const float* wd = a.wd + wo * P_ROWS;
+                const float* wc = Q4 ? a.wc + wo * P_ROWS : nullptr;
+                const float* xst = a.xst + xo;
+                const float* xsumt = Q4 ? a.xsumt + xo : nullptr;
                 for (int b0 = 0; b0 < turn_blocks; b0 += P_CHUNK, c++) {
-                    const uint32_t nblk = max(0, min(P_CHUNK, nb - b0));  // (none in the chunks that fill up a turn)
+                    const uint32_t nblk = uint32_t(max(0, min(P_CHUNK, nb - b0)));  // (none in the chunks that fill up a turn)
                     uint64_t* full = bars.full + stage_of<Q4>(c);
                     if (c >= uint32_t(S::N)) wait_or_abort(bars.empty + stage_of<Q4>(c), stage_par<Q4>(c) ^ 1, bars.abort_flag);
                     uint8_t* st = smem + stage_of<Q4>(c) * S::BYTES;
+                    uint8_t* sc = smem + S::SCALES + c % S::SN * S::SET;
                     const uint32_t wb = nblk * P_A_BLOCK, xb = nblk * N * 64, wf = nblk * P_ROWS * 4, xf = nblk * N * 4;
-                    const size_t wo = wtile * nb + b0, xo = size_t(tile.row0) * nb + size_t(b0) * N;
-                    mbar_expect_tx(full, wb + xb + (wf + xf) * (Q4 ? 2 : 1));
-                    if (nblk == 0) continue;
-                    bulk_copy(st, a.wt + wo * (P_A_BLOCK / 2), wb, full);
-                    bulk_copy(st + S::B, a.xt + xo * 32, xb, full);
-                    bulk_copy(st + S::WD, a.wd + wo * P_ROWS, wf, full);
-                    bulk_copy(st + S::XS, a.xst + xo, xf, full);
-                    if (Q4) {
-                        bulk_copy(st + S::WC, a.wc + wo * P_ROWS, wf, full);
-                        bulk_copy(st + S::XSUM, a.xsumt + xo, xf, full);
+                    if (umma::elect_one()) {
+                        mbar_expect_tx(full, wb + xb + (wf + xf) * (Q4 ? 2 : 1));
+                        if (nblk) {
+                            bulk_copy(st, wt, wb, full);
+                            bulk_copy(st + S::B, xt, xb, full);
+                            bulk_copy(sc, wd, wf, full);
+                            bulk_copy(sc + S::XS, xst, xf, full);
+                            if (Q4) {
+                                bulk_copy(sc + S::WC, wc, wf, full);
+                                bulk_copy(sc + S::XSUM, xsumt, xf, full);
+                            }
+                        }
                     }
+                    __syncwarp();
+                    wt += P_CHUNK * P_A_BLOCK, xt += P_CHUNK * N * 64, wd += P_CHUNK * P_ROWS, xst += P_CHUNK * N;
+                    if (Q4) wc += P_CHUNK * P_ROWS, xsumt += P_CHUNK * N;
                 }
             }
             if (s_abort) {
@@ -513,39 +541,43 @@ __global__ void __launch_bounds__(P_THREADS, 1)
                 for (uint32_t i = c > uint32_t(S::N) ? c - S::N : 0; i < c; i++)
                     mbar_wait_bounded(bars.full + stage_of<Q4>(i), stage_par<Q4>(i));
             }
-        } else if (warp == P_EW + 1 && lane == 0) {
+        } else if (warp == P_EW + 1) {
             // ---- MMA issuer: a block = two K = 16 products into its own TMEM buffer, a commit per chunk
+            const uint32_t sums = warp_uniform(tmem);
             uint32_t c = 0;
             TokenTile ahead = tile_of(a, blockIdx.x, work);
             for (int w = blockIdx.x; w < work; w += gridDim.x) {
-                const uint32_t N = ahead.cols, idesc = umma::idesc_f16(P_ROWS, int(N));
+                const uint32_t N = warp_uniform(ahead.cols), idesc = umma::idesc_f16(P_ROWS, int(N));
                 ahead = tile_of(a, w + gridDim.x, work);
                 for (int b0 = 0; b0 < turn_blocks; b0 += P_CHUNK, c++) {
-                    const int nblk = min(P_CHUNK, nb - b0);
-                    if (c >= uint32_t(P_NGRP)) {
-                        wait_or_abort(bars.tempty + half_of(c), half_par(c) ^ 1, bars.abort_flag);
-                        mbar_arrive_if(bars.empty + stage_of<Q4>(c - P_NGRP), true);
-                    }
+                    const int nblk = nb - b0;
                     wait_or_abort(bars.full + stage_of<Q4>(c), stage_par<Q4>(c), bars.abort_flag);
+                    if (c >= uint32_t(P_NGRP)) wait_or_abort(bars.tempty + half_of(c), half_par(c) ^ 1, bars.abort_flag);
                     umma::fence_after_sync();
+                    // (Low words of the descriptors: address and K stride; the rest is the same for all.)
                     const uint32_t sa = smem_addr(smem + stage_of<Q4>(c) * S::BYTES), sb = sa + S::B;
+                    const uint32_t da = umma::smem_desc_low(sa, P_ROWS * 16), db = umma::smem_desc_low(sb, N * 16);
+                    const uint32_t d = sums + half_of(c) * P_CHUNK * P_TBUF;
+                    if (umma::elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < P_CHUNK; k++) {
-                        if (k < nblk) {
-                            const uint32_t d = tmem + (half_of(c) * P_CHUNK + k) * P_TBUF;
+                        for (int k = 0; k < P_CHUNK; k++) {
+                            if (k < nblk) {
 #pragma unroll
-                            for (int h = 0; h < 2; h++)
-                                umma::mma_f16(d, umma::smem_desc(sa + k * P_A_BLOCK + h * P_ROWS * 32, P_ROWS * 16, 128),
-                                              umma::smem_desc(sb + k * N * 64 + h * N * 32, N * 16, 128), idesc, uint32_t(h));
+                                for (int h = 0; h < 2; h++)
+                                    umma::mma_f16_low(d + k * P_TBUF, da + (k * P_A_BLOCK + h * P_ROWS * 32) / 16, db + (k * 2 + h) * N * 2, idesc, uint32_t(h));
+                            }
                         }
+                        umma::commit(bars.tfull + half_of(c));
+                        mbar_arrive_if(bars.tfull + half_of(c), true);  // (what this warp saw land, the float warps may read)
+                        umma::commit(bars.empty + stage_of<Q4>(c));
                     }
-                    umma::commit(bars.tfull + half_of(c));
-                    mbar_arrive_if(bars.tfull + half_of(c), true);  // (what this thread saw land, the float warps may read)
+                    __syncwarp();
                 }
             }
             if (s_abort) {
                 // Giving up: the MMAs in flight must finish before TMEM is freed.
-                umma::commit(bars.drain);
+                if (umma::elect_one()) umma::commit(bars.drain);
+                __syncwarp();
                 mbar_wait_bounded(bars.drain, 0);
             }
         }

@@ -72,6 +72,27 @@ __device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t a_desc, uint64
         : "memory");
 }
 
+// One lane of a converged warp.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t yes;
+    asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\tselp.u32 %0, 1, 0, e;\n\t}" : "=r"(yes));
+    return yes != 0;
+}
+
+// mma_f16 with descriptors of which only the low words (address, leading offset) differ: SBO 128 bytes, as everywhere here.
+__device__ __forceinline__ uint32_t smem_desc_low(uint32_t smem_addr, uint32_t lbo_bytes) {
+    return ((smem_addr >> 4) & 0x3FFFu) | ((lbo_bytes >> 4) & 0x3FFFu) << 16;
+}
+__device__ __forceinline__ void mma_f16_low(uint32_t tmem_d, uint32_t a_low, uint32_t b_low, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "mov.b64 da, {%1, %6};\n\tmov.b64 db, {%2, %6};\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, {%5, %5, %5, %5}, p;\n\t}"
+        ::"r"(tmem_d), "r"(a_low), "r"(b_low), "r"(idesc), "r"(accumulate), "r"(0u), "n"((128 >> 4) | 1 << 14)
+        : "memory");
+}
+
 // Arrives on an mbarrier once every MMA issued so far by this thread has completed.
 __device__ __forceinline__ void commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
