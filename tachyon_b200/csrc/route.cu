@@ -198,6 +198,7 @@ struct RouteTile {
     static constexpr int REGS_DOTS = TG * TE > 20 ? 176 : 136, REGS_ROWS = 256 - REGS_DOTS;
     static_assert(KC >= MAX_TOPK, "the exponentials of a tile's picks fit where its rows were");
     __host__ __device__ static int key_stride(int experts) { return (experts + 31) / 32 * 32; }
+    static_assert(2 * (X + W) >= int(sizeof(DispatchSmem)), "a dispatch fits where the buffers were");
     __host__ __device__ static size_t bytes(int experts, int topk) {
         return 2 * size_t(X + W) + size_t(TM) * (key_stride(experts) + 2 * topk + 1) * 4;
     }
@@ -444,6 +445,22 @@ __global__ void __launch_bounds__(RT_THREADS, 1) route_tile_kernel(const RouteAr
         a.ids[size_t(t0) * topk + i] = sid[i];
         a.gates[size_t(t0) * topk + i] = __fdiv_rn(sexp[i], sum);
     }
+    // ---- the dispatch of a batch that one CTA can dispatch, by the last CTA to get here (its first 256 threads have a token
+    // each; the others take part in the barriers)
+    if (a.fuse_dispatch) {
+        __shared__ int s_last;
+        __threadfence();  // this CTA's ids are visible before its ticket
+        __syncthreads();
+        if (tid == 0) s_last = atomicAdd(a.ticket, 1) == int(gridDim.x) - 1;
+        __syncthreads();
+        if (s_last) {
+            __threadfence();
+            DispatchSmem& sm = *reinterpret_cast<DispatchSmem*>(rt_smem);
+            dispatch_small_body(sm, a.ids, a.t, experts, topk, a.counts, a.offsets, a.perm, a.pos, a.slot_token, a.active, a.status);
+            if (a.tiles) token_tiles_body(sm.scount, sm.soff, experts, a.tile_cols, a.tiles, a.tile_count, sm.stiles, sm.srows);
+            if (tid == 0) *a.ticket = 0;  // ready for the next launch on this stream
+        }
+    }
 }
 
 // One warp per row.
@@ -506,11 +523,14 @@ int launch_route(const MoeDims& d, const uint16_t* router, const float* bias, co
     if (a.stage_router) smem = staged;
     if (smem < sizeof(DispatchSmem)) smem = sizeof(DispatchSmem);
     const int sms = ws.sms > 0 ? ws.sms : 148;
-    if (a.fuse_dispatch) {
-        // Up to one CTA's worth of tokens: a CTA per token; the last one to finish runs the dispatch.
+    if (a.fuse_dispatch && (t <= 128 || a.scatter.ranks > 0)) {
+        // Few tokens (or rows that go to every rank from here): a CTA per token; the last one to finish runs the dispatch.
+        // (Past 128 the tiles below are ahead, whole blocks of 129 / 200 / 256 tokens in us: 1b shape 69.9 / 74.9 / 87.6 so,
+        // 67.5 / 71.0 / 82.8 in tiles; 64 experts of 2048 x 1024 201 / 205 / 211, 196 / 200 / 205. Up to 128 these kernels only run
+        // with the one-kernel block off.)
         launch_overlapped(route_kernel, dim3(t), dim3(ROUTE_THREADS), smem, stream, a);
     } else {
-        // Larger batches: a CTA per tile of 32, 16, 8 or 4 tokens, the widest that still gives two thirds of the SMs one.
+        // A CTA per tile of 32, 16, 8 or 4 tokens, the widest that still gives two thirds of the SMs one.
         // (The wider the tile, the fewer bytes of shared memory a product costs. 333 tokens of the 1b shape in tiles of 2,
         // which are more than there are SMs: 14.9 us, of 4: 9.7.)
         const int tm = t >= 32 * 2 * sms / 3 ? 32 : t >= 16 * 2 * sms / 3 ? 16 : t >= 8 * 2 * sms / 3 ? 8 : 4;

@@ -38,10 +38,10 @@ def test_blocks_at_the_edges(oracle, ctx, shape, t, skewed):
 
 
 @pytest.mark.parametrize("hidden,experts,topk", [(96, 31, 5), (160, 40, 8), (544, 64, 8), (1056, 130, 8), (64, 256, 32)])
-@pytest.mark.parametrize("t", [261, 803, 1601, 3200])
+@pytest.mark.parametrize("t", [131, 261, 803, 1601, 3200])
 def test_router_tiles_match_the_router_of_one_token(oracle, ctx, hidden, experts, topk, t):
     """Every tile size with a remainder, one to four passes over the experts, rows that end inside a chunk, and experts
-    of equal rows (so equal logits): the routing of the same tokens 200 at a time, bit for bit."""
+    of equal rows (so equal logits): the routing of the same tokens 100 at a time, bit for bit, and their order by expert."""
     router = synth.normal(41, synth.STREAM_ROUTER, experts * hidden).reshape(experts, hidden) * 0.1
     router[experts // 2] = router[3]
     router[experts - 1] = router[0]
@@ -64,9 +64,13 @@ def test_router_tiles_match_the_router_of_one_token(oracle, ctx, hidden, experts
     try:
         ctx.set_decode_block(False)
         whole = routing(x)
-        for lo in range(0, t, 200):
-            for a, b in zip(routing(x[lo:lo + 200]), whole):
-                assert np.array_equal(a, b[lo:lo + 200])
+        offsets, perm = layer.last_dispatch(t)
+        picks = whole[0].reshape(-1)
+        assert np.array_equal(perm, np.argsort(picks, kind="stable"))
+        assert np.array_equal(offsets[1:], np.cumsum(np.bincount(picks, minlength=experts)))
+        for lo in range(0, t, 100):
+            for a, b in zip(routing(x[lo:lo + 100]), whole):
+                assert np.array_equal(a, b[lo:lo + 100])
     finally:
         ctx.set_decode_block(True)
         layer.free()
