@@ -38,12 +38,13 @@ struct tc_ctx {
     tc::PrefillScratch pre;   // token tiles of the tcgen05 path
     std::vector<void*> pre_allocs;
     // Tokens per expert (on average) from which the tcgen05 kernels take over, past the one-kernel block's 128 tokens.
-    // 16 is about where they cross the bandwidth-oriented ones under an even router (us per block, tcgen05 / the
-    // others, 8-bit, 8 picks): 64 experts of 2048 x 1024 at 129 tokens, an average of 16.1: 239 / 250; 128 experts of
-    // 1024 x 512 at 14: 166 / 156, 16: 169 / 163, 20: 171 / 172; 256 of them at 14: 293 / 266, 16: 295 / 281, 20: 303 / 312;
-    // 96 of 2048 x 768, 4 picks, at 13: 283 / 271, 16: 285 / 274, 20: 289 / 330. 4-bit weights cross at the same place;
-    // 32 to 40 experts are past it at 129 tokens (80 / 104, 110 / 135). A router that prefers a few experts puts the
-    // tcgen05 kernels far ahead below the line too: 128 experts at 144 tokens, an average of 9, with a Zipf bias 110 / 447.
+    // Under an even router they cross the bandwidth-oriented ones between 8 and 12 (us per block, tcgen05 / the
+    // others, 8-bit, 8 picks): 64 experts of 2048 x 1024 at 129 tokens, an average of 16.1: 193 / 239; 128 experts of
+    // 1024 x 512 at 9: 129 / 102, 12: 131 / 143, 16: 133 / 154; 256 of them at 8: 228 / 192, 12: 226 / 235, 16: 228 / 266;
+    // 96 of 2048 x 768, 4 picks, at 8: 218 / 163, 10.7: 220 / 225, 16: 221 / 256. 4-bit weights at 9 to 12 (128 experts 128 / 132
+    // at 9). 16 is from slower tcgen05 kernels, which crossed there; between 12 and 16 it now costs 4 to 13 %.
+    // 32 to 40 experts are past it at 129 tokens (64 / 101, 91 / 132). A router that prefers a few experts puts the
+    // tcgen05 kernels far ahead below the line too: 128 experts at 144 tokens, an average of 9, with a Zipf bias 90 / 440.
     // But the counts are on the device and the choice is made on the host, from the average.
     int prefill_min_avg = 16;
     float* host_x = nullptr;  // device staging for the host-buffer entry point (large batches)

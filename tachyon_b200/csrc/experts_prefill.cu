@@ -21,7 +21,6 @@
 //    integers below 2^20, exact in the f32 accumulator, so the sums arrive as floats. With kind::i8
 //    every sum costs a conversion besides (238 cycles per unit); with mma.sync, which would leave the
 //    sums in registers, conversions and a slower instruction (276).
-//  - Block scales travel with the operands, in the same shared-memory stages.
 //  - A finished tile is only parked in shared memory by the float warps; four other warps take it
 //    from there while the next tile's chains run: for gate_up SwiGLU, 8-bit quantization per
 //    32-block (src/kernels.rs:84-98) and the store in the layout the down product reads, so the
@@ -29,14 +28,14 @@
 // Persistent CTAs (one per SM) walk (token tile, 128-row tile) pairs; both rings run across tile
 // boundaries. Roles: warps 0-7 float chains (TMEM lane quadrant = warp % 4, half of the tokens
 // = warp / 4: a row's weight scale, a barrier wait and a release are paid once per 64 outputs of a
-// lane), warp 8 streams operand chunks of 2 blocks, one thread of warp 9 issues the products into a ring
+// lane), warp 8 streams operand chunks of 2 blocks, an elected lane of warp 9 issues the products into a ring
 // of two TMEM halves, warps 12-15 finish tiles. An expert's tokens are cut into tiles of 128 and a
 // remainder of 128, 64 or 32 columns (4-bit: 64 at most, since each output keeps a second chain).
 // Every wait is bounded; TMEM is freed on every path.
 //
-// Measured (granite-1b-a400m, 4096 tokens, int8; 24 us of gate_up tile the activations): gate_up 234 -> 189 us, down 109
-// -> 88; 64 experts of 2048 x 1024: 812 -> 626, 383 -> 293; 40 of 1536 x 512 in 4 bits at 2047 tokens: 276 -> 213, 138 ->
-// 109. A chunk of two blocks takes 750 cycles (188 a unit), a tile 3300 besides, and another 3300 of a scheduler's time go
+// Measured (granite-1b-a400m, 4096 tokens, int8; 24, now 20 us of gate_up tile the activations): gate_up 234 -> 183 us, down
+// 109 -> 86; 64 experts of 2048 x 1024: 812 -> 615, 383 -> 291; 40 of 1536 x 512 in 4 bits at 2047 tokens: 276 -> 209, 138
+// -> 109. A chunk of two blocks takes 750 cycles (188 a unit), a tile 3300 besides, and another 3300 of a scheduler's time go
 // to finishing it in gate_up; 4-bit tiles, of 64 columns, take 480 a unit, where shared memory alone is 395 (192 the
 // scales, 96 operands, 98 copies). Tried: 16 float warps of 32 columns (as before or slower), the loop rolled to a
 // block (bookkeeping: 342 instructions a unit against 177) or to a chunk (211 / 99 us), pieces of 32 values a
