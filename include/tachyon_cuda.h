@@ -134,7 +134,8 @@ int tc_moe_set_router_bias(tc_moe_layer *layer, const float *bias_host);
 int tc_moe_forward(tc_moe_layer *layer, const float *x_dev, int t, float *y_dev);
 /* The whole MLP block of a MoE layer on the residual stream, as
  * src/model.rs:662-681 runs it: y[t,hidden] += moe(rmsnorm(y, norm_weight, eps)).
- * The norm is fused into the router kernel (same arithmetic as tc_rmsnorm). */
+ * The norm is fused into the router kernel (same arithmetic as tc_rmsnorm). y as above; the weight
+ * may stand at any float, in a packed buffer for instance. */
 int tc_moe_block(tc_moe_layer *layer, const float *norm_weight_dev, float eps, int t, float *y_dev);
 /* The same through host buffers: copies x and y in, runs, copies y back, waits. */
 int tc_moe_forward_host(tc_moe_layer *layer, const float *x_host, int t, float *y_host);

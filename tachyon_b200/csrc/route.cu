@@ -204,6 +204,8 @@ struct RouteTile {
     }
 };
 
+__device__ __forceinline__ float4 four_floats(const float* p) { return make_float4(p[0], p[1], p[2], p[3]); }
+
 template <int NG, int TG, int TE, int KC>
 __global__ void __launch_bounds__(RT_THREADS, 1) route_tile_kernel(const RouteArgs a) {
     using L = RouteTile<NG, TG, TE, KC>;
@@ -270,13 +272,16 @@ __global__ void __launch_bounds__(RT_THREADS, 1) route_tile_kernel(const RouteAr
         // This thread stages columns 8 col8 .. of rows row0, row0 + 256 / KV, ... of every chunk.
         const int row0 = rid / KV, col8 = rid % KV;
         const bool stages = rid < TASKS;  // (whole warps)
+        // The caller's weight may stand at any float. (Read so from an aligned one too, it is 1 to 2 us of a stage of 20 to 80.)
+        const bool norm_vec = reinterpret_cast<uintptr_t>(a.norm_w) % 16 == 0;
         float4 ahead[PER][2], nw[2];
         auto request = [&](int c) {
             const int col = c * KC + col8 * 8;
             const bool on = stages && col < hidden;
 #pragma unroll
             for (int h = 0; h < 2; h++) {
-                nw[h] = on && a.norm_w ? *reinterpret_cast<const float4*>(a.norm_w + col + 4 * h) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                nw[h] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (on && a.norm_w) nw[h] = norm_vec ? *reinterpret_cast<const float4*>(a.norm_w + col + 4 * h) : four_floats(a.norm_w + col + 4 * h);
 #pragma unroll
                 for (int i = 0; i < PER; i++) {
                     ahead[i][h] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);

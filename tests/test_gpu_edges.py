@@ -76,6 +76,39 @@ def test_router_tiles_match_the_router_of_one_token(oracle, ctx, hidden, experts
         layer.free()
 
 
+@pytest.mark.parametrize("t", [1, 33, 128, 129, 257, 800, 1600, 3200])
+def test_the_norms_weight_may_stand_at_any_float(oracle, ctx, t):
+    """A norm's weight that is a slice of a packed buffer, 4, 8 or 12 bytes past a 16-byte boundary: the same bits as
+    from an aligned one in every kernel that reads it (the one-kernel block, the router of a token, all router tiles)."""
+    shape = MoeShape("slice", 544, 8, 2, 32, fmt="q8")
+    lw = layer_weights(oracle, shape, 17)
+    x = workloads.hidden_states(shape, t, seed=t)
+    norm = (1.0 + 0.1 * synth.normal(7, synth.STREAM_HIDDEN, shape.hidden)).astype(np.float32)
+    ctx.set_arithmetic(ctx.ARITH_FAST)
+    layer = make_layer(ctx, lw, shape.topk, t)
+
+    def block(off):
+        packed = ctx.to_device(np.concatenate([np.full(off, 7.0, np.float32), norm, np.full(4, 7.0, np.float32)]))
+        assert packed.ptr % 16 == 0
+        y = ctx.to_device(x)
+        assert ctx.lib.tc_moe_block(layer.handle, packed.ptr + 4 * off, 1e-6, t, y.ptr) == 0
+        out = (y.get(), *layer.last_routing(t))
+        for d in (y, packed):
+            d.free()
+        return out
+
+    try:
+        for one_kernel in (True, False):
+            ctx.set_decode_block(one_kernel)
+            aligned = block(0)
+            for off in (1, 2, 3):
+                for a, b in zip(aligned, block(off)):
+                    assert np.array_equal(a, b)
+    finally:
+        ctx.set_decode_block(True)
+        layer.free()
+
+
 @pytest.mark.parametrize("t", [1, 128, 129])
 def test_host_buffers_at_the_edges(oracle, ctx, t):
     lw = layer_weights(oracle, ODD_Q8, 17)
