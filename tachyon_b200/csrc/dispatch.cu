@@ -113,14 +113,17 @@ namespace {
 // Large batches in one kernel, a CTA per expert: expert e's slots start after all the slots of lower
 // experts, so a CTA that counts the ids below e and those equal to e as it reads them needs nothing from the
 // others. A warp owns a contiguous range of the slots (read twice: count, then place), which keeps the
-// order; the hits go to shared memory first, and the three stores and the division by topk are made by a thread per
-// slot. (Made where a hit was found, under a mask in two of three groups of 32 ids, they were 13 of the kernel's 21
-// thousand cycles: 4096 tokens of 8 picks of 32 experts 15 us, now 13, of 64 experts 16.6, now 14.8.) The last CTA to finish lists the experts that have tokens and, when asked, cuts the token tiles.
+// order. The hits of an expert with up to DISPATCH_E_HELD slots go to shared memory first, and the three stores and the
+// division by topk are made by a thread per slot. (Made where a hit was found, under a mask in two of three groups of 32
+// ids, they were 13 of the kernel's 21 thousand cycles: 4096 tokens of 8 picks of 32 experts 15 us, now 13, of 64 experts
+// 16.6, now 14.8.) More slots than that are placed where they are found: held part by part, they took a walk over all ids
+// for every part (65536 tokens of 8 picks of 32 experts 209 us, now 166, with a Zipf bias on the router 485, now 192).
+// The last CTA to finish lists the experts that have tokens and, when asked, cuts the token tiles.
 // (Three passes with a histogram per 256 tokens, most of it launches and a serial scan, against every CTA
 // reading all ids, 128 KB from L2: router and dispatch of 4096 tokens of the 1b shape 68 to 58 us.)
 constexpr int DISPATCH_E_THREADS = 1024;
 constexpr int DISPATCH_E_WARPS = DISPATCH_E_THREADS / 32;
-constexpr int DISPATCH_E_HELD = 8192;  // an expert's slots held in shared memory at a time
+constexpr int DISPATCH_E_HELD = 8192;  // the most slots of an expert that shared memory holds
 
 struct DispatchArgs {
     const uint32_t* ids;
@@ -175,30 +178,36 @@ __global__ void __launch_bounds__(DISPATCH_E_THREADS) dispatch_experts_kernel(co
     const uint32_t h = s_hits[lane], first = __reduce_add_sync(0xffffffffu, s_below[lane]);
     uint32_t at = first + __reduce_add_sync(0xffffffffu, lane < warp ? h : 0u);
     const uint32_t total = __reduce_add_sync(0xffffffffu, h);
-    // The expert's slots in order, DISPATCH_E_HELD at a time, into shared memory; then a thread per slot.
-    for (uint32_t from = first; from < first + total; from += DISPATCH_E_HELD) {
-        const uint32_t most = min(first + total - from, uint32_t(DISPATCH_E_HELD));
-        for (uint32_t k = tid; k < most; k += DISPATCH_E_THREADS) s_slots[k] = 0xffffffffu;  // (none: see below)
+    // (The bounds below: after a wait for another rank has run out, its ids may still arrive between the two reads.)
+    auto place = [&](uint32_t p, uint32_t i) {
+        a.perm[p] = i;
+        a.slot_token[p] = i / uint32_t(a.topk);
+        a.pos[i] = p;
+    };
+    if (total <= uint32_t(DISPATCH_E_HELD)) {
+        for (uint32_t k = tid; k < total; k += DISPATCH_E_THREADS) s_slots[k] = 0xffffffffu;  // (none)
         __syncthreads();
-        uint32_t p = at - from;  // wraps for slots of earlier rounds
+        uint32_t p = at - first;
         if (hits) {
             walk([&](int i, uint32_t id) {
                 const unsigned ballot = __ballot_sync(0xffffffffu, id == e);
                 const uint32_t k = p + __popc(ballot & ((1u << lane) - 1u));
-                // (The bound: after a wait for another rank has run out, its ids may still arrive between the two reads.)
-                if (id == e && k < most) s_slots[k] = uint32_t(i);
+                if (id == e && k < total) s_slots[k] = uint32_t(i);
                 p += __popc(ballot);
             });
         }
         __syncthreads();
-        for (uint32_t k = tid; k < most; k += DISPATCH_E_THREADS) {
+        for (uint32_t k = tid; k < total; k += DISPATCH_E_THREADS) {
             const uint32_t i = s_slots[k];
-            if (i >= uint32_t(a.slots)) continue;
-            a.perm[from + k] = i;
-            a.slot_token[from + k] = i / uint32_t(a.topk);
-            a.pos[i] = from + k;
+            if (i < uint32_t(a.slots)) place(first + k, i);
         }
-        __syncthreads();
+    } else if (hits) {
+        walk([&](int i, uint32_t id) {
+            const unsigned ballot = __ballot_sync(0xffffffffu, id == e);
+            const uint32_t p = at + __popc(ballot & ((1u << lane) - 1u));
+            if (id == e && p < first + total) place(p, uint32_t(i));
+            at += __popc(ballot);
+        });
     }
     if (tid == 0) {
         a.counts[e] = total;
