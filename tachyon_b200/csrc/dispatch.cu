@@ -116,8 +116,9 @@ namespace {
 // order. The hits of an expert with up to DISPATCH_E_HELD slots go to shared memory first, and the three stores and the
 // division by topk are made by a thread per slot. (Made where a hit was found, under a mask in two of three groups of 32
 // ids, they were 13 of the kernel's 21 thousand cycles: 4096 tokens of 8 picks of 32 experts 15 us, now 13, of 64 experts
-// 16.6, now 14.8.) More slots than that are placed where they are found: held part by part, they took a walk over all ids
-// for every part (65536 tokens of 8 picks of 32 experts 209 us, now 166, with a Zipf bias on the router 485, now 192).
+// 16.6, now 14.8.) The slots of an expert with more are placed where they are found: held part by part, they took a walk over
+// all ids for every part (router and dispatch of 65536 tokens of 256 columns, 8 picks of 32 experts, 411 us, now 366, with a
+// Zipf bias on the router 691, now 399).
 // The last CTA to finish lists the experts that have tokens and, when asked, cuts the token tiles.
 // (Three passes with a histogram per 256 tokens, most of it launches and a serial scan, against every CTA
 // reading all ids, 128 KB from L2: router and dispatch of 4096 tokens of the 1b shape 68 to 58 us.)
@@ -135,6 +136,32 @@ struct DispatchArgs {
     int tile_cols;
     int *ticket, *status;
 };
+
+// The warp's slots of expert e, among lo .. hi - 1, straight to their places: from `at`, before `end`. Not inlined, and the
+// other form below a loop that runs once: inlined, or as straight code, the kernel takes 32 registers instead of 51, two CTAs fit an SM,
+// both go where the router leaves room first, and router and dispatch of 4096 tokens of the 1b shape take 45 us instead of 40.
+__device__ __noinline__ void place_as_found(const uint32_t* ids, uint32_t* perm, uint32_t* slot_token, uint32_t* pos, uint32_t topk,
+                                            uint32_t e, int lo, int hi, uint32_t at, uint32_t end) {
+    const int lane = threadIdx.x & 31;
+    constexpr int HELD = 8;
+#pragma unroll 1
+    for (int i0 = lo; i0 < hi; i0 += 32 * HELD) {
+        uint32_t id[HELD];
+#pragma unroll
+        for (int u = 0; u < HELD; u++) {
+            const int i = i0 + 32 * u + lane;
+            id[u] = i < hi ? __ldcg(ids + i) : 0xffffffffu;
+        }
+#pragma unroll
+        for (int u = 0; u < HELD; u++) {
+            const uint32_t i = i0 + 32 * u + lane;
+            const unsigned ballot = __ballot_sync(0xffffffffu, id[u] == e);
+            const uint32_t p = at + __popc(ballot & ((1u << lane) - 1u));
+            if (id[u] == e && p < end) perm[p] = i, slot_token[p] = i / topk, pos[i] = p;
+            at += __popc(ballot);
+        }
+    }
+}
 
 __global__ void __launch_bounds__(DISPATCH_E_THREADS) dispatch_experts_kernel(const DispatchArgs a, const PeerWait pw) {
     __shared__ uint32_t s_hits[DISPATCH_E_WARPS], s_below[DISPATCH_E_WARPS];
@@ -178,36 +205,31 @@ __global__ void __launch_bounds__(DISPATCH_E_THREADS) dispatch_experts_kernel(co
     const uint32_t h = s_hits[lane], first = __reduce_add_sync(0xffffffffu, s_below[lane]);
     uint32_t at = first + __reduce_add_sync(0xffffffffu, lane < warp ? h : 0u);
     const uint32_t total = __reduce_add_sync(0xffffffffu, h);
-    // (The bounds below: after a wait for another rank has run out, its ids may still arrive between the two reads.)
-    auto place = [&](uint32_t p, uint32_t i) {
-        a.perm[p] = i;
-        a.slot_token[p] = i / uint32_t(a.topk);
-        a.pos[i] = p;
-    };
-    if (total <= uint32_t(DISPATCH_E_HELD)) {
-        for (uint32_t k = tid; k < total; k += DISPATCH_E_THREADS) s_slots[k] = 0xffffffffu;  // (none)
+    // (The bounds: after a wait for another rank has run out, its ids may still arrive between the two reads.)
+    const bool held = total <= uint32_t(DISPATCH_E_HELD);
+    if (!held && hits) place_as_found(a.ids, a.perm, a.slot_token, a.pos, a.topk, e, lo, hi, at, first + total);
+    for (uint32_t from = first; held && from < first + total; from += DISPATCH_E_HELD) {
+        const uint32_t most = min(first + total - from, uint32_t(DISPATCH_E_HELD));
+        for (uint32_t k = tid; k < most; k += DISPATCH_E_THREADS) s_slots[k] = 0xffffffffu;  // (none)
         __syncthreads();
-        uint32_t p = at - first;
+        uint32_t p = at - from;
         if (hits) {
             walk([&](int i, uint32_t id) {
                 const unsigned ballot = __ballot_sync(0xffffffffu, id == e);
                 const uint32_t k = p + __popc(ballot & ((1u << lane) - 1u));
-                if (id == e && k < total) s_slots[k] = uint32_t(i);
+                if (id == e && k < most) s_slots[k] = uint32_t(i);
                 p += __popc(ballot);
             });
         }
         __syncthreads();
-        for (uint32_t k = tid; k < total; k += DISPATCH_E_THREADS) {
+        for (uint32_t k = tid; k < most; k += DISPATCH_E_THREADS) {
             const uint32_t i = s_slots[k];
-            if (i < uint32_t(a.slots)) place(first + k, i);
+            if (i >= uint32_t(a.slots)) continue;
+            a.perm[from + k] = i;
+            a.slot_token[from + k] = i / uint32_t(a.topk);
+            a.pos[i] = from + k;
         }
-    } else if (hits) {
-        walk([&](int i, uint32_t id) {
-            const unsigned ballot = __ballot_sync(0xffffffffu, id == e);
-            const uint32_t p = at + __popc(ballot & ((1u << lane) - 1u));
-            if (id == e && p < first + total) place(p, uint32_t(i));
-            at += __popc(ballot);
-        });
+        __syncthreads();
     }
     if (tid == 0) {
         a.counts[e] = total;

@@ -109,16 +109,17 @@ def test_the_norms_weight_may_stand_at_any_float(oracle, ctx, t):
         layer.free()
 
 
-@pytest.mark.parametrize("topk", [1, 2])
-@pytest.mark.parametrize("t", [8192, 8193, 17000])
-def test_dispatch_of_an_expert_with_more_slots_than_are_held(oracle, ctx, t, topk):
-    """Up to 8192 slots of an expert go through shared memory, more straight to their places: every token on
-    expert 1, so 8192 slots, one more, and twice as many, beside experts with the rest of the slots or none."""
-    shape = MoeShape("crowd", 32, 3, topk, 32, fmt="q8")
+@pytest.mark.parametrize("experts,topk,t", [
+    (3, 1, 8192), (3, 1, 8193), (3, 2, 8192), (3, 2, 17000), (200, 2, 8192), (200, 2, 8193), (200, 1, 20001),
+])
+def test_dispatch_of_an_expert_with_more_slots_than_are_held(oracle, ctx, experts, topk, t):
+    """An expert's slots go through shared memory up to 8192 of them and straight to their places beyond: every token on
+    expert 1, so as many slots, one more, and twice as many, beside the rest of the slots."""
+    shape = MoeShape("crowd", 32, experts, topk, 32, fmt="q8")
     lw = layer_weights(oracle, shape, 3)
     ctx.set_arithmetic(ctx.ARITH_FAST)
     layer = make_layer(ctx, lw, topk, t)
-    layer.set_router_bias(np.array([0.0, 1e6, 0.0], np.float32))
+    layer.set_router_bias(np.where(np.arange(experts) == 1, 1e6, 0.0).astype(np.float32))
     x = ctx.to_device(workloads.hidden_states(shape, t, seed=t))
     y = ctx.to_device(np.zeros((t, 32), np.float32))
     try:
@@ -127,7 +128,7 @@ def test_dispatch_of_an_expert_with_more_slots_than_are_held(oracle, ctx, t, top
         offsets, perm = layer.last_dispatch(t)
         assert np.array_equal(ids[:, 0], np.full(t, 1))
         assert np.array_equal(perm, np.argsort(ids.reshape(-1), kind="stable"))
-        assert np.array_equal(offsets[1:], np.cumsum(np.bincount(ids.reshape(-1), minlength=3)))
+        assert np.array_equal(offsets[1:], np.cumsum(np.bincount(ids.reshape(-1), minlength=experts)))
     finally:
         layer.free()
         x.free()
