@@ -337,7 +337,7 @@ bool ws_reserve(tc_ctx* ctx, const tc::MoeDims& d, int max_tokens) {
               ws_alloc(ctx, w.hs, slots * pad8(n.inter / 32)) &&
               ws_alloc(ctx, w.hsum, slots * pad8(n.inter / 32)) &&
               ws_alloc(ctx, w.out, slots * n.hidden) &&
-              ws_alloc(ctx, w.ticket, size_t(1)) && ws_alloc(ctx, w.grid_sync, size_t(tc::GRID_SYNC_WORDS));
+              ws_alloc(ctx, w.ticket, size_t(tc::route_tickets(T, ctx->sms))) && ws_alloc(ctx, w.grid_sync, size_t(tc::GRID_SYNC_WORDS));
     if (!ok) {
         ws_release(ctx);
         w = before;
@@ -347,7 +347,7 @@ bool ws_reserve(tc_ctx* ctx, const tc::MoeDims& d, int max_tokens) {
     cudaStreamSynchronize(ctx->stream);
     for (void* p : before_allocs) cudaFree(p);
     w.status = ctx->status;
-    cudaMemset(w.ticket, 0, sizeof(int));
+    cudaMemset(w.ticket, 0, tc::route_tickets(T, ctx->sms) * sizeof(int));
     cudaMemset(w.grid_sync, 0, tc::GRID_SYNC_WORDS * sizeof(uint32_t));
     w.max_tokens = T;
     w.sms = ctx->sms;
@@ -462,7 +462,7 @@ int tc_sync(tc_ctx* ctx) {
     }
     if (worst) {
         // A kernel that gave up may have left its arrival counters part-way: start clean.
-        if (ctx->ws.ticket) cudaMemset(ctx->ws.ticket, 0, sizeof(int));
+        if (ctx->ws.ticket) cudaMemset(ctx->ws.ticket, 0, tc::route_tickets(ctx->ws.max_tokens, ctx->sms) * sizeof(int));
         if (ctx->ws.grid_sync) cudaMemset(ctx->ws.grid_sync, 0, tc::GRID_SYNC_WORDS * sizeof(uint32_t));
         if (ctx->self_window) {
             cudaMemset(ctx->self_window, 0, SELF_FLAG_BYTES);

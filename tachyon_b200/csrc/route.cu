@@ -18,6 +18,7 @@
 // The softmax exponential is evaluated in double precision and rounded to
 // float; the CPU path calls libm's expf. The two agree except where expf
 // itself is not correctly rounded, hence the 1e-5 tolerance on gates.
+#include <algorithm>
 #include <type_traits>
 
 #include "dispatch_common.cuh"
@@ -47,7 +48,9 @@ struct RouteArgs {
     // dispatch outputs, used when fused
     int fuse_dispatch;
     int stage_router;      // the router matrix fits in shared memory beside the row: stage it with bulk copies
+    int part_experts;      // tile kernel: the experts of one CTA (blockIdx.y * part_experts and on)
     int* ticket;
+    int* tile_tickets;     // [tiles] the same among the CTAs of a tile
     int* status;
     uint32_t *counts, *offsets, *perm, *pos, *slot_token;
     int* active;
@@ -174,7 +177,9 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // q with lanes 4 q .. 4 q + 3, over chunks of KC columns that stand in shared memory twice over. While eight warps work on a
 // chunk, eight others bring the next: the rows through registers, normed and quantized on the way, the router's
 // by asynchronous copies. Then a warp per token ranks the logits, and every pick gets its gate from a thread of its
-// own. Experts beyond the 64 / NG x TE of a pass take another pass over the columns.
+// own. More experts than the 64 / NG x TE of a CTA are split over CTAs (SPLIT), whose last one makes the picks.
+// (One CTA in several passes over the columns: 256 experts of 1024 columns, router and dispatch, 2500 tokens 278 us, now
+// 110, 129 tokens 57, now 25; 128 experts, 4800 tokens 189, now 117; 65 experts, 2500 tokens 91, now 66.)
 //
 // Bound by shared memory, 16 TG + 8 TE bytes a thread for 2 TG TE packed products: at 4 x 4 a step of sixteen columns is 24
 // cycles of it a warp against 16 of the FP32 pipe, at 4 x 8 32 against 32; with whole rows and the whole matrix staged
@@ -190,7 +195,7 @@ constexpr int RT_HALF = 256, RT_THREADS = 2 * RT_HALF;  // the threads of either
 
 template <int NG, int TG, int TE, int KC>
 struct RouteTile {
-    static constexpr int TM = NG * TG, EG = RT_HALF / 4 / NG, EP = EG * TE;  // tokens, expert groups, experts of a pass
+    static constexpr int TM = NG * TG, EG = RT_HALF / 4 / NG, EP = EG * TE;  // tokens, expert groups, most experts
     static constexpr int XSTRIDE = KC / QK * ROW_PAD_BLOCK;  // floats per staged row piece
     static constexpr int WSTRIDE = KC * 2 + 32;  // bytes per staged router row piece: four neighbouring rows on distinct banks
     static constexpr int X = TM * XSTRIDE * 4, W = EP * WSTRIDE;             // bytes of a buffer
@@ -206,7 +211,7 @@ struct RouteTile {
 
 __device__ __forceinline__ float4 four_floats(const float* p) { return make_float4(p[0], p[1], p[2], p[3]); }
 
-template <int NG, int TG, int TE, int KC>
+template <int NG, int TG, int TE, int KC, bool SPLIT>
 __global__ void __launch_bounds__(RT_THREADS, 1) route_tile_kernel(const RouteArgs a) {
     using L = RouteTile<NG, TG, TE, KC>;
     constexpr int TM = L::TM, EG = L::EG, KV = KC / 8;
@@ -225,20 +230,22 @@ __global__ void __launch_bounds__(RT_THREADS, 1) route_tile_kernel(const RouteAr
     const int t0 = blockIdx.x * TM, nt = min(TM, a.t - t0);
     const int padded = (nb + SUPER - 1) / SUPER * SUPER;
     const int chunks = (hidden + KC - 1) / KC;
+    const int e_lo = SPLIT ? blockIdx.y * a.part_experts : 0, n_e = SPLIT ? min(a.part_experts, experts - e_lo) : experts;
+    const bool first = !SPLIT || blockIdx.y == 0;  // of the tile's CTAs: the one that quantizes
     const bool dots = tid < RT_HALF;
     const int rid = tid - RT_HALF;  // of the threads that bring the rows
     grid_launch_dependents();
-    auto stage_router = [&](int e_lo, int c) {
-        const int n = min(L::EP, experts - e_lo), vecs = min(KC, hidden - c * KC) / 8;
+    auto stage_router = [&](int c) {
+        const int vecs = min(KC, hidden - c * KC) / 8;
         uint8_t* dst = wbuf + (c & 1) * L::W;
 #pragma unroll 4
-        for (int i = rid; i < n * KV; i += RT_HALF) {
+        for (int i = rid; i < n_e * KV; i += RT_HALF) {
             const int e = i / KV, v = i % KV;
             if (v < vecs) cp_async16(dst + e * L::WSTRIDE + v * 16, a.router + size_t(e_lo + e) * hidden + c * KC + v * 8);
         }
         cp_async_commit();
     };
-    if (!dots) stage_router(0, 0);  // (a constant: before the wait)
+    if (!dots) stage_router(0);  // (a constant: before the wait)
     grid_dependency_wait();
 
     // ---- 1 / rms of the rows, a warp per token, several at a time
@@ -342,80 +349,74 @@ __global__ void __launch_bounds__(RT_THREADS, 1) route_tile_kernel(const RouteAr
                 a.xs[token * padded + b] = d, a.xsum[token * padded + b] = su;  // (zeros up to whole super-blocks)
             }
         };
-        for (int e_lo = 0; e_lo < experts; e_lo += L::EP) {
-            if (e_lo > 0) stage_router(e_lo, 0);
-            request(0);
+        request(0);
 #pragma unroll 1
-            for (int c = 0; c <= chunks; c++) {  // chunk c goes in while c - 1 is worked on
-                if (c > 0 && c < chunks) stage_router(e_lo, c);
-                if (stages && c < chunks) {
-                    stage_rows(c);
-                    if (c + 1 < chunks) request(c + 1);
-                }
-                if (c > 0 && e_lo == 0) quantize_rows(c - 1);
-                cp_async_wait_all();
-                __syncthreads();
+        for (int c = 0; c <= chunks; c++) {  // chunk c goes in while c - 1 is worked on
+            if (c > 0 && c < chunks) stage_router(c);
+            if (stages && c < chunks) {
+                stage_rows(c);
+                if (c + 1 < chunks) request(c + 1);
             }
+            if (c > 0 && first) quantize_rows(c - 1);
+            cp_async_wait_all();
+            __syncthreads();
         }
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(L::REGS_DOTS));
         const int quad = tid >> 2, q = tid & 3, tg = quad / EG, eg = quad % EG;  // tokens tg + NG i, experts eg + EG j
-        for (int e_lo = 0; e_lo < experts; e_lo += L::EP) {
-            const int n_e = min(L::EP, experts - e_lo);
-            float2 acc[TG][TE][2];
+        float2 acc[TG][TE][2];
 #pragma unroll
-            for (int i = 0; i < TG; i++)
+        for (int i = 0; i < TG; i++)
 #pragma unroll
-                for (int j = 0; j < TE; j++) acc[i][j][0] = acc[i][j][1] = make_float2(0.0f, 0.0f);
-            __syncthreads();
+            for (int j = 0; j < TE; j++) acc[i][j][0] = acc[i][j][1] = make_float2(0.0f, 0.0f);
+        __syncthreads();
 #pragma unroll 1
-            for (int c = 0; c < chunks; c++) {
-                const float* xr = xbuf + (c & 1) * (L::X / 4) + tg * L::XSTRIDE + q * 4;
-                const uint8_t* wr = wbuf + (c & 1) * L::W + eg * L::WSTRIDE + q * 8;
-                const int steps = min(KC, hidden - c * KC) / 16;
+        for (int c = 0; c < chunks; c++) {
+            const float* xr = xbuf + (c & 1) * (L::X / 4) + tg * L::XSTRIDE + q * 4;
+            const uint8_t* wr = wbuf + (c & 1) * L::W + eg * L::WSTRIDE + q * 8;
+            const int steps = min(KC, hidden - c * KC) / 16;
 #pragma unroll(TG * TE < 16 ? 8 : 2)
-                for (int s = 0; s < steps; s++) {
-                    float4 xv[TG];
+            for (int s = 0; s < steps; s++) {
+                float4 xv[TG];
 #pragma unroll
-                    for (int i = 0; i < TG; i++)
-                        xv[i] = *reinterpret_cast<const float4*>(xr + i * NG * L::XSTRIDE + s / 2 * ROW_PAD_BLOCK + s % 2 * 16);
+                for (int i = 0; i < TG; i++)
+                    xv[i] = *reinterpret_cast<const float4*>(xr + i * NG * L::XSTRIDE + s / 2 * ROW_PAD_BLOCK + s % 2 * 16);
 #pragma unroll
-                    for (int j = 0; j < TE; j++) {  // (experts past the last read what the buffer holds; nothing is made of it)
-                        const uint2 w = *reinterpret_cast<const uint2*>(wr + j * EG * L::WSTRIDE + s * 32);
-                        const float2 w01 = make_float2(bf16_lo(w.x), bf16_hi(w.x)), w23 = make_float2(bf16_lo(w.y), bf16_hi(w.y));
+                for (int j = 0; j < TE; j++) {  // (experts past the last read what the buffer holds; nothing is made of it)
+                    const uint2 w = *reinterpret_cast<const uint2*>(wr + j * EG * L::WSTRIDE + s * 32);
+                    const float2 w01 = make_float2(bf16_lo(w.x), bf16_hi(w.x)), w23 = make_float2(bf16_lo(w.y), bf16_hi(w.y));
 #pragma unroll
-                        for (int i = 0; i < TG; i++) {
-                            acc[i][j][0] = fma2(w01, make_float2(xv[i].x, xv[i].y), acc[i][j][0]);
-                            acc[i][j][1] = fma2(w23, make_float2(xv[i].z, xv[i].w), acc[i][j][1]);
-                        }
+                    for (int i = 0; i < TG; i++) {
+                        acc[i][j][0] = fma2(w01, make_float2(xv[i].x, xv[i].y), acc[i][j][0]);
+                        acc[i][j][1] = fma2(w23, make_float2(xv[i].z, xv[i].w), acc[i][j][1]);
                     }
                 }
-                __syncthreads();
             }
-#pragma unroll
-            for (int i = 0; i < TG; i++)
-#pragma unroll
-                for (int j = 0; j < TE; j++) {
-                    // The two 8-lane accumulators added lane-wise, then the hsum tree.
-                    const float lanes[4] = {acc[i][j][0].x, acc[i][j][0].y, acc[i][j][1].x, acc[i][j][1].y};
-                    float v[4], sv[4];
-#pragma unroll
-                    for (int l = 0; l < 4; l++) v[l] = lanes[l] + __shfl_xor_sync(0xffffffffu, lanes[l], 2);
-#pragma unroll
-                    for (int l = 0; l < 4; l++) sv[l] = v[l] + __shfl_xor_sync(0xffffffffu, v[l], 1);
-                    float y = (sv[0] + sv[2]) + (sv[1] + sv[3]);
-                    y = y + 0.0f;  // the dot's scalar tail is an empty sum
-                    const int token = tg + NG * i, e = eg + EG * j;
-                    if (q == 0 && token < nt && e < n_e) {
-                        if (a.bias) y = y + a.bias[e_lo + e];
-                        skey[token * kstride + e_lo + e] = total_key(y);
-                        if (a.logits) a.logits[size_t(t0 + token) * experts + e_lo + e] = y;
-                    }
-                }
+            __syncthreads();
         }
+#pragma unroll
+        for (int i = 0; i < TG; i++)
+#pragma unroll
+            for (int j = 0; j < TE; j++) {
+                // The two 8-lane accumulators added lane-wise, then the hsum tree.
+                const float lanes[4] = {acc[i][j][0].x, acc[i][j][0].y, acc[i][j][1].x, acc[i][j][1].y};
+                float v[4], sv[4];
+#pragma unroll
+                for (int l = 0; l < 4; l++) v[l] = lanes[l] + __shfl_xor_sync(0xffffffffu, lanes[l], 2);
+#pragma unroll
+                for (int l = 0; l < 4; l++) sv[l] = v[l] + __shfl_xor_sync(0xffffffffu, v[l], 1);
+                float y = (sv[0] + sv[2]) + (sv[1] + sv[3]);
+                y = y + 0.0f;  // the dot's scalar tail is an empty sum
+                const int token = tg + NG * i, e = eg + EG * j;
+                if (q == 0 && token < nt && e < n_e) {
+                    if (a.bias) y = y + a.bias[e_lo + e];
+                    skey[token * kstride + e_lo + e] = total_key(y);
+                    if (a.logits) a.logits[size_t(t0 + token) * experts + e_lo + e] = y;
+                }
+            }
     }
     // Scale rows are padded with zeros to whole super-blocks; those past the last chunk's columns:
-    if (!dots && padded > chunks * (KC / QK)) {
+    if (!dots && first && padded > chunks * (KC / QK)) {
         const int n = padded - chunks * (KC / QK);
         for (int i = rid; i < nt * n; i += RT_HALF) {
             const size_t at = size_t(t0 + i / n) * padded + chunks * (KC / QK) + i % n;
@@ -423,48 +424,63 @@ __global__ void __launch_bounds__(RT_THREADS, 1) route_tile_kernel(const RouteAr
             a.xsum[at] = 0.0f;
         }
     }
-    __syncthreads();  // the keys are complete
-
-    // ---- ranks: larger key first, lower expert first among equals; a warp per token and 32 experts
-    const int groups = (experts + 31) / 32;
+    __shared__ int s_last;
+    auto last_to_get_here = [&](int* ticket, unsigned n) {  // of n CTAs, whose writes the last one then sees
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) s_last = atomicAdd(ticket, 1) == int(n) - 1;
+        __syncthreads();
+        if (s_last) __threadfence();
+        return s_last != 0;
+    };
+    // ---- picks and gates
+    if (!SPLIT) {
+        __syncthreads();  // the keys are complete
+        // ranks: larger key first, lower expert first among equals; a warp per token and 32 experts
+        const int groups = (experts + 31) / 32;
 #pragma unroll 1
-    for (int i = warp; i < nt * groups; i += RT_THREADS / 32) {
-        const int token = i / groups, g = i - token * groups, e = g * 32 + lane;
-        const int* keys = skey + token * kstride;
-        const int key = keys[e];
-        const int rank = rank_in_order(keys, experts, g, key, e < experts, lane);
-        if (e < experts && rank < topk) {
-            sid[token * topk + rank] = uint32_t(e);
-            sval[token * topk + rank] = __int_as_float(key ^ int(unsigned(key >> 31) >> 1));  // (total_key is its own inverse)
+        for (int i = warp; i < nt * groups; i += RT_THREADS / 32) {
+            const int token = i / groups, g = i - token * groups, e = g * 32 + lane;
+            const int* keys = skey + token * kstride;
+            const int key = keys[e];
+            const int rank = rank_in_order(keys, experts, g, key, e < experts, lane);
+            if (e < experts && rank < topk) {
+                sid[token * topk + rank] = uint32_t(e);
+                sval[token * topk + rank] = __int_as_float(key ^ int(unsigned(key >> 31) >> 1));  // (total_key is its own inverse)
+            }
         }
-    }
-    __syncthreads();
-    // ---- gates: softmax over a token's picks, the top score as the maximum, the sum taken in score order
-    float* sexp = xbuf;  // (no longer read)
-    for (int i = tid; i < nt * topk; i += RT_THREADS) sexp[i] = exp_nonpositive_f64(sval[i] - sval[i / topk * topk]);
-    __syncthreads();
-    for (int i = tid; i < nt * topk; i += RT_THREADS) {
-        const float* ex = sexp + i / topk * topk;
-        float sum = 0.0f;
-        for (int j = 0; j < topk; j++) sum = sum + ex[j];
-        a.ids[size_t(t0) * topk + i] = sid[i];
-        a.gates[size_t(t0) * topk + i] = __fdiv_rn(sexp[i], sum);
+        __syncthreads();
+        // gates: softmax over a token's picks, the top score as the maximum, the sum taken in score order
+        float* sexp = xbuf;  // (no longer read)
+        for (int i = tid; i < nt * topk; i += RT_THREADS) sexp[i] = exp_nonpositive_f64(sval[i] - sval[i / topk * topk]);
+        __syncthreads();
+        for (int i = tid; i < nt * topk; i += RT_THREADS) {
+            const float* ex = sexp + i / topk * topk;
+            float sum = 0.0f;
+            for (int j = 0; j < topk; j++) sum = sum + ex[j];
+            a.ids[size_t(t0) * topk + i] = sid[i];
+            a.gates[size_t(t0) * topk + i] = __fdiv_rn(sexp[i], sum);
+        }
+    } else {
+        // By the last of the tile's CTAs, from the logits as they all stored them, a warp per token. (The ranking above grows with
+        // the square of the experts: every key against every other.)
+        if (!last_to_get_here(a.tile_tickets + blockIdx.x, gridDim.y)) return;
+        if (tid == 0) a.tile_tickets[blockIdx.x] = 0;  // ready for the next launch on this stream
+        float* slog = reinterpret_cast<float*>(skey);
+        for (int token = warp; token < nt; token += RT_THREADS / 32) {
+            for (int e = lane; e < experts; e += 32) slog[token * kstride + e] = __ldcg(a.logits + size_t(t0 + token) * experts + e);
+            __syncwarp();
+            const size_t at = size_t(t0 + token) * topk;
+            route_topk_gates(slog + token * kstride, experts, topk, a.ids + at, a.gates + at, lane);
+        }
     }
     // ---- the dispatch of a batch that one CTA can dispatch, by the last CTA to get here (its first 256 threads have a token
     // each; the others take part in the barriers)
-    if (a.fuse_dispatch) {
-        __shared__ int s_last;
-        __threadfence();  // this CTA's ids are visible before its ticket
-        __syncthreads();
-        if (tid == 0) s_last = atomicAdd(a.ticket, 1) == int(gridDim.x) - 1;
-        __syncthreads();
-        if (s_last) {
-            __threadfence();
-            DispatchSmem& sm = *reinterpret_cast<DispatchSmem*>(rt_smem);
-            dispatch_small_body(sm, a.ids, a.t, experts, topk, a.counts, a.offsets, a.perm, a.pos, a.slot_token, a.active, a.status);
-            if (a.tiles) token_tiles_body(sm.scount, sm.soff, experts, a.tile_cols, a.tiles, a.tile_count, sm.stiles, sm.srows);
-            if (tid == 0) *a.ticket = 0;  // ready for the next launch on this stream
-        }
+    if (a.fuse_dispatch && last_to_get_here(a.ticket, gridDim.x)) {
+        DispatchSmem& sm = *reinterpret_cast<DispatchSmem*>(rt_smem);
+        dispatch_small_body(sm, a.ids, a.t, experts, topk, a.counts, a.offsets, a.perm, a.pos, a.slot_token, a.active, a.status);
+        if (a.tiles) token_tiles_body(sm.scount, sm.soff, experts, a.tile_cols, a.tiles, a.tile_count, sm.stiles, sm.srows);
+        if (tid == 0) *a.ticket = 0;  // ready for the next launch on this stream
     }
 }
 
@@ -487,11 +503,19 @@ __global__ void rmsnorm_kernel(const float* x, const float* __restrict__ w, floa
 void init_kernels_route() {
     cudaFuncSetAttribute(route_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ROUTE_SMEM_LIMIT));
     auto opt_in = [](auto kernel) { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ROUTE_SMEM_LIMIT)); };
-    opt_in(route_tile_kernel<8, 4, 4, 128>), opt_in(route_tile_kernel<8, 4, 5, 128>), opt_in(route_tile_kernel<8, 4, 8, 128>);
-    opt_in(route_tile_kernel<8, 2, 4, 128>), opt_in(route_tile_kernel<8, 2, 5, 128>), opt_in(route_tile_kernel<8, 2, 8, 128>);
-    opt_in(route_tile_kernel<8, 1, 4, 256>), opt_in(route_tile_kernel<8, 1, 5, 256>), opt_in(route_tile_kernel<8, 1, 8, 256>);
-    opt_in(route_tile_kernel<4, 1, 2, 512>), opt_in(route_tile_kernel<4, 1, 3, 512>), opt_in(route_tile_kernel<4, 1, 4, 512>);
+    auto every_width = [&](auto split) {
+        constexpr bool S = decltype(split)::value;
+        opt_in(route_tile_kernel<8, 4, 5, 128, S>), opt_in(route_tile_kernel<8, 4, 8, 128, S>);
+        opt_in(route_tile_kernel<8, 2, 5, 128, S>), opt_in(route_tile_kernel<8, 2, 8, 128, S>);
+        opt_in(route_tile_kernel<8, 1, 5, 256, S>), opt_in(route_tile_kernel<8, 1, 8, 256, S>);
+        opt_in(route_tile_kernel<4, 1, 3, 512, S>), opt_in(route_tile_kernel<4, 1, 4, 512, S>);
+    };
+    every_width(std::false_type{}), every_width(std::true_type{});
+    opt_in(route_tile_kernel<8, 4, 4, 128, false>), opt_in(route_tile_kernel<8, 2, 4, 128, false>);
+    opt_in(route_tile_kernel<8, 1, 4, 256, false>), opt_in(route_tile_kernel<4, 1, 2, 512, false>);
 }
+
+int route_tickets(int max_tokens, int sms) { return 1 + std::max(sms, max_tokens / 32 + 1); }
 
 int launch_route(const MoeDims& d, const uint16_t* router, const float* bias, const float* x,
                  const float* norm_w, float eps, int t, Workspace& ws, cudaStream_t stream) {
@@ -513,6 +537,7 @@ int launch_route(const MoeDims& d, const uint16_t* router, const float* bias, co
     a.xsum = ws.xsum;
     a.fuse_dispatch = t <= DISPATCH_THREADS;
     a.ticket = ws.ticket;
+    a.tile_tickets = ws.ticket + 1;
     a.status = ws.status;
     a.counts = ws.counts;
     a.offsets = ws.offsets;
@@ -535,28 +560,34 @@ int launch_route(const MoeDims& d, const uint16_t* router, const float* bias, co
         // with the one-kernel block off.)
         launch_overlapped(route_kernel, dim3(t), dim3(ROUTE_THREADS), smem, stream, a);
     } else {
-        // A CTA per tile of 32, 16, 8 or 4 tokens, the widest that still gives two thirds of the SMs one.
-        // (The wider the tile, the fewer bytes of shared memory a product costs. 333 tokens of the 1b shape in tiles of 2,
-        // which are more than there are SMs: 14.9 us, of 4: 9.7.)
-        const int tm = t >= 32 * 2 * sms / 3 ? 32 : t >= 16 * 2 * sms / 3 ? 16 : t >= 8 * 2 * sms / 3 ? 8 : 4;
-        auto go = [&](auto kernel, size_t smem_bytes) {
-            launch_overlapped(kernel, dim3((t + tm - 1) / tm), dim3(RT_THREADS), smem_bytes, stream, a);
-        };
-        auto tile = [&](auto ng, auto tg, auto te, auto kc) {
+        // A CTA per tile of 4, 8, 16 or 32 tokens and up to 64 experts: the narrowest tile whose CTAs all run at once (one
+        // fills an SM), else the widest, whose products cost the fewest bytes of shared memory. The line lies where a second
+        // wave begins: router and dispatch of the 1b shape in us, one wave of the wider tile / two of the narrower, at 600 tokens 23 / 25,
+        // 1300 29 / 32, 2500 38 / 43; 64 experts of 2048 columns 37 / 43, 53 / 62, 79 / 93.
+        const int parts = (d.experts + 63) / 64;
+        a.part_experts = (d.experts + parts - 1) / parts;
+        int tm = 4;
+        while (tm < 32 && (t + tm - 1) / tm * parts > sms) tm *= 2;
+        auto tile = [&](auto ng, auto tg, auto te, auto kc, auto split) {
             constexpr int NG = decltype(ng)::value, TG = decltype(tg)::value, TE = decltype(te)::value, KC = decltype(kc)::value;
-            go(route_tile_kernel<NG, TG, TE, KC>, RouteTile<NG, TG, TE, KC>::bytes(d.experts, d.topk));
+            launch_overlapped(route_tile_kernel<NG, TG, TE, KC, decltype(split)::value>, dim3((t + tm - 1) / tm, parts),
+                              dim3(RT_THREADS), RouteTile<NG, TG, TE, KC>::bytes(d.experts, d.topk), stream, a);
         };
-        auto eight_groups = [&](auto tg, auto kc) {
-            if (d.experts <= 32) tile(Int<8>{}, tg, Int<4>{}, kc);
-            else if (d.experts <= 40) tile(Int<8>{}, tg, Int<5>{}, kc);
-            else tile(Int<8>{}, tg, Int<8>{}, kc);
+        // (Experts cut in parts are 33 to 64 each.)
+        auto widths = [&](auto split) {
+            const int n = a.part_experts;
+            if (tm == 4) n <= 48 ? tile(Int<4>{}, Int<1>{}, Int<3>{}, Int<512>{}, split) : tile(Int<4>{}, Int<1>{}, Int<4>{}, Int<512>{}, split);
+            else if (tm == 8) n <= 40 ? tile(Int<8>{}, Int<1>{}, Int<5>{}, Int<256>{}, split) : tile(Int<8>{}, Int<1>{}, Int<8>{}, Int<256>{}, split);
+            else if (tm == 16) n <= 40 ? tile(Int<8>{}, Int<2>{}, Int<5>{}, Int<128>{}, split) : tile(Int<8>{}, Int<2>{}, Int<8>{}, Int<128>{}, split);
+            else n <= 40 ? tile(Int<8>{}, Int<4>{}, Int<5>{}, Int<128>{}, split) : tile(Int<8>{}, Int<4>{}, Int<8>{}, Int<128>{}, split);
         };
-        if (tm == 32) eight_groups(Int<4>{}, Int<128>{});
-        else if (tm == 16) eight_groups(Int<2>{}, Int<128>{});
-        else if (tm == 8) eight_groups(Int<1>{}, Int<256>{});
-        else if (d.experts <= 32) tile(Int<4>{}, Int<1>{}, Int<2>{}, Int<512>{});
-        else if (d.experts <= 48) tile(Int<4>{}, Int<1>{}, Int<3>{}, Int<512>{});
-        else tile(Int<4>{}, Int<1>{}, Int<4>{}, Int<512>{});
+        const std::false_type whole;
+        if (parts > 1) widths(std::true_type{});
+        else if (d.experts > 32) widths(whole);
+        else if (tm == 4) tile(Int<4>{}, Int<1>{}, Int<2>{}, Int<512>{}, whole);
+        else if (tm == 8) tile(Int<8>{}, Int<1>{}, Int<4>{}, Int<256>{}, whole);
+        else if (tm == 16) tile(Int<8>{}, Int<2>{}, Int<4>{}, Int<128>{}, whole);
+        else tile(Int<8>{}, Int<4>{}, Int<4>{}, Int<128>{}, whole);
     }
     int launched = 1;
     // (Expert parallel over peer windows: the dispatch runs later, over every rank's tokens.)

@@ -37,42 +37,95 @@ def test_blocks_at_the_edges(oracle, ctx, shape, t, skewed):
     check_block(oracle, ctx, shape, lw, workloads.hidden_states(shape, t, seed=t), bias=bias, arith="fast")
 
 
-@pytest.mark.parametrize("hidden,experts,topk", [(96, 31, 5), (160, 40, 8), (544, 64, 8), (1056, 130, 8), (64, 256, 32)])
-@pytest.mark.parametrize("t", [131, 261, 803, 1601, 3200])
-def test_router_tiles_match_the_router_of_one_token(oracle, ctx, hidden, experts, topk, t):
-    """Every tile size with a remainder, one to four passes over the experts, rows that end inside a chunk, and experts
-    of equal rows (so equal logits): the routing of the same tokens 100 at a time, bit for bit, and their order by expert."""
+def block_in_one_and_by_100(ctx, layer, x, norm):
+    """Everything a block leaves behind, of the whole batch (the router's tiles) and of 100 tokens at a time (the router of
+    one token), both on the kernels that read the router's 8-bit rows with their padded scales."""
+    def run(rows):
+        y = ctx.to_device(rows)
+        layer.block(norm, 1e-6, y)
+        ids, gates, _, logits = layer.last_routing(len(rows))
+        out = [ids, gates, logits, y.get()]
+        y.free()
+        return out
+
+    ctx.set_decode_block(False)
+    ctx.set_prefill_threshold(1 << 30)
+    try:
+        whole = run(x)
+        dispatch = layer.last_dispatch(len(x))
+        parts = [run(x[lo:lo + 100]) for lo in range(0, len(x), 100)]
+    finally:
+        ctx.set_decode_block(True)
+        ctx.set_prefill_threshold(16)
+    return whole, [np.concatenate(p) for p in zip(*parts)], dispatch
+
+
+@pytest.mark.parametrize("hidden,experts,topk,fmt", [
+    (96, 31, 5, "q4"), (160, 40, 8, "q8"), (544, 64, 8, "q4"), (96, 65, 9, "q4"), (1056, 130, 8, "q8"), (64, 256, 32, "q8"),
+])
+@pytest.mark.parametrize("t", [131, 261, 500, 803, 1601, 3200])
+def test_router_tiles_match_the_router_of_one_token(oracle, ctx, hidden, experts, topk, fmt, t):
+    """Every tile size with a remainder, experts in one CTA and split over two to four, rows that end inside a chunk and inside
+    a super-block, and experts of equal rows (so equal logits): the block of the same tokens 100 at a time, bit for bit,
+    and their order by expert."""
     router = synth.normal(41, synth.STREAM_ROUTER, experts * hidden).reshape(experts, hidden) * 0.1
     router[experts // 2] = router[3]
     router[experts - 1] = router[0]
-    shape = MoeShape("tiles", hidden, experts, topk, 32, fmt="q8")
+    shape = MoeShape("tiles", hidden, experts, topk, 32, fmt=fmt)
     lw = layer_weights(oracle, shape, 3)
     lw = workloads.LayerWeights(weights.Matrix.from_f32(router.reshape(-1), experts, hidden, "bf16"), lw.gate_up, lw.down)
     x = workloads.hidden_states(shape, t, seed=t)
     x[5] = 0.0  # (all logits equal)
     norm = ctx.to_device((1.0 + 0.1 * synth.normal(7, synth.STREAM_HIDDEN, hidden)).astype(np.float32))
     ctx.set_arithmetic(ctx.ARITH_FAST)
+    # Longer rows before: what they leave in the scratch must not show.
+    long = MoeShape("long", 2080, 2, 1, 32, fmt=fmt)
+    before = make_layer(ctx, layer_weights(oracle, long, 3), 1, t)
     layer = make_layer(ctx, lw, topk, t)
-
-    def routing(rows):
-        y = ctx.to_device(rows)
-        layer.block(norm, 1e-6, y)
-        ids, gates, _, logits = layer.last_routing(len(rows))
-        y.free()
-        return ids, gates, logits
-
     try:
-        ctx.set_decode_block(False)
-        whole = routing(x)
-        offsets, perm = layer.last_dispatch(t)
+        rows = ctx.to_device(workloads.hidden_states(long, t, seed=1))
+        before.block(ctx.to_device(np.ones(2080, np.float32)), 1e-6, rows)
+        rows.free()
+        whole, parts, (offsets, perm) = block_in_one_and_by_100(ctx, layer, x, norm)
         picks = whole[0].reshape(-1)
         assert np.array_equal(perm, np.argsort(picks, kind="stable"))
         assert np.array_equal(offsets[1:], np.cumsum(np.bincount(picks, minlength=experts)))
-        for lo in range(0, t, 100):
-            for a, b in zip(routing(x[lo:lo + 100]), whole):
-                assert np.array_equal(a, b[lo:lo + 100])
+        for a, b in zip(whole, parts):
+            assert np.array_equal(a, b)
     finally:
-        ctx.set_decode_block(True)
+        layer.free()
+        before.free()
+
+
+@pytest.mark.parametrize("experts", [32, 130])
+@pytest.mark.parametrize("t", [131, 1601, 4000])
+def test_router_tiles_on_rows_that_are_not_finite(oracle, ctx, experts, t):
+    """NaN, infinite, tiny and overflowing rows: the same picks, gates and output rows as from the router of one token,
+    and the rows beside them untouched by it."""
+    shape = MoeShape("odd-rows", 160, experts, 4, 32, fmt="q8")
+    lw = layer_weights(oracle, shape, 3)
+    clean = workloads.hidden_states(shape, t, seed=t)
+    x = clean.copy()
+    odd = [3, 17, 40, 66, 90, 127, t - 1]
+    x[3, 7] = np.nan
+    x[17, ::3] = np.inf
+    x[40, 5] = -np.inf
+    x[66] = 1e-41
+    x[90] = 3e38
+    x[127] = -0.0
+    x[t - 1] = np.nan
+    norm = ctx.to_device((1.0 + 0.1 * synth.normal(7, synth.STREAM_HIDDEN, 160)).astype(np.float32))
+    ctx.set_arithmetic(ctx.ARITH_FAST)
+    layer = make_layer(ctx, lw, 4, t)
+    try:
+        whole, parts, _ = block_in_one_and_by_100(ctx, layer, x, norm)
+        for a, b in zip(whole, parts):
+            assert np.array_equal(a, b, equal_nan=True)
+        assert all(len(set(p)) == 4 and max(p) < experts for p in whole[0].tolist())
+        rest = np.setdiff1d(np.arange(t), odd)
+        for a, b in zip(whole, block_in_one_and_by_100(ctx, layer, clean, norm)[0]):
+            assert np.array_equal(a[rest], b[rest])
+    finally:
         layer.free()
 
 
