@@ -61,17 +61,6 @@ __device__ __forceinline__ void mma_s8(uint32_t tmem_d, uint64_t a_desc, uint64_
         : "memory");
 }
 
-// The same with f16 operands, one K = 16 step.
-__device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                        uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-        ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
-        : "memory");
-}
-
 // One lane of a converged warp.
 __device__ __forceinline__ bool elect_one() {
     uint32_t yes;
@@ -79,7 +68,8 @@ __device__ __forceinline__ bool elect_one() {
     return yes != 0;
 }
 
-// mma_f16 with descriptors of which only the low words (address, leading offset) differ: SBO 128 bytes, as everywhere here.
+// The same with f16 operands, one K = 16 step. Of the descriptors only the low words (address, leading offset) are given;
+// the high one is that of every operand tile here: SBO 128 bytes, version, no swizzle.
 __device__ __forceinline__ uint32_t smem_desc_low(uint32_t smem_addr, uint32_t lbo_bytes) {
     return ((smem_addr >> 4) & 0x3FFFu) | ((lbo_bytes >> 4) & 0x3FFFu) << 16;
 }
@@ -103,20 +93,9 @@ __device__ __forceinline__ void commit(uint64_t* bar) {
 __device__ __forceinline__ void fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// 16 lanes (the lower or upper half of this warp's quadrant, by taddr's lane) x 64, 32 or 16 consecutive columns of
+// 16 lanes (the lower or upper half of this warp's quadrant, by taddr's lane) x 32 or 16 consecutive columns of
 // f32 values, in the order of an m16n8 accumulator: v[4 j], v[4 j + 1] are row lane / 4, columns 8 j + 2 (lane % 4)
 // and the next; v[4 j + 2], v[4 j + 3] the same of row lane / 4 + 8.
-__device__ __forceinline__ void ld_half_f32(uint32_t taddr, float (&v)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.16x256b.x8.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]),
-          "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15]),
-          "=f"(v[16]), "=f"(v[17]), "=f"(v[18]), "=f"(v[19]), "=f"(v[20]), "=f"(v[21]), "=f"(v[22]), "=f"(v[23]),
-          "=f"(v[24]), "=f"(v[25]), "=f"(v[26]), "=f"(v[27]), "=f"(v[28]), "=f"(v[29]), "=f"(v[30]), "=f"(v[31])
-        : "r"(taddr)
-        : "memory");
-}
 __device__ __forceinline__ void ld_half_f32(uint32_t taddr, float (&v)[16]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
@@ -134,24 +113,9 @@ __device__ __forceinline__ void ld_half_f32(uint32_t taddr, float (&v)[8]) {
         : "r"(taddr)
         : "memory");
 }
-__device__ __forceinline__ void ld_half_f32(uint32_t taddr, float (&v)[4]) {
-    asm volatile("tcgen05.ld.sync.aligned.16x256b.x1.b32 {%0, %1, %2, %3}, [%4];"
-                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
-                 : "r"(taddr)
-                 : "memory");
-}
 
 // Waits for this thread's TMEM loads. The values pass through the statement so
 // that no use of them can be scheduled above the wait.
-__device__ __forceinline__ void wait_ld(float (&v)[32]) {
-    asm volatile("tcgen05.wait::ld.sync.aligned;"
-                 : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]), "+f"(v[6]), "+f"(v[7]),
-                   "+f"(v[8]), "+f"(v[9]), "+f"(v[10]), "+f"(v[11]), "+f"(v[12]), "+f"(v[13]), "+f"(v[14]), "+f"(v[15]),
-                   "+f"(v[16]), "+f"(v[17]), "+f"(v[18]), "+f"(v[19]), "+f"(v[20]), "+f"(v[21]), "+f"(v[22]), "+f"(v[23]),
-                   "+f"(v[24]), "+f"(v[25]), "+f"(v[26]), "+f"(v[27]), "+f"(v[28]), "+f"(v[29]), "+f"(v[30]), "+f"(v[31])
-                 :
-                 : "memory");
-}
 __device__ __forceinline__ void wait_ld(float (&v)[16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;"
                  : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]), "+f"(v[6]), "+f"(v[7]),
@@ -164,9 +128,6 @@ __device__ __forceinline__ void wait_ld(float (&v)[8]) {
                  : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]), "+f"(v[6]), "+f"(v[7])
                  :
                  : "memory");
-}
-__device__ __forceinline__ void wait_ld(float (&v)[4]) {
-    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]) : : "memory");
 }
 
 // Byte offset of (row, k) in a block's operand tile of `rows` rows x 32 f16.

@@ -39,17 +39,20 @@ umma_selftest_kernel(const uint16_t* __restrict__ a_tile, const uint16_t* __rest
     __syncthreads();
     umma::fence_after_sync();
     const uint32_t tmem = s_tmem;
-    if (warp == 0 && lane == 0) {
+    if (warp == 0) {  // an elected lane of a converged warp, as the issuing warp of those kernels
+        const uint32_t da = umma::smem_desc_low(smem_addr(s_a), 128 * 16), db = umma::smem_desc_low(smem_addr(s_b), N * 16);
+        if (umma::elect_one()) {
 #pragma unroll
-        for (int h = 0; h < 2; h++)
-            umma::mma_f16(tmem, umma::smem_desc(smem_addr(s_a) + h * 128 * 32, 128 * 16, 128),
-                          umma::smem_desc(smem_addr(s_b) + h * N * 32, N * 16, 128), umma::idesc_f16(128, N), uint32_t(h));
-        umma::commit(&s_bar);
+            for (int h = 0; h < 2; h++)
+                umma::mma_f16_low(tmem, da + h * 128 * 2, db + h * N * 2, umma::idesc_f16(128, N), uint32_t(h));
+            umma::commit(&s_bar);
+        }
+        __syncwarp();
     }
     const bool landed = mbar_wait_bounded(&s_bar, 0);
     umma::fence_after_sync();
     if (landed) {
-        // As the prefill kernels read them: a half of the rows at a time, here once 32 and twice 16 of every 64 columns.
+        // A half of the rows at a time, in the two widths those kernels use: 32 columns, and twice 16, of every 64.
         const uint32_t base = tmem + (uint32_t(warp * 32) << 16);
         auto read = [&](int c0, int h, auto& v) {
             constexpr int n = sizeof(v) / sizeof(float);
@@ -66,15 +69,10 @@ umma_selftest_kernel(const uint16_t* __restrict__ a_tile, const uint16_t* __rest
         for (int c0 = 0; c0 < N; c0 += 64) {
 #pragma unroll
             for (int h = 0; h < 2; h++) {
-                if (c0 > 0) {
-                    float v[32];
-                    read(c0, h, v);
-                } else {
-                    float v[16], lo[8], hi[8];
-                    read(0, h, v);
-                    read(32, h, lo);
-                    read(48, h, hi);
-                }
+                float v[16], lo[8], hi[8];
+                read(c0, h, v);
+                read(c0 + 32, h, lo);
+                read(c0 + 48, h, hi);
             }
         }
     } else if (tid == 0) {
