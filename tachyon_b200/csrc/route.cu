@@ -88,51 +88,36 @@ __global__ void __launch_bounds__(ROUTE_THREADS) route_kernel(const RouteArgs a)
     // The router matrix is a constant: it streams in while the kernel in front of this
     // one (the previous block's combine) finishes. Everything below reads its output.
     grid_dependency_wait();
-    // A CTA walks tokens blockIdx.x, blockIdx.x + gridDim.x, ...: one each for batches of up to a few
-    // CTAs per SM, several for prefill-size batches (the staged router matrix is then read once per
-    // CTA instead of once per token). The next token's row is requested before this one is worked on.
-    bool w_landed = true;
-    constexpr int ROW_VEC = 4;  // float4 per thread held ahead: rows of up to 4096 floats
-    float4 ahead[ROW_VEC];
-    auto request_row = [&](int token) {
+    const int token = blockIdx.x;
+    const float* xin = a.x + size_t(token) * hidden;
+    constexpr int ROW_VEC = 4;  // float4 per thread asked for at a time
+    for (int c0 = tid * 4; c0 < hidden; c0 += ROW_VEC * ROUTE_THREADS * 4) {
+        float4 v[ROW_VEC];
 #pragma unroll
         for (int i = 0; i < ROW_VEC; i++) {
-            const int c = (tid + i * ROUTE_THREADS) * 4;
-            if (token < a.t && c < hidden)
-                ahead[i] = *reinterpret_cast<const float4*>(a.x + size_t(token) * hidden + c);
+            const int c = c0 + i * ROUTE_THREADS * 4;
+            if (c < hidden) v[i] = *reinterpret_cast<const float4*>(xin + c);
         }
-    };
-    const bool rows_ahead = hidden <= ROW_VEC * ROUTE_THREADS * 4;
-    if (rows_ahead) request_row(blockIdx.x);
-    for (int token = blockIdx.x; token < a.t; token += gridDim.x) {
-        if (token != int(blockIdx.x)) __syncthreads();  // the previous token's row and logits are no longer read
-        if (rows_ahead) {
 #pragma unroll
-            for (int i = 0; i < ROW_VEC; i++) {
-                const int c = (tid + i * ROUTE_THREADS) * 4;
-                if (c < hidden) *reinterpret_cast<float4*>(xrow + c) = ahead[i];
-            }
-            request_row(token + gridDim.x);
-        } else {
-            const float* xin = a.x + size_t(token) * hidden;
-            for (int c = tid * 4; c < hidden; c += ROUTE_THREADS * 4)
-                *reinterpret_cast<float4*>(xrow + c) = *reinterpret_cast<const float4*>(xin + c);
+        for (int i = 0; i < ROW_VEC; i++) {
+            const int c = c0 + i * ROUTE_THREADS * 4;
+            if (c < hidden) *reinterpret_cast<float4*>(xrow + c) = v[i];
         }
-        __syncthreads();
-        if (a.norm_w) route_norm_row(xrow, hidden, a.norm_w, a.eps, &s_inv, tid, ROUTE_THREADS);
+    }
+    __syncthreads();
+    if (a.norm_w) route_norm_row(xrow, hidden, a.norm_w, a.eps, &s_inv, tid, ROUTE_THREADS);
 
-        if (a.stage_router && token == int(blockIdx.x)) w_landed = mbar_wait_bounded(&s_wbar, 0);
-        route_logits(a.router, a.stage_router && w_landed ? wsm : nullptr, wstride, xrow, a.bias, hidden, 0, experts,
-                     slog, a.logits ? a.logits + size_t(token) * experts : nullptr, tid, ROUTE_THREADS);
-        __syncthreads();
+    const bool w_landed = !a.stage_router || mbar_wait_bounded(&s_wbar, 0);
+    route_logits(a.router, a.stage_router && w_landed ? wsm : nullptr, wstride, xrow, a.bias, hidden, 0, experts,
+                 slog, a.logits ? a.logits + size_t(token) * experts : nullptr, tid, ROUTE_THREADS);
+    __syncthreads();
 
-        // Warp 0 ranks the logits while warps 1.. quantize the row (the two do not depend on each other).
-        if (warp == 0)
-            route_topk_gates(slog, experts, topk, a.ids + size_t(token) * topk, a.gates + size_t(token) * topk, lane);
-        const int padded = (hidden / QK + SUPER - 1) / SUPER * SUPER;
-        route_quantize_row(xrow, hidden, a.xq + size_t(token) * hidden, a.xs + size_t(token) * padded,
-                           a.xsum + size_t(token) * padded, warp, lane, 1, ROUTE_THREADS / 32 - 1);
-    }  // tokens of this CTA
+    // Warp 0 ranks the logits while warps 1.. quantize the row (the two do not depend on each other).
+    if (warp == 0)
+        route_topk_gates(slog, experts, topk, a.ids + size_t(token) * topk, a.gates + size_t(token) * topk, lane);
+    const int padded = (hidden / QK + SUPER - 1) / SUPER * SUPER;
+    route_quantize_row(xrow, hidden, a.xq + size_t(token) * hidden, a.xs + size_t(token) * padded,
+                       a.xsum + size_t(token) * padded, warp, lane, 1, ROUTE_THREADS / 32 - 1);
 
     // ---- the dispatch, by the last CTA to get here (batches of up to one CTA's worth of tokens).
     if (a.stage_router && !w_landed) {
@@ -556,8 +541,9 @@ int launch_route(const MoeDims& d, const uint16_t* router, const float* bias, co
     if (a.fuse_dispatch && (t <= 128 || a.scatter.ranks > 0)) {
         // Few tokens (or rows that go to every rank from here): a CTA per token; the last one to finish runs the dispatch.
         // (Past 128 the tiles below are ahead, whole blocks of 129 / 200 / 256 tokens in us: 1b shape 69.9 / 74.9 / 87.6 so,
-        // 67.5 / 71.0 / 82.8 in tiles; 64 experts of 2048 x 1024 201 / 205 / 211, 196 / 200 / 205. Up to 128 these kernels only run
-        // with the one-kernel block off.)
+        // 67.5 / 71.0 / 82.8 in tiles; 64 experts of 2048 x 1024 201 / 205 / 211, 196 / 200 / 205. Up to 128 these kernels run
+        // where the one-kernel block does not: switched off, the CPU's order of lanes, the two matrices in different formats, rows
+        // longer than it takes.)
         launch_overlapped(route_kernel, dim3(t), dim3(ROUTE_THREADS), smem, stream, a);
     } else {
         // A CTA per tile of 4, 8, 16 or 32 tokens and up to 64 experts: the narrowest tile whose CTAs all run at once (one
