@@ -12,7 +12,7 @@
 // (picks, rows, residual row), during two of which nothing large is on its way: so the residual row and all that
 // belongs to the picks are asked for together, and a thread takes 16 bytes of the row (256 threads went over a row of 1536
 // floats twice, the second time half empty). 4096 tokens of the 1b shape 37 -> 33 us, 2047 of the 3b shape 29.5 -> 25,
-// 4096 of 2048 columns 62 -> 60; 33, 25 and 59 are 167, 126 and 335 MB: 5 to 5.7 TB/s.
+// 4096 of 2048 columns 62 -> 60: 167, 126 and 335 MB, 5.0 to 5.6 TB/s.
 #include "common.cuh"
 
 namespace tc {

@@ -10,7 +10,8 @@
 // What bounds it, in cycles per 128 x 64 x 32 unit and SM: that float work, two packed FP32 operations per output pair
 // and block, 128 (and 34 of the finishing warps); the reads of tensor memory, 128 (the 16-lane shape moves half of what
 // the 32-lane one does) beside the products' own 37; and shared memory at 128 bytes a clock: 64 for the products'
-// operands, 66 for the copies that bring them, 80 for the scales. So:
+// operands, 66 for the copies that bring them, 80 for the scales (if lanes that read the same word cost as much as lanes
+// that do not; the measured 188 a unit, less than the sum, says that they cost less). So:
 //  - A lane has 4 rows x 16 tokens (the 16x256b shape), 20 words of scales per 64 outputs. With a row of 64 tokens
 //    (32x32b) they were 65 words: 272 cycles of shared memory a unit beside the other 130, in units of 365 to 430.
 //  - The float loop's code is 4 blocks long with constant addresses, a barrier test and an arrival per 2 blocks;
@@ -36,8 +37,8 @@
 // Measured (granite-1b-a400m, 4096 tokens, int8; 24, now 20 us of gate_up tile the activations): gate_up 234 -> 183 us, down
 // 109 -> 86; 64 experts of 2048 x 1024: 812 -> 615, 383 -> 291; 40 of 1536 x 512 in 4 bits at 2047 tokens: 276 -> 209, 138
 // -> 109. A chunk of two blocks takes 750 cycles (188 a unit), a tile 3300 besides, and another 3300 of a scheduler's time go
-// to finishing it in gate_up; 4-bit tiles, of 64 columns, take 480 a unit, where shared memory alone is 395 (192 the
-// scales, 96 operands, 98 copies). Tried: 16 float warps of 32 columns (as before or slower), the loop rolled to a
+// to finishing it in gate_up; 4-bit tiles, of 64 columns, take 480 a unit, where shared memory alone is up to 386 (192 the
+// scales, counted as above, 96 operands, 98 copies). Tried: 16 float warps of 32 columns (as before or slower), the loop rolled to a
 // block (bookkeeping: 342 instructions a unit against 177) or to a chunk (211 / 99 us), pieces of 32 values a
 // lane (spills), a block's scales read a block ahead (spills), 4-bit tiles of 128 columns (spills), remainders of 65 to 96
 // tokens as 64 + 32 columns (333 tokens 42 + 25 -> 54 + 31 us: a narrow tile costs nearly as much as a wide one), the widest
