@@ -39,12 +39,15 @@ struct tc_ctx {
     std::vector<void*> pre_allocs;
     // Tokens per expert (on average) from which the tcgen05 kernels take over, past the one-kernel block's 128 tokens.
     // Under an even router they cross the bandwidth-oriented ones between 8 and 12 (us per block, tcgen05 / the
-    // others, 8-bit, 8 picks): 64 experts of 2048 x 1024 at 129 tokens, an average of 16.1: 193 / 239; 128 experts of
-    // 1024 x 512 at 9: 129 / 102, 12: 131 / 143, 16: 133 / 154; 256 of them at 8: 228 / 192, 12: 226 / 235, 16: 228 / 266;
-    // 96 of 2048 x 768, 4 picks, at 8: 218 / 163, 10.7: 220 / 225, 16: 221 / 256. 4-bit weights at 9 to 12 (128 experts 128 / 132
-    // at 9). 16 is from slower tcgen05 kernels, which crossed there; between 12 and 16 it now costs 4 to 13 %.
-    // 32 to 40 experts are past it at 129 tokens (64 / 101, 91 / 132). A router that prefers a few experts puts the
-    // tcgen05 kernels far ahead below the line too: 128 experts at 144 tokens, an average of 9, with a Zipf bias 90 / 440.
+    // others, 8-bit, 8 picks): 64 experts of 2048 x 1024 at 129 tokens, an average of 16.1: 190 / 241; 128 experts of
+    // 1024 x 512 at 9: 121 / 117, 12: 123 / 136, 14: 124 / 142, just below 16: 125 / 143; 256 of them at 8: 200 / 175, 12: 202 / 214,
+    // 14: 203 / 229, just below 16: 205 / 247; 96 of 2048 x 768, 4 picks, at 8: 203 / 175, 10.7: 205 / 208, 12: 203 / 220, 14: 213 / 238,
+    // just below 16: 214 / 264. In 4 bits, 128 experts at 9: 119 / 129, 14: 120 / 140, just below 16: 121 / 151; 256 at 8: 200 / 176, 12: 204 / 225.
+    // 16 is from slower tcgen05 kernels, which crossed there: a block now takes 6 to 14 % longer at 12 than it would with them, 12 to 17 %
+    // at 14, 14 to 24 % just below 16.
+    // 32 to 40 experts are past it at 129 tokens (63 / 97, 91 / 137). A router that prefers a few experts puts the
+    // tcgen05 kernels far ahead below the line too: with a Zipf bias 128 experts at 144 tokens, an average of 9, 78 / 434, 96 experts at
+    // 10.7 121 / 1543.
     // But the counts are on the device and the choice is made on the host, from the average.
     int prefill_min_avg = 16;
     float* host_x = nullptr;  // device staging for the host-buffer entry point (large batches)
@@ -337,7 +340,8 @@ bool ws_reserve(tc_ctx* ctx, const tc::MoeDims& d, int max_tokens) {
               ws_alloc(ctx, w.hs, slots * pad8(n.inter / 32)) &&
               ws_alloc(ctx, w.hsum, slots * pad8(n.inter / 32)) &&
               ws_alloc(ctx, w.out, slots * n.hidden) &&
-              ws_alloc(ctx, w.ticket, size_t(tc::route_tickets(T, ctx->sms))) && ws_alloc(ctx, w.grid_sync, size_t(tc::GRID_SYNC_WORDS));
+              ws_alloc(ctx, w.ticket, size_t(1)) && ws_alloc(ctx, w.grid_sync, size_t(tc::GRID_SYNC_WORDS)) &&
+              ws_alloc(ctx, w.tile_tickets, tc::route_tile_tickets(T, ctx->sms));
     if (!ok) {
         ws_release(ctx);
         w = before;
@@ -347,7 +351,8 @@ bool ws_reserve(tc_ctx* ctx, const tc::MoeDims& d, int max_tokens) {
     cudaStreamSynchronize(ctx->stream);
     for (void* p : before_allocs) cudaFree(p);
     w.status = ctx->status;
-    cudaMemset(w.ticket, 0, tc::route_tickets(T, ctx->sms) * sizeof(int));
+    cudaMemset(w.ticket, 0, sizeof(int));
+    cudaMemset(w.tile_tickets, 0, tc::route_tile_tickets(T, ctx->sms) * sizeof(int));
     cudaMemset(w.grid_sync, 0, tc::GRID_SYNC_WORDS * sizeof(uint32_t));
     w.max_tokens = T;
     w.sms = ctx->sms;
@@ -462,7 +467,9 @@ int tc_sync(tc_ctx* ctx) {
     }
     if (worst) {
         // A kernel that gave up may have left its arrival counters part-way: start clean.
-        if (ctx->ws.ticket) cudaMemset(ctx->ws.ticket, 0, tc::route_tickets(ctx->ws.max_tokens, ctx->sms) * sizeof(int));
+        if (ctx->ws.ticket) cudaMemset(ctx->ws.ticket, 0, sizeof(int));
+        if (ctx->ws.tile_tickets)
+            cudaMemset(ctx->ws.tile_tickets, 0, tc::route_tile_tickets(ctx->ws.max_tokens, ctx->sms) * sizeof(int));
         if (ctx->ws.grid_sync) cudaMemset(ctx->ws.grid_sync, 0, tc::GRID_SYNC_WORDS * sizeof(uint32_t));
         if (ctx->self_window) {
             cudaMemset(ctx->self_window, 0, SELF_FLAG_BYTES);

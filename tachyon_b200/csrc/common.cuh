@@ -100,7 +100,8 @@ struct Workspace {
     float* hsum = nullptr;        // [T*k, pad8(I/32)]
     float* out = nullptr;         // [T*k, H] expert outputs, sorted order
     int* status = nullptr;        // device status word
-    int* ticket = nullptr;        // [route_tickets] arrival counters of the router CTAs: all, then those of a tile (zero between launches)
+    int* ticket = nullptr;        // arrival counter of the router CTAs (zero between launches)
+    int* tile_tickets = nullptr;  // [route_tile_tickets] the same among the CTAs of a router tile
     uint32_t* grid_sync = nullptr;  // [GRID_SYNC_WORDS] arrival counters of the one-kernel decode block (zero between launches)
     TokenTile* tiles = nullptr;   // when set: the dispatch also cuts the experts' tokens into tiles of up to
     int* tile_count = nullptr;    // tile_cols columns for the tensor-core kernels
@@ -139,7 +140,7 @@ enum : int {
 // x is the block's normed input, or (norm_w set) the residual stream to be
 // RMS-normed first. Batches of up to 256 tokens are dispatched by the same
 // kernel; larger ones by launch_dispatch, which this then calls.
-int route_tickets(int max_tokens, int sms);
+size_t route_tile_tickets(int max_tokens, int sms);
 int launch_route(const MoeDims& d, const uint16_t* router, const float* bias, const float* x,
                  const float* norm_w, float eps, int t, Workspace& ws, cudaStream_t stream);
 
